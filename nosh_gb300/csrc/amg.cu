@@ -728,8 +728,7 @@ __device__ __forceinline__ void tail_rows(const Team &tm, const LevelDesc<T> &A,
     if (i < A.n)
       for (int32_t k = A.rp[i] + li; k < A.rp[i + 1]; k += tpr) {
         const C2<T> v = A.off[k], xv = x[A.ci[k]];
-        sr += v.x * xv.x - v.y * xv.y;
-        si += v.x * xv.y + v.y * xv.x;
+        row_mac(sr, si, v, xv);
       }
     for (int off = tpr >> 1; off > 0; off >>= 1) {
       sr += __shfl_xor_sync(0xffffffffu, sr, off);

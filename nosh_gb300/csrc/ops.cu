@@ -456,10 +456,8 @@ __global__ void __launch_bounds__(128) residual_pair_kernel(
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         if (k0 + u < e) {
-          ar += v[u].x * p[u].x - v[u].y * p[u].y;
-          ai += v[u].x * p[u].y + v[u].y * p[u].x;
-          br += v[u].x * q[u].x - v[u].y * q[u].y;
-          bi += v[u].x * q[u].y + v[u].y * q[u].x;
+          row_mac(ar, ai, v[u], p[u]);
+          row_mac(br, bi, v[u], q[u]);
         }
       }
     }

@@ -188,6 +188,23 @@ struct PartOf<Op, A, decltype((void)sizeof(typename Op::Part), void())> {
   using type = typename Op::Part;
 };
 
+// One nonzero of a row sum: (sr, si) += v x (complex).  In FP64 each component
+// is two chained FMAs: GB300's FP64 pipe takes 16 cycles of an SM per warp
+// instruction and bounds these kernels, so four instructions a nonzero
+// instead of the six that adding the rounded product takes (mul, fma, add
+// per component), with one rounding less.  In FP32 the pipe is not the
+// bound; the product is formed first.
+__device__ __forceinline__ void row_mac(float &sr, float &si, const C2<float> &v, const C2<float> &x) {
+  sr += v.x * x.x - v.y * x.y;
+  si += v.x * x.y + v.y * x.x;
+}
+__device__ __forceinline__ void row_mac(double &sr, double &si, const C2<double> &v, const C2<double> &x) {
+  sr = fma(v.x, x.x, sr);
+  si = fma(v.x, x.y, si);
+  sr = fma(-v.y, x.y, sr);
+  si = fma(v.y, x.x, si);
+}
+
 // Op must provide:
 //   static constexpr bool kReduce;
 //   struct Pre;                                  -- the row's epilogue operands
@@ -417,8 +434,7 @@ __global__ void __launch_bounds__(block_threads<T>(), sizeof(T) == 4 ? 5 : 1)
           for (int u = 0; u < kBatch; u++) {
             if (u < cnt) {
               const C2<T> v = s_val[k0 + u * R];
-              sr += v.x * xv[u].x - v.y * xv[u].y;
-              si += v.x * xv[u].y + v.y * xv[u].x;
+              row_mac(sr, si, v, xv[u]);
             }
           }
         }
@@ -426,8 +442,7 @@ __global__ void __launch_bounds__(block_threads<T>(), sizeof(T) == 4 ? 5 : 1)
         for (int k = b + lane_r; k < e; k += R) {
           const C2<T> v = ldg(val + k);
           const C2<T> xv = ldg(x + __ldg(ci + k));
-          sr += v.x * xv.x - v.y * xv.y;
-          si += v.x * xv.y + v.y * xv.x;
+          row_mac(sr, si, v, xv);
         }
       }
     }
@@ -519,8 +534,7 @@ __global__ void __launch_bounds__(kWarpThreads)
         for (int kk = k[q] + 16; kk < e[q]; kk += 16) {
           const C2<T> vv = ldg(val + kk);
           const C2<T> xx = ldg(x + __ldg(ci + kk));
-          sr += vv.x * xx.x - vv.y * xx.y;
-          si += vv.x * xx.y + vv.y * xx.x;
+          row_mac(sr, si, vv, xx);
         }
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) {
