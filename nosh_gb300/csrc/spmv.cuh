@@ -5,9 +5,9 @@
 // persistent over row blocks.  A row block's nonzeros [rp[r0], rp[r1]) are
 // contiguous: one thread stages them into shared memory with two bulk
 // asynchronous copies (TMA, cp.async.bulk: column ids and complex values)
-// completing on an mbarrier, double-buffered so that the copy of the CTA's
-// next row block overlaps the current one's arithmetic.  The threads of a
-// row then reduce its nonzeros out of shared memory and gather x through
+// completing on an mbarrier; in FP32 double-buffered, so that the copy of the
+// CTA's next row block overlaps the current one's arithmetic (stage_count).
+// The threads of a row then reduce its nonzeros out of shared memory and gather x through
 // the read-only path.  A row block whose nonzeros exceed the staging
 // capacity reads them directly.
 #pragma once
@@ -302,12 +302,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
 }
 
 // Shared memory of one staging buffer (column ids, then complex values) for
-// a capacity of cap nonzeros (a multiple of 4); the kernel uses two.
+// a capacity of cap nonzeros (a multiple of 4); the kernel uses
+// stage_count<T>() of them.
 template <typename T>
 __host__ __device__ constexpr size_t stage_bytes(int cap) {
   return (size_t)cap * (sizeof(int32_t) + sizeof(C2<T>));
 }
-// Largest staging capacity: two buffers within 96 KB.
+// Staging buffers of a CTA.  FP32: two, the next row block's copy under the
+// current one's gathers.  FP64: one.  Two FP64 buffers of a tetrahedral mesh
+// (72 KB) left three CTAs on an SM, and the FP64 pipe, which bounds the
+// kernel, idle a quarter of the time; one buffer fits five (register bound),
+// whose gathers and copies overlap one another.  J rebuild + apply at 160^3
+// 776 -> 699 us, FP64 V-cycles at 48^3 925 -> 868 us; six CTAs (80 registers)
+// gained 1 % more there and lost 3 % on a 32^3 continuation.
+template <typename T>
+__host__ __device__ constexpr int stage_count() {
+  return sizeof(T) == 4 ? 2 : 1;
+}
+// CTAs per SM the staged kernel is compiled for (its register budget).
+template <typename T>
+__host__ __device__ constexpr int stage_ctas() {
+  return sizeof(T) == 4 ? 5 : 4;
+}
+// Largest staging capacity of one buffer: 48 KB.
 template <typename T>
 __host__ __device__ constexpr int stage_limit() {
   return (int)((48 * 1024) / (sizeof(int32_t) + sizeof(C2<T>))) & ~3;
@@ -321,7 +338,7 @@ constexpr int kStageErrorSlot = 15;
 constexpr int kStageWaitSlot = 14;
 
 template <typename T, class Op>
-__global__ void __launch_bounds__(block_threads<T>(), sizeof(T) == 4 ? 5 : 1)
+__global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     row_block_apply(int N, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
                     const C2<T> *__restrict__ val, const C2<T> *__restrict__ x, int cap,
                     Op op, double *partials, unsigned *counter, double *red_out) {
@@ -388,10 +405,11 @@ __global__ void __launch_bounds__(block_threads<T>(), sizeof(T) == 4 ? 5 : 1)
     if (o != 0u) limit = o - 1u;
   }
   int stage = 0;
-  for (int rb = rb0; rb < rb_end; rb = nxt(rb), stage ^= 1) {
+  constexpr bool kTwo = stage_count<T>() == 2;
+  for (int rb = rb0; rb < rb_end; rb = nxt(rb), stage ^= (kTwo ? 1 : 0)) {
     // the other buffer was released by the barrier that ended the previous
     // iteration: start the next row block's copy into it
-    if (threadIdx.x == 0 && nxt(rb) < rb_end) issue(nxt(rb), stage ^ 1);
+    if (kTwo && threadIdx.x == 0 && nxt(rb) < rb_end) issue(nxt(rb), stage ^ 1);
     int ks, n;
     range(rb, ks, n);
     constexpr int R = row_threads<T>();
@@ -401,7 +419,7 @@ __global__ void __launch_bounds__(block_threads<T>(), sizeof(T) == 4 ? 5 : 1)
     const bool staged = n > 0 && n <= cap;
     cur_staged = staged;
     next_staged = false;
-    if (nxt(rb) < rb_end) {
+    if (kTwo && nxt(rb) < rb_end) {
       int ks2, n2;
       range(nxt(rb), ks2, n2);
       next_staged = n2 > 0 && n2 <= cap;
@@ -453,7 +471,8 @@ __global__ void __launch_bounds__(block_threads<T>(), sizeof(T) == 4 ? 5 : 1)
       si += __shfl_xor_sync(0xffffffffu, si, o);
     }
     if (row < N && lane_r == 0) part += (typename PartOf<Op, A>::type)op.finish(row, sr, si, pre);
-    __syncthreads();  // this buffer is refilled two row blocks later
+    __syncthreads();  // the buffer's readers are done: it may be refilled
+    if (!kTwo && threadIdx.x == 0 && nxt(rb) < rb_end) issue(nxt(rb), 0);
   }
   if (!ok) {
     // a wait gave up: record it, give the copies still in flight (this row
@@ -588,7 +607,7 @@ void launch_spmv(bool warp, int N, const int32_t *rp, const int32_t *ci, const C
                                      100 * 1024));
       attr_set = true;
     }
-    const size_t smem = 2 * stage_bytes<T>(cap);
+    const size_t smem = stage_count<T>() * stage_bytes<T>(cap);
     launch_dep(overlap, row_block_apply<T, Op>,
                dim3(row_grid((const void *)row_block_apply<T, Op>, block_threads<T>(), smem, N)),
                dim3(block_threads<T>()), smem, st, N, rp, ci, val, x, cap, op, partials, counter, red_out);
