@@ -30,7 +30,10 @@ using namespace dev;
 
 namespace {
 
-constexpr int64_t kTailMax = 1024;   // levels this small run in one CTA
+// The largest level that the resident V-cycle starts on, and the largest mesh
+// that it takes whole.
+constexpr int64_t kTailMax = 1024;
+constexpr int64_t kResidentMax = 0;
 
 struct HostLevel {
   int64_t n = 0;
@@ -647,199 +650,451 @@ struct DenseMap {
   const int64_t *rowoff;
   const int32_t *bstart, *bdim;
 };
-template <typename T>
-__device__ __forceinline__ T dense_row(const DenseMap &D, const T *__restrict__ Ainv, int64_t i,
-                                       const T *__restrict__ b) {
-  const T *a = Ainv + D.rowoff[i];
-  const T *bb = b + D.bstart[i];
-  const int m = D.bdim[i];
-  T s = 0;
-  for (int j = 0; j < m; j++) s += a[j] * bb[j];
-  return s;
-}
-
+// x = Ainv b, a half-warp per real row (a batch's coarsest level, or a
+// hierarchy of one level)
+constexpr int kDenseLanes = 16;
 template <typename T>
 __global__ void dense_matvec(int m, const T *__restrict__ Ainv, DenseMap D, const T *__restrict__ b,
-                             T *__restrict__ x) {
+                             T *__restrict__ x, const int *halt) {
   dep_sync();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-    x[i] = dense_row(D, Ainv, i, b);
+  if (halt && *halt >= 2) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kDenseLanes, li = t % kDenseLanes;
+  T s = 0;
+  if (i < m) {
+    const T *a = Ainv + D.rowoff[i], *bb = b + D.bstart[i];
+    const int n = D.bdim[i];
+#pragma unroll 4
+    for (int j = li; j < n; j += kDenseLanes) s = fma(a[j], bb[j], s);
+  }
+#pragma unroll
+  for (int o = kDenseLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (i < m && li == 0) x[i] = s;
 }
 
-// ---- coarse-level tail: every level from `lt` down, in one launch (one CTA,
-// or one thread-block cluster)
+// ---- the resident V-cycle: every level from `lt` down, in one launch of one
+// thread-block cluster.
+//
+// The coarse levels are latency: a few hundred to a thousand rows, five SpMVs
+// each.  A launch per step costs about 3 us; one CTA for all of them left the
+// FP64 pipe of a single SM as the bound (a 900-node level of the 65^2 square:
+// 65 us a cycle, 79 % of that pipe).  Here the rows of a level are spread over
+// the CTAs of a cluster (16, which needs the opt-in above the portable 8) and
+// each level's vectors live in shared memory, replicated in every CTA: a row's
+// result is stored to all CTAs (DSMEM), a hardware cluster barrier ends the
+// phase, and every gather is a local shared-memory read.  Each CTA's rows of
+// the operators are staged in its shared memory while the predecessor runs.
+//
+// A row is summed by LN lanes: even lanes its real component, odd lanes its
+// imaginary one (two FMAs a nonzero each, no reduction between the two), and
+// LN/2 parts of the row.  FP64 takes just enough lanes for a warp on each of
+// the SM's four FP64 pipes, since idle lanes of a warp cost as much as busy
+// ones and every shuffle step of a wider split is more FP64 adds; FP32 splits
+// up to sixteen ways.
+constexpr int kTailThreads = 512;
+constexpr int kTailSmem = 200 * 1024;  // shared memory of one CTA, at most
+
 template <typename T>
 struct LevelDesc {
-  int64_t n;
+  int n, rw;  // rows, rows per CTA (CTA r owns [r rw, (r + 1) rw))
+  int staged;  // this CTA's rows of the operator are staged
   const int32_t *rp, *ci;
   const C2<T> *off;
   const T *dia, *dinv, *coef;
-  C2<T> *b, *x, *x2, *d, *res;
   const int32_t *agg, *mem_ptr, *mem_idx;  // transfer to the next level
+  // shared-memory byte offsets: two replicated vectors, the own rows' right-
+  // hand side and Chebyshev direction, the own rows of the operator (row
+  // pointers, columns, values, diagonal blocks and their inverses), this
+  // level's aggregates, the own members of this level's nodes (a list over
+  // the finer level)
+  uint32_t xa, xb, b, d, s_rp, s_ci, s_off, s_dia, s_agg, s_mp, s_mi;
 };
 
+enum TailHead { kHeadRestrict = 0, kHeadVector = 1, kHeadLanczos = 2 };
+enum TailOut { kOutProlong = 0, kOutVector = 1, kOutMinres = 2 };
 
-// The threads that run the tail: one CTA (barrier: __syncthreads), or the
-// CTAs of one thread-block cluster (barrier: the hardware cluster barrier,
-// whose arrive/wait pair has release/acquire semantics at cluster scope, so
-// the vectors one CTA writes to global memory are visible to the others
-// after it).  A cluster spreads the coarse levels' SpMVs over several SMs,
-// whose L2 bandwidth one SM alone does not have.
-struct CtaTeam {
-  __device__ int rank() const { return threadIdx.x; }
-  __device__ int size() const { return blockDim.x; }
-  __device__ void sync() const { __syncthreads(); }
+// Where the resident cycle starts and ends: the finer level's residual,
+// iterate and aggregates (restriction in, prolongation out), or a vector in
+// and out (the whole V-cycle, lt = 0), the MINRES step's Lanczos vector in and
+// its Givens step out.
+template <typename T>
+struct TailArgs {
+  int head, out;
+  const C2<T> *f_res;
+  C2<T> *f_x;
+  const int32_t *f_agg, *f_mp, *f_mi;
+  int64_t f_n;
+  const C2<T> *b;      // kHeadVector; kHeadLanczos: J z
+  C2<T> *r_old;        // kHeadLanczos: r_old in, the new Lanczos vector out
+  const C2<T> *r_cur;
+  C2<T> *z;            // kOutVector, kOutMinres
+  MinresScalars *ms;
 };
-struct ClusterTeam {
-  int r, n;  // CTA rank in the cluster, CTAs in the cluster
-  __device__ static ClusterTeam here() {
+
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+
+__device__ __forceinline__ void st_cluster(uint32_t addr, int rank, C2<float> v) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(ra), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, int rank, C2<double> v) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};\n" ::"r"(ra), "d"(v.x), "d"(v.y) : "memory");
+}
+
+// sign flip by the sign bit (a select between a value and its negative costs
+// an FP64 instruction otherwise)
+__device__ __forceinline__ float flip(float v, unsigned mask) { return __uint_as_float(__float_as_uint(v) ^ mask); }
+__device__ __forceinline__ double flip(double v, unsigned mask) {
+  return __hiloint2double(__double2hiint(v) ^ (int)mask, __double2loint(v));
+}
+
+template <typename T>
+struct Resident {
+  unsigned char *sm;
+  uint32_t sm_addr;
+  int rank, nct;  // CTA of the cluster, CTAs in it
+  int lane, warp, nwarps;
+
+  struct View {
+    const int32_t *rp, *ci;
+    const C2<T> *off;
+    const T *dia, *dinv;
+  };
+  __device__ C2<T> *vec(uint32_t o) const { return reinterpret_cast<C2<T> *>(sm + o); }
+  __device__ T *own(uint32_t o) const { return reinterpret_cast<T *>(sm + o); }
+  __device__ int rows_of(const LevelDesc<T> &A) const { return max(0, min(A.rw, A.n - rank * A.rw)); }
+  __device__ View view(const LevelDesc<T> &A) const {
+    const int r0 = rank * A.rw;
+    if (A.staged)
+      return View{(const int32_t *)(sm + A.s_rp), (const int32_t *)(sm + A.s_ci), (const C2<T> *)(sm + A.s_off),
+                  (const T *)(sm + A.s_dia), (const T *)(sm + A.s_dia) + 3 * A.rw};
+    return View{A.rp + r0, A.ci, A.off, A.dia + 3 * (int64_t)r0, A.dinv + 3 * (int64_t)r0};
+  }
+  // lanes per row for rw rows a CTA
+  __device__ static int lanes_for(int rw) {
+    const int cap = sizeof(T) == 8 ? 128 : kTailThreads;
+    int ln = 2;
+    while (ln < 16 && rw * ln * 2 <= cap) ln *= 2;
+    return ln;
+  }
+  // f(i, c, p, P, ok) for the own rows i < m, LN lanes a row (component c,
+  // part p of P); rows past m run with ok = false on the lanes of a warp that
+  // has a row
+  template <class F>
+  __device__ void rows(int m, int LN, F &&f) const {
+    const int rpw = 32 / LN, li = lane % LN;
+    for (int base = warp * rpw; base < m; base += nwarps * rpw) {
+      const int i = base + lane / LN;
+      const bool ok = i < m;
+      f(ok ? i : m - 1, li & 1, li >> 1, LN >> 1, ok);
+      __syncwarp();
+    }
+  }
+  __device__ static T parts_sum(T v, int P) {
+    for (int o = 2; o < 2 * P; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+  // component c of the off-diagonal row sum over x
+  __device__ static T row_sum(const View &A, int i, int c, int p, int P, const C2<T> *x) {
+    const unsigned sg = c ? 0u : 0x80000000u;
+    T acc = 0;
+    const int e = A.rp[i + 1];
+#pragma unroll 4
+    for (int k = A.rp[i] + p; k < e; k += P) {
+      const C2<T> v = A.off[k], xv = x[A.ci[k]];
+      acc = fma(v.x, c ? xv.y : xv.x, acc);
+      acc = fma(flip(v.y, sg), c ? xv.x : xv.y, acc);
+    }
+    return parts_sum(acc, P);
+  }
+  // component c of a list's sum over src
+  __device__ static T list_sum(const int32_t *mp, const int32_t *mi, int i, int c, int p, int P, const C2<T> *src) {
+    T acc = 0;
+    const int e = mp[i + 1];
+#pragma unroll 4
+    for (int k = mp[i] + p; k < e; k += P) {
+      const T *s = reinterpret_cast<const T *>(src + mi[k]);
+      acc += s[c];
+    }
+    return parts_sum(acc, P);
+  }
+  // the row's value, component c in v, to element `row` of the replicated
+  // vector at byte offset o of every CTA
+  __device__ void spread(uint32_t o, int row, int c, int p, int P, T v, bool ok) const {
+    const T other = __shfl_xor_sync(0xffffffffu, v, 1);
+    const C2<T> w = c ? C2<T>{other, v} : C2<T>{v, other};
+    if (!ok) return;
+    for (int q = 2 * p + c; q < nct; q += 2 * P) st_cluster(sm_addr + o + row * (uint32_t)sizeof(C2<T>), q, w);
+  }
+  __device__ void phase_end() const {
+    cluster_arrive();
+    cluster_wait();
+  }
+};
+
+// own rows of a level's operator (and its lists) into shared memory; the
+// members of its nodes over the finer level (mp, mi: null for the first)
+template <typename T>
+__device__ __forceinline__ void tail_stage(const Resident<T> &R, const LevelDesc<T> &A, bool matrix,
+                                           const int32_t *mp, const int32_t *mi) {
+  const int r0 = R.rank * A.rw, m = R.rows_of(A);
+  const int t = threadIdx.x, st = blockDim.x;
+  if (mp && m > 0) {
+    int32_t *smp = (int32_t *)(R.sm + A.s_mp), *smi = (int32_t *)(R.sm + A.s_mi);
+    const int b = mp[r0], e = mp[r0 + m];
+    for (int q = t; q <= m; q += st) smp[q] = mp[r0 + q] - b;
+    for (int q = t; q < e - b; q += st) smi[q] = mi[b + q];
+  }
+  if (!matrix) return;
+  if (A.agg)
+    for (int q = t; q < A.n; q += st) ((int32_t *)(R.sm + A.s_agg))[q] = A.agg[q];
+  if (!A.staged || m == 0) return;
+  int32_t *srp = (int32_t *)(R.sm + A.s_rp), *sci = (int32_t *)(R.sm + A.s_ci);
+  C2<T> *so = (C2<T> *)(R.sm + A.s_off);
+  T *sd = (T *)(R.sm + A.s_dia);
+  const int b = A.rp[r0], e = A.rp[r0 + m];
+  for (int q = t; q <= m; q += st) srp[q] = A.rp[r0 + q] - b;
+  for (int q = t; q < e - b; q += st) {
+    sci[q] = A.ci[b + q];
+    so[q] = A.off[b + q];
+  }
+  for (int q = t; q < 3 * m; q += st) {
+    sd[q] = A.dia[3 * (int64_t)r0 + q];
+    sd[3 * A.rw + q] = A.dinv[3 * (int64_t)r0 + q];
+  }
+}
+
+// One Chebyshev step of the own rows: x_in (replicated) -> x_out (spread);
+// the new iterate's component is handed to `last` instead when given.
+template <typename T, class Last>
+__device__ __forceinline__ void tail_cheb(const Resident<T> &R, const LevelDesc<T> &A, int k, uint32_t xin,
+                                          uint32_t xout, bool final_step, Last &&last) {
+  const typename Resident<T>::View V = R.view(A);
+  const int r0 = R.rank * A.rw, m = R.rows_of(A), LN = R.lanes_for(A.rw);
+  const C2<T> *x = R.vec(xin);
+  T *bo = R.own(A.b), *dn = R.own(A.d);
+  const T c1 = k == 0 ? (T)0 : A.coef[2 * k], c2 = k == 0 ? A.coef[0] : A.coef[2 * k + 1];
+  R.rows(m, LN, [&](int i, int c, int p, int P, bool ok) {
+    const T s = R.row_sum(V, i, c, p, P, x);
+    const T *xi = reinterpret_cast<const T *>(x + r0 + i);
+    const T xc = xi[c], xo = xi[c ^ 1];
+    const T rc = bo[2 * i + c] - (s + V.dia[3 * i + c] * xc + V.dia[3 * i + 2] * xo);
+    const T ro = __shfl_xor_sync(0xffffffffu, rc, 1);
+    const T z = V.dinv[3 * i + c] * rc + V.dinv[3 * i + 2] * ro;
+    const T dold = k == 0 ? (T)0 : dn[2 * i + c];
+    const T dv = k == 0 ? c2 * z : c1 * dold + c2 * z;
+    __syncwarp();  // every part has read the old direction
+    if (ok && p == 0) dn[2 * i + c] = dv;
+    const T xn = xc + dv;
+    if (final_step) last(i, c, p, xn, ok);
+    else R.spread(xout, r0 + i, c, p, P, xn, ok);
+  });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTailThreads)
+    resident_vcycle(const LevelDesc<T> *__restrict__ lv_g, int lt, int L, int deg, const T *__restrict__ Ainv,
+                    DenseMap D, uint32_t s_bd, uint32_t s_xd, TailArgs<T> a, const int *halt) {
+  extern __shared__ __align__(16) unsigned char tail_sm[];
+  __shared__ LevelDesc<T> lv[16];
+  __shared__ double s_dot[16];
+  __shared__ double s32[32];
+  Resident<T> R;
+  R.sm = tail_sm;
+  R.sm_addr = smem_addr(tail_sm);
+  {
     unsigned r, n;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
-    return ClusterTeam{(int)r, (int)n};
+    R.rank = (int)r;
+    R.nct = (int)n;
   }
-  __device__ int rank() const { return r * (int)blockDim.x + (int)threadIdx.x; }
-  __device__ int size() const { return n * (int)blockDim.x; }
-  __device__ void sync() const {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-  }
-};
-
-// Threads per row for a tail level of n rows: the largest power of two
-// <= 32 that still leaves a thread group per row, so the short serial chains
-// of the coarse rows (and aggregates) are split across lanes.
-template <class Team>
-__device__ __forceinline__ int tail_tpr(const Team &tm, int64_t n) {
-  int t = 1;
-  while (t < 32 && (int64_t)(tm.size() / (2 * t)) >= n) t *= 2;
-  return t;
-}
-
-// For every row i < n: the row's off-diagonal sum over x, reduced across its
-// tpr lanes, then epi(i, sr, si) on the group's first lane.
-template <typename T, class Team, class F>
-__device__ __forceinline__ void tail_rows(const Team &tm, const LevelDesc<T> &A, const C2<T> *x, F &&epi) {
-  const int tpr = tail_tpr(tm, A.n);
-  const int groups = tm.size() / tpr, g = tm.rank() / tpr, li = tm.rank() % tpr;
-  for (int64_t base = 0; base < A.n; base += groups) {
-    const int64_t i = base + g;
-    T sr = 0, si = 0;
-    if (i < A.n)
-      for (int32_t k = A.rp[i] + li; k < A.rp[i + 1]; k += tpr) {
-        const C2<T> v = A.off[k], xv = x[A.ci[k]];
-        row_mac(sr, si, v, xv);
-      }
-    for (int off = tpr >> 1; off > 0; off >>= 1) {
-      sr += __shfl_xor_sync(0xffffffffu, sr, off);
-      si += __shfl_xor_sync(0xffffffffu, si, off);
-    }
-    if (i < A.n && li == 0) epi(i, sr, si);
-  }
-}
-
-template <typename T, class Team>
-__device__ __forceinline__ void tail_body(const Team &tm, const LevelDesc<T> *lv, int lt, int L, int deg,
-                                          const T *__restrict__ Ainv, const DenseMap &D) {
-  const int tid = tm.rank(), bs = tm.size();
-  for (int l = lt; l < L - 1; l++) {
-    const LevelDesc<T> A = lv[l];
-    C2<T> *cur = (deg % 2) ? A.x : A.x2, *oth = (deg % 2) ? A.x2 : A.x;
-    for (int64_t i = tid; i < A.n; i += bs) cheb_first_elem<T>(i, A.dinv, A.coef[0], A.b[i], A.d, cur);
-    tm.sync();
-    for (int k = 1; k < deg; k++) {
-      tail_rows<T>(tm, A, cur, [&](int64_t i, T sr, T si) {
-        cheb_elem<T>(i, k, sr, si, A.dia, A.dinv, A.coef, A.b, cur, A.d, oth);
-      });
-      tm.sync();
-      C2<T> *t = cur;
-      cur = oth;
-      oth = t;
-    }
-    tail_rows<T>(tm, A, A.x, [&](int64_t i, T sr, T si) {
-      const C2<T> xi = A.x[i], bi = A.b[i];
-      const T d0r = A.dia[3 * i], d0i = A.dia[3 * i + 1], d1b = A.dia[3 * i + 2];
-      A.res[i] = C2<T>{bi.x - (sr + d0r * xi.x + d1b * xi.y), bi.y - (si + d1b * xi.x + d0i * xi.y)};
-    });
-    tm.sync();
-    // restriction: aggregate sums, split across lanes like the rows
-    const LevelDesc<T> Cl = lv[l + 1];
-    {
-      const int tpr = tail_tpr(tm, Cl.n);
-      const int groups = bs / tpr, g = tid / tpr, li = tid % tpr;
-      for (int64_t base = 0; base < Cl.n; base += groups) {
-        const int64_t a = base + g;
-        T sr = 0, si = 0;
-        if (a < Cl.n)
-          for (int32_t q = A.mem_ptr[a] + li; q < A.mem_ptr[a + 1]; q += tpr) {
-            const C2<T> v = A.res[A.mem_idx[q]];
-            sr += v.x;
-            si += v.y;
-          }
-        for (int off = tpr >> 1; off > 0; off >>= 1) {
-          sr += __shfl_xor_sync(0xffffffffu, sr, off);
-          si += __shfl_xor_sync(0xffffffffu, si, off);
-        }
-        if (a < Cl.n && li == 0) Cl.b[a] = C2<T>{sr, si};
-      }
-    }
-    tm.sync();
-  }
+  R.lane = threadIdx.x & 31;
+  R.warp = threadIdx.x >> 5;
+  R.nwarps = blockDim.x >> 5;
+  cluster_arrive();  // every CTA has started before any remote store: waited for below
   {
-    const LevelDesc<T> C = lv[L - 1];
-    const int m = (int)(2 * C.n);
-    const T *b = reinterpret_cast<const T *>(C.b);
-    T *x = reinterpret_cast<T *>(C.x);
-    for (int i = tid; i < m; i += bs) x[i] = dense_row(D, Ainv, i, b);
-    tm.sync();
+    const int nw = (int)(sizeof(LevelDesc<T>) / 4) * (L - lt);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(lv_g + lt);
+    for (int q = threadIdx.x; q < nw; q += blockDim.x) reinterpret_cast<uint32_t *>(lv + lt)[q] = src[q];
   }
-  for (int l = L - 2; l >= lt; l--) {
-    const LevelDesc<T> A = lv[l];
-    const C2<T> *xc = lv[l + 1].x;
-    for (int64_t i = tid; i < A.n; i += bs) {
-      const C2<T> c = xc[A.agg[i]];
-      C2<T> v = A.x[i];
-      v.x += c.x;
-      v.y += c.y;
-      A.x[i] = v;
+  __syncthreads();
+  // the operators and lists were written before the launch this one follows:
+  // staged while that one finishes
+  for (int l = lt; l < L; l++) {
+    const int32_t *mp = l > lt ? lv[l - 1].mem_ptr : a.f_mp, *mi = l > lt ? lv[l - 1].mem_idx : a.f_mi;
+    tail_stage<T>(R, lv[l], l < L - 1, mp, mi);
+  }
+  dep_sync();
+  __syncthreads();
+  const bool stop = (halt && *halt >= 2) || (a.head == kHeadLanczos && a.ms->done >= 2);
+  cluster_wait();
+  if (stop) return;  // every CTA alike, before any remote store
+  // down: level l's right-hand side is in its own rows, the first Chebyshev
+  // step (x = c0 D^-1 b) is spread with it
+  auto start_level = [&](int l, int i, int c, int p, int P, T bc, bool ok) {
+    const LevelDesc<T> &A = lv[l];
+    const int r0 = R.rank * A.rw;
+    if (l == L - 1) {
+      R.spread(s_bd, r0 + i, c, p, P, bc, ok);
+      return;
     }
-    tm.sync();
-    C2<T> *cur = A.x, *oth = A.x2;
-    for (int k = 0; k < deg; k++) {
-      tail_rows<T>(tm, A, cur, [&](int64_t i, T sr, T si) {
-        cheb_elem<T>(i, k, sr, si, A.dia, A.dinv, A.coef, A.b, cur, A.d, oth);
-      });
-      tm.sync();
-      C2<T> *t = cur;
+    const typename Resident<T>::View V = R.view(A);
+    const T bo = __shfl_xor_sync(0xffffffffu, bc, 1);
+    const T x = A.coef[0] * (V.dinv[3 * i + c] * bc + V.dinv[3 * i + 2] * bo);
+    if (ok && p == 0) {
+      R.own(A.b)[2 * i + c] = bc;
+      R.own(A.d)[2 * i + c] = x;
+    }
+    R.spread(deg % 2 == 1 ? A.xb : A.xa, r0 + i, c, p, P, x, ok);
+  };
+  {
+    const LevelDesc<T> &A = lv[lt];
+    const int r0 = R.rank * A.rw, m = R.rows_of(A), LN = R.lanes_for(A.rw);
+    T la0 = 0, la1 = 0, la2 = 0;
+    if (a.head == kHeadLanczos) {
+      const T *la = lanczos_coef<T>(a.ms);
+      la0 = la[0];
+      la1 = la[1];
+      la2 = la[2];
+    }
+    R.rows(m, LN, [&](int i, int c, int p, int P, bool ok) {
+      T bc;
+      if (a.head == kHeadRestrict) {
+        bc = R.list_sum((const int32_t *)(R.sm + A.s_mp), (const int32_t *)(R.sm + A.s_mi), i, c, p, P, a.f_res);
+      } else {
+        const int64_t e = 2 * (int64_t)(r0 + i) + c;
+        bc = reinterpret_cast<const T *>(a.b)[e];
+        if (a.head == kHeadLanczos) {
+          T *ro = reinterpret_cast<T *>(a.r_old);
+          bc = la0 * bc - la1 * ro[e] - la2 * reinterpret_cast<const T *>(a.r_cur)[e];
+          __syncwarp();  // every part has read r_old
+          if (ok && p == 0) ro[e] = bc;
+        }
+      }
+      start_level(lt, i, c, p, P, bc, ok);
+    });
+  }
+  R.phase_end();
+  for (int l = lt; l < L - 1; l++) {
+    const LevelDesc<T> &A = lv[l];
+    uint32_t cur = deg % 2 == 1 ? A.xb : A.xa, oth = deg % 2 == 1 ? A.xa : A.xb;
+    for (int k = 1; k < deg; k++) {
+      tail_cheb<T>(R, A, k, cur, oth, false, [](int, int, int, T, bool) {});
+      R.phase_end();
+      const uint32_t t = cur;
       cur = oth;
       oth = t;
     }
-    if (cur != A.x) {
-      for (int64_t i = tid; i < A.n; i += bs) A.x[i] = cur[i];
-      tm.sync();
+    // the residual over xa (the pre-smoothed iterate is xb)
+    {
+      const typename Resident<T>::View V = R.view(A);
+      const int r0 = R.rank * A.rw, m = R.rows_of(A), LN = R.lanes_for(A.rw);
+      const C2<T> *x = R.vec(A.xb);
+      const T *bo = R.own(A.b);
+      R.rows(m, LN, [&](int i, int c, int p, int P, bool ok) {
+        const T s = R.row_sum(V, i, c, p, P, x);
+        const T *xi = reinterpret_cast<const T *>(x + r0 + i);
+        const T rc = bo[2 * i + c] - (s + V.dia[3 * i + c] * xi[c] + V.dia[3 * i + 2] * xi[c ^ 1]);
+        R.spread(A.xa, r0 + i, c, p, P, rc, ok);
+      });
+    }
+    R.phase_end();
+    {
+      const LevelDesc<T> &C = lv[l + 1];
+      const C2<T> *res = R.vec(A.xa);
+      R.rows(R.rows_of(C), R.lanes_for(C.rw), [&](int i, int c, int p, int P, bool ok) {
+        const T bc = R.list_sum((const int32_t *)(R.sm + C.s_mp), (const int32_t *)(R.sm + C.s_mi), i, c, p, P, res);
+        start_level(l + 1, i, c, p, P, bc, ok);
+      });
+    }
+    R.phase_end();
+  }
+  // the coarsest level: its dense inverse, real rows split over 16 lanes
+  {
+    const LevelDesc<T> &C = lv[L - 1];
+    const T *bd = reinterpret_cast<const T *>(tail_sm + s_bd);
+    const int m2 = 2 * R.rows_of(C), i0 = 2 * R.rank * C.rw, li = R.lane & 15;
+    for (int base = 2 * R.warp; base < m2; base += 2 * R.nwarps) {
+      const int i = base + (R.lane >> 4);  // a warp holds both components of a node
+      const int64_t row = i0 + i;
+      const T *av = Ainv + D.rowoff[row], *bb = bd + D.bstart[row];
+      const int m = D.bdim[row];
+      T s = 0;
+#pragma unroll 4
+      for (int j = li; j < m; j += 16) s = fma(av[j], bb[j], s);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const T other = __shfl_xor_sync(0xffffffffu, s, 16);
+      const C2<T> w = R.lane < 16 ? C2<T>{s, other} : C2<T>{other, s};
+      if (R.lane < R.nct) st_cluster(R.sm_addr + s_xd + (uint32_t)(row >> 1) * (uint32_t)sizeof(C2<T>), R.lane, w);
     }
   }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(1024) tail_vcycle(const LevelDesc<T> *__restrict__ lv, int lt, int L,
-                                                    int deg, const T *__restrict__ Ainv, DenseMap D,
-                                                    const int *halt) {
-  dep_sync();
-  if (halt && *halt >= 2) return;
-  tail_body(CtaTeam{}, lv, lt, L, deg, Ainv, D);
-}
-
-// The same over a thread-block cluster (launched with a cluster dimension
-// equal to the grid): the halt flag is read by every CTA alike, so the
-// cluster leaves or stays together.
-template <typename T>
-__global__ void __launch_bounds__(1024) tail_vcycle_cluster(const LevelDesc<T> *__restrict__ lv, int lt, int L,
-                                                            int deg, const T *__restrict__ Ainv, DenseMap D,
-                                                            const int *halt) {
-  dep_sync();
-  if (halt && *halt >= 2) return;
-  tail_body(ClusterTeam::here(), lv, lt, L, deg, Ainv, D);
+  R.phase_end();
+  uint32_t xc = s_xd;
+  double part = 0.0;
+  for (int l = L - 2; l >= lt; l--) {
+    const LevelDesc<T> &A = lv[l];
+    // coarse correction on the CTA's own copy of the whole vector
+    {
+      C2<T> *x = R.vec(A.xb);
+      const C2<T> *c = R.vec(xc);
+      const int32_t *ag = (const int32_t *)(R.sm + A.s_agg);
+      for (int j = threadIdx.x; j < A.n; j += blockDim.x) {
+        const C2<T> e = c[ag[j]];
+        C2<T> v = x[j];
+        v.x += e.x;
+        v.y += e.y;
+        x[j] = v;
+      }
+    }
+    __syncthreads();
+    uint32_t in = A.xb, out = A.xa;
+    const int r0 = R.rank * A.rw;
+    for (int k = 0; k < deg; k++) {
+      const bool fin = l == lt && k == deg - 1 && a.out != kOutProlong;
+      tail_cheb<T>(R, A, k, in, out, fin, [&](int i, int c, int p, T xn, bool ok) {
+        if (!ok || p != 0) return;
+        reinterpret_cast<T *>(a.z)[2 * (int64_t)(r0 + i) + c] = xn;
+        if (a.out == kOutMinres) part += (double)R.own(A.b)[2 * i + c] * (double)xn;
+      });
+      if (!fin) R.phase_end();
+      const uint32_t t = in;
+      in = out;
+      out = t;
+    }
+    xc = in;
+  }
+  if (a.out == kOutProlong) {
+    const C2<T> *c = R.vec(xc);
+    for (int64_t j = (int64_t)R.rank * blockDim.x + threadIdx.x; j < a.f_n; j += (int64_t)R.nct * blockDim.x) {
+      const C2<T> e = c[a.f_agg[j]];
+      C2<T> v = a.f_x[j];
+      v.x += e.x;
+      v.y += e.y;
+      a.f_x[j] = v;
+    }
+  } else if (a.out == kOutMinres) {
+    // <r, z>: the CTAs' sums in CTA order, then the Givens step
+    const double s = block_sum(part, s32);
+    if (threadIdx.x == 0) {
+      uint32_t ra;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(smem_addr(&s_dot[R.rank])), "r"(0));
+      asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(ra), "d"(s) : "memory");
+    }
+    R.phase_end();
+    if (R.rank == 0 && threadIdx.x == 0) {
+      dep_trigger();
+      double t = 0.0;
+      for (int q = 0; q < R.nct; q++) t += s_dot[q];
+      minres_advance(a.ms, t);
+    }
+  }
 }
 
 // plain MINRES pieces for the single-level case
@@ -889,6 +1144,19 @@ struct AmgLevel {
   bool tuned32 = false, tuned64 = false;
   // transfer to the next level
   DevBuf<int32_t> agg, mem_ptr, mem_idx, seg_ptr, seg_idx, intra_ptr, intra_idx;
+  // host copies for the resident cycle's layout (levels and transfers small
+  // enough for it)
+  std::vector<int32_t> h_rp, h_mem_ptr;
+};
+
+// One layout of the resident V-cycle: its first level, the level descriptors
+// and the shared memory of a CTA.
+template <typename T>
+struct TailPlan {
+  int lt = -1;  // -1: none
+  size_t smem = 0;
+  uint32_t s_bd = 0, s_xd = 0;
+  DevBuf<LevelDesc<T>> desc;
 };
 
 template <typename T>
@@ -899,7 +1167,9 @@ struct AmgVals {
   std::vector<DevBuf<T>> dia;      // level >= 1
   std::vector<DevBuf<T>> dinv, coef;
   std::vector<DevBuf<C2<T>>> b, x, x2, d, res;
-  DevBuf<LevelDesc<T>> desc;       // for the coarse-level tail
+  // the resident V-cycle's layouts: [0] in use, [1] the one that keeps the
+  // fine level on the grid (kernel timing of a mesh that [0] takes whole)
+  TailPlan<T> plan[2];
   // row sums of |K_ij| on the fine level for its Gershgorin bound, computed
   // once: |K_ij| = |alpha_ij| does not depend on mu (the phase factor has
   // modulus one), so only the diagonal blocks change between refreshes
@@ -937,14 +1207,16 @@ struct Amg::Impl {
   // launches return at once once the solve has converged
   const int *halt = nullptr;
   template <typename T> void prime();
-  // CTAs of the coarse-level tail, FP32 and FP64 (a thread-block cluster
-  // when > 1).  The FP64 tail of a tetrahedral mesh runs on a cluster of 8:
-  // the coarse SpMVs' FP64 arithmetic then spreads over 8 SMs (plain FP64
-  // continuation at 64^3: 68.2 -> 71.2 steps/s).  The
-  // FP32 tail stays on one CTA, whose vectors stay in its L1 between phases:
-  // clusters of 8 and 16 took the learned line from 671 to 649 and 647
-  // steps/s (in-place A/B).
-  int tail_ctas[2] = {1, 1};
+  void choose_cluster();
+  int tail_ctas = 1;        // CTAs of the resident cycle's cluster
+  bool grid_coarse = false;  // coarsest level too large for it: dense kernel on the grid
+  template <typename T> size_t tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32_t *bd, uint32_t *xd);
+  template <typename T> void build_plan(TailPlan<T> &P, int first);
+  template <typename T> const TailPlan<T> &plan() {
+    AmgVals<T> &V = vals<T>();
+    return V.plan[V.plan[1].lt >= 0 && (nls.timers[0].on || nls.timers[1].on) ? 1 : 0];
+  }
+  template <typename T> void launch_tail(const TailPlan<T> &P, const TailArgs<T> &a, bool overlap);
   // V-cycle launches overlap their predecessors (launch_dep) unless the
   // handle turned that off or times kernels with events between launches
   bool ovl() const { return nls.overlap_launches && !nls.timers[0].on && !nls.timers[1].on; }
@@ -1029,15 +1301,27 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
       A.intra_idx.upload(h.intra_idx, st);
     }
   }
-  // the fine level always runs on the whole grid; the first level at or
-  // below kTailMax nodes and everything under it run in one CTA
+  for (int l = 0; l < L; l++) {
+    if (H[l].n <= std::max(kTailMax, kResidentMax)) I.lev[l].h_rp = H[l].rp;
+    if (l + 1 < L && H[l + 1].n <= std::max(kTailMax, kResidentMax)) I.lev[l].h_mem_ptr = H[l].mem_ptr;
+  }
+  // The resident cycle starts on the first level small enough for it whose
+  // vectors, with those of the levels below, fit a CTA's shared memory in
+  // FP64; the levels above it run on the whole grid.
+  I.choose_cluster();
   I.lt = L - 1;
-  for (int l = 1; l < L; l++)
-    if (I.lev[l].n <= kTailMax) {
+  I.grid_coarse = L < 2;
+  for (int l = 0; l < L; l++) {
+    if (I.lev[l].n > (l == 0 ? kResidentMax : kTailMax)) {
+      if (l == L - 1) I.grid_coarse = true;
+      continue;
+    }
+    if (I.tail_layout<double>(l, nullptr, nullptr, nullptr) <= (size_t)kTailSmem) {
       I.lt = l;
       break;
     }
-  if (I.lt < 1) I.lt = L - 1;
+    if (l == L - 1) I.grid_coarse = true;
+  }
   I.lmax_bits.alloc(L);
   I.lmax.alloc(L);
   {
@@ -1125,32 +1409,18 @@ void Amg::Impl::ensure_vals() {
     }
     V.dinv[l].alloc(3 * n);
     V.coef[l].alloc(2 * std::max(opt.smooth_degree, 1) + 2);
+    // (levels inside the resident cycle keep their vectors in shared memory)
+    if (l > 0 && l >= lt && !grid_coarse) continue;
     V.b[l].alloc(n);
     V.x[l].alloc(n);
     V.x2[l].alloc(n);
     V.d[l].alloc(n);
     V.res[l].alloc(n);
   }
-  std::vector<LevelDesc<T>> desc(L);
-  for (int l = 0; l < L; l++) {
-    LevelDesc<T> &D = desc[l];
-    D.n = lev[l].n;
-    D.rp = lev[l].rp;
-    D.ci = lev[l].ci;
-    D.off = off<T>(l);
-    D.dia = dia<T>(l);
-    D.dinv = V.dinv[l].p;
-    D.coef = V.coef[l].p;
-    D.b = V.b[l].p;
-    D.x = V.x[l].p;
-    D.x2 = V.x2[l].p;
-    D.d = V.d[l].p;
-    D.res = V.res[l].p;
-    D.agg = lev[l].agg.p;
-    D.mem_ptr = lev[l].mem_ptr.p;
-    D.mem_idx = lev[l].mem_idx.p;
+  if (!grid_coarse) {
+    build_plan<T>(V.plan[0], lt);
+    if (lt == 0) build_plan<T>(V.plan[1], 1);
   }
-  V.desc.upload(desc, nls.stream);
   nls.sync();
   prime<T>();
   V.ready = true;
@@ -1248,13 +1518,16 @@ void Amg::Impl::prime() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
   NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, ResidOp<T>>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-  tail_ctas[sizeof(T) == 8] = 1;
-  const int L = (int)lev.size();
-  if (sizeof(T) == 8 && L >= 2 && lt < L) {
-    constexpr int c = 8;  // portable cluster size
+}
+
+// The cluster's size: 16 CTAs (above the portable 8) when the device runs
+// them at the layouts' largest shared memory, else 8, else one.
+void Amg::Impl::choose_cluster() {
+  auto fits = [&](int c, const void *k) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(c);
-    cfg.blockDim = dim3(1024);
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = kTailSmem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = c;
@@ -1262,15 +1535,104 @@ void Amg::Impl::prime() {
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int nc = 0;
-    const bool ok = cudaOccupancyMaxActiveClusters(&nc, tail_vcycle_cluster<T>, &cfg) == cudaSuccess && nc > 0;
-    cudaGetLastError();  // a device without clusters of 8 keeps the one-CTA tail
-    // tetrahedral hierarchies only: their coarse rows hold about twice the
-    // nonzeros of triangular ones, and the FP64 tail of a 2-D 65 x 65 mesh
-    // lost more to the cluster barriers than it gained (FP64 Newton solve
-    // 111.8 -> 104.4 solves/s), while the 64^3 one gained
-    if (ok && nls.mesh->nvc == 4) tail_ctas[1] = c;
+    int n = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return ok;
+  };
+  const void *ks[2] = {(const void *)resident_vcycle<float>, (const void *)resident_vcycle<double>};
+  for (const void *k : ks) {
+    NOSH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
+    NOSH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   }
+  tail_ctas = 1;
+  for (int c : {16, 8})
+    if (fits(c, ks[0]) && fits(c, ks[1])) {
+      tail_ctas = c;
+      break;
+    }
+}
+
+// Shared-memory layout of a resident cycle that starts on level `first`;
+// returns the bytes its vectors and lists need (the operators' rows are
+// staged level by level while they fit).
+template <typename T>
+size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32_t *bd, uint32_t *xd) {
+  const int L = (int)lev.size(), C = tail_ctas;
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o += (bytes + 15) / 16 * 16;
+    return (uint32_t)at;
+  };
+  // the longest of the CTAs' ranges of a CSR's entries
+  auto longest = [&](const std::vector<int32_t> &ptr, int n, int rw) {
+    int m = 0;
+    for (int r = 0; r * rw < n; r++) m = std::max(m, ptr[std::min(n, (r + 1) * rw)] - ptr[r * rw]);
+    return (size_t)m;
+  };
+  std::vector<LevelDesc<T>> D(L);
+  for (int l = first; l < L; l++) {
+    LevelDesc<T> &A = D[l];
+    A = LevelDesc<T>{};
+    A.n = (int)lev[l].n;
+    A.rw = (A.n + C - 1) / C;
+    if (l > first || first > 0) {
+      A.s_mp = take(4 * (size_t)(A.rw + 1));
+      A.s_mi = take(4 * longest(lev[l - 1].h_mem_ptr, A.n, A.rw));
+    }
+    if (l == L - 1) break;
+    A.xa = take(sizeof(C2<T>) * (size_t)A.n);
+    A.xb = take(sizeof(C2<T>) * (size_t)A.n);
+    A.b = take(sizeof(C2<T>) * (size_t)A.rw);
+    A.d = take(sizeof(C2<T>) * (size_t)A.rw);
+    A.s_agg = take(4 * (size_t)A.n);
+  }
+  const uint32_t b0 = take(sizeof(C2<T>) * (size_t)D[L - 1].n), x0 = take(sizeof(C2<T>) * (size_t)D[L - 1].n);
+  const size_t need = o;
+  if (bd) *bd = b0;
+  if (xd) *xd = x0;
+  if (!desc) return need;
+  AmgVals<T> &V = vals<T>();
+  for (int l = first; l < L; l++) {
+    LevelDesc<T> &A = D[l];
+    A.rp = lev[l].rp;
+    A.ci = lev[l].ci;
+    A.off = off<T>(l);
+    A.dia = dia<T>(l);
+    A.dinv = V.dinv[l].p;
+    A.coef = V.coef[l].p;
+    A.agg = lev[l].agg.p;
+    A.mem_ptr = lev[l].mem_ptr.p;
+    A.mem_idx = lev[l].mem_idx.p;
+    if (l == L - 1) break;
+    const size_t nz = longest(lev[l].h_rp, A.n, A.rw), before = o;
+    A.s_rp = take(4 * (size_t)(A.rw + 1));
+    A.s_ci = take(4 * nz);
+    A.s_off = take(sizeof(C2<T>) * nz);
+    A.s_dia = take(6 * sizeof(T) * (size_t)A.rw);
+    if (o <= (size_t)kTailSmem) A.staged = 1;
+    else o = before;
+  }
+  *desc = std::move(D);
+  return o;
+}
+
+template <typename T>
+void Amg::Impl::build_plan(TailPlan<T> &P, int first) {
+  std::vector<LevelDesc<T>> d;
+  P.smem = tail_layout<T>(first, &d, &P.s_bd, &P.s_xd);
+  P.desc.upload(d, nls.stream);
+  nls.sync();
+  P.lt = first;
+}
+
+template <typename T>
+void Amg::Impl::launch_tail(const TailPlan<T> &P, const TailArgs<T> &a, bool overlap) {
+  launch_cluster_dep(overlap, tail_ctas, resident_vcycle<T>, dim3(kTailThreads), P.smem, nls.stream,
+                     (const LevelDesc<T> *)P.desc.p, P.lt, (int)lev.size(), std::max(opt.smooth_degree, 1),
+                     dense_inv<T>(), dmap(), P.s_bd, P.s_xd, a, halt);
+  ++nls.launch_count;
 }
 
 template <typename T, class Op>
@@ -1318,31 +1680,39 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
   rows<T>(l, x, rop);
   if (tm) tm->end(st, (deg - 1) * cheb_bytes + res_bytes, deg);
   const AmgLevel &Cl = lev[l + 1];
-  if (l + 1 < lt) {
-    // restriction + first step of level l+1, whose pre-smoothing must end in
-    // its x buffer
-    C2<T> *first = (deg % 2 == 1) ? V.x[l + 1].p : V.x2[l + 1].p;
-    launch_dep(ovl(), restrict_first<T>, dim3(div_up(Cl.n * kAggLanes, B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
-               A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p, V.coef[l + 1].p, V.d[l + 1].p, first,
-               halt);
-    ++nls.launch_count;
-    descend_ascend<T>(l + 1, V.b[l + 1].p, V.x[l + 1].p, nullptr);
+  const TailPlan<T> &P = plan<T>();
+  if (!grid_coarse && l + 1 == P.lt) {
+    TailArgs<T> a{};
+    a.head = kHeadRestrict;
+    a.out = kOutProlong;
+    a.f_res = V.res[l].p;
+    a.f_x = x;
+    a.f_agg = A.agg.p;
+    a.f_mp = A.mem_ptr.p;
+    a.f_mi = A.mem_idx.p;
+    a.f_n = A.n;
+    launch_tail<T>(P, a, ovl());
   } else {
-    launch_dep(ovl(), restrict_kernel<T>, dim3(div_up(Cl.n * kAggLanes, B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
-               A.mem_idx.p, V.res[l].p, V.b[l + 1].p, halt);
-    ++nls.launch_count;
-    const int tc = tail_ctas[sizeof(T) == 8];
-    if (tc > 1)
-      launch_cluster_dep(ovl(), tc, tail_vcycle_cluster<T>, dim3(1024), 0, st, V.desc.p, lt, L, deg,
-                         dense_inv<T>(), dmap(), halt);
-    else
-      launch_dep(ovl(), tail_vcycle<T>, dim3(1), dim3(1024), 0, st, V.desc.p, lt, L, deg, dense_inv<T>(), dmap(),
-               halt);
+    if (l + 1 < L - 1) {
+      // restriction + first step of level l+1, whose pre-smoothing must end
+      // in its x buffer
+      C2<T> *first = (deg % 2 == 1) ? V.x[l + 1].p : V.x2[l + 1].p;
+      launch_dep(ovl(), restrict_first<T>, dim3(div_up(Cl.n * kAggLanes, B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
+                 A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p, V.coef[l + 1].p, V.d[l + 1].p, first,
+                 halt);
+      ++nls.launch_count;
+      descend_ascend<T>(l + 1, V.b[l + 1].p, V.x[l + 1].p, nullptr);
+    } else {
+      launch_dep(ovl(), restrict_kernel<T>, dim3(div_up(Cl.n * kAggLanes, B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
+                 A.mem_idx.p, V.res[l].p, V.b[l + 1].p, halt);
+      const int m = (int)(2 * Cl.n);
+      launch_dep(ovl(), dense_matvec<T>, dim3(div_up(m * kDenseLanes, B)), dim3(B), 0, st, m, dense_inv<T>(), dmap(),
+                 (const T *)V.b[l + 1].p, (T *)V.x[l + 1].p, halt);
+      nls.launch_count += 2;
+    }
+    launch_dep(ovl(), prolong_kernel<T>, dim3(div_up(A.n, B)), dim3(B), 0, st, A.n, A.agg.p, V.x[l + 1].p, x, halt);
     ++nls.launch_count;
   }
-  launch_dep(ovl(), prolong_kernel<T>, dim3(div_up(A.n, B)), dim3(B), 0, st, A.n, A.agg.p, V.x[l + 1].p, x,
-             halt);
-  ++nls.launch_count;
   cur = x;
   oth = V.x2[l].p;
   if (tm) tm->begin(st);
@@ -1372,9 +1742,21 @@ void Amg::apply(const T *r, T *z) {
   const AmgLevel &A = I.lev[0];
   if (L == 1) {
     const int m2 = (int)(2 * A.n);
-    launch_dep(I.ovl(), dense_matvec<T>, dim3(div_up(m2, 128)), dim3(128), 0, st, m2, I.dense_inv<T>(), I.dmap(),
-               r, z);
+    launch_dep(I.ovl(), dense_matvec<T>, dim3(div_up(m2 * kDenseLanes, 256)), dim3(256), 0, st, m2,
+               I.dense_inv<T>(), I.dmap(), r, z, (const int *)nullptr);
     ++I.nls.launch_count;
+    NOSH_CUDA(cudaGetLastError());
+    return;
+  }
+  if (const TailPlan<T> &P = I.plan<T>(); P.lt == 0) {
+    // the whole cycle resident; no overlap: it stages the block inverses,
+    // which the refresh before it may have written
+    TailArgs<T> a{};
+    a.head = kHeadVector;
+    a.out = kOutVector;
+    a.b = (const C2<T> *)r;
+    a.z = (C2<T> *)z;
+    I.launch_tail<T>(P, a, false);
     NOSH_CUDA(cudaGetLastError());
     return;
   }
@@ -1430,13 +1812,27 @@ void Amg::apply_minres(MinresScalars *ms, const T *u, T *r_old, const T *r_cur, 
     NOSH_CUDA(cudaGetLastError());
     return;
   }
+  I.halt = &ms->done;
+  if (const TailPlan<T> &P = I.plan<T>(); P.lt == 0) {
+    TailArgs<T> a{};
+    a.head = kHeadLanczos;
+    a.out = kOutMinres;
+    a.b = (const C2<T> *)u;
+    a.r_old = (C2<T> *)r_old;
+    a.r_cur = (const C2<T> *)r_cur;
+    a.z = (C2<T> *)z_out;
+    a.ms = ms;
+    I.launch_tail<T>(P, a, I.ovl());
+    I.halt = nullptr;
+    NOSH_CUDA(cudaGetLastError());
+    return;
+  }
   const int deg = std::max(I.opt.smooth_degree, 1);
   // the fine level's right-hand side is r_new itself: point b[0] at r_old
   C2<T> *first = (deg % 2 == 1) ? (C2<T> *)z_out : V.x2[0].p;
   launch_dep(I.ovl(), lanczos_first<T>, dim3(div_up(A.n, 256)), dim3(256), 0, st, A.n, ms, (const C2<T> *)u,
              (C2<T> *)r_old, (const C2<T> *)r_cur, V.dinv[0].p, V.coef[0].p, V.d[0].p, first);
   ++I.nls.launch_count;
-  I.halt = &ms->done;
   I.descend_ascend<T>(0, (const C2<T> *)r_old, (C2<T> *)z_out, ms);
   I.halt = nullptr;
   NOSH_CUDA(cudaGetLastError());
