@@ -161,7 +161,7 @@ int nosh_nls_system_iterations(nosh_nls nls, int *newton_iters, int *krylov_iter
 int nosh_nls_system_norms(nosh_nls nls, double *norms);
 /* The preconditioner hierarchy (after the first rebuild): number of
  * levels, their sizes (nodes; up to max_sizes entries) and the first level
- * run by the single-CTA tail kernel.  num_levels is 0 before the first
+ * run by the resident coarse-cycle kernel (0: the whole V-cycle).  num_levels is 0 before the first
  * rebuild. */
 int nosh_nls_amg_levels(nosh_nls nls, int *num_levels, int64_t *sizes,
                         int max_sizes, int *tail_level);

@@ -31,9 +31,13 @@ using namespace dev;
 namespace {
 
 // The largest level that the resident V-cycle starts on, and the largest mesh
-// that it takes whole.
+// that it takes whole.  Measured per MINRES iteration, whole against from
+// level 1 on: 17^2 25 / 36 us (FP64) and 21 / 30 (mixed), 45^2 41 / 45 and
+// 30 / 35, 11^3 cubes 35 / 43 and 23 / 30; a 65^2 square's rows (265 a CTA)
+// are more than one pass of the CTA.  Levels of 2048 and 4096 nodes in it gained
+// nothing on 32^3 and 48^3 (their SpMVs fill the grid by then).
 constexpr int64_t kTailMax = 1024;
-constexpr int64_t kResidentMax = 0;
+constexpr int64_t kResidentMax = 2048;
 
 struct HostLevel {
   int64_t n = 0;
@@ -460,6 +464,7 @@ struct ResidOp {
   const C2<T> *b, *x;
   C2<T> *res;
   const int *halt = nullptr;
+  bool trigger = false;
   struct Pre {
     C2<T> xi, bi;
     T d0r, d0i, d1b;
@@ -676,13 +681,20 @@ __global__ void dense_matvec(int m, const T *__restrict__ Ainv, DenseMap D, cons
 //
 // The coarse levels are latency: a few hundred to a thousand rows, five SpMVs
 // each.  A launch per step costs about 3 us; one CTA for all of them left the
-// FP64 pipe of a single SM as the bound (a 900-node level of the 65^2 square:
+// FP64 pipe of a single SM as the bound (a 737-node level of the 65^2 square:
 // 65 us a cycle, 79 % of that pipe).  Here the rows of a level are spread over
 // the CTAs of a cluster (16, which needs the opt-in above the portable 8) and
 // each level's vectors live in shared memory, replicated in every CTA: a row's
-// result is stored to all CTAs (DSMEM), a hardware cluster barrier ends the
-// phase, and every gather is a local shared-memory read.  Each CTA's rows of
-// the operators are staged in its shared memory while the predecessor runs.
+// result is sent to all CTAs by asynchronous stores that complete on the
+// phase's mbarrier in the receiving CTA, and every gather is a local shared-
+// memory read.  A CTA goes on as soon as it has the whole vector; a cluster
+// barrier per phase instead measured 1000-1400 cycles of each phase's 2800.
+// Each CTA's rows of the operators are staged in its shared memory while the
+// predecessor (which triggers this launch at its start) runs.
+//
+// A vector may be overwritten by other CTAs as soon as they have the vector
+// of the phase that reads it: each sends its rows of that phase only after
+// its own reads, and nobody goes on without all rows.
 //
 // A row is summed by LN lanes: even lanes its real component, odd lanes its
 // imaginary one (two FMAs a nonzero each, no reduction between the two), and
@@ -692,11 +704,12 @@ __global__ void dense_matvec(int m, const T *__restrict__ Ainv, DenseMap D, cons
 // up to sixteen ways.
 constexpr int kTailThreads = 512;
 constexpr int kTailSmem = 200 * 1024;  // shared memory of one CTA, at most
+constexpr int kMaxDegree = 8;          // of the smoother (nosh_nls_set_amg_options)
 
 template <typename T>
 struct LevelDesc {
-  int n, rw;  // rows, rows per CTA (CTA r owns [r rw, (r + 1) rw))
-  int staged;  // this CTA's rows of the operator are staged
+  int n, rw;   // rows, rows per CTA (CTA r owns [r rw, (r + 1) rw))
+  int lnb;     // log2 of the lanes per row
   const int32_t *rp, *ci;
   const C2<T> *off;
   const T *dia, *dinv, *coef;
@@ -728,22 +741,42 @@ struct TailArgs {
   const C2<T> *r_cur;
   C2<T> *z;            // kOutVector, kOutMinres
   MinresScalars *ms;
+  unsigned *fail;      // set when a wait for a phase's vector gives up
 };
+
+// The coarsest level's dense inverse in shared memory (byte offsets): the own
+// real rows, packed as in global memory, and their (offset, first column,
+// columns); staged when it fits.
+struct TailDense {
+  uint32_t s_bd, s_xd, s_a, s_map;
+  int staged;
+};
+
+// phases of a level: the first step, deg - 1 pre-smoothing steps, the
+// residual, deg post-smoothing steps; two for the coarsest level
+__host__ __device__ constexpr int tail_phases(int levels, int deg) { return (levels - 1) * (2 * deg + 1) + 2; }
 
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
 }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
-
-__device__ __forceinline__ void st_cluster(uint32_t addr, int rank, C2<float> v) {
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, int rank) {
   uint32_t ra;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(ra), "f"(v.x), "f"(v.y) : "memory");
+  asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
+  return ra;
 }
-__device__ __forceinline__ void st_cluster(uint32_t addr, int rank, C2<double> v) {
-  uint32_t ra;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(addr), "r"(rank));
-  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};\n" ::"r"(ra), "d"(v.x), "d"(v.y) : "memory");
+// store to another CTA's shared memory, completing on its mbarrier
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t bar, int rank, C2<float> v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];\n" ::"r"(
+                   map_rank(addr, rank)),
+               "f"(v.x), "f"(v.y), "r"(map_rank(bar, rank))
+               : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t bar, int rank, C2<double> v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];\n" ::"r"(
+                   map_rank(addr, rank)),
+               "d"(v.x), "d"(v.y), "r"(map_rank(bar, rank))
+               : "memory");
 }
 
 // sign flip by the sign bit (a select between a value and its negative costs
@@ -753,160 +786,195 @@ __device__ __forceinline__ double flip(double v, unsigned mask) {
   return __hiloint2double(__double2hiint(v) ^ (int)mask, __double2loint(v));
 }
 
-template <typename T>
-struct Resident {
-  unsigned char *sm;
-  uint32_t sm_addr;
-  int rank, nct;  // CTA of the cluster, CTAs in it
-  int lane, warp, nwarps;
+extern __shared__ __align__(16) unsigned char tail_sm[];
+template <typename V>
+__device__ __forceinline__ V &tail_at(uint32_t o, int i = 0) {
+  return *(reinterpret_cast<V *>(tail_sm + o) + i);
+}
 
-  struct View {
-    const int32_t *rp, *ci;
-    const C2<T> *off;
-    const T *dia, *dinv;
-  };
-  __device__ C2<T> *vec(uint32_t o) const { return reinterpret_cast<C2<T> *>(sm + o); }
-  __device__ T *own(uint32_t o) const { return reinterpret_cast<T *>(sm + o); }
-  __device__ int rows_of(const LevelDesc<T> &A) const { return max(0, min(A.rw, A.n - rank * A.rw)); }
-  __device__ View view(const LevelDesc<T> &A) const {
-    const int r0 = rank * A.rw;
-    if (A.staged)
-      return View{(const int32_t *)(sm + A.s_rp), (const int32_t *)(sm + A.s_ci), (const C2<T> *)(sm + A.s_off),
-                  (const T *)(sm + A.s_dia), (const T *)(sm + A.s_dia) + 3 * A.rw};
-    return View{A.rp + r0, A.ci, A.off, A.dia + 3 * (int64_t)r0, A.dinv + 3 * (int64_t)r0};
+// The cluster as one thread sees it.
+struct TailTeam {
+  uint32_t sm_addr, bars;
+  int rank, nct;  // CTA of the cluster, CTAs in it
+  int lane, warp;
+  unsigned *fail;
+  template <typename T>
+  __device__ __forceinline__ int rows_of(const LevelDesc<T> &A) const {
+    return max(0, min(A.rw, A.n - rank * A.rw));
   }
-  // lanes per row for rw rows a CTA
-  __device__ static int lanes_for(int rw) {
-    const int cap = sizeof(T) == 8 ? 128 : kTailThreads;
-    int ln = 2;
-    while (ln < 16 && rw * ln * 2 <= cap) ln *= 2;
-    return ln;
+  // the value of row `row`, component c in v, to the replicated vector at byte
+  // offset o of every CTA (phase ph); the row's lanes share the CTAs
+  template <typename T>
+  __device__ __forceinline__ void spread(int ph, uint32_t o, int row, int li, int LN, T v, bool ok) const {
+    const T other = __shfl_xor_sync(0xffffffffu, v, 1);
+    const C2<T> w = (li & 1) ? C2<T>{other, v} : C2<T>{v, other};
+    if (!ok) return;
+    const uint32_t at = sm_addr + o + row * (uint32_t)sizeof(C2<T>), bar = bars + 8u * ph;
+    for (int q = li; q < nct; q += LN) st_async(at, bar, q, w);
   }
-  // f(i, c, p, P, ok) for the own rows i < m, LN lanes a row (component c,
-  // part p of P); rows past m run with ok = false on the lanes of a warp that
-  // has a row
-  template <class F>
-  __device__ void rows(int m, int LN, F &&f) const {
-    const int rpw = 32 / LN, li = lane % LN;
-    for (int base = warp * rpw; base < m; base += nwarps * rpw) {
-      const int i = base + lane / LN;
-      const bool ok = i < m;
-      f(ok ? i : m - 1, li & 1, li >> 1, LN >> 1, ok);
-      __syncwarp();
+  // the whole vector of phase ph has arrived here
+  __device__ __forceinline__ void wait(int ph) const {
+    const uint32_t a = bars + 8u * ph;
+    for (uint32_t it = 0; it < kStageWaitPolls; it++) {
+      uint32_t done;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+          " selp.u32 %0, 1, 0, p;\n}\n"
+          : "=r"(done)
+          : "r"(a)
+          : "memory");
+      if (done) return;
     }
+    atomicOr(fail, 1u);
   }
-  __device__ static T parts_sum(T v, int P) {
-    for (int o = 2; o < 2 * P; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+};
+
+// This thread's part of a level: one component of part p of one own row (a
+// level has at most kTailRows rows a CTA, so one pass covers them).  The first
+// kLaneNz nonzeros and the row's diagonal blocks are held in registers for the
+// phases of one visit to the level: a phase is a chain of dependent
+// instructions on a few warps, and loading them anew in each took half of it.
+// Warps without a row do nothing; the spare lanes of a warp with one repeat
+// its last row without storing, so that every lane takes part in the shuffles.
+constexpr int kTailRows = kTailThreads / 2;
+constexpr int kLaneNz = 8;
+template <typename T>
+struct TailLane {
+  bool act, ok;  // the warp has a row; this lane's is its own
+  int i, row, li, LN, c, P;
+  uint32_t xo[kLaneNz];  // byte offsets into a replicated vector
+  T vr[kLaneNz], vi[kLaneNz];  // the value; its imaginary part with the component's sign
+  int k, e;              // nonzeros past the registers (staged, step P)
+  T dd, df, id, jf;      // diagonal block and inverse: own component, coupling
+  __device__ __forceinline__ void place(const TailTeam &R, const LevelDesc<T> &A) {
+    const int m = R.rows_of(A);
+    LN = 1 << A.lnb;
+    P = LN >> 1;
+    li = R.lane & (LN - 1);
+    c = li & 1;
+    const int i0 = R.warp << (5 - A.lnb);
+    act = i0 < m;
+    const int at = i0 + (R.lane >> A.lnb);
+    ok = at < m;
+    i = ok ? at : m - 1;
+    row = R.rank * A.rw + i;
+  }
+  __device__ __forceinline__ void load(const LevelDesc<T> &A) {
+    if (!act) return;
+    const unsigned sg = c ? 0u : 0x80000000u;
+    e = tail_at<int32_t>(A.s_rp, i + 1);
+    k = tail_at<int32_t>(A.s_rp, i) + (li >> 1);
+#pragma unroll
+    for (int u = 0; u < kLaneNz; u++) {
+      xo[u] = (uint32_t)row * (uint32_t)sizeof(C2<T>);  // (times zero: the row's own value)
+      vr[u] = vi[u] = 0;
+      if (k < e) {
+        xo[u] = (uint32_t)tail_at<int32_t>(A.s_ci, k) * (uint32_t)sizeof(C2<T>);
+        const C2<T> v = tail_at<C2<T>>(A.s_off, k);
+        vr[u] = v.x;
+        vi[u] = flip(v.y, sg);
+        k += P;
+      }
+    }
+    dd = tail_at<T>(A.s_dia, 3 * i + c);
+    df = tail_at<T>(A.s_dia, 3 * i + 2);
+    id = tail_at<T>(A.s_dia, 3 * A.rw + 3 * i + c);
+    jf = tail_at<T>(A.s_dia, 3 * A.rw + 3 * i + 2);
+  }
+  __device__ __forceinline__ T parts_sum(T v) const {
+    for (int o = 2; o < LN; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
   }
-  // component c of the off-diagonal row sum over x
-  __device__ static T row_sum(const View &A, int i, int c, int p, int P, const C2<T> *x) {
+  // component c of the off-diagonal row sum over the vector at offset x
+  __device__ __forceinline__ T row_sum(const LevelDesc<T> &A, uint32_t x) const {
+    C2<T> xv[kLaneNz];
+#pragma unroll
+    for (int u = 0; u < kLaneNz; u++) xv[u] = tail_at<C2<T>>(x + xo[u]);
+    T s0 = 0, s1 = 0;
+#pragma unroll
+    for (int u = 0; u < kLaneNz; u++) {
+      s0 = fma(vr[u], c ? xv[u].y : xv[u].x, s0);
+      s1 = fma(vi[u], c ? xv[u].x : xv[u].y, s1);
+    }
     const unsigned sg = c ? 0u : 0x80000000u;
-    T acc = 0;
-    const int e = A.rp[i + 1];
-#pragma unroll 4
-    for (int k = A.rp[i] + p; k < e; k += P) {
-      const C2<T> v = A.off[k], xv = x[A.ci[k]];
-      acc = fma(v.x, c ? xv.y : xv.x, acc);
-      acc = fma(flip(v.y, sg), c ? xv.x : xv.y, acc);
+    for (int q = k; q < e; q += P) {
+      const C2<T> v = tail_at<C2<T>>(A.s_off, q), y = tail_at<C2<T>>(x, tail_at<int32_t>(A.s_ci, q));
+      s0 = fma(v.x, c ? y.y : y.x, s0);
+      s1 = fma(flip(v.y, sg), c ? y.x : y.y, s1);
     }
-    return parts_sum(acc, P);
+    return parts_sum(s0 + s1);
   }
-  // component c of a list's sum over src
-  __device__ static T list_sum(const int32_t *mp, const int32_t *mi, int i, int c, int p, int P, const C2<T> *src) {
+  // component c of the own node's sum over its members (lists at A.s_mp,
+  // A.s_mi) of the finer vector `at(j)` gives
+  template <class F>
+  __device__ __forceinline__ T members(const LevelDesc<T> &A, F &&at) const {
     T acc = 0;
-    const int e = mp[i + 1];
-#pragma unroll 4
-    for (int k = mp[i] + p; k < e; k += P) {
-      const T *s = reinterpret_cast<const T *>(src + mi[k]);
-      acc += s[c];
+    const int last = tail_at<int32_t>(A.s_mp, i + 1);
+    constexpr int U = 8;  // loads under way at once
+    for (int k0 = tail_at<int32_t>(A.s_mp, i) + (li >> 1); k0 < last; k0 += U * P) {
+      T v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = at(tail_at<int32_t>(A.s_mi, min(k0 + u * P, last - 1)));
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (k0 + u * P < last) acc += v[u];
     }
-    return parts_sum(acc, P);
-  }
-  // the row's value, component c in v, to element `row` of the replicated
-  // vector at byte offset o of every CTA
-  __device__ void spread(uint32_t o, int row, int c, int p, int P, T v, bool ok) const {
-    const T other = __shfl_xor_sync(0xffffffffu, v, 1);
-    const C2<T> w = c ? C2<T>{other, v} : C2<T>{v, other};
-    if (!ok) return;
-    for (int q = 2 * p + c; q < nct; q += 2 * P) st_cluster(sm_addr + o + row * (uint32_t)sizeof(C2<T>), q, w);
-  }
-  __device__ void phase_end() const {
-    cluster_arrive();
-    cluster_wait();
+    return parts_sum(acc);
   }
 };
 
 // own rows of a level's operator (and its lists) into shared memory; the
 // members of its nodes over the finer level (mp, mi: null for the first)
 template <typename T>
-__device__ __forceinline__ void tail_stage(const Resident<T> &R, const LevelDesc<T> &A, bool matrix,
-                                           const int32_t *mp, const int32_t *mi) {
+__device__ __forceinline__ void tail_stage(const TailTeam &R, const LevelDesc<T> &A, bool matrix,
+                                           const int32_t *mp, const int32_t *mi, int t, int st) {
   const int r0 = R.rank * A.rw, m = R.rows_of(A);
-  const int t = threadIdx.x, st = blockDim.x;
-  if (mp && m > 0) {
-    int32_t *smp = (int32_t *)(R.sm + A.s_mp), *smi = (int32_t *)(R.sm + A.s_mi);
-    const int b = mp[r0], e = mp[r0 + m];
-    for (int q = t; q <= m; q += st) smp[q] = mp[r0 + q] - b;
-    for (int q = t; q < e - b; q += st) smi[q] = mi[b + q];
-  }
+  if (matrix)
+    for (int q = t; q < A.n; q += st) tail_at<int32_t>(A.s_agg, q) = A.agg[q];
+  if (m == 0) return;
+  const int mb = mp ? mp[r0] : 0, me = mp ? mp[r0 + m] : 0;
+  const int b = matrix ? A.rp[r0] : 0, e = matrix ? A.rp[r0 + m] : 0;
+  if (mp)
+    for (int q = t; q <= m; q += st) tail_at<int32_t>(A.s_mp, q) = mp[r0 + q] - mb;
+  for (int q = t; q < me - mb; q += st) tail_at<int32_t>(A.s_mi, q) = mi[mb + q];
   if (!matrix) return;
-  if (A.agg)
-    for (int q = t; q < A.n; q += st) ((int32_t *)(R.sm + A.s_agg))[q] = A.agg[q];
-  if (!A.staged || m == 0) return;
-  int32_t *srp = (int32_t *)(R.sm + A.s_rp), *sci = (int32_t *)(R.sm + A.s_ci);
-  C2<T> *so = (C2<T> *)(R.sm + A.s_off);
-  T *sd = (T *)(R.sm + A.s_dia);
-  const int b = A.rp[r0], e = A.rp[r0 + m];
-  for (int q = t; q <= m; q += st) srp[q] = A.rp[r0 + q] - b;
+  for (int q = t; q <= m; q += st) tail_at<int32_t>(A.s_rp, q) = A.rp[r0 + q] - b;
   for (int q = t; q < e - b; q += st) {
-    sci[q] = A.ci[b + q];
-    so[q] = A.off[b + q];
+    tail_at<int32_t>(A.s_ci, q) = A.ci[b + q];
+    tail_at<C2<T>>(A.s_off, q) = A.off[b + q];
   }
   for (int q = t; q < 3 * m; q += st) {
-    sd[q] = A.dia[3 * (int64_t)r0 + q];
-    sd[3 * A.rw + q] = A.dinv[3 * (int64_t)r0 + q];
+    tail_at<T>(A.s_dia, q) = A.dia[3 * (int64_t)r0 + q];
+    tail_at<T>(A.s_dia, 3 * A.rw + q) = A.dinv[3 * (int64_t)r0 + q];
   }
 }
 
-// One Chebyshev step of the own rows: x_in (replicated) -> x_out (spread);
-// the new iterate's component is handed to `last` instead when given.
-template <typename T, class Last>
-__device__ __forceinline__ void tail_cheb(const Resident<T> &R, const LevelDesc<T> &A, int k, uint32_t xin,
-                                          uint32_t xout, bool final_step, Last &&last) {
-  const typename Resident<T>::View V = R.view(A);
-  const int r0 = R.rank * A.rw, m = R.rows_of(A), LN = R.lanes_for(A.rw);
-  const C2<T> *x = R.vec(xin);
-  T *bo = R.own(A.b), *dn = R.own(A.d);
-  const T c1 = k == 0 ? (T)0 : A.coef[2 * k], c2 = k == 0 ? A.coef[0] : A.coef[2 * k + 1];
-  R.rows(m, LN, [&](int i, int c, int p, int P, bool ok) {
-    const T s = R.row_sum(V, i, c, p, P, x);
-    const T *xi = reinterpret_cast<const T *>(x + r0 + i);
-    const T xc = xi[c], xo = xi[c ^ 1];
-    const T rc = bo[2 * i + c] - (s + V.dia[3 * i + c] * xc + V.dia[3 * i + 2] * xo);
-    const T ro = __shfl_xor_sync(0xffffffffu, rc, 1);
-    const T z = V.dinv[3 * i + c] * rc + V.dinv[3 * i + 2] * ro;
-    const T dold = k == 0 ? (T)0 : dn[2 * i + c];
-    const T dv = k == 0 ? c2 * z : c1 * dold + c2 * z;
-    __syncwarp();  // every part has read the old direction
-    if (ok && p == 0) dn[2 * i + c] = dv;
-    const T xn = xc + dv;
-    if (final_step) last(i, c, p, xn, ok);
-    else R.spread(xout, r0 + i, c, p, P, xn, ok);
-  });
+// Chebyshev step k of the lane's row: the iterate at offset x -> its new
+// value (component c), d the direction, b the right-hand side
+template <typename T>
+__device__ __forceinline__ T tail_cheb(const TailLane<T> &Q, const LevelDesc<T> &A, const T *coef, int k, uint32_t x,
+                                       T b, T &d) {
+  const C2<T> xi = tail_at<C2<T>>(x, Q.row);
+  const T xc = Q.c ? xi.y : xi.x, xo = Q.c ? xi.x : xi.y;
+  const T rc = (b - (Q.dd * xc + Q.df * xo)) - Q.row_sum(A, x);
+  const T ro = __shfl_xor_sync(0xffffffffu, rc, 1);
+  const T z = Q.id * rc + Q.jf * ro;
+  d = k == 0 ? coef[0] * z : coef[2 * k] * d + coef[2 * k + 1] * z;
+  return xc + d;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kTailThreads)
     resident_vcycle(const LevelDesc<T> *__restrict__ lv_g, int lt, int L, int deg, const T *__restrict__ Ainv,
-                    DenseMap D, uint32_t s_bd, uint32_t s_xd, TailArgs<T> a, const int *halt) {
-  extern __shared__ __align__(16) unsigned char tail_sm[];
+                    DenseMap D, TailDense td, uint32_t s_bar, TailArgs<T> a, const int *halt) {
   __shared__ LevelDesc<T> lv[16];
+  __shared__ T s_coef[16][2 * kMaxDegree];
   __shared__ double s_dot[16];
   __shared__ double s32[32];
-  Resident<T> R;
-  R.sm = tail_sm;
+  TailTeam R;
   R.sm_addr = smem_addr(tail_sm);
+  R.bars = R.sm_addr + s_bar;
+  R.fail = a.fail;
   {
     unsigned r, n;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -916,184 +984,235 @@ __global__ void __launch_bounds__(kTailThreads)
   }
   R.lane = threadIdx.x & 31;
   R.warp = threadIdx.x >> 5;
-  R.nwarps = blockDim.x >> 5;
-  cluster_arrive();  // every CTA has started before any remote store: waited for below
   {
     const int nw = (int)(sizeof(LevelDesc<T>) / 4) * (L - lt);
     const uint32_t *src = reinterpret_cast<const uint32_t *>(lv_g + lt);
     for (int q = threadIdx.x; q < nw; q += blockDim.x) reinterpret_cast<uint32_t *>(lv + lt)[q] = src[q];
   }
   __syncthreads();
+  const int per = 2 * deg + 1, nph = tail_phases(L - lt, deg);
+  // every phase's mbarrier expects its whole vector
+  for (int q = threadIdx.x; q < nph; q += blockDim.x) {
+    uint64_t *bar = &tail_at<uint64_t>(s_bar, q);
+    const int l = q < nph - 2 ? lt + q / per : L - 1;
+    mbar_init(bar);
+    mbar_expect_tx(bar, (uint32_t)(lv[l].n * (int)sizeof(C2<T>)));
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  cluster_arrive();  // (waited for below) every CTA's mbarriers are ready before any store to it
   // the operators and lists were written before the launch this one follows:
-  // staged while that one finishes
+  // staged while that one runs
   for (int l = lt; l < L; l++) {
     const int32_t *mp = l > lt ? lv[l - 1].mem_ptr : a.f_mp, *mi = l > lt ? lv[l - 1].mem_idx : a.f_mi;
-    tail_stage<T>(R, lv[l], l < L - 1, mp, mi);
+    // (the first level by three quarters of the warps, the others by the rest)
+    constexpr int kFirst = kTailThreads / 4 * 3;
+    const int t = (int)threadIdx.x - (l > lt ? kFirst : 0);
+    if (t >= 0 && (l > lt || t < kFirst))
+      tail_stage<T>(R, lv[l], l < L - 1, mp, mi, t, l > lt ? kTailThreads - kFirst : kFirst);
   }
+  for (int q = threadIdx.x; q < (L - 1 - lt) * 2 * deg; q += blockDim.x) {
+    const int l = lt + q / (2 * deg);
+    s_coef[l][q % (2 * deg)] = lv[l].coef[q % (2 * deg)];
+  }
+  if (td.staged) {
+    const LevelDesc<T> &C = lv[L - 1];
+    const int i0 = 2 * R.rank * C.rw, m2 = 2 * R.rows_of(C);
+    if (m2 > 0) {
+      const int64_t o0 = D.rowoff[i0], o1 = D.rowoff[i0 + m2 - 1] + D.bdim[i0 + m2 - 1];
+      for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+        tail_at<int32_t>(td.s_map, 3 * q) = (int32_t)(D.rowoff[i0 + q] - o0);
+        tail_at<int32_t>(td.s_map, 3 * q + 1) = D.bstart[i0 + q];
+        tail_at<int32_t>(td.s_map, 3 * q + 2) = D.bdim[i0 + q];
+      }
+      for (int q = threadIdx.x; q < (int)(o1 - o0); q += blockDim.x) tail_at<T>(td.s_a, q) = Ainv[o0 + q];
+    }
+  }
+  cluster_wait();
   dep_sync();
   __syncthreads();
-  const bool stop = (halt && *halt >= 2) || (a.head == kHeadLanczos && a.ms->done >= 2);
-  cluster_wait();
-  if (stop) return;  // every CTA alike, before any remote store
-  // down: level l's right-hand side is in its own rows, the first Chebyshev
-  // step (x = c0 D^-1 b) is spread with it
-  auto start_level = [&](int l, int i, int c, int p, int P, T bc, bool ok) {
+  const int done = halt ? *halt : 0;  // (looked at below, with the first loads under way)
+  TailLane<T> Q{};
+  // The start of level l from its right-hand side's component bc: the first
+  // Chebyshev step (x = c0 D^-1 b) is spread; b and d stay with the row.
+  auto start_level = [&](int l, T bc) {
     const LevelDesc<T> &A = lv[l];
-    const int r0 = R.rank * A.rw;
     if (l == L - 1) {
-      R.spread(s_bd, r0 + i, c, p, P, bc, ok);
+      R.spread<T>(nph - 2, td.s_bd, Q.row, Q.li, Q.LN, bc, Q.ok);
       return;
     }
-    const typename Resident<T>::View V = R.view(A);
     const T bo = __shfl_xor_sync(0xffffffffu, bc, 1);
-    const T x = A.coef[0] * (V.dinv[3 * i + c] * bc + V.dinv[3 * i + 2] * bo);
-    if (ok && p == 0) {
-      R.own(A.b)[2 * i + c] = bc;
-      R.own(A.d)[2 * i + c] = x;
+    const T x = s_coef[l][0] * (tail_at<T>(A.s_dia, 3 * A.rw + 3 * Q.i + Q.c) * bc +
+                                tail_at<T>(A.s_dia, 3 * A.rw + 3 * Q.i + 2) * bo);
+    if (Q.ok && Q.li < 2) {
+      tail_at<T>(A.b, 2 * Q.i + Q.c) = bc;
+      tail_at<T>(A.d, 2 * Q.i + Q.c) = x;
     }
-    R.spread(deg % 2 == 1 ? A.xb : A.xa, r0 + i, c, p, P, x, ok);
+    R.spread<T>((l - lt) * per, deg % 2 == 1 ? A.xb : A.xa, Q.row, Q.li, Q.LN, x, Q.ok);
+    __syncwarp();
   };
   {
     const LevelDesc<T> &A = lv[lt];
-    const int r0 = R.rank * A.rw, m = R.rows_of(A), LN = R.lanes_for(A.rw);
-    T la0 = 0, la1 = 0, la2 = 0;
-    if (a.head == kHeadLanczos) {
-      const T *la = lanczos_coef<T>(a.ms);
-      la0 = la[0];
-      la1 = la[1];
-      la2 = la[2];
-    }
-    R.rows(m, LN, [&](int i, int c, int p, int P, bool ok) {
-      T bc;
+    Q.place(R, A);
+    T bc = 0;
+    if (Q.act) {
       if (a.head == kHeadRestrict) {
-        bc = R.list_sum((const int32_t *)(R.sm + A.s_mp), (const int32_t *)(R.sm + A.s_mi), i, c, p, P, a.f_res);
+        const T *res = reinterpret_cast<const T *>(a.f_res);
+        bc = Q.members(A, [&](int j) { return res[2 * (int64_t)j + Q.c]; });
       } else {
-        const int64_t e = 2 * (int64_t)(r0 + i) + c;
+        const int64_t e = 2 * (int64_t)Q.row + Q.c;
         bc = reinterpret_cast<const T *>(a.b)[e];
         if (a.head == kHeadLanczos) {
+          const T *la = lanczos_coef<T>(a.ms);
           T *ro = reinterpret_cast<T *>(a.r_old);
-          bc = la0 * bc - la1 * ro[e] - la2 * reinterpret_cast<const T *>(a.r_cur)[e];
+          bc = la[0] * bc - la[1] * ro[e] - la[2] * reinterpret_cast<const T *>(a.r_cur)[e];
           __syncwarp();  // every part has read r_old
-          if (ok && p == 0) ro[e] = bc;
+          if (Q.ok && Q.li < 2 && done < 2) ro[e] = bc;
         }
       }
-      start_level(lt, i, c, p, P, bc, ok);
-    });
+    }
+    // the recurrence has ended: every CTA leaves alike, before any store to
+    // another
+    if (done >= 2) return;
+    if (Q.act) start_level(lt, bc);
   }
-  R.phase_end();
   for (int l = lt; l < L - 1; l++) {
     const LevelDesc<T> &A = lv[l];
+    int ph = (l - lt) * per;
     uint32_t cur = deg % 2 == 1 ? A.xb : A.xa, oth = deg % 2 == 1 ? A.xa : A.xb;
-    for (int k = 1; k < deg; k++) {
-      tail_cheb<T>(R, A, k, cur, oth, false, [](int, int, int, T, bool) {});
-      R.phase_end();
+    T b = 0, d = 0;
+    Q.load(A);
+    if (Q.act) {
+      b = tail_at<T>(A.b, 2 * Q.i + Q.c);
+      d = tail_at<T>(A.d, 2 * Q.i + Q.c);
+    }
+    for (int k = 1; k < deg; k++, ph++) {
+      R.wait(ph);
+      if (Q.act) {
+        const T x = tail_cheb<T>(Q, A, s_coef[l], k, cur, b, d);
+        R.spread<T>(ph + 1, oth, Q.row, Q.li, Q.LN, x, Q.ok);
+      }
       const uint32_t t = cur;
       cur = oth;
       oth = t;
     }
     // the residual over xa (the pre-smoothed iterate is xb)
-    {
-      const typename Resident<T>::View V = R.view(A);
-      const int r0 = R.rank * A.rw, m = R.rows_of(A), LN = R.lanes_for(A.rw);
-      const C2<T> *x = R.vec(A.xb);
-      const T *bo = R.own(A.b);
-      R.rows(m, LN, [&](int i, int c, int p, int P, bool ok) {
-        const T s = R.row_sum(V, i, c, p, P, x);
-        const T *xi = reinterpret_cast<const T *>(x + r0 + i);
-        const T rc = bo[2 * i + c] - (s + V.dia[3 * i + c] * xi[c] + V.dia[3 * i + 2] * xi[c ^ 1]);
-        R.spread(A.xa, r0 + i, c, p, P, rc, ok);
-      });
+    R.wait(ph++);
+    if (Q.act) {
+      const C2<T> xi = tail_at<C2<T>>(A.xb, Q.row);
+      const T t = b - (Q.dd * (Q.c ? xi.y : xi.x) + Q.df * (Q.c ? xi.x : xi.y));
+      R.spread<T>(ph, A.xa, Q.row, Q.li, Q.LN, t - Q.row_sum(A, A.xb), Q.ok);
     }
-    R.phase_end();
-    {
-      const LevelDesc<T> &C = lv[l + 1];
-      const C2<T> *res = R.vec(A.xa);
-      R.rows(R.rows_of(C), R.lanes_for(C.rw), [&](int i, int c, int p, int P, bool ok) {
-        const T bc = R.list_sum((const int32_t *)(R.sm + C.s_mp), (const int32_t *)(R.sm + C.s_mi), i, c, p, P, res);
-        start_level(l + 1, i, c, p, P, bc, ok);
-      });
-    }
-    R.phase_end();
+    const LevelDesc<T> &C = lv[l + 1];
+    Q.place(R, C);
+    R.wait(ph);
+    if (Q.act) start_level(l + 1, Q.members(C, [&](int j) {
+      const C2<T> v = tail_at<C2<T>>(A.xa, j);
+      return Q.c ? v.y : v.x;
+    }));
   }
   // the coarsest level: its dense inverse, real rows split over 16 lanes
   {
     const LevelDesc<T> &C = lv[L - 1];
-    const T *bd = reinterpret_cast<const T *>(tail_sm + s_bd);
-    const int m2 = 2 * R.rows_of(C), i0 = 2 * R.rank * C.rw, li = R.lane & 15;
-    for (int base = 2 * R.warp; base < m2; base += 2 * R.nwarps) {
+    const int m2 = 2 * R.rows_of(C), li = R.lane & 15;
+    R.wait(nph - 2);
+    for (int base = 2 * R.warp; base < m2; base += 2 * (kTailThreads / 32)) {
       const int i = base + (R.lane >> 4);  // a warp holds both components of a node
-      const int64_t row = i0 + i;
-      const T *av = Ainv + D.rowoff[row], *bb = bd + D.bstart[row];
-      const int m = D.bdim[row];
+      const int row = 2 * R.rank * C.rw + i;
       T s = 0;
+      if (td.staged) {
+        const int o = tail_at<int32_t>(td.s_map, 3 * i), bs = tail_at<int32_t>(td.s_map, 3 * i + 1),
+                  m = tail_at<int32_t>(td.s_map, 3 * i + 2);
 #pragma unroll 4
-      for (int j = li; j < m; j += 16) s = fma(av[j], bb[j], s);
+        for (int j = li; j < m; j += 16) s = fma(tail_at<T>(td.s_a, o + j), tail_at<T>(td.s_bd, bs + j), s);
+      } else {
+        const T *av = Ainv + D.rowoff[row];
+        const int bs = D.bstart[row], m = D.bdim[row];
+#pragma unroll 4
+        for (int j = li; j < m; j += 16) s = fma(av[j], tail_at<T>(td.s_bd, bs + j), s);
+      }
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       const T other = __shfl_xor_sync(0xffffffffu, s, 16);
       const C2<T> w = R.lane < 16 ? C2<T>{s, other} : C2<T>{other, s};
-      if (R.lane < R.nct) st_cluster(R.sm_addr + s_xd + (uint32_t)(row >> 1) * (uint32_t)sizeof(C2<T>), R.lane, w);
+      if (R.lane < R.nct)
+        st_async(R.sm_addr + td.s_xd + (uint32_t)(row >> 1) * (uint32_t)sizeof(C2<T>), R.bars + 8u * (nph - 1),
+                 R.lane, w);
     }
+    R.wait(nph - 1);
   }
-  R.phase_end();
-  uint32_t xc = s_xd;
+  uint32_t xc = td.s_xd;
   double part = 0.0;
+  // the first of this thread's fine elements that the result is added to,
+  // loaded ahead
+  const int64_t j0 = (int64_t)R.rank * blockDim.x + threadIdx.x;
+  int32_t ag0 = 0;
+  C2<T> fx0{0, 0};
+  if (a.out == kOutProlong && j0 < a.f_n) {
+    ag0 = a.f_agg[j0];
+    fx0 = a.f_x[j0];
+  }
   for (int l = L - 2; l >= lt; l--) {
     const LevelDesc<T> &A = lv[l];
-    // coarse correction on the CTA's own copy of the whole vector
-    {
-      C2<T> *x = R.vec(A.xb);
-      const C2<T> *c = R.vec(xc);
-      const int32_t *ag = (const int32_t *)(R.sm + A.s_agg);
+    int ph = (l - lt) * per + deg + 1;  // the first post-smoothing step's
+    T b = 0, d = 0;
+    Q.place(R, A);
+    Q.load(A);
+    if (Q.act) b = tail_at<T>(A.b, 2 * Q.i + Q.c);
+    // coarse correction on the CTA's own copy of the whole vector (a CTA
+    // without rows here sends none, so others may already be overwriting its
+    // copy: it reads the result only)
+    if (R.rows_of(A) > 0)
       for (int j = threadIdx.x; j < A.n; j += blockDim.x) {
-        const C2<T> e = c[ag[j]];
-        C2<T> v = x[j];
-        v.x += e.x;
-        v.y += e.y;
-        x[j] = v;
+        const C2<T> e = tail_at<C2<T>>(xc, tail_at<int32_t>(A.s_agg, j));
+        C2<T> &x = tail_at<C2<T>>(A.xb, j);
+        x = C2<T>{x.x + e.x, x.y + e.y};
       }
-    }
     __syncthreads();
     uint32_t in = A.xb, out = A.xa;
-    const int r0 = R.rank * A.rw;
-    for (int k = 0; k < deg; k++) {
+    for (int k = 0; k < deg; k++, ph++) {
       const bool fin = l == lt && k == deg - 1 && a.out != kOutProlong;
-      tail_cheb<T>(R, A, k, in, out, fin, [&](int i, int c, int p, T xn, bool ok) {
-        if (!ok || p != 0) return;
-        reinterpret_cast<T *>(a.z)[2 * (int64_t)(r0 + i) + c] = xn;
-        if (a.out == kOutMinres) part += (double)R.own(A.b)[2 * i + c] * (double)xn;
-      });
-      if (!fin) R.phase_end();
+      if (Q.act) {
+        const T x = tail_cheb<T>(Q, A, s_coef[l], k, in, b, d);
+        if (!fin) {
+          R.spread<T>(ph, out, Q.row, Q.li, Q.LN, x, Q.ok);
+        } else if (Q.ok && Q.li < 2) {
+          reinterpret_cast<T *>(a.z)[2 * (int64_t)Q.row + Q.c] = x;
+          part = (double)b * (double)x;
+        }
+      }
+      if (!fin) R.wait(ph);
       const uint32_t t = in;
       in = out;
       out = t;
     }
     xc = in;
   }
+  // (no CTA leaves while others may still send to it)
   if (a.out == kOutProlong) {
-    const C2<T> *c = R.vec(xc);
-    for (int64_t j = (int64_t)R.rank * blockDim.x + threadIdx.x; j < a.f_n; j += (int64_t)R.nct * blockDim.x) {
-      const C2<T> e = c[a.f_agg[j]];
-      C2<T> v = a.f_x[j];
-      v.x += e.x;
-      v.y += e.y;
-      a.f_x[j] = v;
+    cluster_arrive();
+    for (int64_t j = j0; j < a.f_n; j += (int64_t)R.nct * blockDim.x) {
+      const C2<T> e = tail_at<C2<T>>(xc, j == j0 ? ag0 : a.f_agg[j]);
+      const C2<T> v = j == j0 ? fx0 : a.f_x[j];
+      a.f_x[j] = C2<T>{v.x + e.x, v.y + e.y};
     }
+    cluster_wait();
   } else if (a.out == kOutMinres) {
     // <r, z>: the CTAs' sums in CTA order, then the Givens step
     const double s = block_sum(part, s32);
-    if (threadIdx.x == 0) {
-      uint32_t ra;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(ra) : "r"(smem_addr(&s_dot[R.rank])), "r"(0));
-      asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(ra), "d"(s) : "memory");
-    }
-    R.phase_end();
+    if (threadIdx.x == 0)
+      asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(map_rank(smem_addr(&s_dot[R.rank]), 0)), "d"(s)
+                   : "memory");
+    cluster_arrive();
+    cluster_wait();
     if (R.rank == 0 && threadIdx.x == 0) {
       dep_trigger();
       double t = 0.0;
       for (int q = 0; q < R.nct; q++) t += s_dot[q];
       minres_advance(a.ms, t);
     }
+  } else {
+    cluster_arrive();
+    cluster_wait();
   }
 }
 
@@ -1155,7 +1274,8 @@ template <typename T>
 struct TailPlan {
   int lt = -1;  // -1: none
   size_t smem = 0;
-  uint32_t s_bd = 0, s_xd = 0;
+  TailDense dense{};
+  uint32_t s_bar = 0;
   DevBuf<LevelDesc<T>> desc;
 };
 
@@ -1210,7 +1330,7 @@ struct Amg::Impl {
   void choose_cluster();
   int tail_ctas = 1;        // CTAs of the resident cycle's cluster
   bool grid_coarse = false;  // coarsest level too large for it: dense kernel on the grid
-  template <typename T> size_t tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32_t *bd, uint32_t *xd);
+  template <typename T> size_t tail_layout(int first, std::vector<LevelDesc<T>> *desc, TailPlan<T> *P);
   template <typename T> void build_plan(TailPlan<T> &P, int first);
   template <typename T> const TailPlan<T> &plan() {
     AmgVals<T> &V = vals<T>();
@@ -1316,7 +1436,7 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
       if (l == L - 1) I.grid_coarse = true;
       continue;
     }
-    if (I.tail_layout<double>(l, nullptr, nullptr, nullptr) <= (size_t)kTailSmem) {
+    if (I.tail_layout<double>(l, nullptr, nullptr) <= (size_t)kTailSmem) {
       I.lt = l;
       break;
     }
@@ -1554,10 +1674,9 @@ void Amg::Impl::choose_cluster() {
 }
 
 // Shared-memory layout of a resident cycle that starts on level `first`;
-// returns the bytes its vectors and lists need (the operators' rows are
-// staged level by level while they fit).
+// returns its bytes (the dense inverse's rows are staged when they fit too).
 template <typename T>
-size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32_t *bd, uint32_t *xd) {
+size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, TailPlan<T> *P) {
   const int L = (int)lev.size(), C = tail_ctas;
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -1577,6 +1696,10 @@ size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32
     A = LevelDesc<T>{};
     A.n = (int)lev[l].n;
     A.rw = (A.n + C - 1) / C;
+    const int cap = sizeof(T) == 8 ? 128 : kTailThreads;
+    if (A.rw > kTailRows) o += kTailSmem;  // more rows than a pass covers: does not fit
+    A.lnb = 1;  // (see the kernel's note on lanes)
+    while (A.lnb < 4 && (A.rw << (A.lnb + 1)) <= cap) ++A.lnb;
     if (l > first || first > 0) {
       A.s_mp = take(4 * (size_t)(A.rw + 1));
       A.s_mi = take(4 * longest(lev[l - 1].h_mem_ptr, A.n, A.rw));
@@ -1587,12 +1710,17 @@ size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32
     A.b = take(sizeof(C2<T>) * (size_t)A.rw);
     A.d = take(sizeof(C2<T>) * (size_t)A.rw);
     A.s_agg = take(4 * (size_t)A.n);
+    const size_t nz = longest(lev[l].h_rp, A.n, A.rw);
+    A.s_rp = take(4 * (size_t)(A.rw + 1));
+    A.s_ci = take(4 * nz);
+    A.s_off = take(sizeof(C2<T>) * nz);
+    A.s_dia = take(6 * sizeof(T) * (size_t)A.rw);
   }
-  const uint32_t b0 = take(sizeof(C2<T>) * (size_t)D[L - 1].n), x0 = take(sizeof(C2<T>) * (size_t)D[L - 1].n);
-  const size_t need = o;
-  if (bd) *bd = b0;
-  if (xd) *xd = x0;
-  if (!desc) return need;
+  const uint32_t bd = take(sizeof(C2<T>) * (size_t)D[L - 1].n), xd = take(sizeof(C2<T>) * (size_t)D[L - 1].n);
+  const uint32_t bar = take(8 * (size_t)tail_phases(L - first, std::max(opt.smooth_degree, 1)));
+  if (!desc) return o;
+  P->dense = TailDense{bd, xd, 0, 0, 0};
+  P->s_bar = bar;
   AmgVals<T> &V = vals<T>();
   for (int l = first; l < L; l++) {
     LevelDesc<T> &A = D[l];
@@ -1605,13 +1733,14 @@ size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32
     A.agg = lev[l].agg.p;
     A.mem_ptr = lev[l].mem_ptr.p;
     A.mem_idx = lev[l].mem_idx.p;
-    if (l == L - 1) break;
-    const size_t nz = longest(lev[l].h_rp, A.n, A.rw), before = o;
-    A.s_rp = take(4 * (size_t)(A.rw + 1));
-    A.s_ci = take(4 * nz);
-    A.s_off = take(sizeof(C2<T>) * nz);
-    A.s_dia = take(6 * sizeof(T) * (size_t)A.rw);
-    if (o <= (size_t)kTailSmem) A.staged = 1;
+  }
+  {
+    // the dense inverse's own rows
+    const int rw2 = 2 * D[L - 1].rw;
+    const size_t before = o;
+    P->dense.s_map = take(12 * (size_t)rw2);
+    P->dense.s_a = take(sizeof(T) * (size_t)rw2 * max_dim);
+    if (o <= (size_t)kTailSmem) P->dense.staged = 1;
     else o = before;
   }
   *desc = std::move(D);
@@ -1621,7 +1750,7 @@ size_t Amg::Impl::tail_layout(int first, std::vector<LevelDesc<T>> *desc, uint32
 template <typename T>
 void Amg::Impl::build_plan(TailPlan<T> &P, int first) {
   std::vector<LevelDesc<T>> d;
-  P.smem = tail_layout<T>(first, &d, &P.s_bd, &P.s_xd);
+  P.smem = tail_layout<T>(first, &d, &P);
   P.desc.upload(d, nls.stream);
   nls.sync();
   P.lt = first;
@@ -1631,7 +1760,7 @@ template <typename T>
 void Amg::Impl::launch_tail(const TailPlan<T> &P, const TailArgs<T> &a, bool overlap) {
   launch_cluster_dep(overlap, tail_ctas, resident_vcycle<T>, dim3(kTailThreads), P.smem, nls.stream,
                      (const LevelDesc<T> *)P.desc.p, P.lt, (int)lev.size(), std::max(opt.smooth_degree, 1),
-                     dense_inv<T>(), dmap(), P.s_bd, P.s_xd, a, halt);
+                     dense_inv<T>(), dmap(), P.dense, P.s_bar, a, halt);
   ++nls.launch_count;
 }
 
@@ -1676,13 +1805,15 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
     rows<T>(l, cur, op);
     std::swap(cur, oth);
   }
-  ResidOp<T> rop{dv, b, x, V.res[l].p, halt};
+  // (the resident cycle stages its operators under the residual's launch)
+  ResidOp<T> rop{dv, b, x, V.res[l].p, halt, !grid_coarse && l + 1 == plan<T>().lt && ovl()};
   rows<T>(l, x, rop);
   if (tm) tm->end(st, (deg - 1) * cheb_bytes + res_bytes, deg);
   const AmgLevel &Cl = lev[l + 1];
   const TailPlan<T> &P = plan<T>();
   if (!grid_coarse && l + 1 == P.lt) {
     TailArgs<T> a{};
+    a.fail = nls.red.counter.p + kStageErrorSlot;
     a.head = kHeadRestrict;
     a.out = kOutProlong;
     a.f_res = V.res[l].p;
@@ -1752,6 +1883,7 @@ void Amg::apply(const T *r, T *z) {
     // the whole cycle resident; no overlap: it stages the block inverses,
     // which the refresh before it may have written
     TailArgs<T> a{};
+    a.fail = I.nls.red.counter.p + kStageErrorSlot;
     a.head = kHeadVector;
     a.out = kOutVector;
     a.b = (const C2<T> *)r;
@@ -1815,6 +1947,7 @@ void Amg::apply_minres(MinresScalars *ms, const T *u, T *r_old, const T *r_cur, 
   I.halt = &ms->done;
   if (const TailPlan<T> &P = I.plan<T>(); P.lt == 0) {
     TailArgs<T> a{};
+    a.fail = I.nls.red.counter.p + kStageErrorSlot;
     a.head = kHeadLanczos;
     a.out = kOutMinres;
     a.b = (const C2<T> *)u;

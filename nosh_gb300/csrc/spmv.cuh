@@ -264,6 +264,23 @@ __device__ __forceinline__ bool halted_early(const Op &op) {
     return false;
   }
 }
+// An Op may carry `bool trigger`: the launch then lets its successor start as
+// soon as all its own CTAs run, for a successor that has work to do before
+// its dep_sync() and leaves room on the SMs (the resident coarse cycle).
+template <class Op, class = void>
+struct HasTrigger {
+  static constexpr bool value = false;
+};
+template <class Op>
+struct HasTrigger<Op, decltype((void)std::declval<Op>().trigger, void())> {
+  static constexpr bool value = true;
+};
+template <class Op>
+__device__ __forceinline__ void early_trigger(const Op &op) {
+  if constexpr (HasTrigger<Op>::value) {
+    if (op.trigger) dep_trigger();
+  }
+}
 // ---- bulk-copy staging (TMA + mbarrier) ------------------------------
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -385,6 +402,7 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
   const bool skip = halted_early(op);
   if (!skip && threadIdx.x == 0 && rb0 < rb_end) issue(rb0, 0);
   dep_sync();
+  early_trigger(op);
   if (halted(op)) {
     // let the copy issued above land before the CTA leaves
     if (!skip && threadIdx.x == 0 && rb0 < rb_end) {
@@ -505,6 +523,7 @@ __global__ void __launch_bounds__(kWarpThreads)
                    unsigned *counter, double *red_out) {
   using A = typename Acc<T>::type;
   dep_sync();
+  early_trigger(op);
   if (halted(op)) return;
   const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4;
   const int nwb = (N + 31) / 32;

@@ -1,0 +1,58 @@
+"""The resident V-cycle (levels in a thread-block cluster's shared memory)
+against the same cycle with its fine level on the grid, and its symmetry.
+
+Small meshes run the whole cycle resident; with kernel timing on the handle
+keeps the fine level on the grid, so the two applies differ in rounding only.
+Sizes sit at the edges: a hierarchy of two levels, fewer rows than CTAs, one
+row more than a multiple of them, the largest mesh taken whole and the one
+after, triangles and tetrahedra, every smoothing degree parity.
+
+Tolerances, before any run: a cycle is about 30 dependent roundings deep and
+its intermediate vectors are within a factor of 100 of its result, so FP64
+1e-12 and FP32 1e-4 of the largest entry; the symmetry defect relative to
+||a|| ||M b|| the same.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+MESHES = {
+    "square9": lambda: O.gen_square(9, 3),
+    "square17": lambda: O.gen_square(17, 1),
+    "square33": lambda: O.gen_square(33, 2),
+    "square45": lambda: O.gen_square(45, 4),
+    "square46": lambda: O.gen_square(46, 4),
+    "square65": lambda: O.gen_square(65, 1),
+    "cube4": lambda: O.gen_cube(4, 5),
+    "cube11": lambda: O.gen_cube(11, 6),
+    "cube17": lambda: O.gen_cube(17, 7),
+}
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3])
+@pytest.mark.parametrize("prec,tol", [(0, 1e-12), (1, 1e-4)])
+@pytest.mark.parametrize("name", sorted(MESHES))
+def test_resident_cycle(name, prec, tol, degree):
+    import nosh_gb300 as ng
+
+    x, c, psi = MESHES[name]()
+    m = O.finish_mesh(x, c)
+    A = O.mvp_constant_curl(m.x)
+    model = ng.nls(ng.mesh(m.x, m.cells), A, -1.0, 1.0, 1.0, mu=0.3, precision=prec)
+    model.set_spmv_schedule(ng.SPMV_STAGED)
+    model.set_amg_options(smooth_degree=degree, coarse_size=40)
+    M = model.create_W_prec()
+    M.rebuild({"g": 1.0, "mu": 0.3}, psi)
+    rng = np.random.default_rng(11)
+    a, b = rng.standard_normal((2, 2 * m.N))
+    Ma, Mb = M.apply(a), M.apply(b)
+    assert np.isfinite(Ma).all() and a @ Ma > 0 and b @ Mb > 0
+    assert abs(a @ Mb - b @ Ma) <= tol * np.linalg.norm(a) * np.linalg.norm(Mb)
+    model.profile(True)
+    grid = M.apply(a)
+    model.profile(False)
+    assert np.abs(grid - Ma).max() <= tol * np.abs(grid).max()
+    assert np.array_equal(M.apply(a), Ma)
