@@ -230,15 +230,24 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Block-level sum (blockDim.x multiple of 32, <= 1024); valid in thread 0.
+// Up to eight warps' sums are added by that thread in order: a shuffle tree
+// over them is five dependent FP64 steps whatever their number.
 __device__ __forceinline__ double block_sum(double v, double *smem32) {
   v = warp_sum(v);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
   if (lane == 0) smem32[w] = v;
   __syncthreads();
   double r = 0.0;
-  if (w == 0) {
-    r = (lane < (int)(blockDim.x >> 5)) ? smem32[lane] : 0.0;
+  if (nw <= 8) {
+    if (threadIdx.x == 0) {
+      double t[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) t[k] = k < nw ? smem32[k] : 0.0;
+      r = ((t[0] + t[1]) + (t[2] + t[3])) + (nw > 4 ? (t[4] + t[5]) + (t[6] + t[7]) : 0.0);
+    }
+  } else if (w == 0) {
+    r = lane < nw ? smem32[lane] : 0.0;
     r = warp_sum(r);
   }
   return r;

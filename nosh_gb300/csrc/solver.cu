@@ -53,6 +53,7 @@ __global__ void minres_init(MinresScalars *s, const double *params) {
   s->done = 0;
   s->wx_pending = 0;
   s->oldb = 0.0;
+  s->ioldb = 0.0;
   s->dbar = 0.0;
   s->epsln = 0.0;
   s->oldeps = 0.0;
@@ -66,10 +67,12 @@ __global__ void minres_init(MinresScalars *s, const double *params) {
     s->flag = isnan(rz) || isinf(rz) ? NOSH_ERR_NAN : NOSH_ERR_BREAKDOWN;
     s->done = 2;
     s->beta1 = s->beta = s->phibar = 0.0;
+    s->ibeta = 0.0;
     return;
   }
   s->beta1 = sqrt(rz);
   s->beta = s->beta1;
+  s->ibeta = rsqrt(rz);
   s->phibar = s->beta1;
   if (rz == 0.0) s->done = 2;  // b == 0: x = 0
 }
@@ -307,10 +310,20 @@ int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &re
     NOSH_CUDA(cudaGraphLaunch(part_exec[h], st));
     s.launch_count += part_kernels[h];
   };
-  // first batch: as many parts as the previous solve used (one chunk at
-  // first); one part per poll when timing, so that every replay's events
-  // are read before the part is replayed again
-  int batch = timed ? 1 : last_its > 0 ? (last_its + kPart - 1) / kPart : kParts;
+  // First batch: the parts this tolerance takes at the previous solve's
+  // convergence rate (one chunk at first).  A part too many costs its
+  // launches, a part too few a round trip to the host, about as much.  One
+  // part per poll when timing, so that every replay's events are read before
+  // the part is replayed again.
+  int batch = kParts;
+  if (timed) {
+    batch = 1;
+  } else if (last_its > 0) {
+    double its = last_its;
+    if (last_rel > 0.0 && last_rel < 0.9 && rtol > 0.0 && rtol < 0.9) its *= std::log(rtol) / std::log(last_rel);
+    its = std::min(its, (double)maxit);
+    batch = std::max(1, (int)std::lround(its / kPart));
+  }
   int it = 0, h = 0;
   bool first = true;
   for (;;) {
@@ -359,6 +372,7 @@ int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &re
   status = h_sc->flag;
   rel_res = h_sc->beta1 > 0 ? h_sc->phibar / h_sc->beta1 : 0.0;
   last_its = h_sc->itn;
+  last_rel = rel_res;
   return h_sc->itn;
 }
 

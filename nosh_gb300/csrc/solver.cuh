@@ -11,8 +11,8 @@ namespace nosh {
 // the SPD preconditioner, vectors in T, scalars in FP64 (minres_state.cuh).
 // Buffer roles repeat every kChunk iterations; the chunk is captured once as
 // kParts CUDA graphs of kPart iterations (replayed in turn).  A solve
-// launches as many parts as the previous solve needed before the host first
-// polls the convergence flag, then one at a time; launches after
+// launches as many parts as the previous solve's convergence rate predicts
+// before the host first polls the convergence flag, then one at a time; launches after
 // convergence return at once (each such iteration still costs its kernels'
 // launches, so parts are kept short).
 template <typename T>
@@ -35,7 +35,8 @@ struct Minres {
   DevBuf<double> params;
   double *h_params = nullptr;
   int64_t part_kernels[kParts] = {};
-  int last_its = 0;  // iterations of the previous solve
+  int last_its = 0;  // iterations of the previous solve, and where it ended
+  double last_rel = 0.0;
   // Kernel timing (the handle's timers on): the graphs are captured with
   // event-record nodes around the timed launches; the pairs of each
   // iteration of each part (per timer) and of the prologue, harvested after
