@@ -249,8 +249,6 @@ __global__ void rap_diag(int64_t na, const int32_t *__restrict__ mptr,
   cdia[3 * a + 2] = d2;
 }
 
-// inverse diagonal blocks and the Gershgorin bound of lambda_max(D^-1 A):
-// 1 + ||D_i^-1||_2 sum_j |a_ij|, reduced by max over rows (arithmetic in T)
 // sum_j |a_ij| per row (the loop dinv_gershgorin runs without rowabs)
 template <typename T>
 __global__ void row_abs_sums(int64_t n, const int32_t *__restrict__ rp, const C2<T> *__restrict__ off,
@@ -265,70 +263,97 @@ __global__ void row_abs_sums(int64_t n, const int32_t *__restrict__ rp, const C2
   out[i] = s;
 }
 
-// (rowabs: the rows' sums of |a_ij| when known, else summed here)
+// The smoother's Chebyshev polynomial on [lmax / ratio, 1.1 lmax]: its
+// centre and half width are multiples of lmax, so everything but 1 / lmax is
+// a constant of the degree and the ratio: coef[0] = c0 / lmax, then per step
+// k >= 1 the pair (p[k] = rho_k rho_{k-1}, q[k] / lmax = 2 rho_k / delta).
+constexpr int kMaxDegree = 8;  // of the smoother (nosh_nls_set_amg_options)
+struct ChebSpec {
+  int deg;
+  double c0, p[kMaxDegree], q[kMaxDegree];
+  static ChebSpec of(int deg, double ratio) {
+    ChebSpec s{};
+    s.deg = deg;
+    const double lmin = 1.0 / (1.1 * ratio), theta = 0.5 * (1.0 + lmin), delta = 0.5 * (1.0 - lmin);
+    const double sigma = theta / delta;
+    double rho = 1.0 / sigma;
+    s.c0 = 1.0 / theta;
+    for (int k = 1; k < deg; k++) {
+      const double rn = 1.0 / (2.0 * sigma - rho);
+      s.p[k] = rn * rho;
+      s.q[k] = 2.0 * rn / delta;
+      rho = rn;
+    }
+    return s;
+  }
+};
+
+__device__ __forceinline__ void inv3(double det, double a, double d, double b, double *o) {
+  const double r = 1.0 / det;  // one FP64 division instead of three
+  o[0] = d * r;
+  o[1] = a * r;
+  o[2] = -b * r;
+}
+__device__ __forceinline__ void inv3(float det, float a, float d, float b, float *o) {
+  o[0] = d / det;
+  o[1] = a / det;
+  o[2] = -b / det;
+}
+
+// Inverse diagonal blocks and the Gershgorin bound of lambda_max(D^-1 A),
+// 1 + ||D_i^-1||_2 sum_j |a_ij| reduced by max over rows (arithmetic in T;
+// rowabs: the rows' sums of |a_ij| when known, else summed here); the last
+// CTA to finish turns it into the level's Chebyshev coefficients.  The bound
+// is compared as the bits of a non-negative double, which order alike: an
+// FP64 maximum would be FP64 instructions.  *lmax_bits and *arrive are zero
+// between launches.
 template <typename T>
-__global__ void dinv_gershgorin(int64_t n, const int32_t *__restrict__ rp,
-                                const C2<T> *__restrict__ off, const T *__restrict__ dia,
-                                T *__restrict__ dinv, unsigned long long *lmax_bits, int *err,
-                                const T *__restrict__ rowabs = nullptr) {
+__global__ void dinv_gershgorin(int64_t n, const int32_t *__restrict__ rp, const C2<T> *__restrict__ off,
+                                const T *__restrict__ dia, T *__restrict__ dinv, unsigned long long *lmax_bits,
+                                unsigned *arrive, int *err, const T *__restrict__ rowabs, ChebSpec spec, T *coef) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double bound = 0.0;
+  unsigned long long v = 0;
   if (i < n) {
     const T a = dia[3 * i], d = dia[3 * i + 1], b = dia[3 * i + 2];
     const T det = a * d - b * b;
-    dinv[3 * i] = d / det;
-    dinv[3 * i + 1] = a / det;
-    dinv[3 * i + 2] = -b / det;
+    inv3(det, a, d, b, dinv + 3 * i);
     const T lmin = (T)0.5 * (a + d) - sqrt((T)0.25 * (a - d) * (a - d) + b * b);
     T s = 0;
     if (rowabs) {
       s = rowabs[i];
     } else {
       for (int32_t k = rp[i]; k < rp[i + 1]; k++) {
-        const C2<T> v = off[k];
-        s += sqrt(v.x * v.x + v.y * v.y);
+        const C2<T> w = off[k];
+        s += sqrt(w.x * w.x + w.y * w.y);
       }
     }
-    bound = (lmin > 0 && det > 0) ? 1.0 + (double)(s / lmin) : 1e300;
+    const double bound = (lmin > 0 && det > 0) ? 1.0 + (double)(s / lmin) : 1e300;
+    v = (unsigned long long)__double_as_longlong(bound);
     // a diagonal block that is not positive definite: the operator is not
     // SPD (a g < 0 regularisation), so neither is the V-cycle
     if (!(lmin > 0 && det > 0)) atomicOr(err, 32);
   }
-  // max over the block, then one atomic per block (non-negative doubles
-  // order like their bit patterns)
-  __shared__ double sm[32];
-  double v = bound;
+  __shared__ unsigned long long sm[32];
+  auto warp_max = [](unsigned long long u) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) u = max(u, __shfl_xor_sync(0xffffffffu, u, o));
+    return u;
+  };
+  v = warp_max(v);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    v = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (threadIdx.x == 0) atomicMax(lmax_bits, (unsigned long long)__double_as_longlong(v));
+  if (threadIdx.x >= 32) return;
+  v = warp_max(threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0ull);
+  if (threadIdx.x != 0) return;
+  atomicMax(lmax_bits, v);
+  if (arrive_acq_rel(arrive) != gridDim.x - 1) return;
+  const double il = 1.0 / (1.1 * __longlong_as_double((long long)atomicExch(lmax_bits, 0ull)));
+  *arrive = 0u;
+  coef[0] = (T)(spec.c0 * il);
+  for (int k = 1; k < spec.deg; k++) {
+    coef[2 * k] = (T)spec.p[k];
+    coef[2 * k + 1] = (T)(spec.q[k] * il);
   }
-}
-
-// Chebyshev coefficients from lambda_max: c[0] = 1/theta, then per step
-// k >= 1 the pair (rho_k rho_{k-1}, 2 rho_k / delta).
-template <typename T>
-__global__ void cheb_coeffs(const unsigned long long *lmax_bits, int deg, double ratio, T *coef,
-                            double *lmax_out) {
-  // smoothing interval [lmax / ratio, 1.1 lmax]
-  const double lmax = 1.1 * __longlong_as_double((long long)*lmax_bits);
-  const double lmin = lmax / (1.1 * ratio);
-  const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
-  const double sigma = theta / delta;
-  double rho = 1.0 / sigma;
-  coef[0] = (T)(1.0 / theta);
-  for (int k = 1; k < deg; k++) {
-    const double rn = 1.0 / (2.0 * sigma - rho);
-    coef[2 * k] = (T)(rn * rho);
-    coef[2 * k + 1] = (T)(2.0 * rn / delta);
-    rho = rn;
-  }
-  *lmax_out = lmax;
 }
 
 // ---- smoother building blocks (shared by the grid kernels and the tail)
@@ -704,7 +729,6 @@ __global__ void dense_matvec(int m, const T *__restrict__ Ainv, DenseMap D, cons
 // up to sixteen ways.
 constexpr int kTailThreads = 512;
 constexpr int kTailSmem = 200 * 1024;  // shared memory of one CTA, at most
-constexpr int kMaxDegree = 8;          // of the smoother (nosh_nls_set_amg_options)
 
 template <typename T>
 struct LevelDesc {
@@ -741,7 +765,7 @@ struct TailArgs {
   const C2<T> *r_cur;
   C2<T> *z;            // kOutVector, kOutMinres
   MinresScalars *ms;
-  unsigned *fail;      // set when a wait for a phase's vector gives up
+  unsigned *fail;      // (pinned host memory) set when a wait for a phase's vector gives up
 };
 
 // The coarsest level's dense inverse in shared memory (byte offsets): the own
@@ -825,7 +849,7 @@ struct TailTeam {
           : "memory");
       if (done) return;
     }
-    atomicOr(fail, 1u);
+    *(volatile unsigned *)fail = 1u;
   }
 };
 
@@ -1304,8 +1328,10 @@ struct Amg::Impl {
   int lt = 1;  // first level handled by the coarse-level tail
   AmgVals<float> vf;
   AmgVals<double> vd;
-  DevBuf<unsigned long long> lmax_bits;  // one per level
-  DevBuf<double> lmax;
+  // per level, zero between refreshes: the Gershgorin bound's bits, arrivals
+  DevBuf<unsigned long long> lmax_bits;
+  DevBuf<unsigned> arrive;
+  ChebSpec cheb;
   DevBuf<double> dense;  // coarsest (2n)^2 FP64
   DevBuf<float> densef;
   // packed block-diagonal coarsest inverse: per block (offset, dim), per real
@@ -1443,7 +1469,10 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
     if (l == L - 1) I.grid_coarse = true;
   }
   I.lmax_bits.alloc(L);
-  I.lmax.alloc(L);
+  I.lmax_bits.zero(st);
+  I.arrive.alloc(L);
+  I.arrive.zero(st);
+  I.cheb = ChebSpec::of(std::max(o.smooth_degree, 1), o.cheb_ratio);
   {
     // the coarsest level's dense inverse: one packed block per system
     const HostLevel &Hc = H.back();
@@ -1569,17 +1598,13 @@ void Amg::refresh() {
     // block-Jacobi inverse and Chebyshev bounds follow it, the coarse
     // operators keep their last Galerkin values (SPD, so the V-cycle stays
     // an SPD preconditioner)
-    NOSH_CUDA(cudaMemsetAsync(I.lmax_bits.p, 0, sizeof(unsigned long long), st));
     dinv_gershgorin<T><<<div_up(I.lev[0].n, 256), 256, 0, st>>>(I.lev[0].n, I.lev[0].rp, I.off<T>(0), I.dia<T>(0),
-                                                                V.dinv[0].p, I.lmax_bits.p, I.err.p,
-                                                                V.rowabs0.p);
-    cheb_coeffs<T><<<1, 1, 0, st>>>(I.lmax_bits.p, std::max(I.opt.smooth_degree, 1), I.opt.cheb_ratio, V.coef[0].p,
-                                    I.lmax.p);
-    I.nls.launch_count += 2;
+                                                                V.dinv[0].p, I.lmax_bits.p, I.arrive.p, I.err.p,
+                                                                V.rowabs0.p, I.cheb, V.coef[0].p);
+    ++I.nls.launch_count;
     NOSH_CUDA(cudaGetLastError());
     return;
   }
-  NOSH_CUDA(cudaMemsetAsync(I.lmax_bits.p, 0, L * sizeof(unsigned long long), st));
   for (int l = 0; l < L; l++) {
     AmgLevel &A = I.lev[l];
     if (l > 0) {
@@ -1593,12 +1618,9 @@ void Amg::refresh() {
       ++I.nls.launch_count;
     }
     if (l < L - 1) {  // the coarsest level is solved directly
-      dinv_gershgorin<T><<<div_up(A.n, 256), 256, 0, st>>>(A.n, A.rp, I.off<T>(l), I.dia<T>(l),
-                                                            V.dinv[l].p, I.lmax_bits.p + l, I.err.p,
-                                                            l == 0 ? (const T *)V.rowabs0.p : nullptr);
-      ++I.nls.launch_count;
-      cheb_coeffs<T><<<1, 1, 0, st>>>(I.lmax_bits.p + l, std::max(I.opt.smooth_degree, 1), I.opt.cheb_ratio,
-                                      V.coef[l].p, I.lmax.p + l);
+      dinv_gershgorin<T><<<div_up(A.n, 256), 256, 0, st>>>(
+          A.n, A.rp, I.off<T>(l), I.dia<T>(l), V.dinv[l].p, I.lmax_bits.p + l, I.arrive.p + l, I.err.p,
+          l == 0 ? (const T *)V.rowabs0.p : nullptr, I.cheb, V.coef[l].p);
       ++I.nls.launch_count;
     }
   }
@@ -1813,7 +1835,7 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
   const TailPlan<T> &P = plan<T>();
   if (!grid_coarse && l + 1 == P.lt) {
     TailArgs<T> a{};
-    a.fail = nls.red.counter.p + kStageErrorSlot;
+    a.fail = nls.h_stage_err;
     a.head = kHeadRestrict;
     a.out = kOutProlong;
     a.f_res = V.res[l].p;
@@ -1883,7 +1905,7 @@ void Amg::apply(const T *r, T *z) {
     // the whole cycle resident; no overlap: it stages the block inverses,
     // which the refresh before it may have written
     TailArgs<T> a{};
-    a.fail = I.nls.red.counter.p + kStageErrorSlot;
+    a.fail = I.nls.h_stage_err;
     a.head = kHeadVector;
     a.out = kOutVector;
     a.b = (const C2<T> *)r;
@@ -1947,7 +1969,7 @@ void Amg::apply_minres(MinresScalars *ms, const T *u, T *r_old, const T *r_cur, 
   I.halt = &ms->done;
   if (const TailPlan<T> &P = I.plan<T>(); P.lt == 0) {
     TailArgs<T> a{};
-    a.fail = I.nls.red.counter.p + kStageErrorSlot;
+    a.fail = I.nls.h_stage_err;
     a.head = kHeadLanczos;
     a.out = kOutMinres;
     a.b = (const C2<T> *)u;

@@ -117,9 +117,13 @@ struct OutVec {
       dev = buf.p;
     }
   }
-  void finish(nosh::NlsImpl &s) {
+  // enqueue the copy back; finish(): and wait
+  void copy_back(nosh::NlsImpl &s) {
     if (dev != user)
       NOSH_CUDA(cudaMemcpyAsync(user, dev, n * sizeof(double), cudaMemcpyDefault, s.stream));
+  }
+  void finish(nosh::NlsImpl &s) {
+    copy_back(s);
     s.sync();
   }
 };
@@ -456,10 +460,8 @@ int nosh_nls_compute_f_norm(nosh_nls nls, const double *x, const double *p, doub
     const double *dx = stage_in(s, x, s.d_in, 2 * s.N);
     OutVec of(s, f, s.d_out, 2 * s.N);
     s.compute_f64(dx, g, mu, of.dev, norm ? 0 : -1);
-    double n2 = 0.0;
-    if (norm) s.red.out.download(&n2, 1, s.stream);
     of.finish(s);
-    if (norm) *norm = std::sqrt(n2);
+    if (norm) *norm = std::sqrt(s.red.host[0]);
   });
 }
 
@@ -573,7 +575,7 @@ int nosh_jacobian_rebuild(nosh_nls nls, const double *p, const double *x) {
     auto &s = N(nls);
     double g, mu;
     read_params(p, g, mu);
-    s.jac_rebuild(stage_in(s, x, s.d_in, 2 * s.N), g, mu);
+    s.jac_rebuild(stage_in(s, x, s.d_in, 2 * s.N), g, mu, s.precision != NOSH_PREC_FP64);
     s.sync();
   });
 }
@@ -584,6 +586,7 @@ int nosh_jacobian_apply(nosh_nls nls, const double *X, double *Y, int nvec, int 
     auto &s = NC(nls);
     check_apply_args(mode, alpha, beta, nvec);
     require(s.jac_ready, "Jacobian not built: call nosh_jacobian_rebuild first");
+    if (s.precision != NOSH_PREC_FP64) s.ensure_diag32();
     for (int k = 0; k < nvec; k++) {
       const double *dx = stage_in(s, X + (size_t)k * 2 * s.N, s.d_in, 2 * s.N);
       OutVec o(s, Y + (size_t)k * 2 * s.N, s.d_out, 2 * s.N);
@@ -594,8 +597,9 @@ int nosh_jacobian_apply(nosh_nls nls, const double *X, double *Y, int nvec, int 
         s.jac_apply<float>(s.d_inf.p, s.d_outf.p);
         nosh::launch_f32_to_f64(s.d_outf.p, o.dev, 2 * s.N, s.stream);
       }
-      o.finish(s);
+      o.copy_back(s);
     }
+    s.sync();  // once: the vectors share the handle's stream and staging buffers
   });
 }
 
@@ -605,7 +609,7 @@ int nosh_keo_regularized_rebuild(nosh_nls nls, const double *p, const double *x)
     auto &s = N(nls);
     double g, mu;
     read_params(p, g, mu);
-    s.reg_rebuild(stage_in(s, x, s.d_in, 2 * s.N), g, mu);
+    s.reg_rebuild(stage_in(s, x, s.d_in, 2 * s.N), g, mu, s.precision != NOSH_PREC_FP64);
     nosh::Amg &amg = nosh::ensure_preconditioner(s);
     if (s.precision == NOSH_PREC_FP64) amg.refresh<double>();
     else amg.refresh<float>();
@@ -619,6 +623,7 @@ int nosh_keo_regularized_apply(nosh_nls nls, const double *X, double *Y, int nve
     auto &s = NC(nls);
     check_apply_args(mode, alpha, beta, nvec);
     require(s.reg_ready && s.amg, "preconditioner not built: call nosh_keo_regularized_rebuild");
+    if (s.precision != NOSH_PREC_FP64) s.ensure_diag32();
     for (int k = 0; k < nvec; k++) {
       const double *dx = stage_in(s, X + (size_t)k * 2 * s.N, s.d_in, 2 * s.N);
       OutVec o(s, Y + (size_t)k * 2 * s.N, s.d_out, 2 * s.N);
@@ -629,8 +634,9 @@ int nosh_keo_regularized_apply(nosh_nls nls, const double *X, double *Y, int nve
         s.amg->apply<float>(s.d_inf.p, s.d_outf.p);
         nosh::launch_f32_to_f64(s.d_outf.p, o.dev, 2 * s.N, s.stream);
       }
-      o.finish(s);
+      o.copy_back(s);
     }
+    s.sync();  // once: the vectors share the handle's stream and staging buffers
   });
 }
 
@@ -653,6 +659,7 @@ int nosh_keo_regularized_smoother_apply(nosh_nls nls, const double *x, double *y
   return guarded([&] {
     auto &s = NC(nls);
     require(s.reg_ready && s.amg, "preconditioner not built: call nosh_keo_regularized_rebuild");
+    if (s.precision != NOSH_PREC_FP64) s.ensure_diag32();
     const double *dx = stage_in(s, x, s.d_in, 2 * s.N);
     OutVec o(s, y, s.d_out, 2 * s.N);
     if (s.precision == NOSH_PREC_FP64) {

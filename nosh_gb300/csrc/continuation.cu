@@ -148,12 +148,12 @@ void ContinuationImpl::extrapolate(int order, double mu_new, double *out) {
 }
 
 namespace {
-double *dots_host(NlsImpl &s, const DotSet &d, int64_t n, double *dev_out, double *host) {
-  dot_set_kernel<<<reduce_grid(n), 256, 0, s.stream>>>(n, d, s.red.partials.p, s.red.counter.p, dev_out);
+double *dots_host(NlsImpl &s, const DotSet &d, int64_t n, double *host) {
+  dot_set_kernel<<<reduce_grid(n), 256, 0, s.stream>>>(n, d, s.red.partials.p, s.red.counter.p, s.red.host);
   ++s.launch_count;
   NOSH_CUDA(cudaGetLastError());
-  NOSH_CUDA(cudaMemcpyAsync(host, dev_out, d.k * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
   s.sync();
+  for (int k = 0; k < d.k; k++) host[k] = s.red.host[k];
   return host;
 }
 void lin3(NlsImpl &s, int64_t n, double *y, double c0, const double *x0, double c1 = 0.0,
@@ -183,7 +183,7 @@ int ContinuationImpl::tangent_direction(const nosh_newton_options &opt, int prec
   d.add(slot(0), out, true);  // <psi0, i v> = -<i psi0, v>
   d.add(slot(0), slot(0));
   double h[6];
-  dots_host(s, d, s.N, dots.p, h);
+  dots_host(s, d, s.N, h);
   NOSH_CHECK(h[1] > 0.0, NOSH_ERR_BREAKDOWN, "tangent at a zero state");
   const double kappa = -h[0] / h[1];
   // out = -(v - kappa i psi0)
@@ -247,7 +247,7 @@ void ContinuationImpl::advance_arclength(double ds, int predictor, double theta_
     DotSet d;
     d.add(tau.p, tau.p);
     if (have_secant) d.add(tau.p, va.p);
-    dots_host(s, d, N, dots.p, h);
+    dots_host(s, d, N, h);
   }
   const double t2 = h[0] * inv_n + th2 * tmu * tmu;
   NOSH_CHECK(t2 > 0.0 && std::isfinite(t2), NOSH_ERR_BREAKDOWN, "zero or non-finite tangent");
@@ -287,7 +287,7 @@ void ContinuationImpl::advance_arclength(double ds, int predictor, double theta_
     DotSet d;
     d.add(tau.p, va.p);
     d.add(tau.p, vb.p);
-    dots_host(s, d, N, dots.p, h);
+    dots_host(s, d, N, h);
     const double den = th2 * tmu - h[1] * inv_n;
     if (!(std::isfinite(den) && den != 0.0)) {
       st.status = NOSH_ERR_BREAKDOWN;  // singular bordered system

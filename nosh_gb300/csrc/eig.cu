@@ -310,8 +310,7 @@ int lowest_eigenpairs(NlsImpl &s, const double *psi_dev, double g, double mu, in
   NOSH_CHECK(k >= 1 && 3 * mb <= kMaxRows && 3 * mb + 1 < n, NOSH_ERR_INVALID,
              "need 1 <= k, 3 (k + guard) <= 64 and 3 (k + guard) + 1 < 2N");
   // FP64 operators at psi
-  s.jac_rebuild(psi_dev, g, mu);
-  s.reg_rebuild(psi_dev, g, mu);
+  s.operators64_rebuild(psi_dev, g, mu);
   ensure_preconditioner(s).refresh<double>();
   BlockOps B(s, n);
   DevBuf<double> U(n), X((size_t)mb * n), AX((size_t)mb * n), P((size_t)mb * n), R((size_t)mb * n);

@@ -1511,7 +1511,7 @@ void Mpnn::Impl::features(const double *const x[4], const double mu[4], double t
                                      (const C2<double> *)target, sq.p, (C2<double> *)vc.p, (C2<double> *)vd.p,
                                      (C2<double> *)vt.p);
     ++s.launch_count;
-    s.jac_rebuild(vt.p, s.g0, t);
+    s.jac_rebuild(vt.p, s.g0, t, false);
     s.jac_apply<double>(vc.p, jc.p);
     s.jac_apply<double>(vd.p, jd.p);
     gram3_kernel<<<reduce_grid(2 * N), 256, 0, st>>>(2 * N, jc.p, jd.p, rd.partials.p, rd.counter.p, gram.p);

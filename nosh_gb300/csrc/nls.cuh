@@ -17,12 +17,23 @@ struct Reducer {
   DevBuf<double> partials;   // >= number of blocks of any reducing launch
   DevBuf<unsigned> counter;  // zero between launches
   DevBuf<double> out;        // result slots
+  // result slots in pinned host memory, written by the finishing thread: a
+  // call that waits for the stream next reads its result without a copy
+  // (each cost about 3 us of the GPU's copy queue and the host)
+  double *host = nullptr;
+  Reducer() = default;
+  Reducer(const Reducer &) = delete;
+  Reducer &operator=(const Reducer &) = delete;
+  ~Reducer() {
+    if (host) cudaFreeHost(host);
+  }
   void init(int max_blocks, int nslots, cudaStream_t s) {
     partials.alloc(max_blocks * 4 + 64);
     counter.alloc(16);
     counter.zero(s);
     out.alloc(nslots);
     out.zero(s);
+    if (!host) NOSH_CUDA(cudaMallocHost(&host, 16 * sizeof(double)));
   }
 };
 
@@ -158,6 +169,10 @@ struct NlsImpl {
   DevBuf<double> d_jd64, d_rd64;  // 3N each
   DevBuf<float> d_jd32, d_rd32;
   bool jac_ready = false, reg_ready = false;
+  // the FP32 blocks belong to the FP64 blocks' state (else ensure_diag32()
+  // rounds them before an FP32 apply)
+  bool jd32_ok = false, rd32_ok = false;
+  void ensure_diag32();
   double reg_g = 0.0;
 
   // staging for host / misaligned vectors
@@ -216,10 +231,10 @@ struct NlsImpl {
   void dkeo_refill(double mu);
   void keo_apply64(const double *x, double *y);
   void dkeo_apply64(const double *x, double *y);
-  // y = F(x); optional ||F||^2 into red.out[slot]; with soff, also the
+  // y = F(x); optional ||F||^2 into red.host[slot]; with soff, also the
   // off-diagonal sums of K x (2N doubles), the base of residual_update
   void compute_f64(const double *x, double g, double mu, double *f, int norm_slot, double *soff = nullptr);
-  // F and ||F||^2 (into red.out[0]; not waited for) of x = x_old + dx, dx
+  // F and ||F||^2 (into red.host[0]; not waited for) of x = x_old + dx, dx
   // an FP32 update already added to x, from soff = the off-diagonal sums of
   // K x_old (updated in place to those of K x): an FP32 SpMV of dx with an
   // FP64 epilogue (ResidualUpdateOp)
@@ -237,11 +252,14 @@ struct NlsImpl {
                      double norms[2], double *sa = nullptr, double *sb = nullptr, bool wait = true);
   // the norms of a residual_pair(..., wait = false): waits, then norms[0..1]
   void residual_pair_norms(double norms[2]);
-  void jac_rebuild(const double *x, double g, double mu);
+  // (want32: the FP32 blocks in the same pass)
+  void jac_rebuild(const double *x, double g, double mu, bool want32);
+  // jac_rebuild and reg_rebuild in one launch, the FP64 blocks only
+  void operators64_rebuild(const double *x, double g, double mu);
   // the FP32 diagonal blocks of J and of the regularised KEO only, for a
   // mixed-precision solve
   void operators32_rebuild(const double *x, double g, double mu);
-  void reg_rebuild(const double *x, double g, double mu);
+  void reg_rebuild(const double *x, double g, double mu, bool want32);
   template <typename T>
   void jac_apply(const T *x, T *y, double *dot_out = nullptr);
   template <typename T>
@@ -251,12 +269,13 @@ struct NlsImpl {
   // full-graph values (with diagonal) in complex_graph order, complex
   void export_values(const C2<double> *offdiag, const double *diag, double *out);
 
-  // Waits for the handle's stream.  A staged SpMV that gave up waiting for
-  // its copies (kStageErrorSlot set) makes it throw NOSH_ERR_CUDA after
-  // clearing the flag and the reduction counters, so the handle stays usable.
+  // Waits for the handle's stream.  A kernel that gave up one of its bounded
+  // waits (a staged SpMV's copies, the resident cycle's vectors) has set
+  // *h_stage_err: then it throws NOSH_ERR_CUDA after clearing the flag and the
+  // reduction counters, so the handle stays usable.
   void sync();
   [[noreturn]] void stage_failure();
-  unsigned *h_stage_err = nullptr;  // pinned, one word
+  unsigned *h_stage_err = nullptr;  // pinned, one word, written by the failing kernel
   // diagnostics: bound of the staging waits (polls; < 0 restores the default)
   void set_stage_wait_limit(int64_t polls);
   // index-check mode: the KEO graph is validated on the device before every

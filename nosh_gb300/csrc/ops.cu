@@ -134,85 +134,73 @@ __global__ void dkeo_assemble64(int64_t E, const double *__restrict__ alpha,
 }
 
 // ------------------------------------------------------------ diagonals
-// jacobian_operator::rebuild_diags_ (src/jacobian_operator.cpp:184-197),
-// with K_ii folded in: [[d0r, d1b], [d1b, d0i]].
-__global__ void jac_diag_kernel(int64_t N, const double *__restrict__ kdiag,
-                                const double *__restrict__ cvt, const double *__restrict__ V,
-                                double g, const C2<double> *__restrict__ x, double *d64,
+// Per vertex, [[a, c], [c, b]] with K_ii folded in:
+//   Jacobian (rebuild_diags_, src/jacobian_operator.cpp:184-197):
+//     K_ii + cv t (V + 2 g |x|^2) +- g cv t (x_r^2 - x_i^2), c = 2 g cv t x_r x_i
+//   regularised KEO (src/keo_regularized.cpp:233-258), for g > 0: the same
+//     without V; K_ii alone otherwise.
+// Both are (K_ii [+ cv t V]) + g cv t (3 x_r^2 + x_i^2) and its mirror image:
+// eleven FP64 instructions for one, thirteen for both (the sums as written
+// above took eighteen and thirty-two), and FP64 instructions bound these
+// kernels: at 160^3 the Jacobian's blocks took 116 us for 47 us of traffic.
+struct DiagTerms {
+  double gw, s1, s2, c;
+};
+__device__ __forceinline__ DiagTerms diag_terms(const C2<double> &p, double w, double g) {
+  const double xx = p.x * p.x, yy = p.y * p.y, gw = g * w;
+  return DiagTerms{gw, fma(3.0, xx, yy), fma(3.0, yy, xx), (gw * p.x) * (p.y + p.y)};
+}
+template <typename T>
+__device__ __forceinline__ void put3(T *d, int64_t k, double a, double b, double c) {
+  d[3 * k] = (T)a;
+  d[3 * k + 1] = (T)b;
+  d[3 * k + 2] = (T)c;
+}
+
+// Jacobian blocks in FP64 and, for a mixed-precision handle, FP32
+__global__ void jac_diag_kernel(int64_t N, const double *__restrict__ kdiag, const double *__restrict__ cvt,
+                                const double *__restrict__ V, double g, const C2<double> *__restrict__ x, double *d64,
                                 float *d32) {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const C2<double> p = x[k];
   const double w = cvt[k];
-  const double al = w * (V[k] + g * 2.0 * (p.x * p.x + p.y * p.y));
-  const double rx2 = g * w * (p.x * p.x - p.y * p.y);
-  const double a = kdiag[k] + al + rx2, b = kdiag[k] + al - rx2, c = g * w * (2.0 * p.x * p.y);
-  d64[3 * k] = a;
-  d64[3 * k + 1] = b;
-  d64[3 * k + 2] = c;
-  d32[3 * k] = (float)a;
-  d32[3 * k + 1] = (float)b;
-  d32[3 * k + 2] = (float)c;
+  const DiagTerms t = diag_terms(x[k], w, g);
+  const double kv = fma(w, V[k], kdiag[k]), a = fma(t.gw, t.s1, kv), b = fma(t.gw, t.s2, kv);
+  put3(d64, k, a, b, t.c);
+  if (d32) put3(d32, k, a, b, t.c);
 }
 
-// keo_regularized::rebuild (src/keo_regularized.cpp:233-258): + g cv t
-// [[2|x|^2 + gamma, beta], [beta, 2|x|^2 - gamma]] when g > 0.
-__global__ void reg_diag_kernel(int64_t N, const double *__restrict__ kdiag,
-                                const double *__restrict__ cvt, double g,
+// regularised KEO blocks, likewise
+__global__ void reg_diag_kernel(int64_t N, const double *__restrict__ kdiag, const double *__restrict__ cvt, double g,
                                 const C2<double> *__restrict__ x, double *d64, float *d32) {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= N) return;
-  double a = kdiag[k], b = kdiag[k], c = 0.0;
+  double a = kdiag[k], b = a, c = 0.0;
   if (g > 0.0) {
-    const C2<double> p = x[k];
-    const double w = g * cvt[k];
-    const double al = w * 2.0 * (p.x * p.x + p.y * p.y);
-    const double be = w * (2.0 * p.x * p.y);
-    const double ga = w * (p.x * p.x - p.y * p.y);
-    a += al + ga;
-    b += al - ga;
-    c = be;
+    const DiagTerms t = diag_terms(x[k], cvt[k], g);
+    b = fma(t.gw, t.s2, a);
+    a = fma(t.gw, t.s1, a);
+    c = t.c;
   }
-  d64[3 * k] = a;
-  d64[3 * k + 1] = b;
-  d64[3 * k + 2] = c;
-  d32[3 * k] = (float)a;
-  d32[3 * k + 1] = (float)b;
-  d32[3 * k + 2] = (float)c;
+  put3(d64, k, a, b, c);
+  if (d32) put3(d32, k, a, b, c);
 }
 
-// Both FP32 diagonal blocks (Jacobian and regularised KEO) in one pass, for
-// the mixed-precision Newton step's operators: the arithmetic of the two
-// kernels above (so the FP32 blocks are bitwise theirs), the FP64 blocks not
-// written.  (The same formulas in FP32 arithmetic saved a few more
-// microseconds but moved the Krylov counts of the 64^3 continuation.)
-__global__ void jac_reg_diag32_kernel(int64_t N, const double *__restrict__ kdiag, const double *__restrict__ cvt,
-                                      const double *__restrict__ V, double g, const C2<double> *__restrict__ x,
-                                      float *jd32, float *rd32) {
+// Both blocks of a Newton step's operators in one pass, in the step's
+// precision (the FP64 arithmetic either way; the same formulas in FP32
+// arithmetic moved the Krylov counts of the 64^3 continuation).
+template <typename T>
+__global__ void jac_reg_diag_kernel(int64_t N, const double *__restrict__ kdiag, const double *__restrict__ cvt,
+                                    const double *__restrict__ V, double g, const C2<double> *__restrict__ x, T *jd,
+                                    T *rd) {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const C2<double> p = x[k];
   const double w = cvt[k], kd = kdiag[k];
-  {
-    const double al = w * (V[k] + g * 2.0 * (p.x * p.x + p.y * p.y));
-    const double rx2 = g * w * (p.x * p.x - p.y * p.y);
-    jd32[3 * k] = (float)(kd + al + rx2);
-    jd32[3 * k + 1] = (float)(kd + al - rx2);
-    jd32[3 * k + 2] = (float)(g * w * (2.0 * p.x * p.y));
-  }
-  double a = kd, b = kd, c = 0.0;
-  if (g > 0.0) {
-    const double wg = g * w;
-    const double al = wg * 2.0 * (p.x * p.x + p.y * p.y);
-    const double be = wg * (2.0 * p.x * p.y);
-    const double ga = wg * (p.x * p.x - p.y * p.y);
-    a += al + ga;
-    b += al - ga;
-    c = be;
-  }
-  rd32[3 * k] = (float)a;
-  rd32[3 * k + 1] = (float)b;
-  rd32[3 * k + 2] = (float)c;
+  const DiagTerms t = diag_terms(x[k], w, g);
+  const double kv = fma(w, V[k], kd);
+  put3(jd, k, fma(t.gw, t.s1, kv), fma(t.gw, t.s2, kv), t.c);
+  if (g > 0.0) put3(rd, k, fma(t.gw, t.s1, kd), fma(t.gw, t.s2, kd), t.c);
+  else put3(rd, k, kd, kd, 0.0);
 }
 
 // dF/dp diagonal terms (src/model_evaluator_nls.cpp:665-691): out +=
@@ -397,32 +385,39 @@ template bool pick_warp_schedule<float>(int, const int32_t *, const int32_t *, c
 template bool pick_warp_schedule<double>(int, const int32_t *, const int32_t *, const C2<double> *, int, double *,
                                          unsigned *, cudaStream_t);
 
+namespace {
+// CTAs of a kernel the device holds at once.  The runtime's occupancy query
+// costs more than the launch it precedes, and the answer depends on the
+// kernel, its launch shape and the device only: kept per thread.
+int64_t resident_ctas(const void *kernel, int threads, size_t smem) {
+  struct Entry {
+    const void *kernel;
+    int threads, device;
+    size_t smem;
+    int64_t ctas;
+  };
+  thread_local std::vector<Entry> seen;
+  int d = 0;
+  NOSH_CUDA(cudaGetDevice(&d));
+  for (const Entry &e : seen)
+    if (e.kernel == kernel && e.smem == smem && e.threads == threads && e.device == d) return e.ctas;
+  int sms = 0, per_sm = 0;
+  NOSH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d));
+  NOSH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+  if (seen.size() >= 256) seen.clear();
+  seen.push_back({kernel, threads, d, smem, (int64_t)std::max(per_sm, 1) * sms});
+  return seen.back().ctas;
+}
+}  // namespace
+
 int warp_grid(const void *kernel, int64_t n_rows) {
-  static int sms = 0;
-  if (sms == 0) {
-    int d = 0;
-    NOSH_CUDA(cudaGetDevice(&d));
-    NOSH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d));
-  }
-  int per_sm = 0;
-  NOSH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarpThreads, 0));
   const int64_t blocks = (n_rows + kWarpThreads - 1) / kWarpThreads;
-  const int64_t cap = (int64_t)std::max(per_sm, 1) * sms;
-  return (int)std::max<int64_t>(1, std::min(blocks, cap));
+  return (int)std::max<int64_t>(1, std::min(blocks, resident_ctas(kernel, kWarpThreads, 0)));
 }
 
 int row_grid(const void *kernel, int threads, size_t smem, int64_t n_rows) {
-  static int sms = 0;
-  if (sms == 0) {
-    int d = 0;
-    NOSH_CUDA(cudaGetDevice(&d));
-    NOSH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d));
-  }
-  int per_sm = 0;
-  NOSH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   const int64_t blocks = (n_rows + kRows - 1) / kRows;
-  const int64_t cap = (int64_t)std::max(per_sm, 1) * sms;
-  return (int)std::max<int64_t>(1, std::min(blocks, cap));
+  return (int)std::max<int64_t>(1, std::min(blocks, resident_ctas(kernel, threads, smem)));
 }
 }  // namespace dev
 
@@ -623,6 +618,8 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
   red.init(div_up(N, kRows) + div_up(N, 256) + 1024, 64, s);
   NOSH_CUDA(cudaMallocHost(&h_stage_err, sizeof(unsigned)));
   *h_stage_err = 0u;
+  NOSH_CUDA(cudaMemcpyAsync(red.counter.p + kStageErrorSlot, &h_stage_err, sizeof(h_stage_err),
+                            cudaMemcpyHostToDevice, s));
   cap32 = staging_cap<float>(*m);
   cap64 = staging_cap<double>(*m);
   tune_schedules();
@@ -718,22 +715,19 @@ NlsImpl::~NlsImpl() {
 }
 
 void NlsImpl::sync() {
-  if (!h_stage_err || !red.counter.p) {
+  if (!h_stage_err) {
     NOSH_CUDA(cudaStreamSynchronize(stream));
     return;
   }
-  NOSH_CUDA(cudaMemcpyAsync(h_stage_err, red.counter.p + kStageErrorSlot, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                            stream));
   NOSH_CUDA(cudaStreamSynchronize(stream));
   if (*h_stage_err) stage_failure();
 }
 
 void NlsImpl::stage_failure() {
   // the CTAs that left early never reached their grid reductions: reset the
-  // arrival counters they left behind along with the flag (the wait-bound
-  // override in kStageWaitSlot stays)
-  NOSH_CUDA(cudaMemsetAsync(red.counter.p, 0, kStageWaitSlot * sizeof(unsigned), stream));
-  NOSH_CUDA(cudaMemsetAsync(red.counter.p + kStageErrorSlot, 0, sizeof(unsigned), stream));
+  // arrival counters they left behind along with the flag (its address and
+  // the wait-bound override stay)
+  NOSH_CUDA(cudaMemsetAsync(red.counter.p, 0, kStageErrorSlot * sizeof(unsigned), stream));
   NOSH_CUDA(cudaStreamSynchronize(stream));
   if (h_stage_err) *h_stage_err = 0;
   throw Error(NOSH_ERR_CUDA,
@@ -791,7 +785,7 @@ void NlsImpl::compute_f64(const double *x, double g, double mu, double *f, int n
   const int cap = cap64;
   if (norm_slot >= 0) {
     ResidualOp<true> op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f, (C2<double> *)soff};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap, red.out.p + norm_slot);
+    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap, red.host + norm_slot);
   } else {
     ResidualOp<false> op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f,
                          (C2<double> *)soff};
@@ -802,7 +796,7 @@ void NlsImpl::compute_f64(const double *x, double g, double mu, double *f, int n
 void NlsImpl::residual_update(const double *x, const float *dx, double g, double mu, double *f, double *soff) {
   if (!(keo_mu == mu)) keo_refill(mu);
   ResidualUpdateOp op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f, (C2<double> *)soff};
-  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)dx, op, cap32, red.out.p);
+  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)dx, op, cap32, red.host);
 }
 
 namespace {
@@ -851,17 +845,16 @@ void NlsImpl::residual_pair(const double *xa, const double *xb, double g, double
   residual_pair_kernel<<<div_up(N, 128), 128, 0, stream>>>(
       (int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo64.p, d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)xa,
       (const C2<double> *)xb, (C2<double> *)fa, (C2<double> *)fb, (C2<double> *)sa, (C2<double> *)sb,
-      red.partials.p, red.counter.p, red.out.p);
+      red.partials.p, red.counter.p, red.host);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
   if (wait) residual_pair_norms(norms);
 }
 
 void NlsImpl::residual_pair_norms(double norms[2]) {
-  red.out.download(norms, 2, stream);
   sync();
-  norms[0] = std::sqrt(norms[0]);
-  norms[1] = std::sqrt(norms[1]);
+  norms[0] = std::sqrt(red.host[0]);
+  norms[1] = std::sqrt(red.host[1]);
 }
 
 void NlsImpl::dfdp64(const double *x, double g, double mu, int param, double *out) {
@@ -874,34 +867,59 @@ void NlsImpl::dfdp64(const double *x, double g, double mu, int param, double *ou
   NOSH_CUDA(cudaGetLastError());
 }
 
-void NlsImpl::jac_rebuild(const double *x, double g, double mu) {
+void NlsImpl::jac_rebuild(const double *x, double g, double mu, bool want32) {
   if (!(keo_mu == mu)) keo_refill(mu);
-  jac_diag_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, d_V.p, g,
-                                                       (const C2<double> *)x, d_jd64.p, d_jd32.p);
+  jac_diag_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x,
+                                                       d_jd64.p, want32 ? d_jd32.p : nullptr);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
   jac_ready = true;
+  jd32_ok = want32;
 }
 
 void NlsImpl::operators32_rebuild(const double *x, double g, double mu) {
   if (!(keo_mu == mu)) keo_refill(mu);
-  jac_reg_diag32_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, d_V.p, g,
-                                                             (const C2<double> *)x, d_jd32.p, d_rd32.p);
+  jac_reg_diag_kernel<float><<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, d_V.p, g,
+                                                                  (const C2<double> *)x, d_jd32.p, d_rd32.p);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
   // the FP64 blocks no longer belong to the same state: the operator entry
   // points want their own rebuild
   jac_ready = reg_ready = false;
+  jd32_ok = rd32_ok = true;
 }
 
-void NlsImpl::reg_rebuild(const double *x, double g, double mu) {
+void NlsImpl::operators64_rebuild(const double *x, double g, double mu) {
   if (!(keo_mu == mu)) keo_refill(mu);
-  reg_diag_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, g,
-                                                       (const C2<double> *)x, d_rd64.p, d_rd32.p);
+  jac_reg_diag_kernel<double><<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, d_V.p, g,
+                                                                   (const C2<double> *)x, d_jd64.p, d_rd64.p);
+  ++launch_count;
+  NOSH_CUDA(cudaGetLastError());
+  reg_g = g;
+  jac_ready = reg_ready = true;
+  jd32_ok = rd32_ok = false;
+}
+
+void NlsImpl::reg_rebuild(const double *x, double g, double mu, bool want32) {
+  if (!(keo_mu == mu)) keo_refill(mu);
+  reg_diag_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, g, (const C2<double> *)x, d_rd64.p,
+                                                       want32 ? d_rd32.p : nullptr);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
   reg_g = g;
   reg_ready = true;
+  rd32_ok = want32;
+}
+
+void NlsImpl::ensure_diag32() {
+  if (jac_ready && !jd32_ok) {
+    launch_f64_to_f32(d_jd64.p, d_jd32.p, 3 * N, stream);
+    jd32_ok = true;
+  }
+  if (reg_ready && !rd32_ok) {
+    launch_f64_to_f32(d_rd64.p, d_rd32.p, 3 * N, stream);
+    rd32_ok = true;
+  }
 }
 
 template <>
@@ -944,25 +962,21 @@ void NlsImpl::reg_apply<float>(const float *x, float *y) {
 
 double NlsImpl::energy(const double *psi) {
   energy_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, mesh->d_cv.p, (const C2<double> *)psi,
-                                                     red.partials.p, red.counter.p, red.out.p);
+                                                     red.partials.p, red.counter.p, red.host);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
-  double e = 0.0;
-  red.out.download(&e, 1, stream);
   sync();
-  return e / cv_sum;
+  return red.host[0] / cv_sum;
 }
 
 double NlsImpl::inner_product(const double *phi, const double *psi) {
   inner_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, mesh->d_cv.p, (const C2<double> *)phi,
                                                     (const C2<double> *)psi, red.partials.p,
-                                                    red.counter.p, red.out.p);
+                                                    red.counter.p, red.host);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
-  double e = 0.0;
-  red.out.download(&e, 1, stream);
   sync();
-  return e / cv_sum;
+  return red.host[0] / cv_sum;
 }
 
 void NlsImpl::export_values(const C2<double> *offdiag, const double *diag, double *out) {

@@ -25,29 +25,27 @@ using namespace dev;
 
 namespace {
 
+// The start of a solve, in one pass: r0 = r1 = scale rhs in the Krylov
+// precision, x = w0 = w1 = w2 = 0 (the copies and memsets it replaces were six
+// nodes of a few us each).
 template <typename T>
-__global__ void dot_kernel(int64_t n, const T *__restrict__ a, const T *__restrict__ b,
-                           double *partials, unsigned *counter, double *out) {
-  double v = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  // two elements per pass, their loads issued first (the per-thread order
-  // stays i, i + stride, ...)
-  for (; i + stride < n; i += 2 * stride) {
-    const T a0 = a[i], b0 = b[i], a1 = a[i + stride], b1 = b[i + stride];
-    v += (double)a0 * (double)b0;
-    v += (double)a1 * (double)b1;
+__global__ void minres_begin(int64_t n, const MinresArgs *args, T *__restrict__ r0, T *__restrict__ r1,
+                             T *__restrict__ x, T *__restrict__ w0, T *__restrict__ w1, T *__restrict__ w2) {
+  const double *rhs = args->rhs;
+  const double scale = args->scale;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const T b = (T)(scale * rhs[i]);
+    r0[i] = b;
+    r1[i] = b;
+    x[i] = w0[i] = w1[i] = w2[i] = (T)0;
   }
-  for (; i < n; i += stride) v += (double)a[i] * (double)b[i];
-  grid_reduce(v, partials, counter, out);
 }
 
-// params = {rtol, maxit} (device memory, written before each solve so the
-// captured prologue graph stays valid)
-__global__ void minres_init(MinresScalars *s, const double *params) {
-  const double rz = s->rz;
-  s->rtol = params[0];
-  s->maxit = (int)params[1];
+// The recurrence's initial state from <b, M b>.
+__device__ __forceinline__ void minres_init(MinresScalars *s, double rz, double rtol, int maxit) {
+  s->rz = rz;
+  s->rtol = rtol;
+  s->maxit = maxit;
   s->itn = 0;
   s->flag = 0;
   s->done = 0;
@@ -75,6 +73,38 @@ __global__ void minres_init(MinresScalars *s, const double *params) {
   s->ibeta = rsqrt(rz);
   s->phibar = s->beta1;
   if (rz == 0.0) s->done = 2;  // b == 0: x = 0
+}
+
+// <b, M b>, then the recurrence's initial state
+template <typename T>
+__global__ void dot_init(int64_t n, const T *__restrict__ a, const T *__restrict__ b, double *partials,
+                         unsigned *counter, MinresScalars *s, const MinresArgs *args) {
+  double v = 0.0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  // two elements per pass, their loads issued first (the per-thread order
+  // stays i, i + stride, ...)
+  for (; i + stride < n; i += 2 * stride) {
+    const T a0 = a[i], b0 = b[i], a1 = a[i + stride], b1 = b[i + stride];
+    v += (double)a0 * (double)b0;
+    v += (double)a1 * (double)b1;
+  }
+  for (; i < n; i += stride) v += (double)a[i] * (double)b[i];
+  double total = 0.0;
+  if (grid_reduce(v, partials, counter, &s->rz, &total)) minres_init(s, total, args->rtol, args->maxit);
+}
+
+// the host's view of the recurrence (pinned memory), before a poll
+__global__ void minres_report(const MinresScalars *s, const int *amg_err, MinresReport *out) {
+  MinresReport r;
+  r.beta1 = s->beta1;
+  r.phibar = s->phibar;
+  r.itn = s->itn;
+  r.done = s->done;
+  r.flag = s->flag;
+  r.wx_pending = s->wx_pending;
+  r.amg_err = *amg_err;
+  *out = r;
 }
 
 // u = J z and <z, u>, with the deferred w/x update of the previous Lanczos
@@ -166,10 +196,8 @@ template <typename T>
 Minres<T>::Minres(NlsImpl &nls) : s(nls), n2(2 * nls.N) {
   for (DevBuf<T> *b : {&r[0], &r[1], &z[0], &z[1], &w[0], &w[1], &w[2], &u, &x}) b->alloc(n2);
   sc.alloc(1);
-  NOSH_CUDA(cudaMallocHost(&h_sc, sizeof(MinresScalars)));
-  NOSH_CUDA(cudaMallocHost(&h_err, 2 * sizeof(int)));
-  NOSH_CUDA(cudaMallocHost(&h_params, 2 * sizeof(double)));
-  params.alloc(2);
+  NOSH_CUDA(cudaMallocHost(&h_rep, sizeof(MinresReport)));
+  NOSH_CUDA(cudaMallocHost(&h_args, sizeof(MinresArgs)));
   NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, JacMinresOp<T>>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
 }
@@ -182,7 +210,6 @@ void Minres<T>::drop_graphs() {
   }
   if (pro_exec) cudaGraphExecDestroy(pro_exec);
   pro_exec = nullptr;
-  pro_b = nullptr;
   for (auto &part : part_ev)
     for (auto &it : part)
       for (auto &v : it) KernelTimer::release(v);
@@ -192,9 +219,8 @@ void Minres<T>::drop_graphs() {
 template <typename T>
 Minres<T>::~Minres() {
   drop_graphs();
-  if (h_params) cudaFreeHost(h_params);
-  if (h_sc) cudaFreeHost(h_sc);
-  if (h_err) cudaFreeHost(h_err);
+  if (h_rep) cudaFreeHost(h_rep);
+  if (h_args) cudaFreeHost(h_args);
 }
 
 // Iteration j of a chunk.  Buffer roles rotate with period 2 (z, r) and 3
@@ -239,10 +265,8 @@ void Minres<T>::wx_final(int j) {
 }
 
 template <typename T>
-int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &rel_res) {
+int Minres<T>::solve(const double *rhs, double scale, double rtol, int maxit, int &status, double &rel_res) {
   cudaStream_t st = s.stream;
-  const int G = vec_grid(n2);
-  const size_t bytes = n2 * sizeof(T);
   MinresScalars *d = sc.p;
   // with kernel timing on, the graphs carry event-record nodes around the
   // timed launches: captured anew when timing is switched
@@ -252,43 +276,28 @@ int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &re
     drop_graphs();
     graphs_timed = timed;
   }
-  h_params[0] = rtol;
-  h_params[1] = (double)maxit;
-  NOSH_CUDA(cudaMemcpyAsync(params.p, h_params, 2 * sizeof(double), cudaMemcpyHostToDevice, st));
-  // prologue: r_old = r_cur = b, x = w = 0, z = M b, beta1^2 = <b, z>; one
-  // captured graph for a given right-hand-side buffer
-  auto prologue = [&] {
-    NOSH_CUDA(cudaMemcpyAsync(r[0].p, b, bytes, cudaMemcpyDeviceToDevice, st));
-    NOSH_CUDA(cudaMemcpyAsync(r[1].p, b, bytes, cudaMemcpyDeviceToDevice, st));
-    for (DevBuf<T> *q : {&x, &w[0], &w[1], &w[2]}) NOSH_CUDA(cudaMemsetAsync(q->p, 0, bytes, st));
+  // (the previous solve has been waited for: the kernels read the arguments
+  // from here)
+  *h_args = MinresArgs{rhs, scale, rtol, maxit};
+  // prologue: r_old = r_cur = b, x = w = 0, z = M b, beta1^2 = <b, z>
+  if (!pro_exec) {
+    for (auto &v : pro_ev) KernelTimer::release(v);
+    cudaGraph_t g;
+    const int64_t before = s.launch_count;
+    NOSH_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    minres_begin<T><<<vec_grid(n2), 256, 0, st>>>(n2, h_args, r[0].p, r[1].p, x.p, w[0].p, w[1].p, w[2].p);
     s.amg->apply<T>(r[1].p, z[0].p);
-    dot_kernel<T><<<reduce_grid(n2), 256, 0, st>>>(n2, r[1].p, z[0].p, s.red.partials.p, s.red.counter.p,
-                                                    &d->rz);
-    minres_init<<<1, 1, 0, st>>>(d, params.p);
+    dot_init<T><<<reduce_grid(n2), 256, 0, st>>>(n2, r[1].p, z[0].p, s.red.partials.p, s.red.counter.p, d, h_args);
     s.launch_count += 2;
-  };
-  {
-    if (!pro_exec || pro_b != b) {
-      if (pro_exec) {
-        NOSH_CUDA(cudaStreamSynchronize(st));
-        NOSH_CUDA(cudaGraphExecDestroy(pro_exec));
-      }
-      for (auto &v : pro_ev) KernelTimer::release(v);
-      cudaGraph_t g;
-      const int64_t before = s.launch_count;
-      NOSH_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      prologue();
-      NOSH_CUDA(cudaStreamEndCapture(st, &g));
-      for (int k = 0; k < 2; k++) pro_ev[k] = s.timers[k].take();
-      pro_kernels = s.launch_count - before;
-      s.launch_count = before;
-      NOSH_CUDA(cudaGraphInstantiate(&pro_exec, g, 0));
-      NOSH_CUDA(cudaGraphDestroy(g));
-      pro_b = b;
-    }
-    NOSH_CUDA(cudaGraphLaunch(pro_exec, st));
-    s.launch_count += pro_kernels;
+    NOSH_CUDA(cudaStreamEndCapture(st, &g));
+    for (int k = 0; k < 2; k++) pro_ev[k] = s.timers[k].take();
+    pro_kernels = s.launch_count - before;
+    s.launch_count = before;
+    NOSH_CUDA(cudaGraphInstantiate(&pro_exec, g, 0));
+    NOSH_CUDA(cudaGraphDestroy(g));
   }
+  NOSH_CUDA(cudaGraphLaunch(pro_exec, st));
+  s.launch_count += pro_kernels;
   NOSH_CUDA(cudaGetLastError());
   if (!part_exec[0]) {
     for (int h = 0; h < kParts; h++) {
@@ -331,10 +340,8 @@ int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &re
     for (int q = 0; q < batch; q++, h = (h + 1) % kParts, it += kPart) launch_part(h);
     batch = 1;
     NOSH_CUDA(cudaGetLastError());
-    NOSH_CUDA(cudaMemcpyAsync(h_sc, d, sizeof(MinresScalars), cudaMemcpyDeviceToHost, st));
-    NOSH_CUDA(cudaMemcpyAsync(h_err, s.amg->error_flag_ptr(), sizeof(int), cudaMemcpyDeviceToHost, st));
-    NOSH_CUDA(cudaMemcpyAsync(h_err + 1, s.red.counter.p + kStageErrorSlot, sizeof(int), cudaMemcpyDeviceToHost,
-                              st));
+    minres_report<<<1, 1, 0, st>>>(d, s.amg->error_flag_ptr(), h_rep);
+    ++s.launch_count;
     NOSH_CUDA(cudaStreamSynchronize(st));
     if (timed) {
       // the launches that did work: iteration g's Jacobian apply runs unless
@@ -344,7 +351,7 @@ int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &re
       if (first)
         for (int k = 0; k < 2; k++)
           for (const auto &p : pro_ev[k]) s.timers[k].harvest(p);
-      const int jac_end = h_sc->itn + (h_sc->done ? 1 : 0);
+      const int jac_end = h_rep->itn + (h_rep->done ? 1 : 0);
       // the solve's first Jacobian apply has no deferred w/x update to apply
       const double jac_first = s.spmv_bytes(2 * sizeof(T), 7 * sizeof(T));
       for (int jj = 0; jj < kPart; jj++) {
@@ -352,28 +359,28 @@ int Minres<T>::solve(const T *b, double rtol, int maxit, int &status, double &re
         if (g < jac_end)
           for (const auto &p : part_ev[h0][jj][NOSH_KERNEL_JACOBIAN])
             s.timers[NOSH_KERNEL_JACOBIAN].harvest(p, g == 0 ? jac_first : -1.0);
-        if (g < h_sc->itn)
+        if (g < h_rep->itn)
           for (const auto &p : part_ev[h0][jj][NOSH_KERNEL_SMOOTHER]) s.timers[NOSH_KERNEL_SMOOTHER].harvest(p);
       }
     }
     first = false;
-    if (h_sc->done || h_err[1] != 0 || it >= maxit + kChunk) break;
+    if (h_rep->done || *s.h_stage_err != 0 || it >= maxit + kChunk) break;
   }
   // converged on the last issued iteration: its w/x update is still due
   // (h is the next part; the last issued iteration ends the part before it)
-  if (h_sc->wx_pending) wx_final(((h + kParts - 1) % kParts + 1) * kPart - 1);
-  if (h_err[1] != 0) s.stage_failure();
-  if (h_err[0] != 0) {
+  if (h_rep->wx_pending) wx_final(((h + kParts - 1) % kParts + 1) * kPart - 1);
+  if (*s.h_stage_err != 0) s.stage_failure();
+  if (h_rep->amg_err != 0) {
     s.amg->clear_error();
     throw Error(NOSH_ERR_BREAKDOWN,
                 "the regularised KEO or a level of its AMG hierarchy is not positive definite "
                 "(a diagonal block or a coarsest pivot)");
   }
-  status = h_sc->flag;
-  rel_res = h_sc->beta1 > 0 ? h_sc->phibar / h_sc->beta1 : 0.0;
-  last_its = h_sc->itn;
+  status = h_rep->flag;
+  rel_res = h_rep->beta1 > 0 ? h_rep->phibar / h_rep->beta1 : 0.0;
+  last_its = h_rep->itn;
   last_rel = rel_res;
-  return h_sc->itn;
+  return h_rep->itn;
 }
 
 template struct Minres<float>;
@@ -412,11 +419,6 @@ __global__ void secant_kernel(int64_t n, const double *__restrict__ c, double r,
   }
 }
 
-template <typename T>
-__global__ void cast_to(int64_t n, const double *__restrict__ a, T *__restrict__ b) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    b[i] = (T)a[i];
-}
 template <typename T>
 __global__ void cast_from(int64_t n, const T *__restrict__ a, double *__restrict__ b) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -481,23 +483,19 @@ NewtonState &state_of(NlsImpl &s) {
 
 double residual_norm(NlsImpl &s, const double *psi, double g, double mu, double *f) {
   s.compute_f64(psi, g, mu, f, 0);
-  double n2 = 0.0;
-  s.red.out.download(&n2, 1, s.stream);
   s.sync();
-  return std::sqrt(n2);
+  return std::sqrt(s.red.host[0]);
 }
 
 // The same for ns.psi, keeping the off-diagonal sums of K psi in ns.soff
 static double residual_norm_kept(NlsImpl &s, NewtonState &ns, double g, double mu) {
   ns.ensure_soff(2 * s.N);
   s.compute_f64(ns.psi.p, g, mu, ns.f.p, 0, ns.soff.p);
-  double n2 = 0.0;
-  s.red.out.download(&n2, 1, s.stream);
   s.sync();
   ns.soff_valid = true;
   ns.soff_fresh = true;
   ns.soff_mu = mu;
-  return std::sqrt(n2);
+  return std::sqrt(s.red.host[0]);
 }
 
 // psi += dx (FP64 += FP32), and ||dx||_2^2 into *out: the per-thread sums
@@ -547,12 +545,11 @@ static double residual_after_update(NlsImpl &s, NewtonState &ns, const T *dx, do
     return residual_norm_kept(s, ns, g, mu);
   }
   axpy_cast_norm<T><<<vec_grid(n2), 256, 0, s.stream>>>(n2, dx, ns.psi.p, s.red.partials.p, s.red.counter.p,
-                                                        s.red.out.p + 1);
+                                                        s.red.host + 1);
   ++s.launch_count;
   s.residual_update(ns.psi.p, (const float *)dx, g, mu, ns.f.p, ns.soff.p);
-  double sq[2] = {0.0, 0.0};  // ||F||^2, ||dx||^2
-  s.red.out.download(sq, 2, s.stream);
   s.sync();
+  const double sq[2] = {s.red.host[0], s.red.host[1]};  // ||F||^2, ||dx||^2
   const double fn = std::sqrt(sq[0]);
   const double e = 3.0 * (s.max_row_nnz() + 1) * std::ldexp(1.0, -24) * s.keo_abs_rowmax() * std::sqrt(sq[1]);
   if (fn <= tol - e || (fn > tol + e && e <= 0.01 * fn)) {
@@ -584,11 +581,10 @@ static void rebuild_operators(NlsImpl &s, const double *psi, double g, double mu
     // the preconditioner's one-time setup (the host aggregation's strength
     // test) reads the FP64 regularised diagonal, which the mixed rebuild
     // does not write: fill it at this state first
-    if (!s.amg) s.reg_rebuild(psi, g, mu);
+    if (!s.amg) s.reg_rebuild(psi, g, mu, false);
     s.operators32_rebuild(psi, g, mu);
   } else {
-    s.jac_rebuild(psi, g, mu);
-    s.reg_rebuild(psi, g, mu);
+    s.operators64_rebuild(psi, g, mu);
   }
   ensure_preconditioner(s).refresh<T>();
 }
@@ -605,13 +601,11 @@ static Minres<T> &minres_of(NlsImpl &s, NewtonState &ns);
 template <>
 Minres<float> &minres_of<float>(NlsImpl &s, NewtonState &ns) {
   if (!ns.m32) ns.m32.reset(new Minres<float>(s));
-  if (ns.b32.n < (size_t)(2 * s.N)) ns.b32.alloc(2 * s.N);
   return *ns.m32;
 }
 template <>
 Minres<double> &minres_of<double>(NlsImpl &s, NewtonState &ns) {
   if (!ns.m64) ns.m64.reset(new Minres<double>(s));
-  if (ns.b64.n < (size_t)(2 * s.N)) ns.b64.alloc(2 * s.N);
   return *ns.m64;
 }
 template <typename T> static DevBuf<T> &rhs_of(NewtonState &ns);
@@ -722,7 +716,6 @@ static void newton_loop(NlsImpl &s, NewtonState &ns, double g, double mu,
     return;
   }
   Minres<T> &mr = minres_of<T>(s, ns);
-  DevBuf<T> &b = rhs_of<T>(ns);
   const int64_t n2 = 2 * s.N;
   const int G = vec_grid(n2);
   double fn = st.f_norm0, fn_prev = fn;
@@ -735,12 +728,10 @@ static void newton_loop(NlsImpl &s, NewtonState &ns, double g, double mu,
     // batched systems: converged ones get a zero right-hand side (their
     // Newton update is zero: the Jacobian is block diagonal)
     if (!s.sys_off.empty()) s.mask_converged(ns.f.p, opt.tol);
-    neg_cast<T><<<G, 256, 0, s.stream>>>(n2, ns.f.p, b.p);
-    ++s.launch_count;
     const double eta = forcing_term(opt, it, fn, fn_prev, sizeof(T) == 4, s.forcing_aim);
     int status = 0;
     double rel = 0.0;
-    const int its = mr.solve(b.p, eta, opt.max_krylov, status, rel);
+    const int its = mr.solve(ns.f.p, -1.0, eta, opt.max_krylov, status, rel);
     st.krylov_iters += its;
     if (status == NOSH_ERR_NAN || status == NOSH_ERR_BREAKDOWN) {
       // the hierarchy's coarse operators are rebuilt in full next time, so
@@ -816,16 +807,13 @@ static void tangent_predict(NlsImpl &s, NewtonState &ns, double g, double mu_cur
   // dx/dmu = -J^-1 dF/dmu at (x, mu_cur) (LOCA tangent predictor; dF/dmu is
   // DkeoDP x, src/model_evaluator_nls.cpp:632-695)
   Minres<T> &mr = minres_of<T>(s, ns);
-  DevBuf<T> &b = rhs_of<T>(ns);
   const int64_t n2 = 2 * s.N;
   const int G = vec_grid(n2);
   rebuild_operators<T>(s, ns.xc.p, g, mu_cur);
   s.dfdp64(ns.xc.p, g, mu_cur, 1, ns.tmp.p);
-  neg_cast<T><<<G, 256, 0, s.stream>>>(n2, ns.tmp.p, b.p);
-  ++s.launch_count;
   int status = 0;
   double rel = 0.0;
-  st.krylov_iters += mr.solve(b.p, sizeof(T) == 4 ? 1e-5 : 1e-8, opt.max_krylov, status, rel);
+  st.krylov_iters += mr.solve(ns.tmp.p, -1.0, sizeof(T) == 4 ? 1e-5 : 1e-8, opt.max_krylov, status, rel);
   NOSH_CHECK(status != NOSH_ERR_NAN && status != NOSH_ERR_BREAKDOWN, status, "tangent solve failed");
   axpy_to<T><<<G, 256, 0, s.stream>>>(n2, dmu, mr.x.p, ns.xc.p, ns.psi.p);
   ++s.launch_count;
@@ -838,14 +826,11 @@ template <typename T>
 static int linear_solve_t(NlsImpl &s, NewtonState &ns, const double *rhs, double *x, double g, double mu,
                           double rtol, int maxit, bool rebuild, int &status) {
   Minres<T> &mr = minres_of<T>(s, ns);
-  DevBuf<T> &b = rhs_of<T>(ns);
   const int64_t n2 = 2 * s.N;
   const int G = vec_grid(n2);
   if (rebuild) rebuild_operators<T>(s, ns.psi.p, g, mu);
-  cast_to<T><<<G, 256, 0, s.stream>>>(n2, rhs, b.p);
-  ++s.launch_count;
   double rel = 0.0;
-  const int its = mr.solve(b.p, rtol, maxit, status, rel);
+  const int its = mr.solve(rhs, 1.0, rtol, maxit, status, rel);
   cast_from<T><<<G, 256, 0, s.stream>>>(n2, mr.x.p, x);
   ++s.launch_count;
   NOSH_CUDA(cudaGetLastError());

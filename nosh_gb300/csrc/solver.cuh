@@ -7,6 +7,17 @@
 
 namespace nosh {
 
+// The recurrence's state as the host polls it, and a solve's arguments.
+struct MinresReport {
+  double beta1, phibar;
+  int itn, done, flag, wx_pending, amg_err;
+};
+struct MinresArgs {
+  const double *rhs;
+  double scale, rtol;
+  int maxit;
+};
+
 // Preconditioned MINRES (Paige-Saunders) on J dx = b with the AMG V-cycle as
 // the SPD preconditioner, vectors in T, scalars in FP64 (minres_state.cuh).
 // Buffer roles repeat every kChunk iterations; the chunk is captured once as
@@ -24,16 +35,15 @@ struct Minres {
   int64_t n2;  // real length (2N)
   DevBuf<T> r[2], z[2], w[3], u, x;
   DevBuf<MinresScalars> sc;
-  MinresScalars *h_sc = nullptr;  // pinned host mirror
-  int *h_err = nullptr;
+  // pinned host memory that the kernels read and write directly: the
+  // recurrence's state at a poll (minres_report), and the solve's arguments,
+  // through which right-hand side, tolerance and limit reach the captured
+  // prologue (initial V-cycle and recurrence set-up)
+  MinresReport *h_rep = nullptr;
+  MinresArgs *h_args = nullptr;
   cudaGraphExec_t part_exec[kParts] = {};
-  // the captured prologue (initial V-cycle and recurrence set-up) for the
-  // right-hand side pro_b; rtol and maxit reach it through `params`
   cudaGraphExec_t pro_exec = nullptr;
-  const T *pro_b = nullptr;
   int64_t pro_kernels = 0;
-  DevBuf<double> params;
-  double *h_params = nullptr;
   int64_t part_kernels[kParts] = {};
   int last_its = 0;  // iterations of the previous solve, and where it ended
   double last_rel = 0.0;
@@ -46,8 +56,9 @@ struct Minres {
   std::vector<KernelTimer::Pair> pro_ev[2];
   explicit Minres(NlsImpl &nls);
   ~Minres();
-  // b: device vector of T (2N); returns iterations; x holds the solution
-  int solve(const T *b, double rtol, int maxit, int &status, double &rel_res);
+  // right-hand side scale * rhs (device, 2N FP64); returns iterations; x
+  // holds the solution
+  int solve(const double *rhs, double scale, double rtol, int maxit, int &status, double &rel_res);
 
  private:
   void iteration(int j);   // issue iteration j (0..kChunk-1) of a chunk

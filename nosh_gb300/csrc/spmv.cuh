@@ -346,9 +346,14 @@ template <typename T>
 __host__ __device__ constexpr int stage_limit() {
   return (int)((48 * 1024) / (sizeof(int32_t) + sizeof(C2<T>))) & ~3;
 }
-// Slot of the per-stream reduction counters that records a staging copy
-// that never completed (checked by the host at its next synchronisation).
-constexpr int kStageErrorSlot = 15;
+// Slots of the reduction counters that hold the address of the host's failure
+// word (pinned memory, read after every synchronisation): a bounded wait that
+// gave up sets it.
+constexpr int kStageErrorSlot = 12;
+__device__ __forceinline__ void stage_fail(const unsigned *counter) {
+  unsigned *const *p = reinterpret_cast<unsigned *const *>(counter + kStageErrorSlot);
+  if (*p) **reinterpret_cast<volatile unsigned *const *>(p) = 1u;
+}
 // Slot holding a diagnostic override of the staging-wait bound: 0 = the
 // default kStageWaitPolls, v > 0 = v - 1 polls.  Read only by launches that
 // stage (cap > 0).
@@ -408,7 +413,7 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     if (!skip && threadIdx.x == 0 && rb0 < rb_end) {
       int ks, n;
       range(rb0, ks, n);
-      if (n > 0 && n <= cap && !mbar_wait(&bar[0], 0u)) atomicOr(counter + kStageErrorSlot, 1u);
+      if (n > 0 && n <= cap && !mbar_wait(&bar[0], 0u)) stage_fail(counter);
     }
     return;
   }
@@ -497,7 +502,7 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     // block's and the next one's) a last wait at the default bound, so no
     // copy lands in shared memory after the CTA has left, and leave (the
     // results of this launch are invalid)
-    if (threadIdx.x == 0) atomicOr(counter + kStageErrorSlot, 1u);
+    if (threadIdx.x == 0) stage_fail(counter);
     if (cur_staged) mbar_wait(&bar[stage], parity[stage]);
     if (next_staged) mbar_wait(&bar[stage ^ 1], parity[stage ^ 1]);
     return;
