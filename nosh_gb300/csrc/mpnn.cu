@@ -32,6 +32,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -74,13 +75,6 @@ struct Layout {
   }
 };
 
-// ------------------------------------------------ tensor-core node GEMM
-// out[r, 0:64] (=, +=) [in0[r, 0:K0], in1[r, 0:K1]] @ W, W stored as
-// Wt[64][K] BF16 (transposed, K = K0 + K1 <= 128, K0, K1 multiples of 16
-// or K1 = 0).  One warp per 16 rows, 4 warps per CTA.  Used by the backward
-// pass (the forward runs in the fused layer kernels below).
-enum Epi { EPI_LINEAR = 0, EPI_ACCUM = 1 };
-
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t *>(&v);
@@ -95,93 +89,27 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(128) gemm64_kernel(int64_t n, const float *__restrict__ in0, int K0,
-                                                     const float *__restrict__ in1, int K1,
-                                                     const __nv_bfloat16 *__restrict__ Wt,
-                                                     float *__restrict__ out) {
-  constexpr int KMAX = 128, LD = KMAX + 8;  // padded rows: conflict-free
-  __shared__ __align__(16) __nv_bfloat16 sW[H * LD];
-  const int K = K0 + K1;
-  for (int q = threadIdx.x; q < H * K; q += blockDim.x) sW[(q / K) * LD + (q % K)] = Wt[q];
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, tig = lane & 3;
-  const int64_t r0 = (blockIdx.x * 4 + warp) * 16;
-  if (r0 >= n) return;
-  const int64_t ra = r0 + g, rb = r0 + g + 8;
-  float acc[8][4];
-#pragma unroll
-  for (int t = 0; t < 8; t++) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-  for (int kk = 0; kk < K; kk += 16) {
-    const float *src = kk < K0 ? in0 : in1;
-    const int ld = kk < K0 ? K0 : K1, kc = kk < K0 ? kk : kk - K0;
-    float2 a[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    if (ra < n) {
-      a[0] = *reinterpret_cast<const float2 *>(src + ra * ld + kc + tig * 2);
-      a[2] = *reinterpret_cast<const float2 *>(src + ra * ld + kc + tig * 2 + 8);
-    }
-    if (rb < n) {
-      a[1] = *reinterpret_cast<const float2 *>(src + rb * ld + kc + tig * 2);
-      a[3] = *reinterpret_cast<const float2 *>(src + rb * ld + kc + tig * 2 + 8);
-    }
-    const uint32_t a0 = pack_bf16(a[0].x, a[0].y), a1 = pack_bf16(a[1].x, a[1].y);
-    const uint32_t a2 = pack_bf16(a[2].x, a[2].y), a3 = pack_bf16(a[3].x, a[3].y);
-#pragma unroll
-    for (int t = 0; t < 8; t++) {
-      const __nv_bfloat16 *w = sW + (t * 8 + g) * LD + kk + tig * 2;
-      const uint32_t b0 = *reinterpret_cast<const uint32_t *>(w);
-      const uint32_t b1 = *reinterpret_cast<const uint32_t *>(w + 8);
-      mma_bf16(acc[t], a0, a1, a2, a3, b0, b1);
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-    const int c = t * 8 + tig * 2;
-#pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int64_t r = half ? rb : ra;
-      if (r >= n) continue;
-      const float v0 = acc[t][2 * half], v1 = acc[t][2 * half + 1];
-      float2 *o = reinterpret_cast<float2 *>(out + r * H + c);
-      if (EPI == EPI_LINEAR) {
-        *o = make_float2(v0, v1);
-      } else {
-        const float2 p = *o;
-        *o = make_float2(p.x + v0, p.y + v1);
-      }
-    }
-  }
-}
-
-// forward operand: W (K x ncols, row-major FP32 inside the parameter
-// vector) -> Wt[64][K] BF16 with Wt[n][k] = W[k][col0 + n]
-__global__ void to_bf16_t(const float *__restrict__ W, int K, int ncols, int col0, __nv_bfloat16 *__restrict__ Wt) {
+// All BF16 operands from the FP32 parameters, one launch: segment q writes
+// rows x K values dst[n * K + k] = src[k * sk + n * sn] (zero for k >= kv):
+// the forward operands transposed (W^T row by row), the backward ones as
+// stored.  (A launch per matrix made 22 of about 2.5 us each an optimiser step.)
+struct CastSeg {
+  int64_t src, dst;
+  int rows, K, kv, sk, sn;
+};
+constexpr int kCastSegs = 1 + 7 * LAYERS;
+struct CastPlan {
+  CastSeg seg[kCastSegs];
+};
+__global__ void cast_operands(CastPlan plan, const float *__restrict__ P, __nv_bfloat16 *__restrict__ wt) {
+  const CastSeg s = plan.seg[blockIdx.y];
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= H * K) return;
-  const int n = q / K, k = q % K;
-  Wt[q] = __float2bfloat16(W[(int64_t)k * ncols + col0 + n]);
+  if (q >= s.rows * s.K) return;
+  const int n = q / s.K, k = q % s.K;
+  wt[s.dst + q] = __float2bfloat16(k < s.kv ? P[s.src + (int64_t)k * s.sk + (int64_t)n * s.sn] : 0.f);
 }
 
-// encoder operand: Wt[n][k] = W[k][n] for k < 8, zero for the padding k < 16
-__global__ void enc_to_bf16(const float *__restrict__ W, __nv_bfloat16 *__restrict__ Wt) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= H * 16) return;
-  const int n = q / 16, k = q % 16;
-  Wt[q] = __float2bfloat16(k < FX ? W[k * H + n] : 0.f);
-}
-
-__global__ void to_bf16_rows(const float *__restrict__ W, int rows, int row0, __nv_bfloat16 *__restrict__ Wt) {
-  // Wt[n][k] = W[row0 + n][k] for a row-major [* x 64] W: the operand of
-  // dIn[:, row0:row0+64] = dOut @ W[row0:row0+64, :]^T
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= H * H) return;
-  const int n = q / H, k = q % H;
-  Wt[q] = __float2bfloat16(W[(int64_t)(row0 + n) * H + k]);
-  (void)rows;
-}
-
-// ------------------------------------------------- fused forward layers
+// ------------------------------------------------- forward layers
 // A CTA of 4 warps owns tiles of 64 consecutive rows (16 per warp); each CTA
 // walks a contiguous range of tiles, so the neighbour rows a tile gathers
 // (mesh-ordered graphs: bands at fixed index offsets) are largely the rows
@@ -193,12 +121,8 @@ __global__ void to_bf16_rows(const float *__restrict__ W, int rows, int row0, __
 constexpr int TILE = 64;
 constexpr int LDU = 2 * H + 8;  // smem row strides (BF16), padded: conflict-free fragment loads
 constexpr int LDAB = H + 8;
-constexpr int LDM = H + 8;
 constexpr int LDE = 16 + 8;
-constexpr size_t kLayerSmem = (size_t)(H * LDU + 2 * H * LDAB + 4 * 16 * LDM) * sizeof(__nv_bfloat16) +
-                              4 * H * sizeof(float);
 constexpr size_t kEncSmem = (size_t)(H * LDE + 2 * H * LDAB) * sizeof(__nv_bfloat16);
-// the update-only layer (M from global memory): no M staging
 constexpr size_t kUpdateSmem = (size_t)(H * LDU + 2 * H * LDAB) * sizeof(__nv_bfloat16) + 4 * H * sizeof(float);
 
 __device__ __forceinline__ void frag_from_c(const float (&v)[8][4], int kk, uint32_t &a0, uint32_t &a1,
@@ -392,9 +316,10 @@ __device__ __forceinline__ void aggregate_row(int64_t r, int64_t n, const int32_
   m[3] = m23.y;
 }
 
-// Inference split of a layer: the aggregation alone, at high occupancy (the
-// fused layer holds 12 warps per SM and waits on the gathers), writing M in
-// BF16 (the update GEMM's operand, rounded as the fused layer rounds it).
+// A layer's aggregation alone, at high occupancy, writing M in BF16 (the
+// operand of the update GEMM and of the weight gradient, which round it to
+// that anyway).  One kernel for aggregation and update held 12 warps per SM
+// and waited on the gathers: 115 us a layer at 48^3 against 42 + 30 us.
 __global__ void __launch_bounds__(256, 4) mp_aggregate_kernel(int64_t n, const int32_t *__restrict__ rp,
                                                            const int32_t *__restrict__ ci,
                                                            const float4 *__restrict__ ef,
@@ -426,37 +351,26 @@ __global__ void __launch_bounds__(256, 4) mp_aggregate_kernel(int64_t n, const i
   }
 }
 
-// One message-passing layer:
-//   M_i = sum_j relu(A_i + B_j + e_ij W_c + b_m)          (FP32 sums)
+// The update of one message-passing layer (M from mp_aggregate_kernel):
 //   R   = relu(bf16([h, M]) @ bf16(W_u) + b_u),  h' = h + R
 // then, for all but the last layer, the next layer's A, B from h'; the last
 // layer writes per-CTA column sums of h' (the mean-pool partials) instead of
-// h'.  TRAIN also stores M and R (FP32) for the backward pass.  PRE_M (the
-// inference split): M comes from mp_aggregate_kernel in BF16 (Mb) and the
-// kernel is the update GEMM alone.
-template <bool TRAIN, bool LAST, bool PRE_M>
-__global__ void __launch_bounds__(128, 3) mp_layer_kernel(
-    int64_t n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const float4 *__restrict__ ef,
-    const float *__restrict__ h, const __half *__restrict__ A, const __half *__restrict__ B,
-    const float *__restrict__ Wc, const float *__restrict__ bm, const __nv_bfloat16 *__restrict__ Wu,
-    const float *__restrict__ bu, const __nv_bfloat16 *__restrict__ Wab, float *__restrict__ h_out,
-    __half *__restrict__ A_out, __half *__restrict__ B_out, float *__restrict__ M_out,
-    float *__restrict__ R_out, float *__restrict__ pool, const __nv_bfloat16 *__restrict__ Mb) {
-  static_assert(!(TRAIN && PRE_M), "training runs the fused layer");
+// h'.  TRAIN also stores R's sign (gate): all the backward pass reads of it,
+// 8 bytes a row instead of 256; bit 2 t + b of word q is column 8 t + 2 q + b.
+template <bool TRAIN, bool LAST>
+__global__ void __launch_bounds__(128, 3)
+    mp_update_kernel(int64_t n, const float *__restrict__ h, const __nv_bfloat16 *__restrict__ Mb,
+                     const __nv_bfloat16 *__restrict__ Wu, const float *__restrict__ bu,
+                     const __nv_bfloat16 *__restrict__ Wab, float *__restrict__ h_out, __half *__restrict__ A_out,
+                     __half *__restrict__ B_out, uint16_t *__restrict__ gate, float *__restrict__ pool) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16 *sWu = reinterpret_cast<__nv_bfloat16 *>(smem_raw);
   __nv_bfloat16 *sWab = sWu + H * LDU;
-  __nv_bfloat16 *sM = sWab + 2 * H * LDAB;
-  float *sPool = reinterpret_cast<float *>(PRE_M ? sM : sM + 4 * 16 * LDM);
+  float *sPool = reinterpret_cast<float *>(sWab + 2 * H * LDAB);
   stage_w(sWu, Wu, H, 2 * H, LDU);
   if (!LAST) stage_w(sWab, Wab, 2 * H, H, LDAB);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  __nv_bfloat16 *sMw = sM + warp * 16 * LDM;
-  // aggregation: a half-warp per row, 4 channels per lane
-  const int hl = lane & 15, half = lane >> 4, c4 = hl * 4;
-  MsgConst mk;
-  if (!PRE_M) msg_const(Wc, bm, c4, mk);
   float psum[8][2];
 #pragma unroll
   for (int t = 0; t < 8; t++) psum[t][0] = psum[t][1] = 0.f;
@@ -465,21 +379,7 @@ __global__ void __launch_bounds__(128, 3) mp_layer_kernel(
   for (int64_t tile = t0; tile < t1; tile++) {
     const int64_t r0 = tile * TILE + warp * 16;
     if (r0 >= n) continue;
-    if (!PRE_M) {
-      for (int p = 0; p < 8; p++) {
-        const int rr = 2 * p + half;
-        const int64_t r = r0 + rr;
-        float m[4];
-        aggregate_row(r, n, rp, ci, ef, A, B, mk, hl, half, c4, m);
-        uint2 mv;
-        *reinterpret_cast<__nv_bfloat162 *>(&mv.x) = __floats2bfloat162_rn(m[0], m[1]);
-        *reinterpret_cast<__nv_bfloat162 *>(&mv.y) = __floats2bfloat162_rn(m[2], m[3]);
-        *reinterpret_cast<uint2 *>(sMw + rr * LDM + c4) = mv;
-        if (TRAIN && r < n) *reinterpret_cast<float4 *>(M_out + r * H + c4) = make_float4(m[0], m[1], m[2], m[3]);
-      }
-    }
-    __syncwarp();
-    // update GEMM: K = 128 = [h (registers) | M (shared memory)]
+    // update GEMM: K = 128 = [h (registers) | M (BF16 rows)]
     const int64_t ra = r0 + g, rb = r0 + g + 8;
     float v[8][4];
 #pragma unroll
@@ -505,22 +405,12 @@ __global__ void __launch_bounds__(128, 3) mp_layer_kernel(
     }
 #pragma unroll
     for (int kk = 0; kk < 4; kk++) {
-      uint32_t a0, a1, a2, a3;
-      if (PRE_M) {
-        // the A-fragment straight from the BF16 rows (zeros past n, as the
-        // fused aggregation gives)
-        const __nv_bfloat16 *ma = Mb + ra * H + kk * 16 + q * 2, *mb = Mb + rb * H + kk * 16 + q * 2;
-        a0 = ra < n ? *reinterpret_cast<const uint32_t *>(ma) : 0u;
-        a1 = rb < n ? *reinterpret_cast<const uint32_t *>(mb) : 0u;
-        a2 = ra < n ? *reinterpret_cast<const uint32_t *>(ma + 8) : 0u;
-        a3 = rb < n ? *reinterpret_cast<const uint32_t *>(mb + 8) : 0u;
-      } else {
-        const __nv_bfloat16 *mrow = sMw + kk * 16 + q * 2;
-        a0 = *reinterpret_cast<const uint32_t *>(mrow + g * LDM);
-        a1 = *reinterpret_cast<const uint32_t *>(mrow + (g + 8) * LDM);
-        a2 = *reinterpret_cast<const uint32_t *>(mrow + g * LDM + 8);
-        a3 = *reinterpret_cast<const uint32_t *>(mrow + (g + 8) * LDM + 8);
-      }
+      // the A-fragment straight from the BF16 rows (zeros past n)
+      const __nv_bfloat16 *ma = Mb + ra * H + kk * 16 + q * 2, *mb = Mb + rb * H + kk * 16 + q * 2;
+      const uint32_t a0 = ra < n ? *reinterpret_cast<const uint32_t *>(ma) : 0u;
+      const uint32_t a1 = rb < n ? *reinterpret_cast<const uint32_t *>(mb) : 0u;
+      const uint32_t a2 = ra < n ? *reinterpret_cast<const uint32_t *>(ma + 8) : 0u;
+      const uint32_t a3 = rb < n ? *reinterpret_cast<const uint32_t *>(mb + 8) : 0u;
 #pragma unroll
       for (int t = 0; t < 8; t++) {
         const __nv_bfloat16 *w = sWu + (t * 8 + g) * LDU + H + kk * 16 + q * 2;
@@ -528,7 +418,7 @@ __global__ void __launch_bounds__(128, 3) mp_layer_kernel(
                  *reinterpret_cast<const uint32_t *>(w + 8));
       }
     }
-    __syncwarp();  // sMw is rewritten by the next tile
+    uint32_t ga = 0u, gb = 0u;
 #pragma unroll
     for (int t = 0; t < 8; t++) {
       const int c = t * 8 + q * 2;
@@ -540,13 +430,17 @@ __global__ void __launch_bounds__(128, 3) mp_layer_kernel(
       v[t][2] = rb < n ? v[t][2] + u2 : 0.f;
       v[t][3] = rb < n ? v[t][3] + u3 : 0.f;
       if (TRAIN) {
-        if (ra < n) *reinterpret_cast<float2 *>(R_out + ra * H + c) = make_float2(u0, u1);
-        if (rb < n) *reinterpret_cast<float2 *>(R_out + rb * H + c) = make_float2(u2, u3);
+        ga |= (u0 > 0.f ? 1u << (2 * t) : 0u) | (u1 > 0.f ? 2u << (2 * t) : 0u);
+        gb |= (u2 > 0.f ? 1u << (2 * t) : 0u) | (u3 > 0.f ? 2u << (2 * t) : 0u);
       }
       if (!LAST) {
         if (ra < n) *reinterpret_cast<float2 *>(h_out + ra * H + c) = make_float2(v[t][0], v[t][1]);
         if (rb < n) *reinterpret_cast<float2 *>(h_out + rb * H + c) = make_float2(v[t][2], v[t][3]);
       }
+    }
+    if (TRAIN) {
+      if (ra < n) gate[ra * 4 + q] = (uint16_t)ga;
+      if (rb < n) gate[rb * 4 + q] = (uint16_t)gb;
     }
     if (LAST) {
 #pragma unroll
@@ -585,312 +479,571 @@ __global__ void __launch_bounds__(128, 3) mp_layer_kernel(
 
 // ------------------------------------------------- edge backward kernels
 // Both walk rows with a half-warp per row (4 channels per lane) and gather
-// the 16 neighbours of a batch before using any (as the forward layer does).
-constexpr int EB_ROWS = 64;  // rows per CTA (16 half-warps x 4)
+// the 16 neighbours of a batch before using any (as the aggregation does).
+// The first decides which messages were positive and keeps the decision, 64
+// bits a nonzero; the second, over the transposed lists, then reads 8 bytes
+// where it would gather a sender's A and form the message again (131 -> 62 us
+// a layer at 48^3).  The gradients go out in BF16, the operand type of the
+// GEMMs that read them.
+constexpr int kEdgeThreads = 256;
 
 __device__ __forceinline__ float4 half4_to_float4(uint2 u) {
   const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
   const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
+__device__ __forceinline__ uint2 float4_to_bf16(const float (&v)[4]) {
+  return make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+}
 
-// dA_i = sum_j dM_i [P_ij > 0] (P_ij = A_i + B_j + e_ij W_c + b_m), and the
-// CTA's partials of dW_c (4 x 64) and db_m (64): 5 x 64 floats per CTA
-__global__ void __launch_bounds__(256) edge_backward_a(int64_t n, const int32_t *__restrict__ rp,
-                                                       const int32_t *__restrict__ ci, const float4 *__restrict__ ef,
-                                                       const __half *__restrict__ A,
-                                                       const __half *__restrict__ B,
-                                                       const float *__restrict__ Wc, const float *__restrict__ bm,
-                                                       const float *__restrict__ dM, float *__restrict__ dA,
-                                                       float *__restrict__ part) {
-  __shared__ float red[16][5][H];
+// dA_i = dM_i * #{j : P_ij > 0} per channel (P_ij = A_i + B_j + e_ij W_c +
+// b_m), gate[k] the signs of nonzero k (bit 16 c + h of the 64: channel 4 h +
+// c), and the CTA's partials of dW_c (4 x 64) and db_m (64): 5 x 64 floats.
+// A row's sums over its neighbours are of the gated features alone; dM, which
+// they share, multiplies once.  The constant feature's weight gradient is the
+// bias's.  The kernel is bound by instruction issue (66 % of the slots, 79
+// instructions a neighbour and lane): packed FP32 pairs, three CTAs an SM with
+// spills, and leaving a batch early were no faster (109, 112 and 122 us
+// against 97-103 at 48^3).
+__global__ void __launch_bounds__(kEdgeThreads, 2)
+    edge_backward_a(int64_t n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                    const float4 *__restrict__ ef, const __half *__restrict__ A, const __half *__restrict__ B,
+                    const float *__restrict__ Wc, const float *__restrict__ bm, const float *__restrict__ dM,
+                    __nv_bfloat16 *__restrict__ dA, uint2 *__restrict__ gate, float *__restrict__ part) {
+  __shared__ __align__(16) float red[16][4][H];
   const int lane = threadIdx.x & 31, hw = threadIdx.x >> 4, hl = lane & 15, half = lane >> 4, c4 = hl * 4;
-  float wc[FE][4], bmv[4];
+  float wc[3][4], base[4];
 #pragma unroll
-  for (int f = 0; f < FE; f++) {
+  for (int f = 0; f < 3; f++) {
     const float4 w = *reinterpret_cast<const float4 *>(Wc + f * H + c4);
     wc[f][0] = w.x; wc[f][1] = w.y; wc[f][2] = w.z; wc[f][3] = w.w;
   }
   {
     const float4 b = *reinterpret_cast<const float4 *>(bm + c4);
-    bmv[0] = b.x; bmv[1] = b.y; bmv[2] = b.z; bmv[3] = b.w;
+    const float4 w = *reinterpret_cast<const float4 *>(Wc + 3 * H + c4);
+    base[0] = b.x + w.x; base[1] = b.y + w.y; base[2] = b.z + w.z; base[3] = b.w + w.w;
   }
-  float gw[5][4];
+  float gw[4][4];
 #pragma unroll
-  for (int f = 0; f < 5; f++) gw[f][0] = gw[f][1] = gw[f][2] = gw[f][3] = 0.f;
-  for (int rr = 0; rr < EB_ROWS / 16; rr++) {
-    const int64_t i = (int64_t)blockIdx.x * EB_ROWS + hw * (EB_ROWS / 16) + rr;
+  for (int f = 0; f < 4; f++) gw[f][0] = gw[f][1] = gw[f][2] = gw[f][3] = 0.f;
+  // each CTA walks one contiguous range of rows, a row pair per warp
+  const int wpc = kEdgeThreads / 32;
+  const int64_t per = ((n + gridDim.x - 1) / gridDim.x + 1) & ~(int64_t)1;
+  const int64_t first = blockIdx.x * per, end = first + per < n ? first + per : n;
+  for (int64_t r0 = first + 2 * (threadIdx.x >> 5); r0 < end; r0 += 2 * wpc) {
+    const int64_t i = r0 + half;
     int32_t beg = 0, deg = 0;
     float a[4] = {0.f, 0.f, 0.f, 0.f}, dm[4] = {0.f, 0.f, 0.f, 0.f};
-    if (i < n) {
+    if (i < end) {
       beg = rp[i];
       deg = rp[i + 1] - beg;
       const float4 av = half4_to_float4(*reinterpret_cast<const uint2 *>(A + i * H + c4));
       const float4 d = *reinterpret_cast<const float4 *>(dM + i * H + c4);
-      a[0] = av.x + bmv[0]; a[1] = av.y + bmv[1]; a[2] = av.z + bmv[2]; a[3] = av.w + bmv[3];
+      a[0] = av.x + base[0]; a[1] = av.y + base[1]; a[2] = av.z + base[2]; a[3] = av.w + base[3];
       dm[0] = d.x; dm[1] = d.y; dm[2] = d.z; dm[3] = d.w;
     }
-    float sacc[4] = {0.f, 0.f, 0.f, 0.f};
+    float es[4][4];  // gated sums of the three features, and the count
+#pragma unroll
+    for (int f = 0; f < 4; f++) es[f][0] = es[f][1] = es[f][2] = es[f][3] = 0.f;
     const int maxdeg = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));
     for (int k0 = 0; k0 < maxdeg; k0 += 16) {
       const bool ok = k0 + hl < deg;
       const int32_t jl = ok ? ci[beg + k0 + hl] : 0;
       const float4 el = ok ? ef[beg + k0 + hl] : make_float4(0.f, 0.f, 0.f, 0.f);
       const int cnt = deg - k0;
-      uint2 bv[16];
+      uint2 mine = make_uint2(0u, 0u);
+      const unsigned pick = half ? 0x7632u : 0x5410u;  // this half's 16 bits of two ballots
 #pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int32_t j = __shfl_sync(0xffffffffu, jl, (half << 4) + u);
-        bv[u] = *reinterpret_cast<const uint2 *>(B + (int64_t)j * H + c4);
-      }
+      for (int u0 = 0; u0 < 16; u0 += 8) {
+        if (u0 >= maxdeg - k0) break;
+        uint2 bv[8];
 #pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int src = (half << 4) + u;
-        const float e[4] = {__shfl_sync(0xffffffffu, el.x, src), __shfl_sync(0xffffffffu, el.y, src),
-                            __shfl_sync(0xffffffffu, el.z, src), __shfl_sync(0xffffffffu, el.w, src)};
-        const float4 b = half4_to_float4(bv[u]);
-        const float bb[4] = {b.x, b.y, b.z, b.w};
-        const bool live = u < cnt;
+        for (int u = 0; u < 8; u++) {
+          const int32_t j = __shfl_sync(0xffffffffu, jl, (half << 4) + u0 + u);
+          bv[u] = *reinterpret_cast<const uint2 *>(B + (int64_t)j * H + c4);
+        }
 #pragma unroll
-        for (int cc = 0; cc < 4; cc++) {
-          const float pv = a[cc] + bb[cc] + e[0] * wc[0][cc] + e[1] * wc[1][cc] + e[2] * wc[2][cc] + e[3] * wc[3][cc];
-          const float gg = (live && pv > 0.f) ? dm[cc] : 0.f;
-          sacc[cc] += gg;
+        for (int u = 0; u < 8; u++) {
+          const int src = (half << 4) + u0 + u;
+          const float e[3] = {__shfl_sync(0xffffffffu, el.x, src), __shfl_sync(0xffffffffu, el.y, src),
+                              __shfl_sync(0xffffffffu, el.z, src)};
+          const float4 b = half4_to_float4(bv[u]);
+          const float bb[4] = {b.x, b.y, b.z, b.w};
+          const bool live = u0 + u < cnt;
+          unsigned bal[4];
 #pragma unroll
-          for (int f = 0; f < FE; f++) gw[f][cc] += e[f] * gg;
-          gw[4][cc] += gg;
+          for (int cc = 0; cc < 4; cc++) {
+            const float pv = fmaf(e[2], wc[2][cc], fmaf(e[1], wc[1][cc], fmaf(e[0], wc[0][cc], a[cc] + bb[cc])));
+            const bool on = live && pv > 0.f;
+            bal[cc] = __ballot_sync(0xffffffffu, on);
+            if (on) {
+              es[0][cc] += e[0];
+              es[1][cc] += e[1];
+              es[2][cc] += e[2];
+              es[3][cc] += 1.f;
+            }
+          }
+          if (hl == u0 + u) {
+            mine.x = __byte_perm(bal[0], bal[1], pick);
+            mine.y = __byte_perm(bal[2], bal[3], pick);
+          }
         }
       }
+      if (ok) gate[beg + k0 + hl] = mine;
     }
-    if (i < n) *reinterpret_cast<float4 *>(dA + i * H + c4) = make_float4(sacc[0], sacc[1], sacc[2], sacc[3]);
+#pragma unroll
+    for (int f = 0; f < 4; f++)
+#pragma unroll
+      for (int cc = 0; cc < 4; cc++) gw[f][cc] = fmaf(es[f][cc], dm[cc], gw[f][cc]);
+    if (i < end) {
+      const float v[4] = {es[3][0] * dm[0], es[3][1] * dm[1], es[3][2] * dm[2], es[3][3] * dm[3]};
+      *reinterpret_cast<uint2 *>(dA + i * H + c4) = float4_to_bf16(v);
+    }
   }
 #pragma unroll
-  for (int f = 0; f < 5; f++)
-#pragma unroll
-    for (int cc = 0; cc < 4; cc++) red[hw][f][c4 + cc] = gw[f][cc];
+  for (int f = 0; f < 4; f++)
+    *reinterpret_cast<float4 *>(&red[hw][f][c4]) = make_float4(gw[f][0], gw[f][1], gw[f][2], gw[f][3]);
   __syncthreads();
   for (int q = threadIdx.x; q < 5 * H; q += blockDim.x) {
+    const int f = min(q / H, 3);
     float t = 0.f;
-    for (int w = 0; w < 16; w++) t += red[w][q / H][q % H];
+    for (int w = 0; w < 16; w++) t += red[w][f][q % H];
     part[(int64_t)blockIdx.x * 5 * H + q] = t;
   }
 }
 
 // dB_j = sum over the rows i that receive from j of dM_i [P_ij > 0]: row j
 // of the symmetric graph lists those i; tr[k] is the position of (i, j)
-__global__ void __launch_bounds__(256) edge_backward_b(int64_t n, const int32_t *__restrict__ rp,
-                                                       const int32_t *__restrict__ ci, const int32_t *__restrict__ tr,
-                                                       const float4 *__restrict__ ef,
-                                                       const __half *__restrict__ A,
-                                                       const __half *__restrict__ B,
-                                                       const float *__restrict__ Wc, const float *__restrict__ bm,
-                                                       const float *__restrict__ dM, float *__restrict__ dB) {
-  const int lane = threadIdx.x & 31, hw = threadIdx.x >> 4, hl = lane & 15, half = lane >> 4, c4 = hl * 4;
-  float wc[FE][4], bmv[4];
-#pragma unroll
-  for (int f = 0; f < FE; f++) {
-    const float4 w = *reinterpret_cast<const float4 *>(Wc + f * H + c4);
-    wc[f][0] = w.x; wc[f][1] = w.y; wc[f][2] = w.z; wc[f][3] = w.w;
-  }
-  {
-    const float4 b = *reinterpret_cast<const float4 *>(bm + c4);
-    bmv[0] = b.x; bmv[1] = b.y; bmv[2] = b.z; bmv[3] = b.w;
-  }
-  for (int rr = 0; rr < EB_ROWS / 16; rr++) {
-    const int64_t j = (int64_t)blockIdx.x * EB_ROWS + hw * (EB_ROWS / 16) + rr;
+__global__ void __launch_bounds__(kEdgeThreads, 2)
+    edge_backward_b(int64_t n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                    const int32_t *__restrict__ tr, const uint2 *__restrict__ gate, const float *__restrict__ dM,
+                    __nv_bfloat16 *__restrict__ dB) {
+  const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4, c4 = hl * 4;
+  const int wpc = kEdgeThreads / 32;
+  const int64_t per = ((n + gridDim.x - 1) / gridDim.x + 1) & ~(int64_t)1;
+  const int64_t first = blockIdx.x * per, end = first + per < n ? first + per : n;
+  for (int64_t r0 = first + 2 * (threadIdx.x >> 5); r0 < end; r0 += 2 * wpc) {
+    const int64_t j = r0 + half;
     int32_t beg = 0, deg = 0;
-    float b[4] = {0.f, 0.f, 0.f, 0.f};
-    if (j < n) {
+    if (j < end) {
       beg = rp[j];
       deg = rp[j + 1] - beg;
-      const float4 bv = half4_to_float4(*reinterpret_cast<const uint2 *>(B + j * H + c4));
-      b[0] = bv.x + bmv[0]; b[1] = bv.y + bmv[1]; b[2] = bv.z + bmv[2]; b[3] = bv.w + bmv[3];
     }
     float sacc[4] = {0.f, 0.f, 0.f, 0.f};
     const int maxdeg = max(deg, __shfl_xor_sync(0xffffffffu, deg, 16));
     for (int k0 = 0; k0 < maxdeg; k0 += 16) {
       const bool ok = k0 + hl < deg;
       const int32_t il = ok ? ci[beg + k0 + hl] : 0;
-      const float4 el = ok ? ef[tr[beg + k0 + hl]] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const int cnt = deg - k0;
-      uint2 av[16];
+      const uint2 gl = ok ? gate[tr[beg + k0 + hl]] : make_uint2(0u, 0u);
       float4 dv[16];
 #pragma unroll
       for (int u = 0; u < 16; u++) {
         const int32_t i = __shfl_sync(0xffffffffu, il, (half << 4) + u);
-        av[u] = *reinterpret_cast<const uint2 *>(A + (int64_t)i * H + c4);
         dv[u] = *reinterpret_cast<const float4 *>(dM + (int64_t)i * H + c4);
       }
 #pragma unroll
       for (int u = 0; u < 16; u++) {
-        const int src = (half << 4) + u;
-        const float e[4] = {__shfl_sync(0xffffffffu, el.x, src), __shfl_sync(0xffffffffu, el.y, src),
-                            __shfl_sync(0xffffffffu, el.z, src), __shfl_sync(0xffffffffu, el.w, src)};
-        const float4 ai = half4_to_float4(av[u]);
-        const float aa[4] = {ai.x, ai.y, ai.z, ai.w}, dd[4] = {dv[u].x, dv[u].y, dv[u].z, dv[u].w};
-        const bool live = u < cnt;
-#pragma unroll
-        for (int cc = 0; cc < 4; cc++) {
-          const float pv = aa[cc] + b[cc] + e[0] * wc[0][cc] + e[1] * wc[1][cc] + e[2] * wc[2][cc] + e[3] * wc[3][cc];
-          sacc[cc] += (live && pv > 0.f) ? dd[cc] : 0.f;
-        }
+        const unsigned lo = __shfl_sync(0xffffffffu, gl.x, (half << 4) + u) >> hl;
+        const unsigned hi = __shfl_sync(0xffffffffu, gl.y, (half << 4) + u) >> hl;
+        if (lo & 1u) sacc[0] += dv[u].x;
+        if (lo & 0x10000u) sacc[1] += dv[u].y;
+        if (hi & 1u) sacc[2] += dv[u].z;
+        if (hi & 0x10000u) sacc[3] += dv[u].w;
       }
     }
-    if (j < n) *reinterpret_cast<float4 *>(dB + j * H + c4) = make_float4(sacc[0], sacc[1], sacc[2], sacc[3]);
+    if (j < end) *reinterpret_cast<uint2 *>(dB + j * H + c4) = float4_to_bf16(sacc);
   }
 }
 
-// part[cta][k][c] = sum over the CTA's rows of in[r][k] * dout[r][c] (c <
-// 64) and, in row K, sum of dout[r][c] (bias gradient).  in = [in0 | in1].
-// part[cta][k][c] = sum over the CTA's rows of in[r][k] * dout[r][c]
-// (c < 64) and, in row K, the sum of dout[r][c] (bias gradient);
-// in = [in0 | in1], K = K0 + K1 <= 143.  Tensor cores: the reduction over
-// rows is the k dimension of m16n8k16 BF16 MMAs (FP32 accumulation), with
-// in^T and dout fragments loaded by ldmatrix.trans from row-major tiles of
-// 64 rows staged in shared memory; a ones column in the staged input makes
-// the bias row.  Each CTA (4 warps) owns a contiguous range of rows and the
-// whole (K+1) x 64 output, warps splitting it by 16-feature tiles.
+// ------------------------------------------- node GEMMs of the backward pass
+// One pass over a layer's rows for everything that reads them: the gradients
+// passed on (dIn = dOut W^T) and the weight gradients (in^T dOut, the rows
+// being the k dimension of the MMAs), m16n8k16 BF16 with FP32 accumulation.
+// A CTA of 8 warps walks a contiguous range of 64-row tiles; per tile the
+// operands are converted to BF16 in shared memory while the next tile's rows
+// are under way (cp.async), warps 0-3 form the passed-on gradients (16 rows
+// each), warps 4-7 the weight gradient, accumulated in registers over the
+// tiles.  As separate kernels (mask, weight gradients, GEMMs) a layer read and
+// wrote 760 MB at 48^3 in 280 us; this way 250 MB.
 constexpr int WG_TILE = 64;
-constexpr int WG_MAXK = 144;
-constexpr int WG_LDI = WG_MAXK + 8;  // padded rows: conflict-free ldmatrix
-constexpr int WG_LDD = 64 + 8;
-constexpr int WG_PARTS = 3 * kNumSMs;
+constexpr int WG_LDF = H + 4;        // staged FP32 rows (floats)
+constexpr int WG_LDD = H + 8;        // BF16 rows of 64 columns, padded: conflict-free ldmatrix
+constexpr int WG_LDI = 2 * H + 8;    // BF16 rows of 128 columns
+constexpr int kNodeThreads = 256;
+constexpr int kUpdOut = (2 * H + 1) * H;  // weight-gradient entries of the update ([h, M] and bias)
+constexpr int kMsgOut = 2 * H * H;        // of the message operands (W_a, W_b)
+// weights (2 x 64 rows), two staged FP32 tiles or one and two BF16 ones, the
+// BF16 operand tiles
+constexpr size_t kUpdBwdSmem = (size_t)2 * H * WG_LDD * 2 + 2 * WG_TILE * WG_LDF * 4 + WG_TILE * H * 2 +
+                               WG_TILE * WG_LDD * 2 + WG_TILE * WG_LDI * 2;
+constexpr size_t kMsgBwdSmem = (size_t)2 * H * WG_LDD * 2 + WG_TILE * WG_LDF * 4 + WG_TILE * WG_LDD * 2 +
+                               2 * WG_TILE * WG_LDI * 2;
 
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool ok) {
+  const int sz = ok ? 16 : 0;  // (zero fill past the last row)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(dst)), "l"(src), "r"(sz) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+// rows [r0, r0 + WG_TILE) of an n x 64 matrix of 4-byte (or 2-byte) values to
+// shared rows of `ld` values
+template <typename V>
+__device__ __forceinline__ void prefetch_rows(V *dst, int ld, const V *src, int64_t r0, int64_t n) {
+  constexpr int per = H * (int)sizeof(V) / 16, vals = 16 / (int)sizeof(V);
+  for (int q = threadIdx.x; q < WG_TILE * per; q += kNodeThreads) {
+    const int rr = q / per, c = (q % per) * vals;
+    const bool ok = r0 + rr < n;
+    cp_async16(dst + rr * ld + c, src + (ok ? r0 + rr : 0) * H + c, ok);
+  }
+}
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_addr(p)));
+}
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const __nv_bfloat16 *p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(smem_addr(p)));
 }
 
-// rows [r0, r0 + WG_TILE) of an n x width FP32 matrix -> BF16 shared-memory
-// columns [col0, col0 + width) (zeros past rend); float4 loads when width is
-// a multiple of 4, float2 otherwise (width is even)
-__device__ __forceinline__ void stage_rows(__nv_bfloat16 *dst, int ld, int col0, const float *__restrict__ src,
-                                           int width, int64_t r0, int64_t rend) {
-  if ((width & 3) == 0) {
-    const int per = width >> 2;
-    for (int q = threadIdx.x; q < WG_TILE * per; q += blockDim.x) {
-      const int rr = q / per, c = (q % per) * 4;
-      const int64_t r = r0 + rr;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < rend) v = *reinterpret_cast<const float4 *>(src + r * width + c);
-      __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(dst + rr * ld + col0 + c);
-      o[0] = __floats2bfloat162_rn(v.x, v.y);
-      o[1] = __floats2bfloat162_rn(v.z, v.w);
-    }
-  } else {
-    const int per = width >> 1;
-    for (int q = threadIdx.x; q < WG_TILE * per; q += blockDim.x) {
-      const int rr = q / per, c = (q % per) * 2;
-      const int64_t r = r0 + rr;
-      float2 v = make_float2(0.f, 0.f);
-      if (r < rend) v = *reinterpret_cast<const float2 *>(src + r * width + c);
-      *reinterpret_cast<__nv_bfloat162 *>(dst + rr * ld + col0 + c) = __floats2bfloat162_rn(v.x, v.y);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(128, 3) wgrad_kernel(int64_t n, const float *__restrict__ in0, int K0,
-                                                    const float *__restrict__ in1, int K1,
-                                                    const float *__restrict__ dout, float *__restrict__ part) {
-  __shared__ __align__(16) __nv_bfloat16 sI[WG_TILE * WG_LDI];
-  __shared__ __align__(16) __nv_bfloat16 sD[WG_TILE * WG_LDD];
-  const int K = K0 + K1;
-  const int KP = (K + 1 + 15) & ~15;
-  const int MT = KP / 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q4 = lane & 3;
-  const int64_t rbeg = n * blockIdx.x / gridDim.x, rend = n * (blockIdx.x + 1) / gridDim.x;
-  float acc[3][8][4];
+// acc (16 x 64 of the warp's rows) += D (16 rows of a BF16 tile, stride ldd) W^T,
+// W as [64][64] BF16 rows [n][k]
+__device__ __forceinline__ void tile_gemm(float (&acc)[8][4], const __nv_bfloat16 *d, int ldd,
+                                          const __nv_bfloat16 *W, int lane) {
+  const int g = lane >> 2, q = lane & 3;
 #pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int t = 0; t < 8; t++) acc[i][t][0] = acc[i][t][1] = acc[i][t][2] = acc[i][t][3] = 0.f;
-  for (int64_t r0 = rbeg; r0 < rend; r0 += WG_TILE) {
-    __syncthreads();
-    stage_rows(sI, WG_LDI, 0, in0, K0, r0, rend);
-    if (K1 > 0) stage_rows(sI, WG_LDI, K0, in1, K1, r0, rend);
-    // the ones column (bias row) and the zero padding up to KP
-    for (int q = threadIdx.x; q < WG_TILE * (KP - K); q += blockDim.x) {
-      const int rr = q / (KP - K), k = K + q % (KP - K);
-      sI[rr * WG_LDI + k] = __float2bfloat16(k == K && r0 + rr < rend ? 1.f : 0.f);
-    }
-    stage_rows(sD, WG_LDD, 0, dout, 64, r0, rend);
-    __syncthreads();
-    const int mi = lane >> 3;
-#pragma unroll
-    for (int ks = 0; ks < WG_TILE / 16; ks++) {
-      uint32_t bfr[8][2];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        uint32_t t[4];
-        const int row = ks * 16 + (lane & 7) + (mi & 1) * 8, col = (2 * j + (mi >> 1)) * 8;
-        ldsm_x4_trans(t, sD + row * WG_LDD + col);
-        bfr[2 * j][0] = t[0];
-        bfr[2 * j][1] = t[1];
-        bfr[2 * j + 1][0] = t[2];
-        bfr[2 * j + 1][1] = t[3];
-      }
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        const int mt = warp + 4 * i;
-        if (mt >= MT) break;
-        uint32_t a[4];
-        const int row = ks * 16 + (lane & 7) + (mi >> 1) * 8, col = mt * 16 + (mi & 1) * 8;
-        ldsm_x4_trans(a, sI + row * WG_LDI + col);
-#pragma unroll
-        for (int t = 0; t < 8; t++) mma_bf16(acc[i][t], a[0], a[1], a[2], a[3], bfr[t][0], bfr[t][1]);
-      }
-    }
-  }
-  // C fragment: feature rows mt*16 + g (+8), columns 8t + 2 q4 (+1)
-  float *out = part + (int64_t)blockIdx.x * (K + 1) * 64;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const int mt = warp + 4 * i;
-    if (mt >= MT) break;
-    const int f0 = mt * 16 + g, f1 = f0 + 8;
+  for (int kk = 0; kk < 4; kk++) {
+    uint32_t a[4];
+    ldsm_x4(a, d + (lane & 15) * ldd + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
     for (int t = 0; t < 8; t++) {
-      const int c = t * 8 + q4 * 2;
-      if (f0 <= K) *reinterpret_cast<float2 *>(out + f0 * 64 + c) = make_float2(acc[i][t][0], acc[i][t][1]);
-      if (f1 <= K) *reinterpret_cast<float2 *>(out + f1 * 64 + c) = make_float2(acc[i][t][2], acc[i][t][3]);
+      const __nv_bfloat16 *w = W + (t * 8 + g) * WG_LDD + kk * 16 + q * 2;
+      mma_bf16(acc[t], a[0], a[1], a[2], a[3], *reinterpret_cast<const uint32_t *>(w),
+               *reinterpret_cast<const uint32_t *>(w + 8));
     }
   }
 }
+// the B fragments (k = 16 rows at ks, columns col0 + 0..63) of a BF16 tile
+__device__ __forceinline__ void tile_bfrag(uint32_t (&b)[8][2], const __nv_bfloat16 *d, int ldd, int ks, int col0,
+                                           int lane) {
+  const int mi = lane >> 3, row = ks * 16 + (lane & 7) + (mi & 1) * 8;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    uint32_t t[4];
+    ldsm_x4_trans(t, d + row * ldd + col0 + (2 * j + (mi >> 1)) * 8);
+    b[2 * j][0] = t[0];
+    b[2 * j][1] = t[1];
+    b[2 * j + 1][0] = t[2];
+    b[2 * j + 1][1] = t[3];
+  }
+}
+// acc += in^T D for the 16 features at column f0 of a BF16 tile, 16 rows at ks
+__device__ __forceinline__ void tile_wgrad(float (&acc)[8][4], const __nv_bfloat16 *in, int ldi, int f0, int ks,
+                                           const uint32_t (&b)[8][2], int lane) {
+  const int mi = lane >> 3, row = ks * 16 + (lane & 7) + (mi >> 1) * 8;
+  uint32_t a[4];
+  ldsm_x4_trans(a, in + row * ldi + f0 + (mi & 1) * 8);
+#pragma unroll
+  for (int t = 0; t < 8; t++) mma_bf16(acc[t], a[0], a[1], a[2], a[3], b[t][0], b[t][1]);
+}
+__device__ __forceinline__ void zero_acc(float (&a)[8][4]) {
+#pragma unroll
+  for (int t = 0; t < 8; t++) a[t][0] = a[t][1] = a[t][2] = a[t][3] = 0.f;
+}
+// a 16 x 64 accumulator tile to rows of 64 floats
+__device__ __forceinline__ void store_acc(float *out, const float (&a)[8][4], int lane) {
+  const int g = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    const int c = t * 8 + q * 2;
+    *reinterpret_cast<float2 *>(out + g * H + c) = make_float2(a[t][0], a[t][1]);
+    *reinterpret_cast<float2 *>(out + (g + 8) * H + c) = make_float2(a[t][2], a[t][3]);
+  }
+}
 
-// grad[dst + q] (+)= sum_b part[b][q], fixed order; q < count.  The bias row
-// (q >= bias_from) goes to grad[bias_dst + q - bias_from] when bias_dst >= 0.
-// Blocks of 32 outputs x 8 partial groups; the groups are combined in a
-// fixed order (deterministic).
-__global__ void reduce_parts(int nparts, int count, const float *__restrict__ part, float *__restrict__ grad,
-                             int64_t dst, int bias_from, int64_t bias_dst, int accumulate) {
+// the lane's part of rows ra, rb of an n x 64 matrix in the accumulator layout
+// (loaded ahead of the GEMM whose result is added to it); with dz, the mean
+// pool's gradient dz inv instead
+__device__ __forceinline__ void load_rows(float (&p)[8][4], const float *src, int64_t ra, int64_t rb, int64_t n, int q,
+                                          const float *dz, float inv) {
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    const int c = t * 8 + q * 2;
+    float2 x = make_float2(0.f, 0.f), y = x;
+    if (dz) {
+      x = y = make_float2(dz[c] * inv, dz[c + 1] * inv);
+    } else {
+      if (ra < n) x = *reinterpret_cast<const float2 *>(src + ra * H + c);
+      if (rb < n) y = *reinterpret_cast<const float2 *>(src + rb * H + c);
+    }
+    p[t][0] = x.x; p[t][1] = x.y; p[t][2] = y.x; p[t][3] = y.y;
+  }
+}
+__device__ __forceinline__ void add_rows(float *dst, const float (&p)[8][4], const float (&a)[8][4], int64_t ra,
+                                         int64_t rb, int64_t n, int q) {
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    const int c = t * 8 + q * 2;
+    if (ra < n) *reinterpret_cast<float2 *>(dst + ra * H + c) = make_float2(p[t][0] + a[t][0], p[t][1] + a[t][1]);
+    if (rb < n) *reinterpret_cast<float2 *>(dst + rb * H + c) = make_float2(p[t][2] + a[t][2], p[t][3] + a[t][3]);
+  }
+}
+
+// Backward of the update: dR = dh gated, dM = dR W_u[64:]^T, dh += dR
+// W_u[:64]^T (dh holds the residual path), and the CTA's partial of dW_u and
+// db_u.  POOL (the last layer): dh is the mean pool's, dz / n in every row.
+template <bool POOL>
+__global__ void __launch_bounds__(kNodeThreads, 2)
+    update_backward(int64_t n, const float *__restrict__ h, const __nv_bfloat16 *__restrict__ Mb,
+                    const uint16_t *__restrict__ gate, const float *__restrict__ dz,
+                    const __nv_bfloat16 *__restrict__ Wm, const __nv_bfloat16 *__restrict__ Wh, float *dH,
+                    float *__restrict__ dM, float *__restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __nv_bfloat16 *sWm = reinterpret_cast<__nv_bfloat16 *>(smem_raw), *sWh = sWm + H * WG_LDD;
+  float *fh = reinterpret_cast<float *>(sWh + H * WG_LDD), *fd = fh + WG_TILE * WG_LDF;
+  __nv_bfloat16 *rm = reinterpret_cast<__nv_bfloat16 *>(fd + WG_TILE * WG_LDF);
+  __nv_bfloat16 *sD = rm + WG_TILE * H, *sI = sD + WG_TILE * WG_LDD;
+  stage_w(sWm, Wm, H, H, WG_LDD);
+  stage_w(sWh, Wh, H, H, WG_LDD);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const float inv = 1.f / (float)n;
+  float wacc[2][8][4];  // warps 4-7: feature tiles w - 4 and w; warp 0: the bias row
+  zero_acc(wacc[0]);
+  zero_acc(wacc[1]);
+  int64_t t0, t1;
+  tile_range((n + WG_TILE - 1) / WG_TILE, t0, t1);
+  auto prefetch = [&](int64_t tile) {
+    const int64_t r0 = tile * WG_TILE;
+    prefetch_rows(fh, WG_LDF, h, r0, n);
+    if (!POOL) prefetch_rows(fd, WG_LDF, (const float *)dH, r0, n);
+    prefetch_rows(rm, H, Mb, r0, n);
+  };
+  if (t0 < t1) prefetch(t0);
+  for (int64_t tile = t0; tile < t1; tile++) {
+    const int64_t r0 = tile * WG_TILE;
+    cp_async_wait();
+    __syncthreads();  // the staged rows are here, and the last tile's operands are used up
+    {
+      // a thread per (row, q): the columns 8 t + 2 q, 8 t + 2 q + 1
+      const int rr = threadIdx.x >> 2, qq = threadIdx.x & 3;
+      const unsigned gt = r0 + rr < n ? gate[(r0 + rr) * 4 + qq] : 0u;
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const int c = t * 8 + qq * 2;
+        const float2 x = *reinterpret_cast<const float2 *>(fh + rr * WG_LDF + c);
+        float2 d;
+        if (POOL) d = make_float2(dz[c] * inv, dz[c + 1] * inv);
+        else d = *reinterpret_cast<const float2 *>(fd + rr * WG_LDF + c);
+        if (!(gt >> (2 * t) & 1u)) d.x = 0.f;
+        if (!(gt >> (2 * t) & 2u)) d.y = 0.f;
+        *reinterpret_cast<uint32_t *>(sI + rr * WG_LDI + c) = pack_bf16(x.x, x.y);
+        *reinterpret_cast<uint32_t *>(sD + rr * WG_LDD + c) = pack_bf16(d.x, d.y);
+      }
+      const uint4 *m = reinterpret_cast<const uint4 *>(rm + rr * H + qq * 16);
+      uint4 *o = reinterpret_cast<uint4 *>(sI + rr * WG_LDI + H + qq * 16);
+      o[0] = m[0];
+      o[1] = m[1];
+    }
+    __syncthreads();
+    if (tile + 1 < t1) prefetch(tile + 1);
+    if (warp < 4) {
+      const int64_t ra = r0 + warp * 16 + g, rb = ra + 8;
+      const __nv_bfloat16 *d = sD + warp * 16 * WG_LDD;
+      float acc[8][4];
+      zero_acc(acc);
+      tile_gemm(acc, d, WG_LDD, sWm, lane);
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const int c = t * 8 + q * 2;
+        if (ra < n) *reinterpret_cast<float2 *>(dM + ra * H + c) = make_float2(acc[t][0], acc[t][1]);
+        if (rb < n) *reinterpret_cast<float2 *>(dM + rb * H + c) = make_float2(acc[t][2], acc[t][3]);
+      }
+      if (warp == 0) {
+        // row 0 of the A fragment all ones: the column sums
+        const uint32_t one = g == 0 ? 0x3f803f80u : 0u;
+#pragma unroll
+        for (int ks = 0; ks < WG_TILE / 16; ks++) {
+          uint32_t b[8][2];
+          tile_bfrag(b, sD, WG_LDD, ks, 0, lane);
+#pragma unroll
+          for (int t = 0; t < 8; t++) mma_bf16(wacc[0][t], one, 0u, one, 0u, b[t][0], b[t][1]);
+        }
+      }
+      float p[8][4];
+      load_rows(p, dH, ra, rb, n, q, POOL ? dz : nullptr, inv);
+      zero_acc(acc);
+      tile_gemm(acc, d, WG_LDD, sWh, lane);
+      add_rows(dH, p, acc, ra, rb, n, q);
+    } else {
+#pragma unroll
+      for (int ks = 0; ks < WG_TILE / 16; ks++) {
+        uint32_t b[8][2];
+        tile_bfrag(b, sD, WG_LDD, ks, 0, lane);
+        tile_wgrad(wacc[0], sI, WG_LDI, (warp - 4) * 16, ks, b, lane);
+        tile_wgrad(wacc[1], sI, WG_LDI, warp * 16, ks, b, lane);
+      }
+    }
+  }
+  float *out = part + (int64_t)blockIdx.x * kUpdOut;
+  if (warp == 0 && g == 0)
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+      *reinterpret_cast<float2 *>(out + 2 * H * H + t * 8 + q * 2) = make_float2(wacc[0][t][0], wacc[0][t][1]);
+  if (warp < 4) return;
+  store_acc(out + (warp - 4) * 16 * H, wacc[0], lane);
+  store_acc(out + warp * 16 * H, wacc[1], lane);
+}
+
+// Backward of the message operands A = h W_a, B = h W_b: dh += dA W_a^T + dB
+// W_b^T, and the CTA's partial of dW_a and dW_b.
+__global__ void __launch_bounds__(kNodeThreads, 2)
+    message_backward(int64_t n, const float *__restrict__ h, const __nv_bfloat16 *__restrict__ dA,
+                     const __nv_bfloat16 *__restrict__ dB, const __nv_bfloat16 *__restrict__ Wa,
+                     const __nv_bfloat16 *__restrict__ Wb, float *__restrict__ dH, float *__restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __nv_bfloat16 *sWa = reinterpret_cast<__nv_bfloat16 *>(smem_raw), *sWb = sWa + H * WG_LDD;
+  float *fh = reinterpret_cast<float *>(sWb + H * WG_LDD);
+  __nv_bfloat16 *sI = reinterpret_cast<__nv_bfloat16 *>(fh + WG_TILE * WG_LDF);
+  __nv_bfloat16 *sD = sI + WG_TILE * WG_LDD;  // two tiles of [dA | dB], in turn
+  stage_w(sWa, Wa, H, H, WG_LDD);
+  stage_w(sWb, Wb, H, H, WG_LDD);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  float wacc[2][8][4];  // warps 4-7: 16 features each, dW_a and dW_b
+  zero_acc(wacc[0]);
+  zero_acc(wacc[1]);
+  int64_t t0, t1;
+  tile_range((n + WG_TILE - 1) / WG_TILE, t0, t1);
+  auto prefetch = [&](int64_t tile) {
+    const int64_t r0 = tile * WG_TILE;
+    __nv_bfloat16 *d = sD + ((tile - t0) & 1) * WG_TILE * WG_LDI;
+    prefetch_rows(fh, WG_LDF, h, r0, n);
+    prefetch_rows(d, WG_LDI, dA, r0, n);
+    prefetch_rows(d + H, WG_LDI, dB, r0, n);
+  };
+  if (t0 < t1) prefetch(t0);
+  for (int64_t tile = t0; tile < t1; tile++) {
+    const int64_t r0 = tile * WG_TILE;
+    const __nv_bfloat16 *d = sD + ((tile - t0) & 1) * WG_TILE * WG_LDI;
+    cp_async_wait();
+    __syncthreads();
+    {
+      const int rr = threadIdx.x >> 2, qq = threadIdx.x & 3;
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const int c = t * 8 + qq * 2;
+        const float2 x = *reinterpret_cast<const float2 *>(fh + rr * WG_LDF + c);
+        *reinterpret_cast<uint32_t *>(sI + rr * WG_LDD + c) = pack_bf16(x.x, x.y);
+      }
+    }
+    __syncthreads();
+    if (tile + 1 < t1) prefetch(tile + 1);
+    if (warp < 4) {
+      const int64_t ra = r0 + warp * 16 + g, rb = ra + 8;
+      float p[8][4], acc[8][4];
+      load_rows(p, dH, ra, rb, n, q, nullptr, 0.f);
+      zero_acc(acc);
+      tile_gemm(acc, d + warp * 16 * WG_LDI, WG_LDI, sWa, lane);
+      tile_gemm(acc, d + warp * 16 * WG_LDI + H, WG_LDI, sWb, lane);
+      add_rows(dH, p, acc, ra, rb, n, q);
+    } else {
+#pragma unroll
+      for (int ks = 0; ks < WG_TILE / 16; ks++) {
+        uint32_t b[8][2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          tile_bfrag(b, d, WG_LDI, ks, e * H, lane);
+          tile_wgrad(wacc[e], sI, WG_LDD, (warp - 4) * 16, ks, b, lane);
+        }
+      }
+    }
+  }
+  if (warp < 4) return;
+  float *out = part + (int64_t)blockIdx.x * kMsgOut;
+#pragma unroll
+  for (int e = 0; e < 2; e++) store_acc(out + e * H * H + (warp - 4) * 16 * H, wacc[e], lane);
+}
+
+// The encoder's weight gradient (X: n x 10, h0 = relu(X W + b)): the CTA's
+// partial of X^T dR (10 x 64) and of dR's column sums, dR = dh [h0 > 0]
+// rounded to BF16 and X too, as the other weight gradients round them.  A
+// thread per (column, row quarter).
+constexpr int kEncOut = (FX + 1) * H;
+__global__ void __launch_bounds__(256) encoder_wgrad(int64_t n, const float *__restrict__ X,
+                                                     const float *__restrict__ h0, const float *__restrict__ dH,
+                                                     float *__restrict__ part) {
+  __shared__ __align__(16) float sX[64][FX + 2];
+  __shared__ float red[4][kEncOut];
+  const int c = threadIdx.x & 63, rq = threadIdx.x >> 6;
+  float acc[FX + 1];
+#pragma unroll
+  for (int f = 0; f <= FX; f++) acc[f] = 0.f;
+  const int64_t rbeg = n * blockIdx.x / gridDim.x, rend = n * (blockIdx.x + 1) / gridDim.x;
+  for (int64_t r0 = rbeg; r0 < rend; r0 += 64) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < 64 * FX; q += 256) {
+      const int64_t r = r0 + q / FX;
+      sX[q / FX][q % FX] = r < rend ? __bfloat162float(__float2bfloat16(X[r0 * FX + q])) : 0.f;
+    }
+    __syncthreads();
+    float hv[16], d[16];
+#pragma unroll
+    for (int b = 0; b < 16; b++) {
+      const int64_t r = min(r0 + rq * 16 + b, rend - 1);
+      hv[b] = h0[r * H + c];
+      d[b] = dH[r * H + c];
+    }
+#pragma unroll
+    for (int b = 0; b < 16; b++) {
+      const int rr = rq * 16 + b;
+      const float v = r0 + rr < rend && hv[b] > 0.f ? __bfloat162float(__float2bfloat16(d[b])) : 0.f;
+      const float4 x0 = *reinterpret_cast<const float4 *>(sX[rr]), x1 = *reinterpret_cast<const float4 *>(sX[rr] + 4);
+      const float2 x2 = *reinterpret_cast<const float2 *>(sX[rr] + 8);
+      const float xs[FX] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, x2.x, x2.y};
+#pragma unroll
+      for (int f = 0; f < FX; f++) acc[f] = fmaf(xs[f], v, acc[f]);
+      acc[FX] += v;
+    }
+  }
+#pragma unroll
+  for (int f = 0; f <= FX; f++) red[rq][f * H + c] = acc[f];
+  __syncthreads();
+  for (int q = threadIdx.x; q < kEncOut; q += 256)
+    part[(int64_t)blockIdx.x * kEncOut + q] = (red[0][q] + red[1][q]) + (red[2][q] + red[3][q]);
+}
+
+// grad[dst + q] = sum_b part[b][q] for q < count, every segment of the pass in
+// one launch: blocks of 32 outputs x 8 partial groups, the groups combined in
+// a fixed order (deterministic).
+constexpr int kGradSegs = 1 + 3 * LAYERS;
+struct GradSeg {
+  const float *part;
+  int64_t dst;
+  int nparts, count, block0;  // block0: the segment's first block
+};
+struct GradPlan {
+  GradSeg seg[kGradSegs];
+};
+__global__ void reduce_parts(GradPlan plan, float *__restrict__ grad) {
   __shared__ float red[8][33];
-  const int q = blockIdx.x * 32 + threadIdx.x;
+  int g = 0;
+  while (g + 1 < kGradSegs && (int)blockIdx.x >= plan.seg[g + 1].block0) g++;
+  const GradSeg sg = plan.seg[g];
+  const int q = ((int)blockIdx.x - sg.block0) * 32 + threadIdx.x;
   float s = 0.f;
-  if (q < count)
-    for (int b = threadIdx.y; b < nparts; b += 8) s += part[(int64_t)b * count + q];
+  if (q < sg.count) {
+#pragma unroll 4
+    for (int b = threadIdx.y; b < sg.nparts; b += 8) s += sg.part[(int64_t)b * sg.count + q];
+  }
   red[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
-  if (threadIdx.y != 0 || q >= count) return;
-  s = ((red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x])) +
+  if (threadIdx.y != 0 || q >= sg.count) return;
+  grad[sg.dst + q] =
+      ((red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x])) +
       ((red[4][threadIdx.x] + red[5][threadIdx.x]) + (red[6][threadIdx.x] + red[7][threadIdx.x]));
-  int64_t o;
-  if (q >= bias_from) {
-    if (bias_dst < 0) return;
-    o = bias_dst + (q - bias_from);
-  } else {
-    o = dst + q;
-  }
-  grad[o] = accumulate ? grad[o] + s : s;
 }
-
-// g *= [r > 0] (relu mask from the post-activation)
-__global__ void relu_mask(int64_t n, const float *__restrict__ r, const float *__restrict__ g,
-                          float *__restrict__ out) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q < n) out[q] = r[q] > 0.f ? g[q] : 0.f;
-}
-
 
 // Adam (Kingma & Ba 2015), bias-corrected, FP32
 __global__ void adam_kernel(int64_t n, float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
@@ -1126,13 +1279,6 @@ __global__ void readout(int nparts, int64_t n, const float *__restrict__ part, c
   }
 }
 
-// dh[i][c] = dz[c] / n (gradient of the mean pool)
-__global__ void pool_backward(int64_t n, const float *__restrict__ dz, float *__restrict__ dh) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q < n * H) dh[q] = dz[q % H] / (float)n;
-}
-
-
 // per-nonzero edge features and the transpose map of the symmetric graph
 __global__ void edge_setup(int64_t nnz, const int32_t *__restrict__ nz_edge, const int32_t *__restrict__ pf,
                            const int32_t *__restrict__ pb, const double *__restrict__ alpha,
@@ -1154,13 +1300,12 @@ __global__ void edge_setup(int64_t nnz, const int32_t *__restrict__ nz_edge, con
 
 inline int vgrid(int64_t n) { return (int)std::min<int64_t>(div_up(n, 256), kNumSMs * 8); }
 
-// resident CTAs of a 128-thread kernel on the whole device, capped by the
-// number of tiles
-int persistent_grid(const void *kernel, size_t smem, int64_t tiles) {
+// resident CTAs of a kernel on the whole device, capped by the number of tiles
+int persistent_grid(const void *kernel, size_t smem, int64_t tiles, int threads = 128) {
   int d = 0, sms = 0, per_sm = 0;
   NOSH_CUDA(cudaGetDevice(&d));
   NOSH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d));
-  NOSH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, smem));
+  NOSH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)std::max(per_sm, 1) * sms));
 }
 
@@ -1189,12 +1334,21 @@ struct Mpnn::Impl {
   int64_t wt_enc, wt_a[LAYERS], wt_b[LAYERS], wt_u[LAYERS], wtb_a[LAYERS], wtb_b[LAYERS], wtb_uh[LAYERS],
       wtb_um[LAYERS];
   // activations (A, B in FP16: the message operands) and gradients
-  DevBuf<float> X, Hs[LAYERS], Mg[LAYERS], R[LAYERS];
+  DevBuf<float> X, Hs[LAYERS];
   DevBuf<__half> A[LAYERS], B[LAYERS];
-  DevBuf<float> dH, dR, dM, dA, dB, dz;
+  DevBuf<__nv_bfloat16> Mb[LAYERS];  // aggregated messages ([0] alone without training)
+  // training only, allocated with the first gradient: the update's signs, the
+  // messages' signs of one layer, gradients, weight-gradient partials
+  DevBuf<uint16_t> gate[LAYERS];
+  DevBuf<uint2> mgate;
+  DevBuf<float> dH, dM, dz;
+  DevBuf<__nv_bfloat16> dA, dB;
   DevBuf<float> part, pool;
-  DevBuf<__nv_bfloat16> Mb;  // inference split: one layer's M in BF16
-  int enc_grid = 0, layer_grid = 0, agg_grid = 0, upd_grid = 0;
+  GradPlan grad_plan{};
+  CastPlan cast_plan{};
+  int cast_max = 0, grad_blocks = 0;
+  int enc_grid = 0, agg_grid = 0, upd_grid = 0, node_grid = 0, edge_grid = 0, encw_grid = 0;
+  void ensure_training();
   int pool_parts = 0;  // pool partial rows written by the last forward
   DevBuf<double> sq, red, dots, Ls, gram, w, loss;
   DevBuf<double> vc, vd, vt, jc, jd;  // training sample fields and their J applies
@@ -1211,9 +1365,6 @@ struct Mpnn::Impl {
   // Lagrange weights (into Ls) and phase factors of x[1..3] (and target)
   // against x[0] (into dots)
   void align(const double *const x[4], const double mu[4], double t, const double *target);
-  void gemm(int epi, const float *in0, int K0, const float *in1, int K1, int64_t wt_off, float *out);
-  void wgrad(const float *in0, int K0, const float *in1, int K1, const float *dout, int ncol, int64_t dst,
-             int64_t bias_dst);
   void readout_launch(bool train);
 };
 
@@ -1283,31 +1434,34 @@ Mpnn::Impl::Impl(NlsImpl &nls) : s(nls), N(nls.N), nnz(2 * nls.E), stream(nls.st
     Hs[l].alloc(N * H);
     A[l].alloc(N * H);
     B[l].alloc(N * H);
-    Mg[l].alloc(N * H);
-    R[l].alloc(N * H);
   }
-  for (DevBuf<float> *b : {&dH, &dR, &dM, &dA, &dB}) b->alloc(N * H);
-  dz.alloc(H);
-  part.alloc(std::max<int64_t>((int64_t)WG_PARTS * (2 * H + 1) * H, div_up(N, 64) * 5 * H) + 64);
+  Mb[0].alloc(N * H);
   const int64_t tiles = div_up(N, (int64_t)TILE);
   enc_grid = persistent_grid((const void *)encode_kernel, kEncSmem, tiles);
-  layer_grid = persistent_grid((const void *)mp_layer_kernel<true, true, false>, kLayerSmem, tiles);
-  for (const void *k : {(const void *)mp_layer_kernel<false, false, false>,
-                        (const void *)mp_layer_kernel<false, true, false>,
-                        (const void *)mp_layer_kernel<true, false, false>})
-    layer_grid = std::min(layer_grid, persistent_grid(k, kLayerSmem, tiles));
-  upd_grid = std::min(persistent_grid((const void *)mp_layer_kernel<false, false, true>, kUpdateSmem, tiles),
-                      persistent_grid((const void *)mp_layer_kernel<false, true, true>, kUpdateSmem, tiles));
+  upd_grid = std::min(persistent_grid((const void *)mp_update_kernel<false, false>, kUpdateSmem, tiles),
+                      persistent_grid((const void *)mp_update_kernel<false, true>, kUpdateSmem, tiles));
+  // 16 rows per CTA pass (8 warps, a half-warp per row)
+  agg_grid = persistent_grid((const void *)mp_aggregate_kernel, 0, div_up(N, 16), 256);
   {
-    int d = 0, sms = 0, per_sm = 0;
-    NOSH_CUDA(cudaGetDevice(&d));
-    NOSH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d));
-    NOSH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mp_aggregate_kernel, 256, 0));
-    // 16 rows per CTA pass (8 warps, a half-warp per row)
-    agg_grid = (int)std::max<int64_t>(1, std::min<int64_t>(div_up(N, 16), (int64_t)std::max(per_sm, 1) * sms));
+    // BF16 operands: the encoder's (10 features padded to 16 with zeros), the
+    // forward matrices transposed, the backward ones as stored
+    int g = 0;
+    auto seg = [&](int64_t src, int64_t dst, int rows, int K, int kv, int sk, int sn) {
+      cast_plan.seg[g++] = CastSeg{src, dst, rows, K, kv, sk, sn};
+      cast_max = std::max(cast_max, rows * K);
+    };
+    seg(L.enc_w, wt_enc, H, 16, FX, H, 1);
+    for (int l = 0; l < LAYERS; l++) {
+      seg(L.wa[l], wt_a[l], H, H, H, H, 1);
+      seg(L.wb[l], wt_b[l], H, H, H, H, 1);
+      seg(L.wu[l], wt_u[l], H, 2 * H, 2 * H, H, 1);
+      seg(L.wa[l], wtb_a[l], H, H, H, 1, H);
+      seg(L.wb[l], wtb_b[l], H, H, H, 1, H);
+      seg(L.wu[l], wtb_uh[l], H, H, H, 1, H);
+      seg(L.wu[l] + H * H, wtb_um[l], H, H, H, 1, H);
+    }
   }
-  Mb.alloc(N * H);
-  pool.alloc((int64_t)std::max(layer_grid, upd_grid) * H);
+  pool.alloc((int64_t)upd_grid * H);
   sq.alloc(6 * N);
   red.alloc(8);
   dots.alloc(8);
@@ -1321,33 +1475,52 @@ Mpnn::Impl::Impl(NlsImpl &nls) : s(nls), N(nls.N), nnz(2 * nls.E), stream(nls.st
 }
 
 void Mpnn::Impl::refresh_bf16() {
-  cudaStream_t st = stream;
-  const float *P = params.p;
-  // encoder: K = 10 features padded to 16 (zero weights in the padding)
-  enc_to_bf16<<<div_up(H * 16, 256), 256, 0, st>>>(P + L.enc_w, wt.p + wt_enc);
-  for (int l = 0; l < LAYERS; l++) {
-    to_bf16_t<<<div_up(H * H, 256), 256, 0, st>>>(P + L.wa[l], H, H, 0, wt.p + wt_a[l]);
-    to_bf16_t<<<div_up(H * H, 256), 256, 0, st>>>(P + L.wb[l], H, H, 0, wt.p + wt_b[l]);
-    to_bf16_t<<<div_up(H * 2 * H, 256), 256, 0, st>>>(P + L.wu[l], 2 * H, H, 0, wt.p + wt_u[l]);
-    // backward operands: dIn = dOut W^T  ->  Wt[n][k] = W[n][k]
-    to_bf16_rows<<<div_up(H * H, 256), 256, 0, st>>>(P + L.wa[l], H, 0, wt.p + wtb_a[l]);
-    to_bf16_rows<<<div_up(H * H, 256), 256, 0, st>>>(P + L.wb[l], H, 0, wt.p + wtb_b[l]);
-    to_bf16_rows<<<div_up(H * H, 256), 256, 0, st>>>(P + L.wu[l], 2 * H, 0, wt.p + wtb_uh[l]);
-    to_bf16_rows<<<div_up(H * H, 256), 256, 0, st>>>(P + L.wu[l], 2 * H, H, wt.p + wtb_um[l]);
-  }
-  s.launch_count += 1 + 7 * LAYERS;
+  cast_operands<<<dim3(div_up(cast_max, 256), kCastSegs), 256, 0, stream>>>(cast_plan, params.p, wt.p);
+  ++s.launch_count;
   NOSH_CUDA(cudaGetLastError());
 }
 
-void Mpnn::Impl::gemm(int epi, const float *in0, int K0, const float *in1, int K1, int64_t wt_off, float *out) {
-  const int grid = div_up(N, 64);
-  cudaStream_t st = stream;
-  const __nv_bfloat16 *W = wt.p + wt_off;
-  switch (epi) {
-    case EPI_LINEAR: gemm64_kernel<EPI_LINEAR><<<grid, 128, 0, st>>>(N, in0, K0, in1, K1, W, out); break;
-    default: gemm64_kernel<EPI_ACCUM><<<grid, 128, 0, st>>>(N, in0, K0, in1, K1, W, out); break;
+// the training pass's buffers, launch shapes and gradient segments
+void Mpnn::Impl::ensure_training() {
+  if (dH.n) return;
+  cudaStream_t st = s.stream;
+  for (int l = 0; l < LAYERS; l++) {
+    if (l > 0) Mb[l].alloc(N * H);
+    gate[l].alloc(4 * N);
   }
-  ++s.launch_count;
+  mgate.alloc(nnz);
+  dM.alloc(N * H);
+  dA.alloc(N * H);
+  dB.alloc(N * H);
+  dz.alloc(H);
+  for (const void *k : {(const void *)update_backward<false>, (const void *)update_backward<true>})
+    NOSH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdBwdSmem));
+  NOSH_CUDA(cudaFuncSetAttribute(message_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMsgBwdSmem));
+  const int64_t tiles = div_up(N, (int64_t)WG_TILE);
+  node_grid = std::min({persistent_grid((const void *)update_backward<false>, kUpdBwdSmem, tiles, kNodeThreads),
+                        persistent_grid((const void *)update_backward<true>, kUpdBwdSmem, tiles, kNodeThreads),
+                        persistent_grid((const void *)message_backward, kMsgBwdSmem, tiles, kNodeThreads)});
+  edge_grid = std::min(persistent_grid((const void *)edge_backward_a, 0, div_up(N, 16), kEdgeThreads),
+                       persistent_grid((const void *)edge_backward_b, 0, div_up(N, 16), kEdgeThreads));
+  encw_grid = (int)std::min<int64_t>(4 * kNumSMs, div_up(N, 64));
+  // every segment's partials side by side, reduced together at the end
+  int64_t o = 0;
+  int g = 0;
+  auto seg = [&](int64_t dst, int nparts, int count) {
+    grad_plan.seg[g++] = GradSeg{(const float *)(o * sizeof(float)), dst, nparts, count, grad_blocks};
+    grad_blocks += div_up(count, 32);
+    o += (int64_t)nparts * count;
+  };
+  for (int l = 0; l < LAYERS; l++) {
+    seg(L.wu[l], node_grid, kUpdOut);    // W_u, b_u
+    seg(L.wc[l], edge_grid, 5 * H);      // W_c, b_m
+    seg(L.wa[l], node_grid, kMsgOut);    // W_a, W_b
+  }
+  seg(L.enc_w, encw_grid, kEncOut);
+  part.alloc(o);
+  for (GradSeg &q : grad_plan.seg) q.part = part.p + (int64_t)((uintptr_t)q.part / sizeof(float));
+  dH.alloc(N * H);
+  NOSH_CUDA(cudaStreamSynchronize(st));
 }
 
 void Mpnn::Impl::readout_launch(bool train) {
@@ -1367,80 +1540,48 @@ void Mpnn::Impl::forward(bool train) {
   ++s.launch_count;
   for (int l = 0; l < LAYERS; l++) {
     const bool last = l == LAYERS - 1;
-    if (train) {
-      // fused layer (it also stores M and R for the backward pass)
-      auto kernel = last ? mp_layer_kernel<true, true, false> : mp_layer_kernel<true, false, false>;
-      kernel<<<layer_grid, 128, kLayerSmem, st>>>(
-          N, m.d_rp.p, m.d_ci.p, ef4, Hs[l].p, A[l].p, B[l].p, P + L.wc[l], P + L.bm[l], wt.p + wt_u[l],
-          P + L.bu[l], last ? nullptr : wt.p + wt_a[l + 1], last ? nullptr : Hs[l + 1].p,
-          last ? nullptr : A[l + 1].p, last ? nullptr : B[l + 1].p, Mg[l].p, R[l].p, pool.p, nullptr);
-      pool_parts = layer_grid;
-    } else {
-      // inference: the aggregation at high occupancy, then the update GEMM
-      // (bitwise the fused layer's result: the same arithmetic and the
-      // same BF16 rounding of M)
-      mp_aggregate_kernel<<<agg_grid, 256, 0, st>>>(N, m.d_rp.p, m.d_ci.p, ef4, A[l].p, B[l].p, P + L.wc[l],
-                                                    P + L.bm[l], Mb.p);
-      auto kernel = last ? mp_layer_kernel<false, true, true> : mp_layer_kernel<false, false, true>;
-      kernel<<<upd_grid, 128, kUpdateSmem, st>>>(
-          N, m.d_rp.p, m.d_ci.p, ef4, Hs[l].p, A[l].p, B[l].p, P + L.wc[l], P + L.bm[l], wt.p + wt_u[l],
-          P + L.bu[l], last ? nullptr : wt.p + wt_a[l + 1], last ? nullptr : Hs[l + 1].p,
-          last ? nullptr : A[l + 1].p, last ? nullptr : B[l + 1].p, nullptr, nullptr, pool.p, Mb.p);
-      pool_parts = upd_grid;
-      ++s.launch_count;
-    }
-    ++s.launch_count;
+    __nv_bfloat16 *M = Mb[train ? l : 0].p;
+    mp_aggregate_kernel<<<agg_grid, 256, 0, st>>>(N, m.d_rp.p, m.d_ci.p, ef4, A[l].p, B[l].p, P + L.wc[l],
+                                                  P + L.bm[l], M);
+    auto kernel = train ? (last ? mp_update_kernel<true, true> : mp_update_kernel<true, false>)
+                        : (last ? mp_update_kernel<false, true> : mp_update_kernel<false, false>);
+    kernel<<<upd_grid, 128, kUpdateSmem, st>>>(N, Hs[l].p, M, wt.p + wt_u[l], P + L.bu[l],
+                                               last ? nullptr : wt.p + wt_a[l + 1], last ? nullptr : Hs[l + 1].p,
+                                               last ? nullptr : A[l + 1].p, last ? nullptr : B[l + 1].p,
+                                               train ? gate[l].p : nullptr, pool.p);
+    pool_parts = upd_grid;
+    s.launch_count += 2;
   }
   NOSH_CUDA(cudaGetLastError());
 }
 
-void Mpnn::Impl::wgrad(const float *in0, int K0, const float *in1, int K1, const float *dout, int ncol,
-                       int64_t dst, int64_t bias_dst) {
-  cudaStream_t st = stream;
-  (void)ncol;  // always H
-  const int nb = (int)std::min<int64_t>(WG_PARTS, std::max<int64_t>(1, div_up(N, 4 * WG_TILE)));
-  const int count = (K0 + K1 + 1) * H;
-  wgrad_kernel<<<nb, 128, 0, st>>>(N, in0, K0, in1, K1, dout, part.p);
-  reduce_parts<<<div_up(count, 32), dim3(32, 8), 0, st>>>(nb, count, part.p, grads.p, dst, (K0 + K1) * H, bias_dst,
-                                                          0);
-  s.launch_count += 2;
-}
-
-// forward must have run; gram holds the sample's Gram scalars
+// forward(true) must have run; gram holds the sample's Gram scalars
 double Mpnn::Impl::backward_and_step(float lr) {
   cudaStream_t st = stream;
   const float *P = params.p;
   MeshImpl &m = *s.mesh;
+  const float4 *ef4 = reinterpret_cast<const float4 *>(ef.p);
   readout_launch(true);  // loss, readout gradients, dz
-  pool_backward<<<div_up(N * H, 256), 256, 0, st>>>(N, dz.p, dH.p);
-  ++s.launch_count;
   for (int l = LAYERS - 1; l >= 0; l--) {
     // h_{l+1} = h_l + R_l, R_l = relu([h_l, M_l] W_u + b_u)
-    relu_mask<<<div_up(N * H, 256), 256, 0, st>>>(N * H, R[l].p, dH.p, dR.p);
-    ++s.launch_count;
-    wgrad(Hs[l].p, H, Mg[l].p, H, dR.p, H, L.wu[l], L.bu[l]);
-    // dM = dR W_u[64:128]^T ; dh += dR W_u[0:64]^T (dh holds the residual path)
-    gemm(EPI_LINEAR, dR.p, H, nullptr, 0, wtb_um[l], dM.p);
-    gemm(EPI_ACCUM, dR.p, H, nullptr, 0, wtb_uh[l], dH.p);
-    const int nb = div_up(N, EB_ROWS);
-    const float4 *ef4 = reinterpret_cast<const float4 *>(ef.p);
-    edge_backward_a<<<nb, 256, 0, st>>>(N, m.d_rp.p, m.d_ci.p, ef4, A[l].p, B[l].p, P + L.wc[l], P + L.bm[l],
-                                        dM.p, dA.p, part.p);
-    reduce_parts<<<div_up(5 * H, 32), dim3(32, 8), 0, st>>>(nb, 5 * H, part.p, grads.p, L.wc[l], 4 * H, L.bm[l],
-                                                             0);
-    edge_backward_b<<<nb, 256, 0, st>>>(N, m.d_rp.p, m.d_ci.p, tr.p, ef4, A[l].p, B[l].p, P + L.wc[l],
-                                        P + L.bm[l], dM.p, dB.p);
-    s.launch_count += 3;
+    float *pu = const_cast<float *>(grad_plan.seg[3 * l].part), *pe = const_cast<float *>(grad_plan.seg[3 * l + 1].part),
+          *pm = const_cast<float *>(grad_plan.seg[3 * l + 2].part);
+    auto upd = l == LAYERS - 1 ? update_backward<true> : update_backward<false>;
+    upd<<<node_grid, kNodeThreads, kUpdBwdSmem, st>>>(N, Hs[l].p, Mb[l].p, gate[l].p, dz.p, wt.p + wtb_um[l],
+                                                      wt.p + wtb_uh[l], dH.p, dM.p, pu);
+    // the messages, by receiver and by sender
+    edge_backward_a<<<edge_grid, kEdgeThreads, 0, st>>>(N, m.d_rp.p, m.d_ci.p, ef4, A[l].p, B[l].p, P + L.wc[l],
+                                                        P + L.bm[l], dM.p, dA.p, mgate.p, pe);
+    edge_backward_b<<<edge_grid, kEdgeThreads, 0, st>>>(N, m.d_rp.p, m.d_ci.p, tr.p, mgate.p, dM.p, dB.p);
     // A = h W_a, B = h W_b
-    wgrad(Hs[l].p, H, nullptr, 0, dA.p, H, L.wa[l], -1);
-    wgrad(Hs[l].p, H, nullptr, 0, dB.p, H, L.wb[l], -1);
-    gemm(EPI_ACCUM, dA.p, H, nullptr, 0, wtb_a[l], dH.p);
-    gemm(EPI_ACCUM, dB.p, H, nullptr, 0, wtb_b[l], dH.p);
+    message_backward<<<node_grid, kNodeThreads, kMsgBwdSmem, st>>>(N, Hs[l].p, dA.p, dB.p, wt.p + wtb_a[l],
+                                                                  wt.p + wtb_b[l], dH.p, pm);
+    s.launch_count += 4;
   }
   // encoder: h0 = relu(X W + b)
-  relu_mask<<<div_up(N * H, 256), 256, 0, st>>>(N * H, Hs[0].p, dH.p, dR.p);
-  ++s.launch_count;
-  wgrad(X.p, FX, nullptr, 0, dR.p, H, L.enc_w, L.enc_b);
+  encoder_wgrad<<<encw_grid, 256, 0, st>>>(N, X.p, Hs[0].p, dH.p, const_cast<float *>(grad_plan.seg[3 * LAYERS].part));
+  reduce_parts<<<grad_blocks, dim3(32, 8), 0, st>>>(grad_plan, grads.p);
+  s.launch_count += 2;
   if (lr > 0.f) {
     adam_t++;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -1450,6 +1591,7 @@ double Mpnn::Impl::backward_and_step(float lr) {
     ++s.launch_count;
     refresh_bf16();
   }
+  NOSH_CUDA(cudaGetLastError());
   double hl = 0.0;
   loss.download(&hl, 1, st);
   NOSH_CUDA(cudaStreamSynchronize(st));
@@ -1575,6 +1717,7 @@ void Mpnn::predict_fields(const double *const x[4], const double mu[4], double m
 double Mpnn::train(const double *const x[4], const double mu[4], const double *target, double mu_t, int iters,
                    double lr) {
   Impl &I = *impl;
+  I.ensure_training();
   I.features(x, mu, mu_t, target);
   double l = std::nan("");
   for (int k = 0; k < iters; k++) {
@@ -1611,6 +1754,7 @@ double Mpnn::loss_and_grad(const float *X, const double *gram, float *grad) {
   Impl &I = *impl;
   I.X.upload(X, I.N * FX, I.s.stream);
   I.gram.upload(gram, 3, I.s.stream);
+  I.ensure_training();
   I.forward(true);
   const double l = I.backward_and_step(0.f);  // gradient only, no step
   I.grads.download(grad, I.L.total, I.s.stream);
