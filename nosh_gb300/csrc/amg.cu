@@ -1388,8 +1388,8 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
   // host copy of the current fine operator (strength tests)
   std::vector<HostLevel> H(1);
   H[0].n = m.N;
-  H[0].rp.assign(m.rp.begin(), m.rp.end());
-  H[0].ci = m.ci;
+  H[0].rp = m.rp();
+  H[0].ci = m.ci();
   {
     std::vector<C2<double>> off(2 * m.E);
     s.d_keo64.download(off.data(), 2 * m.E, st);

@@ -216,7 +216,7 @@ int nosh_mesh_edges(nosh_mesh mesh, int32_t *edges) {
   return guarded([&] {
     auto &m = M(mesh);
     require(edges != nullptr, "null output");
-    std::memcpy(edges, m.edges.data(), m.edges.size() * sizeof(int32_t));
+    std::memcpy(edges, m.edges().data(), 2 * m.E * sizeof(int32_t));
   });
 }
 
@@ -224,8 +224,9 @@ int nosh_mesh_edge_gids_complex(nosh_mesh mesh, int32_t *idx) {
   return guarded([&] {
     auto &m = M(mesh);
     require(idx != nullptr, "null output");
+    const std::vector<int32_t> &ed = m.edges();
     for (int64_t e = 0; e < m.E; e++) {
-      const int32_t g0 = m.edges[2 * e] + 1, g1 = m.edges[2 * e + 1] + 1;  // 1-based GIDs
+      const int32_t g0 = ed[2 * e] + 1, g1 = ed[2 * e + 1] + 1;  // 1-based GIDs
       idx[4 * e + 0] = 2 * g0;
       idx[4 * e + 1] = 2 * g0 + 1;
       idx[4 * e + 2] = 2 * g1;
@@ -237,8 +238,8 @@ int nosh_mesh_edge_gids_complex(nosh_mesh mesh, int32_t *idx) {
 int nosh_mesh_edge_data(nosh_mesh mesh, double *length, double *covolume) {
   return guarded([&] {
     auto &m = M(mesh);
-    if (length) std::memcpy(length, m.h_len.data(), m.E * sizeof(double));
-    if (covolume) std::memcpy(covolume, m.h_covol.data(), m.E * sizeof(double));
+    if (length) std::memcpy(length, m.len().data(), m.E * sizeof(double));
+    if (covolume) std::memcpy(covolume, m.covol().data(), m.E * sizeof(double));
   });
 }
 
@@ -246,7 +247,7 @@ int nosh_mesh_control_volumes(nosh_mesh mesh, double *cv) {
   return guarded([&] {
     auto &m = M(mesh);
     require(cv != nullptr, "null output");
-    std::memcpy(cv, m.h_cv.data(), m.N * sizeof(double));
+    std::memcpy(cv, m.cv().data(), m.N * sizeof(double));
   });
 }
 

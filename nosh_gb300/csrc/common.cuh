@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <stdexcept>
@@ -89,26 +90,20 @@ struct DevBuf {
 bool is_device_pointer(const void *p);
 
 // ------------------------------------------------------- host parallelism
-// Static-partition parallel loop over [0, n) on the host cores (integer mesh
-// work during set-up).
+// f(begin, end) over a static partition of [0, n) on the host cores, at least
+// `grain` elements each (a thread costs about 20 us to start).
 template <class F>
-void parallel_for(int64_t n, F &&f, int64_t grain = 1 << 14) {
-  unsigned hw = std::thread::hardware_concurrency();
-  int64_t nt = hw ? hw : 1;
-  if (nt > 64) nt = 64;
-  if (n < grain * 2 || nt == 1) {
-    for (int64_t i = 0; i < n; i++) f(i);
+void parallel_ranges(int64_t n, int64_t grain, F &&f) {
+  const unsigned hw = std::thread::hardware_concurrency();
+  const int64_t nt = std::min<int64_t>(std::min<int64_t>(hw ? hw : 1, 16), n / grain);
+  if (nt <= 1) {
+    f((int64_t)0, n);
     return;
   }
-  if (nt > n / grain) nt = n / grain;
   std::vector<std::thread> th;
-  th.reserve(nt);
-  for (int64_t t = 0; t < nt; t++) {
-    int64_t b = n * t / nt, e = n * (t + 1) / nt;
-    th.emplace_back([b, e, &f] {
-      for (int64_t i = b; i < e; i++) f(i);
-    });
-  }
+  th.reserve(nt - 1);
+  for (int64_t t = 1; t < nt; t++) th.emplace_back([=, &f] { f(n * t / nt, n * (t + 1) / nt); });
+  f((int64_t)0, n / nt);
   for (auto &x : th) x.join();
 }
 

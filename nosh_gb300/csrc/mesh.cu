@@ -1,5 +1,5 @@
-// Mesh set-up: integer work on the host (edges, KEO graph, edge -> nonzero
-// scatter map), geometry on the GPU in FP64 (edge coefficients, covolumes,
+// Mesh set-up on the GPU: edges, KEO graph and edge -> nonzero scatter map
+// from the cells, then the geometry in FP64 (edge coefficients, covolumes,
 // control volumes).
 //
 // Reference: nosh::mesh + mesh_tri / mesh_tetra (src/mesh.cpp,
@@ -7,19 +7,21 @@
 // MOAB's entity order, which is not reproducible without MOAB; here edges are
 // the canonical sorted pairs (v0 < v1) in lexicographic order, and the KEO
 // graph (sorted columns per row) is identical to Tpetra's after fillComplete.
+//
+// The integer work is a vertex -> cell incidence (counting, scan, scatter),
+// then a warp per vertex that sorts its incident cells (so that every later
+// sum runs in cell order, whatever order the scatter left) and its neighbours.
+// On the host it took 60 of the 75 ms of a 64^3 mesh.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
-#include <numeric>
 
 #include "mesh.cuh"
 
 namespace nosh {
 
 namespace {
-
-constexpr int TRI_PAIRS[3][2] = {{0, 1}, {0, 2}, {1, 2}};
-constexpr int TET_PAIRS[6][2] = {{0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3}};
 
 // local edge k of a simplex joins local vertices (pair0(k), pair1(k)):
 // triangles (0,1),(0,2),(1,2); tetrahedra (0,1),(0,2),(0,3),(1,2),(1,3),(2,3).
@@ -32,7 +34,203 @@ template <int nvc>
 __host__ __device__ constexpr int pair1(int k) {
   return nvc == 3 ? (k == 0 ? 1 : 2) : (k < 3 ? k + 1 : (k == 3 ? 2 : 3));
 }
+// the local edge of local vertices a != b
+template <int nvc>
+__device__ __forceinline__ constexpr int edge_of(int a, int b) {
+  const int lo = a < b ? a : b, hi = a < b ? b : a;
+  return nvc == 3 ? lo + hi - 1 : (lo == 0 ? hi - 1 : lo + hi);
+}
 
+// ------------------------------------------------------------- topology
+__global__ void count_incident(int64_t n, const int32_t *__restrict__ cells, int32_t *cnt) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
+    atomicAdd(cnt + cells[k], 1);
+}
+__global__ void scatter_incident(int64_t n, const int32_t *__restrict__ cells, int32_t *cur, int32_t *vc) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
+    vc[atomicAdd(cur + cells[k], 1)] = (int32_t)k;
+}
+
+// Exclusive scan of n counts (in: int32, out: n + 1 int64 prefix sums stored as
+// V), in tiles of 1024: tile sums, their scan by one CTA, then the tiles.
+constexpr int kScanTile = 1024;
+__device__ __forceinline__ int64_t block_scan(int64_t v, int64_t *sm) {
+  // inclusive over 1024 threads
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) sm[w] = v;
+  __syncthreads();
+  if (w == 0) {
+    int64_t t = sm[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t u = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += u;
+    }
+    sm[lane] = t;
+  }
+  __syncthreads();
+  return v + (w ? sm[w - 1] : 0);
+}
+__global__ void __launch_bounds__(kScanTile) scan_tiles(int64_t n, const int32_t *__restrict__ in, int64_t *tile) {
+  __shared__ int64_t sm[32];
+  const int64_t i = blockIdx.x * (int64_t)kScanTile + threadIdx.x;
+  const int64_t s = block_scan(i < n ? in[i] : 0, sm);
+  if (threadIdx.x == kScanTile - 1) tile[blockIdx.x] = s;
+}
+__global__ void __launch_bounds__(kScanTile) scan_sums(int64_t nt, int64_t *tile) {
+  __shared__ int64_t sm[32];
+  int64_t carry = 0;
+  for (int64_t t0 = 0; t0 < nt; t0 += kScanTile) {
+    const int64_t t = t0 + threadIdx.x;
+    const int64_t v = t < nt ? tile[t] : 0;
+    const int64_t s = block_scan(v, sm);
+    const int64_t total = sm[31];
+    if (t < nt) tile[t] = carry + s - v;
+    carry += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) tile[nt] = carry;
+}
+__global__ void __launch_bounds__(kScanTile) scan_write(int64_t n, const int32_t *__restrict__ in,
+                                                        const int64_t *__restrict__ tile, int32_t *out) {
+  __shared__ int64_t sm[32];
+  const int64_t i = blockIdx.x * (int64_t)kScanTile + threadIdx.x;
+  const int64_t v = i < n ? in[i] : 0;
+  const int64_t s = block_scan(v, sm) + tile[blockIdx.x];
+  if (i < n) out[i] = (int32_t)(s - v);
+  if (i == n - 1) out[n] = (int32_t)s;
+}
+
+// A warp per vertex: its incident (cell, slot) codes sorted in place, and its
+// neighbours (the other vertices of those cells) sorted and without
+// repetition at nb + (nvc - 1) ptr[v], their number and how many are above v.
+// Ranks by counting in shared memory: a vertex of a tetrahedral mesh has some
+// 24 cells and 72 candidates.  Vertices with more than kMaxIncident cells are
+// left to the host, listed in `hubs`.
+constexpr int kMaxIncident = 84;  // 3 x 84 candidates
+constexpr int kNbWarps = 4;
+template <int nvc>
+__global__ void __launch_bounds__(32 * kNbWarps)
+    neighbour_kernel(int64_t N, const int32_t *__restrict__ cells, const int32_t *__restrict__ ptr, int32_t *vc,
+                     int32_t *nb, int32_t *deg, int32_t *up, int32_t *hubs, int *nhubs) {
+  constexpr int kCand = kMaxIncident * 3;
+  __shared__ int32_t s_code[kNbWarps][kMaxIncident], s_cand[kNbWarps][kCand];
+  __shared__ uint8_t s_first[kNbWarps][kCand + 4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t v = blockIdx.x * (int64_t)kNbWarps + w; v < N; v += (int64_t)gridDim.x * kNbWarps) {
+    const int b = ptr[v], d = ptr[v + 1] - b;
+    if (d > kMaxIncident) {
+      if (lane == 0) hubs[atomicAdd(nhubs, 1)] = (int32_t)v;
+      continue;
+    }
+    int32_t *code = s_code[w], *cand = s_cand[w];
+    uint8_t *first = s_first[w];
+    __syncwarp();
+    for (int q = lane; q < d; q += 32) code[q] = vc[b + q];
+    __syncwarp();
+    for (int q = lane; q < d; q += 32) {
+      const int32_t c = code[q];
+      int r = 0;
+      for (int j = 0; j < d; j++) r += code[j] < c;
+      vc[b + r] = c;
+      const int64_t cell = c / nvc;
+      int o = 0;
+#pragma unroll
+      for (int k = 0; k < nvc; k++) {
+        const int32_t u = cells[nvc * cell + k];
+        if (u != (int32_t)v) cand[(nvc - 1) * q + o++] = u;
+      }
+    }
+    __syncwarp();
+    const int m = (nvc - 1) * d;
+    for (int q = lane; q < m; q += 32) {
+      const int32_t c = cand[q];
+      bool f = true;
+      for (int j = 0; j < q; j++) f = f && cand[j] != c;
+      first[q] = f;
+    }
+    __syncwarp();
+    int above = 0, uniq = 0;
+    for (int q = lane; q < m; q += 32) {
+      if (!first[q]) continue;
+      const int32_t c = cand[q];
+      int r = 0;
+      for (int j = 0; j < m; j++) r += first[j] && cand[j] < c;
+      nb[(int64_t)(nvc - 1) * b + r] = c;
+      uniq++;
+      above += c > (int32_t)v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      uniq += __shfl_xor_sync(0xffffffffu, uniq, o);
+      above += __shfl_xor_sync(0xffffffffu, above, o);
+    }
+    if (lane == 0) {
+      deg[v] = uniq;
+      up[v] = above;
+    }
+  }
+}
+
+// rows of the graph and the edges, half a warp per vertex (the upper
+// neighbours of each vertex are its edges, in lexicographic order)
+__global__ void graph_rows(int64_t N, int nvc, const int32_t *__restrict__ ptr, const int32_t *__restrict__ nb,
+                           const int32_t *__restrict__ rp, const int32_t *__restrict__ up,
+                           const int32_t *__restrict__ ebase, int32_t *ci, int32_t *edges, int32_t *pos_fwd,
+                           int32_t *nz_edge) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, v = t >> 4;
+  if (v >= N) return;
+  const int b = rp[v], d = rp[v + 1] - b, low = d - up[v];
+  const int32_t *src = nb + (int64_t)(nvc - 1) * ptr[v];
+  for (int q = (int)(t & 15); q < d; q += 16) {
+    const int32_t c = src[q];
+    ci[b + q] = c;
+    if (q >= low) {
+      const int e = ebase[v] + q - low;
+      edges[2 * (int64_t)e] = (int32_t)v;
+      edges[2 * (int64_t)e + 1] = c;
+      pos_fwd[e] = b + q;
+      nz_edge[b + q] = e;
+    }
+  }
+}
+// the nonzero of (v1, v0) of each edge, by bisection of row v1; and the row
+// lengths that the SpMV's staging wants
+__global__ void graph_back(int64_t E, const int32_t *__restrict__ edges, const int32_t *__restrict__ rp,
+                           const int32_t *__restrict__ ci, int32_t *pos_bwd, int32_t *nz_edge) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  const int32_t v = edges[2 * e], w = edges[2 * e + 1];
+  int lo = rp[w], hi = rp[w + 1];
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ci[mid] < v) lo = mid + 1;
+    else hi = mid;
+  }
+  pos_bwd[e] = lo;
+  nz_edge[lo] = ~(int32_t)e;
+}
+__global__ void row_extents(int64_t N, const int32_t *__restrict__ rp, int *out) {
+  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  int row = 0, block = 0;
+  if (v < N) {
+    row = rp[v + 1] - rp[v];
+    if (v % 128 == 0) block = rp[min(N, v + 128)] - (rp[v] & ~3);
+  }
+  row = __reduce_max_sync(0xffffffffu, row);
+  block = __reduce_max_sync(0xffffffffu, block);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(out, row);
+    if (block > 0) atomicMax(out + 1, block);
+  }
+}
+
+// ------------------------------------------------------------- geometry
 struct V3 {
   double x, y, z;
 };
@@ -46,20 +244,21 @@ __device__ __forceinline__ V3 cross(V3 a, V3 b) {
 }
 __device__ __forceinline__ double norm(V3 a) { return sqrt(dot(a, a)); }
 
-// In-place Cholesky solve of the SPD system A c = r (n <= 6), fully unrolled.
-// The edge-coefficient matrix A_ij = (e_i . e_j)^2 is the Gram matrix of the
+// In-place Cholesky solve of the SPD system A c = r (lower triangle of A, n <=
+// 6), fully unrolled, the pivots' reciprocal roots instead of divisions.  The
+// edge-coefficient matrix A_ij = (e_i . e_j)^2 is the Gram matrix of the
 // rank-one tensors e_i e_i^T, SPD for a non-degenerate simplex.
 template <int n>
 __device__ __forceinline__ bool chol_solve(double (&A)[n][n], double (&r)[n]) {
+  bool ok = true;
 #pragma unroll
   for (int j = 0; j < n; j++) {
     double d = A[j][j];
 #pragma unroll
     for (int k = 0; k < j; k++) d -= A[j][k] * A[j][k];
-    if (!(d > 0.0)) return false;
-    d = sqrt(d);
-    A[j][j] = d;
-    const double inv = 1.0 / d;
+    ok = ok && d > 0.0;
+    const double inv = rsqrt(d);
+    A[j][j] = inv;
 #pragma unroll
     for (int i = j + 1; i < n; i++) {
       double s = A[i][j];
@@ -73,143 +272,176 @@ __device__ __forceinline__ bool chol_solve(double (&A)[n][n], double (&r)[n]) {
     double s = r[i];
 #pragma unroll
     for (int k = 0; k < i; k++) s -= A[i][k] * r[k];
-    r[i] = s / A[i][i];
+    r[i] = s * A[i][i];
   }
 #pragma unroll
   for (int i = n - 1; i >= 0; i--) {
     double s = r[i];
 #pragma unroll
     for (int k = i + 1; k < n; k++) s -= A[k][i] * r[k];
-    r[i] = s / A[i][i];
+    r[i] = s * A[i][i];
   }
-  return true;
-}
-
-// Triangle circumcenter in barycentric form (src/mesh.cpp:897-928).
-__device__ __forceinline__ V3 tri_cc(V3 n0, V3 n1, V3 n2, int *err) {
-  const V3 a = n0 - n1, b = n1 - n2, c = n2 - n0;
-  const V3 ab = cross(a, b);
-  const double omega = 2.0 * dot(ab, ab);
-  // degenerate triangle (the reference tests |omega| < 1e-10 absolutely,
-  // src/mesh.cpp:917-927; a scale-free test keeps fine meshes valid)
-  if (!(omega > 1.0e-20 * dot(a, a) * dot(b, b))) atomicOr(err, 1);
-  const double al = -dot(b, b) * dot(a, c) / omega;
-  const double be = -dot(c, c) * dot(b, a) / omega;
-  const double ga = -dot(a, a) * dot(c, b) / omega;
-  return al * n0 + be * n1 + ga * n2;
+  return ok;
 }
 
 // Per simplex: edge coefficients (src/mesh_tri.cpp:107-151,
 // src/mesh_tetra.cpp:107-160) times edge length, one value per local edge,
 // and the control-volume share of each local vertex (circumcentric
 // splitting, src/mesh.cpp:931-1027, src/mesh_tetra.cpp:196-331).
+//
+// The kernel is bound by FP64 instructions, so every quantity comes from the
+// inner products of the edges.  In a triangle the signed distance
+// of the circumcentre from edge e is |e| / 2 times the cotangent of the
+// opposite angle, so an edge's share is |e|^2 cot / 8 to either end.  In a
+// tetrahedron the piece of the dual face of edge e that lies in face F is the
+// triangle of the edge's midpoint, F's circumcentre and the cell's: half of
+// (|e| / 2) cot_F(e) times the signed height h_F of the cell's circumcentre
+// over F, and with cot = (a . b) / |N|, h = (w . N) / |N| (N = F's normal,
+// twice its area, towards the opposite vertex; w from F to the circumcentre)
+// no square root is left: a share of |e|^2 / 24 (a . b) (w . N) / |N|^2 to
+// either end.  About 490 FP64 instructions a tetrahedron; with every
+// circumcentre, norm and cross product formed as such it took 1960 (5.46 ms at
+// 64^3).
 template <int nvc>
-__global__ void cell_geometry_kernel(int64_t T, const int32_t *__restrict__ cells,
-                                     const double *__restrict__ x,
-                                     double *__restrict__ coef_len,
-                                     double *__restrict__ cv_part, int *err) {
+__global__ void cell_geometry_kernel(int64_t T, const int32_t *__restrict__ cells, const double *__restrict__ x,
+                                     double *__restrict__ coef_len, double *__restrict__ cv_part, int *err) {
   constexpr int ne = nvc == 3 ? 3 : 6;
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= T) return;
   V3 v[nvc];
 #pragma unroll
   for (int k = 0; k < nvc; k++) v[k] = ld3(x + 3 * (int64_t)cells[nvc * c + k]);
-  V3 ev[ne];
+  // edge vectors and their inner products (lower triangle); the first nvc - 1
+  // edges are those at vertex 0
+  V3 r[ne];
+  double g[ne][ne];
+#pragma unroll
+  for (int i = 0; i < ne; i++) r[i] = v[pair1<nvc>(i)] - v[pair0<nvc>(i)];
+#pragma unroll
+  for (int i = 0; i < ne; i++)
+#pragma unroll
+    for (int j = 0; j <= i; j++) g[i][j] = dot(r[i], r[j]);
+  // (v_a - v_b) . (v_a - v_c)
+  auto ip = [&](int a, int b, int c) {
+    const int p = edge_of<nvc>(a, b), q = edge_of<nvc>(a, c);
+    const double d = g[p > q ? p : q][p > q ? q : p];
+    return (a < b) == (a < c) ? d : -d;
+  };
+  double l2[ne];  // squared edge lengths
+#pragma unroll
+  for (int k = 0; k < ne; k++) l2[k] = g[k][k];
   double len[ne];
 #pragma unroll
-  for (int k = 0; k < ne; k++) {
-    ev[k] = v[pair0<nvc>(k)] - v[pair1<nvc>(k)];
-    len[k] = norm(ev[k]);
-  }
-  double vol;
+  for (int k = 0; k < ne; k++) len[k] = sqrt(l2[k]);
+  double vol, t = 0.0, nn = 0.0;
+  V3 n12, n20, n01;
   if (nvc == 3) {
-    vol = 0.5 * norm(cross(ev[0], ev[1]));
+    const V3 cr = cross(r[0], r[1]);
+    nn = dot(cr, cr);
+    vol = 0.5 * sqrt(nn);
+    // degenerate triangle (the reference tests |omega| < 1e-10 absolutely,
+    // src/mesh.cpp:917-927; a scale-free test keeps fine meshes valid)
+    if (!(2.0 * nn > 1.0e-20 * (l2[0] * l2[2]))) atomicOr(err, 1);
   } else {
+    n12 = cross(r[1], r[2]);
+    n20 = cross(r[2], r[0]);
+    n01 = cross(r[0], r[1]);
+    t = dot(r[0], n12);
     // local edges 0,1,2 share local vertex 0: never coplanar
-    const double t = dot(ev[0], cross(ev[1], ev[2]));
     if (fabs(t) / (len[0] * len[1] * len[2]) < 1.0e-5) atomicOr(err, 2);
-    vol = fabs(t) / 6.0;
+    if (!(2.0 * fabs(t) > 1.0e-10 * (len[0] * len[1] * len[2]))) atomicOr(err, 8);
+    vol = fabs(t) * (1.0 / 6.0);
   }
-  double A[ne][ne], r[ne];
-#pragma unroll
-  for (int i = 0; i < ne; i++) {
-    const double a = dot(ev[i], ev[i]);
-    r[i] = vol * a;
-#pragma unroll
-    for (int j = 0; j < ne; j++) {
-      const double d = dot(ev[i], ev[j]);
-      A[i][j] = d * d;
-    }
-  }
-  if (!chol_solve<ne>(A, r)) atomicOr(err, 4);
-#pragma unroll
-  for (int k = 0; k < ne; k++) coef_len[ne * c + k] = r[k] * len[k];
-
-  // control volumes
   double share[nvc];
 #pragma unroll
   for (int k = 0; k < nvc; k++) share[k] = 0.0;
   if (nvc == 3) {
-    const V3 cc = tri_cc(v[0], v[1], v[2], err);
+    // |e|^2 cot / 8, cot = (x_0 - o) . (x_1 - o) / (2 area)
+    const double q = 0.125 / (2.0 * vol);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       const int e0 = pair0<3>(k), e1 = pair1<3>(k), o = 3 - e0 - e1;
-      const V3 mp = 0.5 * (v[e0] + v[e1]);
-      const double coedge = norm(mp - cc);
-      const V3 cell_n = cross(v[o] - v[e0], mp - v[e0]);
-      const V3 cc_n = cross(cc - v[e0], mp - v[e0]);
-      const double cov = copysign(coedge, dot(cc_n, cell_n));
-      const double pyr = 0.5 * len[k] * cov / 2;
-      share[e0] += pyr;
-      share[e1] += pyr;
+      const double s = q * (l2[k] * ip(o, e0, e1));
+      share[e0] += s;
+      share[e1] += s;
     }
   } else {
-    // tetrahedron circumcenter (src/mesh_tetra.cpp:377-415)
-    const V3 r0 = v[1] - v[0], r1 = v[2] - v[0], r2 = v[3] - v[0];
-    const V3 c12 = cross(r1, r2), c20 = cross(r2, r0), c01 = cross(r0, r1);
-    const double omega = 2.0 * dot(r0, c12);
-    if (!(fabs(omega) > 1.0e-10 * norm(r0) * norm(r1) * norm(r2))) atomicOr(err, 8);
-    const V3 cc = v[0] + (dot(r0, r0) / omega) * c12 + (dot(r1, r1) / omega) * c20 +
-                  (dot(r2, r2) / omega) * c01;
+    // circumcentre - v_0 (src/mesh_tetra.cpp:377-415)
+    const double h = 0.5 / t;
+    const V3 w = (g[0][0] * h) * n12 + (g[1][1] * h) * n20 + (g[2][2] * h) * n01;
+    const double sg = t > 0.0 ? 1.0 : -1.0;
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
-      const int e0 = pair0<4>(k), e1 = pair1<4>(k);
-      int o0 = -1, o1 = -1;
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (q != e0 && q != e1) {
-          if (o0 < 0) o0 = q;
-          else o1 = q;
-        }
-      const V3 x0 = v[e0], x1 = v[e1], p0 = v[o0], p1 = v[o1];
-      const V3 mp = 0.5 * (x0 + x1);
-      const V3 f0 = tri_cc(x0, x1, p0, err), f1 = tri_cc(x0, x1, p1, err);
-      const V3 gauge = cross(p0 - mp, p1 - mp);
-      const double a0 = 0.5 * norm(mp - f0) * norm(f0 - cc);
-      const double a1 = 0.5 * norm(mp - f1) * norm(f1 - cc);
-      const double cov = copysign(a0, dot(cross(f0 - mp, cc - mp), gauge)) +
-                         copysign(a1, dot(cross(cc - mp, f1 - mp), gauge));
-      const double pyr = 0.5 * len[k] * cov / 3;
-      share[e0] += pyr;
-      share[e1] += pyr;
+    for (int f = 0; f < 4; f++) {
+      // face opposite vertex f, its normal towards f (t = r_0 . n12 > 0 for
+      // the orientation below), w relative to one of its vertices
+      V3 N;
+      double wn;
+      if (f == 0) {
+        N = V3{-(n12.x + n20.x + n01.x), -(n12.y + n20.y + n01.y), -(n12.z + n20.z + n01.z)};
+        wn = dot(w, N) + t;  // (w - r_0) . N, r_0 . N = -t
+      } else {
+        N = f == 1 ? n12 : f == 2 ? n20 : n01;
+        wn = dot(w, N);
+      }
+      const double n2 = dot(N, N);
+      const double q = sg * wn / (24.0 * n2);
+      const int a = f == 0 ? 1 : 0, b = f <= 1 ? 2 : 1, d = f <= 2 ? 3 : 2;
+      // edges (a,b), (a,d), (b,d) with the angles at d, b, a
+      const double lab = l2[a == 0 ? b - 1 : a + b], lad = l2[a == 0 ? d - 1 : a + d], lbd = l2[b + d];
+      if (!(2.0 * n2 > 1.0e-20 * (lbd * fmax(lab, lad)))) atomicOr(err, 1);
+      const double sab = q * (lab * ip(d, a, b)), sad = q * (lad * ip(b, a, d)), sbd = q * (lbd * ip(a, b, d));
+      share[a] += sab + sad;
+      share[b] += sab + sbd;
+      share[d] += sad + sbd;
     }
   }
 #pragma unroll
   for (int k = 0; k < nvc; k++) cv_part[nvc * c + k] = share[k];
+  double A[ne][ne], rhs[ne];
+#pragma unroll
+  for (int i = 0; i < ne; i++) {
+    rhs[i] = vol * l2[i];
+#pragma unroll
+    for (int j = 0; j <= i; j++) A[i][j] = g[i][j] * g[i][j];
+  }
+  if (!chol_solve<ne>(A, rhs)) atomicOr(err, 4);
+#pragma unroll
+  for (int k = 0; k < ne; k++) coef_len[ne * c + k] = rhs[k] * len[k];
 }
 
-// out[i] = sum_{j in [ptr[i], ptr[i+1])} src[idx[j]] in list order
-// (deterministic segmented sum; the lists are in cell order, the order in
-// which the reference accumulates).
-__global__ void segmented_gather_sum(int64_t n, const int64_t *__restrict__ ptr,
-                                     const int32_t *__restrict__ idx,
-                                     const double *__restrict__ src,
-                                     double *__restrict__ out) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// Covolume of each edge: the coefficients of the cells around it, found among
+// the cells incident to its end with fewer of them, in cell order (the order
+// in which the reference accumulates; deterministic).
+template <int nvc>
+__global__ void edge_covolumes(int64_t E, const int32_t *__restrict__ edges, const int32_t *__restrict__ cells,
+                               const int32_t *__restrict__ ptr, const int32_t *__restrict__ vc,
+                               const double *__restrict__ coef_len, double *__restrict__ covol) {
+  constexpr int ne = nvc == 3 ? 3 : 6;
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  int32_t v = edges[2 * e], w = edges[2 * e + 1];
+  if (ptr[w + 1] - ptr[w] < ptr[v + 1] - ptr[v]) {
+    const int32_t t = v;
+    v = w, w = t;
+  }
   double s = 0.0;
-  for (int64_t j = ptr[i]; j < ptr[i + 1]; j++) s += src[idx[j]];
-  out[i] = s;
+  for (int j = ptr[v]; j < ptr[v + 1]; j++) {
+    const int32_t k = vc[j], c = k / nvc, a = k - c * nvc;
+#pragma unroll
+    for (int b = 0; b < nvc; b++)
+      if (cells[(int64_t)nvc * c + b] == w) s += coef_len[(int64_t)ne * c + edge_of<nvc>(a, b)];
+  }
+  covol[e] = s;
+}
+
+// out[v] = sum of the vertex's shares in cell order
+__global__ void vertex_sum(int64_t N, const int32_t *__restrict__ ptr, const int32_t *__restrict__ vc,
+                           const double *__restrict__ src, double *__restrict__ out) {
+  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (v >= N) return;
+  double s = 0.0;
+  for (int j = ptr[v]; j < ptr[v + 1]; j++) s += src[vc[j]];
+  out[v] = s;
 }
 
 __global__ void edge_length_kernel(int64_t E, const int32_t *__restrict__ edges,
@@ -232,7 +464,27 @@ void MeshImpl::validate(int64_t n_vertices, const int32_t *cells, int64_t n_cell
   NOSH_CHECK(n_cells * verts_per_cell < (int64_t)1 << 31 && n_vertices < (int64_t)1 << 30,
              NOSH_ERR_INVALID, "mesh too large for 32-bit indices");
   const int nvc = verts_per_cell;
-  // bounds of every index before anything is uploaded
+  // one pass without branches over everything, on the host's cores when the
+  // mesh is large; only a bad mesh is gone through again for its first fault
+  std::atomic<int> bad{0};
+  parallel_ranges(n_cells, 1 << 17, [&](int64_t b, int64_t e) {
+    unsigned f = 0;
+    for (int64_t k = nvc * b; k < nvc * e; k++) f |= (unsigned)((uint32_t)cells[k] >= (uint32_t)n_vertices);
+    if (nvc == 3) {
+      for (int64_t c = b; c < e; c++) {
+        const int32_t *q = cells + 3 * c;
+        f |= (unsigned)((q[0] == q[1]) | (q[0] == q[2]) | (q[1] == q[2]));
+      }
+    } else {
+      for (int64_t c = b; c < e; c++) {
+        const int32_t *q = cells + 4 * c;
+        f |= (unsigned)((q[0] == q[1]) | (q[0] == q[2]) | (q[0] == q[3]) | (q[1] == q[2]) | (q[1] == q[3]) |
+                        (q[2] == q[3]));
+      }
+    }
+    if (f) bad.store(1);
+  });
+  if (!bad.load()) return;
   for (int64_t k = 0; k < nvc * n_cells; k++)
     NOSH_CHECK(cells[k] >= 0 && cells[k] < n_vertices, NOSH_ERR_INVALID,
                "cell vertex index out of range at entry " + std::to_string(k));
@@ -251,12 +503,9 @@ MeshImpl::MeshImpl(const double *coords, int64_t n_vertices, const int32_t *cell
   ne = nvc == 3 ? 3 : 6;
   N = n_vertices;
   T = n_cells;
-  x.assign(coords, coords + 3 * N);
-  cells.assign(cells_in, cells_in + nvc * T);
   NOSH_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   try {
-    build_topology();
-    build_geometry();
+    build(coords, cells_in);
   } catch (...) {
     // a throwing constructor runs no destructor: release the stream here
     // (the device buffers free themselves)
@@ -271,157 +520,130 @@ MeshImpl::~MeshImpl() {
   if (stream) cudaStreamDestroy(stream);
 }
 
-void MeshImpl::build_topology() {
-  // vertex -> (cell*nvc + slot) incidence, in cell order
-  vc_ptr.assign(N + 1, 0);
-  for (int64_t k = 0; k < nvc * T; k++) vc_ptr[cells[k] + 1]++;
-  for (int64_t i = 0; i < N; i++) vc_ptr[i + 1] += vc_ptr[i];
-  vc_idx.resize(nvc * T);
-  {
-    std::vector<int64_t> fill(vc_ptr.begin(), vc_ptr.end() - 1);
-    for (int64_t k = 0; k < nvc * T; k++) vc_idx[fill[cells[k]]++] = (int32_t)k;
-  }
-  // neighbour sets: per vertex, sorted unique vertices of incident cells
-  auto neighbours = [&](int64_t v, std::vector<int32_t> &buf) {
-    buf.clear();
-    for (int64_t j = vc_ptr[v]; j < vc_ptr[v + 1]; j++) {
-      const int64_t c = vc_idx[j] / nvc;
+namespace {
+// exclusive scan of in[0..n) into out[0..n] on the stream; the total is left
+// in tile[number of tiles]
+int64_t scan(int64_t n, const int32_t *in, int32_t *out, int64_t *tile, cudaStream_t s) {
+  const int64_t nt = div_up(n, kScanTile);
+  scan_tiles<<<(unsigned)nt, kScanTile, 0, s>>>(n, in, tile);
+  scan_sums<<<1, kScanTile, 0, s>>>(nt, tile);
+  scan_write<<<(unsigned)nt, kScanTile, 0, s>>>(n, in, tile, out);
+  return nt;
+}
+inline int wide_grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(div_up(n, 256), 16 * kNumSMs)); }
+
+// The vertices with too many cells for the warp kernel: sorted codes and
+// neighbours from the host.
+void solve_hubs(int nvc, const int32_t *cells, const std::vector<int32_t> &hubs, const DevBuf<int32_t> &ptr,
+                DevBuf<int32_t> &vc, DevBuf<int32_t> &nb, DevBuf<int32_t> &deg, DevBuf<int32_t> &up, cudaStream_t s) {
+  std::vector<int32_t> code, u;
+  for (const int32_t v : hubs) {
+    int32_t pb[2];
+    NOSH_CUDA(cudaMemcpyAsync(pb, ptr.p + v, sizeof(pb), cudaMemcpyDeviceToHost, s));
+    NOSH_CUDA(cudaStreamSynchronize(s));
+    code.resize(pb[1] - pb[0]);
+    NOSH_CUDA(cudaMemcpyAsync(code.data(), vc.p + pb[0], code.size() * 4, cudaMemcpyDeviceToHost, s));
+    NOSH_CUDA(cudaStreamSynchronize(s));
+    std::sort(code.begin(), code.end());
+    u.clear();
+    for (const int32_t k : code)
       for (int q = 0; q < nvc; q++) {
-        const int32_t w = cells[nvc * c + q];
-        if (w != v) buf.push_back(w);
+        const int32_t w = cells[(int64_t)(k / nvc) * nvc + q];
+        if (w != v) u.push_back(w);
       }
-    }
-    std::sort(buf.begin(), buf.end());
-    buf.erase(std::unique(buf.begin(), buf.end()), buf.end());
-  };
-  std::vector<int32_t> deg(N), up(N);
-  parallel_for(N, [&](int64_t v) {
-    thread_local std::vector<int32_t> buf;
-    neighbours(v, buf);
-    deg[v] = (int32_t)buf.size();
-    up[v] = (int32_t)(buf.end() - std::upper_bound(buf.begin(), buf.end(), (int32_t)v));
-  });
-  rp.assign(N + 1, 0);
-  edge_base.assign(N + 1, 0);
-  for (int64_t v = 0; v < N; v++) {
-    rp[v + 1] = rp[v] + deg[v];
-    edge_base[v + 1] = edge_base[v] + up[v];
-  }
-  NOSH_CHECK(rp[N] < (int64_t)1 << 31, NOSH_ERR_INVALID, "too many edges");
-  E = edge_base[N];
-  ci.resize(rp[N]);
-  parallel_for(N, [&](int64_t v) {
-    thread_local std::vector<int32_t> buf;
-    neighbours(v, buf);
-    std::copy(buf.begin(), buf.end(), ci.begin() + rp[v]);
-  });
-  // edges in lexicographic order: the upper neighbours of each vertex
-  edges.resize(2 * E);
-  pos_fwd.resize(E);
-  pos_bwd.resize(E);
-  nz_edge.resize(rp[N]);
-  parallel_for(N, [&](int64_t v) {
-    const int32_t *b = ci.data() + rp[v], *e = ci.data() + rp[v + 1];
-    const int32_t *u = std::upper_bound(b, e, (int32_t)v);
-    int64_t id = edge_base[v];
-    for (const int32_t *q = u; q < e; q++, id++) {
-      edges[2 * id] = (int32_t)v;
-      edges[2 * id + 1] = *q;
-      pos_fwd[id] = (int32_t)(q - ci.data());
-      const int32_t *wb = ci.data() + rp[*q], *we = ci.data() + rp[*q + 1];
-      pos_bwd[id] = (int32_t)(std::lower_bound(wb, we, (int32_t)v) - ci.data());
-    }
-  });
-  parallel_for(E, [&](int64_t e) {
-    nz_edge[pos_fwd[e]] = (int32_t)e;
-    nz_edge[pos_bwd[e]] = ~(int32_t)e;
-  });
-  // cell -> edge ids
-  const int(*pairs)[2] = nvc == 3 ? TRI_PAIRS : TET_PAIRS;
-  cell_edges.resize(ne * T);
-  parallel_for(T, [&](int64_t c) {
-    for (int k = 0; k < ne; k++) {
-      int32_t a = cells[nvc * c + pairs[k][0]], b = cells[nvc * c + pairs[k][1]];
-      const int32_t lo = std::min(a, b), hi = std::max(a, b);
-      const int32_t *rb = ci.data() + rp[lo], *re = ci.data() + rp[lo + 1];
-      const int32_t *u = std::upper_bound(rb, re, lo);
-      cell_edges[ne * c + k] = (int32_t)(edge_base[lo] + (std::lower_bound(u, re, hi) - u));
-    }
-  });
-  // edge -> (cell*ne + slot) incidence in cell order (covolume accumulation)
-  ec_ptr.assign(E + 1, 0);
-  for (int64_t k = 0; k < ne * T; k++) ec_ptr[cell_edges[k] + 1]++;
-  for (int64_t e = 0; e < E; e++) ec_ptr[e + 1] += ec_ptr[e];
-  ec_idx.resize(ne * T);
-  {
-    std::vector<int64_t> fill(ec_ptr.begin(), ec_ptr.end() - 1);
-    for (int64_t k = 0; k < ne * T; k++) ec_idx[fill[cell_edges[k]]++] = (int32_t)k;
+    std::sort(u.begin(), u.end());
+    u.erase(std::unique(u.begin(), u.end()), u.end());
+    const int32_t d = (int32_t)u.size(), a = (int32_t)(u.end() - std::upper_bound(u.begin(), u.end(), v));
+    NOSH_CUDA(cudaMemcpyAsync(vc.p + pb[0], code.data(), code.size() * 4, cudaMemcpyHostToDevice, s));
+    NOSH_CUDA(cudaMemcpyAsync(nb.p + (int64_t)(nvc - 1) * pb[0], u.data(), u.size() * 4, cudaMemcpyHostToDevice, s));
+    NOSH_CUDA(cudaMemcpyAsync(deg.p + v, &d, 4, cudaMemcpyHostToDevice, s));
+    NOSH_CUDA(cudaMemcpyAsync(up.p + v, &a, 4, cudaMemcpyHostToDevice, s));
+    NOSH_CUDA(cudaStreamSynchronize(s));
   }
 }
+}  // namespace
 
-void MeshImpl::build_geometry() {
+void MeshImpl::build(const double *coords, const int32_t *cells) {
   cudaStream_t s = stream;
-  d_x.upload(x, s);
-  d_edges.upload(edges, s);
+  const int64_t nk = nvc * T;
   DevBuf<int32_t> d_cells;
-  d_cells.upload(cells, s);
-  DevBuf<double> coef_len(ne * T), cv_part(nvc * T);
-  DevBuf<int> err(1);
-  err.zero(s);
+  d_cells.upload(cells, nk, s);
+  d_x.upload(coords, 3 * N, s);
+  // geometry of the cells
+  DevBuf<double> coef_len(ne * T), cv_part(nk);
+  DevBuf<int> flags(4);  // geometry errors, hubs, longest row, longest row block
+  flags.zero(s);
   const int B = 128;
   if (nvc == 3)
-    cell_geometry_kernel<3><<<div_up(T, B), B, 0, s>>>(T, d_cells.p, d_x.p, coef_len.p, cv_part.p, err.p);
+    cell_geometry_kernel<3><<<div_up(T, B), B, 0, s>>>(T, d_cells.p, d_x.p, coef_len.p, cv_part.p, flags.p);
   else
-    cell_geometry_kernel<4><<<div_up(T, B), B, 0, s>>>(T, d_cells.p, d_x.p, coef_len.p, cv_part.p, err.p);
+    cell_geometry_kernel<4><<<div_up(T, B), B, 0, s>>>(T, d_cells.p, d_x.p, coef_len.p, cv_part.p, flags.p);
+  // vertex -> (cell, slot) incidence and neighbours
+  DevBuf<int32_t> cnt(N), ptr(N + 1), vc(nk), nb((nvc - 1) * nk), deg(N), up(N), hubs(N), ebase(N + 1);
+  DevBuf<int64_t> tile(div_up(N, kScanTile) + 1);
+  cnt.zero(s);
+  count_incident<<<wide_grid(nk), 256, 0, s>>>(nk, d_cells.p, cnt.p);
+  scan(N, cnt.p, ptr.p, tile.p, s);
+  NOSH_CUDA(cudaMemcpyAsync(cnt.p, ptr.p, N * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+  scatter_incident<<<wide_grid(nk), 256, 0, s>>>(nk, d_cells.p, cnt.p, vc.p);
+  const int ng = (int)std::min<int64_t>(div_up(N, kNbWarps), 1 << 20);
+  if (nvc == 3)
+    neighbour_kernel<3><<<ng, 32 * kNbWarps, 0, s>>>(N, d_cells.p, ptr.p, vc.p, nb.p, deg.p, up.p, hubs.p,
+                                                     flags.p + 1);
+  else
+    neighbour_kernel<4><<<ng, 32 * kNbWarps, 0, s>>>(N, d_cells.p, ptr.p, vc.p, nb.p, deg.p, up.p, hubs.p,
+                                                     flags.p + 1);
   NOSH_CUDA(cudaGetLastError());
+  int h[4] = {0, 0, 0, 0};
+  flags.download(h, 2, s);
+  NOSH_CUDA(cudaStreamSynchronize(s));
+  NOSH_CHECK(h[0] == 0, NOSH_ERR_MESH, "degenerate cell(s) in the mesh (flags " + std::to_string(h[0]) + ")");
+  if (h[1] > 0) {
+    std::vector<int32_t> hv(h[1]);
+    hubs.download(hv.data(), hv.size(), s);
+    NOSH_CUDA(cudaStreamSynchronize(s));
+    solve_hubs(nvc, cells, hv, ptr, vc, nb, deg, up, s);
+  }
+  // row pointers and first edges
+  d_rp.alloc(N + 1);
+  int64_t total[2];
+  NOSH_CUDA(cudaMemcpyAsync(&total[0], tile.p + scan(N, deg.p, d_rp.p, tile.p, s), sizeof(int64_t),
+                            cudaMemcpyDeviceToHost, s));
+  NOSH_CUDA(cudaMemcpyAsync(&total[1], tile.p + scan(N, up.p, ebase.p, tile.p, s), sizeof(int64_t),
+                            cudaMemcpyDeviceToHost, s));
+  row_extents<<<div_up(N, 256), 256, 0, s>>>(N, d_rp.p, flags.p + 2);
+  flags.download(h, 4, s);
+  NOSH_CUDA(cudaStreamSynchronize(s));
+  NOSH_CHECK(total[0] < (int64_t)1 << 31, NOSH_ERR_INVALID, "too many edges");
+  E = total[1];
+  max_row = h[2];
+  max_block = h[3];
+  // column indices padded by kPad entries so that 128-bit staged loads of a
+  // row block may run past its end
+  d_ci.alloc(2 * E + kPad);
+  NOSH_CUDA(cudaMemsetAsync(d_ci.p + 2 * E, 0, kPad * sizeof(int32_t), s));
+  d_edges.alloc(2 * E);
+  d_pos_fwd.alloc(E);
+  d_pos_bwd.alloc(E);
+  d_nz_edge.alloc(2 * E);
   d_len.alloc(E);
   d_covol.alloc(E);
   d_cv.alloc(N);
+  graph_rows<<<div_up(16 * N, 256), 256, 0, s>>>(N, nvc, ptr.p, nb.p, d_rp.p, up.p, ebase.p, d_ci.p, d_edges.p,
+                                                 d_pos_fwd.p, d_nz_edge.p);
+  graph_back<<<div_up(E, 256), 256, 0, s>>>(E, d_edges.p, d_rp.p, d_ci.p, d_pos_bwd.p, d_nz_edge.p);
   edge_length_kernel<<<div_up(E, 256), 256, 0, s>>>(E, d_edges.p, d_x.p, d_len.p);
-  {
-    DevBuf<int64_t> p(E + 1);
-    DevBuf<int32_t> idx;
-    p.upload(ec_ptr, s);
-    idx.upload(ec_idx, s);
-    segmented_gather_sum<<<div_up(E, 256), 256, 0, s>>>(E, p.p, idx.p, coef_len.p, d_covol.p);
-    DevBuf<int64_t> vp(N + 1);
-    DevBuf<int32_t> vidx;
-    vp.upload(vc_ptr, s);
-    vidx.upload(vc_idx, s);
-    segmented_gather_sum<<<div_up(N, 256), 256, 0, s>>>(N, vp.p, vidx.p, cv_part.p, d_cv.p);
-    NOSH_CUDA(cudaGetLastError());
-    int herr = 0;
-    err.download(&herr, 1, s);
-    NOSH_CUDA(cudaStreamSynchronize(s));
-    NOSH_CHECK(herr == 0, NOSH_ERR_MESH,
-               "degenerate cell(s) in the mesh (flags " + std::to_string(herr) + ")");
-  }
-  // device copies of the KEO graph / scatter map used by every operator
-  {
-    std::vector<int32_t> rp32(rp.begin(), rp.end());
-    d_rp.upload(rp32, s);
-    NOSH_CUDA(cudaStreamSynchronize(s));
-  }
-  // column indices padded by kPad entries so that 128-bit staged loads of a
-  // row block may run past its end
-  d_ci.alloc(ci.size() + kPad);
-  NOSH_CUDA(cudaMemsetAsync(d_ci.p, 0, (ci.size() + kPad) * sizeof(int32_t), s));
-  NOSH_CUDA(cudaMemcpyAsync(d_ci.p, ci.data(), ci.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  d_pos_fwd.upload(pos_fwd, s);
-  d_pos_bwd.upload(pos_bwd, s);
-  d_nz_edge.upload(nz_edge, s);
-  NOSH_CUDA(cudaStreamSynchronize(s));
-  // host copies of the geometry for the query entry points
-  h_len.resize(E);
-  h_covol.resize(E);
-  h_cv.resize(N);
-  d_len.download(h_len.data(), E, s);
-  d_covol.download(h_covol.data(), E, s);
-  d_cv.download(h_cv.data(), N, s);
+  if (nvc == 3)
+    edge_covolumes<3><<<div_up(E, 256), 256, 0, s>>>(E, d_edges.p, d_cells.p, ptr.p, vc.p, coef_len.p, d_covol.p);
+  else
+    edge_covolumes<4><<<div_up(E, 256), 256, 0, s>>>(E, d_edges.p, d_cells.p, ptr.p, vc.p, coef_len.p, d_covol.p);
+  vertex_sum<<<div_up(N, 256), 256, 0, s>>>(N, ptr.p, vc.p, cv_part.p, d_cv.p);
+  NOSH_CUDA(cudaGetLastError());
   NOSH_CUDA(cudaStreamSynchronize(s));
 }
 
-void MeshImpl::complex_graph(int32_t *row_ptr, int32_t *cols) const {
+void MeshImpl::complex_graph(int32_t *row_ptr, int32_t *cols) {
+  const std::vector<int32_t> &rp = this->rp(), &ci = this->ci();
   row_ptr[0] = 0;
   for (int64_t v = 0; v < N; v++) {
     const int64_t b = rp[v], e = rp[v + 1], o = row_ptr[v];

@@ -1,5 +1,7 @@
-// Mesh handle: host integer data + device geometry / KEO graph.
+// Mesh handle: device geometry and KEO graph, host copies on demand.
 #pragma once
+
+#include <mutex>
 
 #include "common.cuh"
 
@@ -9,28 +11,15 @@ struct MeshImpl {
   int nvc = 0, ne = 0;  // vertices / edges per cell
   int64_t N = 0, E = 0, T = 0;
   cudaStream_t stream = nullptr;
+  // the longest row of the off-diagonal KEO graph, and the longest 4-aligned
+  // range of nonzeros of 128 consecutive rows from a multiple of 128
+  int max_row = 0, max_block = 0;
 
-  // host: input and integer work
-  std::vector<double> x;          // 3N
-  std::vector<int32_t> cells;     // nvc*T
-  std::vector<int32_t> edges;     // 2E, v0 < v1, lexicographic
-  std::vector<int32_t> cell_edges;  // ne*T
-  std::vector<int64_t> edge_base;   // N+1: first edge id whose v0 == v
-  // off-diagonal KEO graph ("adjacency CSR"): row v = sorted neighbours
-  std::vector<int64_t> rp;        // N+1
-  std::vector<int32_t> ci;        // 2E
-  std::vector<int32_t> nz_edge;   // 2E: edge of each nonzero (~e if row is v1)
-  std::vector<int32_t> pos_fwd, pos_bwd;  // E: nonzero of (v0,v1) / (v1,v0)
-  std::vector<int64_t> vc_ptr;    // N+1, vertex -> cell*nvc+slot (cell order)
-  std::vector<int32_t> vc_idx;
-  std::vector<int64_t> ec_ptr;    // E+1, edge -> cell*ne+slot (cell order)
-  std::vector<int32_t> ec_idx;
-  std::vector<double> h_len, h_covol, h_cv;
-
-  // device
+  // device: coordinates, edges (v0 < v1, lexicographic), geometry, the
+  // off-diagonal KEO graph (row v: its sorted neighbours), each nonzero's edge
+  // (~e if the row is v1), the nonzeros of (v0, v1) and (v1, v0) of each edge
   DevBuf<double> d_x, d_len, d_covol, d_cv;
   DevBuf<int32_t> d_edges;
-  DevBuf<int64_t> d_rp64;
   DevBuf<int32_t> d_rp, d_ci, d_nz_edge, d_pos_fwd, d_pos_bwd;
 
   // expects a description that validate() accepted
@@ -44,12 +33,33 @@ struct MeshImpl {
   MeshImpl(const MeshImpl &) = delete;
   MeshImpl &operator=(const MeshImpl &) = delete;
 
+  // host copies, fetched from the device on first use (a mesh may serve
+  // several handles and threads)
+  const std::vector<int32_t> &edges() { return fetch(h_edges_, d_edges, 2 * E); }
+  const std::vector<int32_t> &rp() { return fetch(h_rp_, d_rp, N + 1); }
+  const std::vector<int32_t> &ci() { return fetch(h_ci_, d_ci, 2 * E); }
+  const std::vector<double> &len() { return fetch(h_len_, d_len, E); }
+  const std::vector<double> &covol() { return fetch(h_covol_, d_covol, E); }
+  const std::vector<double> &cv() { return fetch(h_cv_, d_cv, N); }
+
   // complex graph with the diagonal (row_ptr[N+1], cols[N+2E])
-  void complex_graph(int32_t *row_ptr, int32_t *cols) const;
+  void complex_graph(int32_t *row_ptr, int32_t *cols);
 
  private:
-  void build_topology();
-  void build_geometry();
+  std::mutex fetch_mtx_;
+  std::vector<int32_t> h_edges_, h_rp_, h_ci_;
+  std::vector<double> h_len_, h_covol_, h_cv_;
+  template <typename V>
+  const std::vector<V> &fetch(std::vector<V> &h, const DevBuf<V> &d, int64_t n) {
+    std::lock_guard<std::mutex> lock(fetch_mtx_);
+    if ((int64_t)h.size() != n) {
+      h.resize(n);
+      NOSH_CUDA(cudaMemcpyAsync(h.data(), d.p, n * sizeof(V), cudaMemcpyDeviceToHost, stream));
+      NOSH_CUDA(cudaStreamSynchronize(stream));
+    }
+    return h;
+  }
+  void build(const double *coords, const int32_t *cells);
 };
 
 }  // namespace nosh

@@ -1377,11 +1377,12 @@ Mpnn::Impl::Impl(NlsImpl &nls) : s(nls), N(nls.N), nnz(2 * nls.E), stream(nls.st
   s.d_alpha.download(alpha.data(), s.E, st);
   s.d_p.download(p.data(), s.E, st);
   s.sync();
+  const std::vector<double> &len = m.len();
   double sa = 0, sp = 0, sl = 0;
   for (int64_t e = 0; e < s.E; e++) {
     sa += std::fabs(alpha[e]);
     sp += p[e] * p[e];
-    sl += m.h_len[e];
+    sl += len[e];
   }
   const double ia = sa > 0 ? s.E / sa : 1.0, ip = sp > 0 ? 1.0 / std::sqrt(sp / s.E) : 1.0,
                il = sl > 0 ? s.E / sl : 1.0;

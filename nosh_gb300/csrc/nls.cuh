@@ -242,9 +242,8 @@ struct NlsImpl {
   // bounds for residual_update's rounding (computed once): the largest row
   // sum of |K| (mu-independent: |K_ij| = |alpha_ij|) and the longest row
   double keo_abs_rowmax();
-  int max_row_nnz();
+  int max_row_nnz() const { return mesh->max_row; }
   double abs_rowmax_ = -1.0;
-  int max_row_nnz_ = -1;
   void dfdp64(const double *x, double g, double mu, int param, double *out);
   // F(xa) into fa and F(xb) into fb in one pass, norms[0..1] = their norms
   // (synchronises); with sa / sb, also the off-diagonal sums of K xa / K xb

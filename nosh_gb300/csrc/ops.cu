@@ -231,6 +231,13 @@ __global__ void energy_kernel(int64_t N, const double *__restrict__ cv,
   grid_reduce(v, partials, counter, out);
 }
 
+__global__ void sum_kernel(int64_t n, const double *__restrict__ a, double *partials, unsigned *counter, double *out) {
+  double v = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    v += a[i];
+  grid_reduce(v, partials, counter, out);
+}
+
 __global__ void inner_kernel(int64_t N, const double *__restrict__ cv,
                              const C2<double> *__restrict__ a, const C2<double> *__restrict__ b,
                              double *partials, unsigned *counter, double *out) {
@@ -271,13 +278,8 @@ __global__ void export_kernel(int64_t N, const int32_t *__restrict__ rp,
 template <typename T>
 int staging_cap(const MeshImpl &m) {
   // largest staged range of any row block, capped by the shared memory
-  int64_t mx = 0;
-  for (int64_t r0 = 0; r0 < m.N; r0 += kRows) {
-    const int64_t r1 = std::min<int64_t>(m.N, r0 + kRows);
-    mx = std::max<int64_t>(mx, m.rp[r1] - (m.rp[r0] & ~(int64_t)3));
-  }
-  mx = (mx + 3) & ~(int64_t)3;
-  return (int)std::min<int64_t>(mx, stage_limit<T>());
+  static_assert(kRows == 128, "MeshImpl::max_block is of 128 rows");
+  return (int)std::min<int64_t>((m.max_block + 3) & ~3, stage_limit<T>());
 }
 
 template <typename T, class Op>
@@ -623,8 +625,11 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
   cap32 = staging_cap<float>(*m);
   cap64 = staging_cap<double>(*m);
   tune_schedules();
-  for (double c : m->h_cv) cv_sum += c;
+  sum_kernel<<<reduce_grid(N), 256, 0, s>>>(N, m->d_cv.p, red.partials.p, red.counter.p, red.host);
+  ++launch_count;
+  NOSH_CUDA(cudaGetLastError());
   sync();
+  cv_sum = red.host[0];
 }
 
 void NlsImpl::set_systems(const int64_t *offsets, int64_t num, const double *mu) {
@@ -634,7 +639,7 @@ void NlsImpl::set_systems(const int64_t *offsets, int64_t num, const double *mu)
     NOSH_CHECK(offsets[q + 1] > offsets[q], NOSH_ERR_INVALID, "every system needs at least one vertex");
   // edge -> system, and no edge between two systems
   std::vector<int32_t> es(E);
-  const std::vector<int32_t> &ed = mesh->edges;  // 2E, sorted pairs
+  const std::vector<int32_t> &ed = mesh->edges();  // 2E, sorted pairs
   for (int64_t e = 0; e < E; e++) {
     const int64_t a = ed[2 * e], b = ed[2 * e + 1];
     const int64_t sa = std::upper_bound(offsets, offsets + num + 1, a) - offsets - 1;
@@ -702,7 +707,13 @@ void NlsImpl::tune_schedules() {
   } else {
     warp32 = pick_warp_schedule<float>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo32.p, cap32, red.partials.p,
                                        red.counter.p, stream);
-    warp64 = pick_warp_schedule<double>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo64.p, cap64, red.partials.p,
+    // FP64 rows of a mesh graph are never faster in the warp schedule, whose
+    // shuffles of sums go through the FP64 pipe: 127 us against 55 at 64^3 (14
+    // neighbours), 21 against 8.7 at 17^2 (6).  Timing both took 3.8 ms of a
+    // 64^3 handle's set-up; only longer rows, where a half-warp has more than
+    // two rounds of work a row, are still timed.
+    warp64 = mesh->max_row > 32 &&
+             pick_warp_schedule<double>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo64.p, cap64, red.partials.p,
                                         red.counter.p, stream);
   }
 }
@@ -828,15 +839,6 @@ double NlsImpl::keo_abs_rowmax() {
   std::memcpy(&v, &h, sizeof(v));
   abs_rowmax_ = v * (1.0 + std::ldexp(1.0, -22));
   return abs_rowmax_;
-}
-
-int NlsImpl::max_row_nnz() {
-  if (max_row_nnz_ < 0) {
-    int m = 0;
-    for (int64_t i = 0; i < N; i++) m = std::max(m, (int)(mesh->rp[i + 1] - mesh->rp[i]));
-    max_row_nnz_ = m;
-  }
-  return max_row_nnz_;
 }
 
 void NlsImpl::residual_pair(const double *xa, const double *xb, double g, double mu, double *fa, double *fb,
