@@ -11,7 +11,9 @@
 // The integer work is a vertex -> cell incidence (counting, scan, scatter),
 // then a warp per vertex that sorts its incident cells (so that every later
 // sum runs in cell order, whatever order the scatter left) and its neighbours.
-// On the host it took 60 of the 75 ms of a 64^3 mesh.
+// At 64^3 (1.57 M tetrahedra) 0.65 ms on the device, 60 of the 75 ms of the
+// whole mesh on the host's cores; the mesh now takes 4.9 ms, half of them the
+// copies of its description.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -111,7 +113,8 @@ __global__ void __launch_bounds__(kScanTile) scan_write(int64_t n, const int32_t
 // repetition at nb + (nvc - 1) ptr[v], their number and how many are above v.
 // Ranks by counting in shared memory: a vertex of a tetrahedral mesh has some
 // 24 cells and 72 candidates.  Vertices with more than kMaxIncident cells are
-// left to the host, listed in `hubs`.
+// left to the host, listed in `hubs`.  Bound by the counting loops (0.49 ms at
+// 64^3).
 constexpr int kMaxIncident = 84;  // 3 x 84 candidates
 constexpr int kNbWarps = 4;
 template <int nvc>
@@ -299,9 +302,9 @@ __device__ __forceinline__ bool chol_solve(double (&A)[n][n], double (&r)[n]) {
 // over F, and with cot = (a . b) / |N|, h = (w . N) / |N| (N = F's normal,
 // twice its area, towards the opposite vertex; w from F to the circumcentre)
 // no square root is left: a share of |e|^2 / 24 (a . b) (w . N) / |N|^2 to
-// either end.  About 490 FP64 instructions a tetrahedron; with every
-// circumcentre, norm and cross product formed as such it took 1960 (5.46 ms at
-// 64^3).
+// either end.  486 FP64 instructions a warp, 1.37 ms at 64^3 (81 % of the FP64
+// pipe's rate); with every circumcentre, norm and cross product formed as such
+// 1962 and 5.46 ms.
 template <int nvc>
 __global__ void cell_geometry_kernel(int64_t T, const int32_t *__restrict__ cells, const double *__restrict__ x,
                                      double *__restrict__ coef_len, double *__restrict__ cv_part, int *err) {
@@ -411,7 +414,9 @@ __global__ void cell_geometry_kernel(int64_t T, const int32_t *__restrict__ cell
 
 // Covolume of each edge: the coefficients of the cells around it, found among
 // the cells incident to its end with fewer of them, in cell order (the order
-// in which the reference accumulates; deterministic).
+// in which the reference accumulates; deterministic).  Bound by the latency of
+// the cells' gathers: 0.34 ms at 64^3, without the lists of cells of each edge
+// that the host took 25 ms to make.
 template <int nvc>
 __global__ void edge_covolumes(int64_t E, const int32_t *__restrict__ edges, const int32_t *__restrict__ cells,
                                const int32_t *__restrict__ ptr, const int32_t *__restrict__ vc,
