@@ -443,6 +443,27 @@ __global__ void lanczos_first(int64_t n, const MinresScalars *__restrict__ s,
   cheb_first_elem<T>(i, dinv, coef[0], bi, d, x);
 }
 
+// The same for a union of systems: each vertex takes its system's
+// coefficients, a frozen system's new vector is zero.
+template <typename T>
+__global__ void lanczos_first_sys(int64_t n, const int32_t *__restrict__ vsys, const MinresScalars *__restrict__ sc,
+                                  const C2<T> *__restrict__ u, C2<T> *__restrict__ r_old,
+                                  const C2<T> *__restrict__ r_cur, const T *__restrict__ dinv,
+                                  const T *__restrict__ coef, C2<T> *__restrict__ d, C2<T> *__restrict__ x,
+                                  const int *halt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const MinresScalars *s = sc + (i < n ? vsys[i] : 0);
+  dep_sync();
+  if (i >= n || (halt && *halt >= 2)) return;
+  const C2<T> ui = u[i], ro = r_old[i], rc = r_cur[i];
+  const T *la = lanczos_coef<T>(s);
+  const T a = la[0], bb = la[1], c = la[2];
+  C2<T> bi{a * ui.x - bb * ro.x - c * rc.x, a * ui.y - bb * ro.y - c * rc.y};
+  if (s->done >= 2) bi = C2<T>{0, 0};
+  r_old[i] = bi;
+  cheb_first_elem<T>(i, dinv, coef[0], bi, d, x);
+}
+
 // Chebyshev step with SpMV (grid kernel epilogue)
 template <typename T>
 struct ChebOp {
@@ -481,6 +502,25 @@ struct ChebMinresOp {
   __device__ void hook(double total) const { minres_advance(s, total); }
 };
 
+// The fine level's last step of a batch: also rowdot[i] = <b_i, x_i>.
+template <typename T>
+struct ChebRowDotOp {
+  static constexpr bool kReduce = false;
+  const T *dia, *dinv, *coef;
+  int step;
+  const C2<T> *b, *xin;
+  C2<T> *d, *xout;
+  double *rowdot;
+  const int *halt = nullptr;
+  using Pre = ChebPre<T>;
+  __device__ Pre load(int i) const { return cheb_load<T>(i, step, dia, dinv, b, xin, d); }
+  __device__ double finish(int i, T sr, T si, const Pre &p) const {
+    const C2<T> z = cheb_apply<T>(i, step, sr, si, p, coef, d, xout);
+    rowdot[i] = (double)p.bi.x * (double)z.x + (double)p.bi.y * (double)z.y;
+    return 0.0;
+  }
+};
+
 // res = b - A x
 template <typename T>
 struct ResidOp {
@@ -502,44 +542,63 @@ struct ResidOp {
   }
 };
 
-// Restriction: aggregate sums of the finer level's residual, a half-warp
-// per aggregate (lanes take every 16th member, then a shuffle tree), so the
-// coarse levels' few thousand aggregates spread over the whole GPU instead
-// of a few dozen CTAs each walking its members serially.
-constexpr int kAggLanes = 16;
-template <typename T>
+// Restriction: aggregate sums of the finer level's residual, LN lanes per
+// aggregate and then a shuffle tree, so the coarse levels' few thousand
+// aggregates spread over the whole GPU instead of a few dozen CTAs each
+// walking its members serially.  In FP32 a lane takes every LN-th member, both
+// components.  In FP64 the launch's time is that of its additions, and a lane
+// pair takes the two components of every LN / 2-th member: half the additions
+// of the tree.  The two restrictions of a cycle over 226 K vertices of
+// triangle meshes 9.0 -> 6.3 us each; 6.1 us at 32^3 tetrahedral, where 4 lanes
+// with both components took 8.6.
+template <typename T, int LN>
 __device__ __forceinline__ C2<T> aggregate_sum(int64_t a, int64_t na, int li, const int32_t *__restrict__ mptr,
                                                const int32_t *__restrict__ midx, const C2<T> *__restrict__ r) {
+  if (sizeof(T) == 8) {
+    const T *rc = reinterpret_cast<const T *>(r) + (li & 1);
+    T s = 0;
+    if (a < na)
+      for (int32_t q = mptr[a] + (li >> 1); q < mptr[a + 1]; q += LN / 2) s += rc[2 * (int64_t)midx[q]];
+#pragma unroll
+    for (int o = LN / 2; o > 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return C2<T>{s, __shfl_xor_sync(0xffffffffu, s, 1)};
+  }
   T sr = 0, si = 0;
   if (a < na)
-    for (int32_t q = mptr[a] + li; q < mptr[a + 1]; q += kAggLanes) {
+    for (int32_t q = mptr[a] + li; q < mptr[a + 1]; q += LN) {
       const C2<T> v = r[midx[q]];
       sr += v.x;
       si += v.y;
     }
 #pragma unroll
-  for (int o = kAggLanes / 2; o > 0; o >>= 1) {
+  for (int o = LN / 2; o > 0; o >>= 1) {
     sr += __shfl_xor_sync(0xffffffffu, sr, o);
     si += __shfl_xor_sync(0xffffffffu, si, o);
   }
   return C2<T>{sr, si};
 }
-
+// Lanes per aggregate: half of them where an aggregate has few members (of a
+// triangle mesh some 9, of a tetrahedral one some 25) and the sums are FP64.
 template <typename T>
+inline bool few_members(int64_t n, int64_t na) {
+  return sizeof(T) == 8 && n <= 14 * na;
+}
+
+template <typename T, int LN>
 __global__ void restrict_kernel(int64_t na, const int32_t *__restrict__ mptr,
                                 const int32_t *__restrict__ midx, const C2<T> *__restrict__ r,
                                 C2<T> *__restrict__ rc, const int *halt) {
   dep_sync();
   if (halt && *halt >= 2) return;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t a = t / kAggLanes;
-  const int li = (int)(t % kAggLanes);
-  const C2<T> b = aggregate_sum<T>(a, na, li, mptr, midx, r);
+  const int64_t a = t / LN;
+  const int li = (int)(t % LN);
+  const C2<T> b = aggregate_sum<T, LN>(a, na, li, mptr, midx, r);
   if (a < na && li == 0) rc[a] = b;
 }
 
 // restriction fused with the coarse level's first Chebyshev step
-template <typename T>
+template <typename T, int LN>
 __global__ void restrict_first(int64_t na, const int32_t *__restrict__ mptr,
                                const int32_t *__restrict__ midx, const C2<T> *__restrict__ r,
                                C2<T> *__restrict__ rc, const T *__restrict__ dinv,
@@ -548,9 +607,9 @@ __global__ void restrict_first(int64_t na, const int32_t *__restrict__ mptr,
   dep_sync();
   if (halt && *halt >= 2) return;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t a = t / kAggLanes;
-  const int li = (int)(t % kAggLanes);
-  const C2<T> b = aggregate_sum<T>(a, na, li, mptr, midx, r);
+  const int64_t a = t / LN;
+  const int li = (int)(t % LN);
+  const C2<T> b = aggregate_sum<T, LN>(a, na, li, mptr, midx, r);
   if (a < na && li == 0) {
     rc[a] = b;
     cheb_first_elem<T>(a, dinv, coef[0], b, d, x);
@@ -1348,7 +1407,8 @@ struct Amg::Impl {
   template <typename T> const T *dia(int l);
   template <typename T> const T *dense_inv();
   template <typename T, class Op> void rows(int l, const C2<T> *x, const Op &op);
-  template <typename T> void descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *ms);
+  template <typename T>
+  void descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *ms, double *rowdot = nullptr);
   // the MINRES state's `done` while a MINRES V-cycle is being issued: its
   // launches return at once once the solve has converged
   const int *halt = nullptr;
@@ -1798,9 +1858,10 @@ void Amg::Impl::rows(int l, const C2<T> *x, const Op &op) {
 
 // Level l of the V-cycle after its first Chebyshev step: finish the
 // pre-smoothing (its result ends in x), coarse correction, post-smoothing.
-// With ms != nullptr the fine level's last step also advances MINRES.
+// With ms != nullptr the fine level's last step also advances MINRES, with
+// rowdot != nullptr it writes each vertex's <b, x>.
 template <typename T>
-void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *ms) {
+void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *ms, double *rowdot) {
   AmgVals<T> &V = vals<T>();
   AmgLevel &A = lev[l];
   cudaStream_t st = nls.stream;
@@ -1846,17 +1907,18 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
     a.f_n = A.n;
     launch_tail<T>(P, a, ovl());
   } else {
+    const bool few = few_members<T>(A.n, Cl.n);
     if (l + 1 < L - 1) {
       // restriction + first step of level l+1, whose pre-smoothing must end
       // in its x buffer
       C2<T> *first = (deg % 2 == 1) ? V.x[l + 1].p : V.x2[l + 1].p;
-      launch_dep(ovl(), restrict_first<T>, dim3(div_up(Cl.n * kAggLanes, B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
+      launch_dep(ovl(), few ? restrict_first<T, 8> : restrict_first<T, 16>, dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
                  A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p, V.coef[l + 1].p, V.d[l + 1].p, first,
                  halt);
       ++nls.launch_count;
       descend_ascend<T>(l + 1, V.b[l + 1].p, V.x[l + 1].p, nullptr);
     } else {
-      launch_dep(ovl(), restrict_kernel<T>, dim3(div_up(Cl.n * kAggLanes, B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
+      launch_dep(ovl(), few ? restrict_kernel<T, 8> : restrict_kernel<T, 16>, dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
                  A.mem_idx.p, V.res[l].p, V.b[l + 1].p, halt);
       const int m = (int)(2 * Cl.n);
       launch_dep(ovl(), dense_matvec<T>, dim3(div_up(m * kDenseLanes, B)), dim3(B), 0, st, m, dense_inv<T>(), dmap(),
@@ -1872,6 +1934,9 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
   for (int k = 0; k < deg; k++) {
     if (ms && k == deg - 1) {
       ChebMinresOp<T> op{dv, V.dinv[l].p, V.coef[l].p, k, b, cur, V.d[l].p, oth, ms, halt};
+      rows<T>(l, cur, op);
+    } else if (rowdot && k == deg - 1) {
+      ChebRowDotOp<T> op{dv, V.dinv[l].p, V.coef[l].p, k, b, cur, V.d[l].p, oth, rowdot, halt};
       rows<T>(l, cur, op);
     } else {
       ChebOp<T> op{dv, V.dinv[l].p, V.coef[l].p, k, b, cur, V.d[l].p, oth, halt};
@@ -1993,12 +2058,35 @@ void Amg::apply_minres(MinresScalars *ms, const T *u, T *r_old, const T *r_cur, 
   NOSH_CUDA(cudaGetLastError());
 }
 
+template <typename T>
+bool Amg::apply_batch(const int32_t *vsys, const MinresScalars *sc, const int *halt, const T *u, T *r_old,
+                      const T *r_cur, T *z_out, double *rowdot) {
+  Impl &I = *impl;
+  AmgVals<T> &V = I.vals<T>();
+  if (I.lev.size() == 1 || I.plan<T>().lt == 0) return false;
+  const AmgLevel &A = I.lev[0];
+  const int deg = std::max(I.opt.smooth_degree, 1);
+  C2<T> *first = (deg % 2 == 1) ? (C2<T> *)z_out : V.x2[0].p;
+  I.halt = halt;
+  launch_dep(I.ovl(), lanczos_first_sys<T>, dim3(div_up(A.n, 256)), dim3(256), 0, I.nls.stream, A.n, vsys, sc,
+             (const C2<T> *)u, (C2<T> *)r_old, (const C2<T> *)r_cur, V.dinv[0].p, V.coef[0].p, V.d[0].p, first, halt);
+  ++I.nls.launch_count;
+  I.descend_ascend<T>(0, (const C2<T> *)r_old, (C2<T> *)z_out, nullptr, rowdot);
+  I.halt = nullptr;
+  NOSH_CUDA(cudaGetLastError());
+  return true;
+}
+
 template void Amg::refresh<float>();
 template void Amg::refresh<double>();
 template void Amg::apply<float>(const float *, float *);
 template void Amg::apply<double>(const double *, double *);
 template void Amg::presmooth<float>(const float *, float *);
 template void Amg::presmooth<double>(const double *, double *);
+template bool Amg::apply_batch<float>(const int32_t *, const MinresScalars *, const int *, const float *, float *,
+                                      const float *, float *, double *);
+template bool Amg::apply_batch<double>(const int32_t *, const MinresScalars *, const int *, const double *, double *,
+                                       const double *, double *, double *);
 template void Amg::apply_minres<float>(MinresScalars *, const float *, float *, const float *, float *);
 template void Amg::apply_minres<double>(MinresScalars *, const double *, double *, const double *, double *);
 

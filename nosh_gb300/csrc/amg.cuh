@@ -36,6 +36,14 @@ struct Amg {
   // One MINRES Lanczos step fused around the V-cycle (see amg.cu)
   template <typename T>
   void apply_minres(MinresScalars *ms, const T *u, T *r_old, const T *r_cur, T *z_out);
+  // The same for a union of systems, each with its own recurrence (state
+  // sc[vsys[i]] of vertex i): r_old <- the new Lanczos vector (zero for a
+  // frozen system), z_out <- V-cycle(r_old), rowdot[i] = <r_old, z_out>_i.
+  // The launches return at once while *halt >= 2 (halt may be null).  False, with nothing
+  // launched, for a hierarchy without a fine level on the grid.
+  template <typename T>
+  bool apply_batch(const int32_t *vsys, const MinresScalars *sc, const int *halt, const T *u, T *r_old,
+                   const T *r_cur, T *z_out, double *rowdot);
   int num_levels() const;
   int64_t level_size(int l) const;
   int tail_level() const;

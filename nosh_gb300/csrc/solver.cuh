@@ -66,6 +66,14 @@ struct Minres {
   void drop_graphs();
 };
 
+// State of a batch on the device: its relative tolerance (read by the
+// captured chunk), sum_s beta1_s^2, and 0 while systems run, 1 once the last
+// one is to be frozen at its next Lanczos step, 2 once it is
+struct BatchState {
+  double eta, den;
+  int halt;
+};
+
 // Batched independent solves: one Paige-Saunders recurrence per system
 // over the shared vectors (minres_sys.cu).
 template <typename T>
@@ -78,12 +86,11 @@ struct MinresSys {
   DevBuf<int32_t> vsys, csys, schunk;
   DevBuf<int64_t> cstart;
   DevBuf<unsigned> counter;
-  DevBuf<int> active;
+  DevBuf<BatchState> state;
   int nchunks = 0;
   std::vector<MinresScalars> h_sc;
   int *h_active = nullptr, *h_err = nullptr;
-  double *h_eta = nullptr;
-  DevBuf<double> eta;  // the batch's tolerance (read by the captured chunk)
+  BatchState *h_state = nullptr;
   cudaGraphExec_t chunk_exec = nullptr;
   int64_t chunk_kernels = 0;
   int chunk_maxit = -1;
@@ -97,6 +104,7 @@ struct MinresSys {
             int &status);
 
  private:
+  bool ovl() const;
   void reduce(int mode, int maxit);
   void iteration(int j, int maxit);
 };
