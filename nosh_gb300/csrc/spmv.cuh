@@ -5,9 +5,8 @@
 // persistent over row blocks.  A row block's nonzeros [rp[r0], rp[r1]) are
 // contiguous: one thread stages them into shared memory with two bulk
 // asynchronous copies (TMA, cp.async.bulk: column ids and complex values)
-// completing on an mbarrier; in FP32 double-buffered, so that the copy of the
-// CTA's next row block overlaps the current one's arithmetic (stage_count).
-// The threads of a row then reduce its nonzeros out of shared memory and gather x through
+// completing on an mbarrier; the several CTAs of an SM overlap one another's
+// copies and arithmetic (stage_ctas).  The threads of a row then reduce its nonzeros out of shared memory and gather x through
 // the read-only path.  A row block whose nonzeros exceed the staging
 // capacity reads them directly.
 #pragma once
@@ -318,28 +317,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
   return false;
 }
 
-// Shared memory of one staging buffer (column ids, then complex values) for
-// a capacity of cap nonzeros (a multiple of 4); the kernel uses
-// stage_count<T>() of them.
+// Shared memory of a CTA's staging buffer (column ids, then complex values)
+// for a capacity of cap nonzeros (a multiple of 4).
 template <typename T>
 __host__ __device__ constexpr size_t stage_bytes(int cap) {
   return (size_t)cap * (sizeof(int32_t) + sizeof(C2<T>));
 }
-// Staging buffers of a CTA.  FP32: two, the next row block's copy under the
-// current one's gathers.  FP64: one.  Two FP64 buffers of a tetrahedral mesh
-// (72 KB) left three CTAs on an SM, and the FP64 pipe, which bounds the
-// kernel, idle a quarter of the time; one buffer fits five (register bound),
-// whose gathers and copies overlap one another.  J rebuild + apply at 160^3
-// 776 -> 699 us, FP64 V-cycles at 48^3 925 -> 868 us; six CTAs (80 registers)
-// gained 1 % more there and lost 3 % on a 32^3 continuation.
-template <typename T>
-__host__ __device__ constexpr int stage_count() {
-  return sizeof(T) == 4 ? 2 : 1;
-}
-// CTAs per SM the staged kernel is compiled for (its register budget).
+// CTAs per SM the staged kernel is compiled for (its register budget).  A CTA
+// has one buffer, and the other CTAs of its SM run under its copies: two
+// buffers left room for fewer CTAs, and the gathers, whose latency bounds the
+// FP32 kernel, and the FP64 pipe, which bounds the other, waited.
+// FP64, a tetrahedral mesh: two buffers (72 KB) fit three CTAs, one fits five
+// (register bound).  J rebuild + apply at 160^3 776 -> 699 us, V-cycles at 48^3
+// 925 -> 868 us; six CTAs (80 registers) gained 1 % more there and lost 3 % on a
+// 32^3 continuation.
+// FP32: two buffers with 16 gathers in flight a row (88 registers) fit five
+// CTAs, one with 8 gathers (72 registers) seven.  A mixed continuation step at
+// 64^3 73.3 -> 70.5 ms; one buffer with 16 gathers and five or six CTAs 71.1
+// and 71.9, with 8 gathers and eight CTAs (64 registers) 71.2.
 template <typename T>
 __host__ __device__ constexpr int stage_ctas() {
-  return sizeof(T) == 4 ? 5 : 4;
+  return sizeof(T) == 4 ? 7 : 4;
 }
 // Largest staging capacity of one buffer: 48 KB.
 template <typename T>
@@ -366,12 +364,10 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
                     Op op, double *partials, unsigned *counter, double *red_out) {
   using A = typename Acc<T>::type;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bar[2];
-  const size_t buf = stage_bytes<T>(cap);
+  __shared__ __align__(8) uint64_t bar;
   const int nblocks = (N + kRows - 1) / kRows;
   if (threadIdx.x == 0) {
-    mbar_init(&bar[0]);
-    mbar_init(&bar[1]);
+    mbar_init(&bar);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
@@ -383,16 +379,15 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     ks = k0 & ~3;  // 16-byte aligned start for both arrays
     n = k1 - ks;
   };
-  auto issue = [&](int rb, int stage) {
+  auto issue = [&](int rb) {
     int ks, n;
     range(rb, ks, n);
     if (n > 0 && n <= cap) {
-      unsigned char *base = smem_raw + stage * buf;
       const uint32_t cb = (uint32_t)(((n + 3) >> 2) * 16);                   // column ids
       const uint32_t vb = (uint32_t)(((size_t)n * sizeof(C2<T>) + 15) / 16 * 16);  // values
-      mbar_expect_tx(&bar[stage], cb + vb);
-      bulk_g2s(base, ci + ks, cb, &bar[stage]);
-      bulk_g2s(base + (size_t)cap * sizeof(int32_t), val + ks, vb, &bar[stage]);
+      mbar_expect_tx(&bar, cb + vb);
+      bulk_g2s(smem_raw, ci + ks, cb, &bar);
+      bulk_g2s(smem_raw + (size_t)cap * sizeof(int32_t), val + ks, vb, &bar);
     }
   };
   // The first row block's copy is issued before dep_sync(): the matrix (row
@@ -405,7 +400,7 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
   const int rb0 = blockIdx.x, rb_end = nblocks;
   auto nxt = [&](int rb) { return rb + (int)gridDim.x; };
   const bool skip = halted_early(op);
-  if (!skip && threadIdx.x == 0 && rb0 < rb_end) issue(rb0, 0);
+  if (!skip && threadIdx.x == 0 && rb0 < rb_end) issue(rb0);
   dep_sync();
   early_trigger(op);
   if (halted(op)) {
@@ -413,58 +408,45 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     if (!skip && threadIdx.x == 0 && rb0 < rb_end) {
       int ks, n;
       range(rb0, ks, n);
-      if (n > 0 && n <= cap && !mbar_wait(&bar[0], 0u)) stage_fail(counter);
+      if (n > 0 && n <= cap && !mbar_wait(&bar, 0u)) stage_fail(counter);
     }
     return;
   }
   typename PartOf<Op, A>::type part = 0;
-  uint32_t parity[2] = {0u, 0u};
+  uint32_t parity = 0u;
   bool ok = true;
-  // copies issued and not yet waited for: the current and the next row block
-  bool cur_staged = false, next_staged = false;
+  bool staged = false;  // the current row block's copy was issued
   uint32_t limit = kStageWaitPolls;
   if (cap > 0) {
     const unsigned o = __ldcg(counter + kStageWaitSlot);
     if (o != 0u) limit = o - 1u;
   }
-  int stage = 0;
-  constexpr bool kTwo = stage_count<T>() == 2;
-  for (int rb = rb0; rb < rb_end; rb = nxt(rb), stage ^= (kTwo ? 1 : 0)) {
-    // the other buffer was released by the barrier that ended the previous
-    // iteration: start the next row block's copy into it
-    if (kTwo && threadIdx.x == 0 && nxt(rb) < rb_end) issue(nxt(rb), stage ^ 1);
+  for (int rb = rb0; rb < rb_end; rb = nxt(rb)) {
     int ks, n;
     range(rb, ks, n);
     constexpr int R = row_threads<T>();
     const int row = rb * kRows + (int)threadIdx.x / R, lane_r = (int)threadIdx.x % R;
     typename Op::Pre pre{};
     if (row < N && lane_r == 0) pre = op.load(row);
-    const bool staged = n > 0 && n <= cap;
-    cur_staged = staged;
-    next_staged = false;
-    if (kTwo && nxt(rb) < rb_end) {
-      int ks2, n2;
-      range(nxt(rb), ks2, n2);
-      next_staged = n2 > 0 && n2 <= cap;
-    }
-    const bool arrived = staged ? mbar_wait(&bar[stage], parity[stage], limit) : true;
+    staged = n > 0 && n <= cap;
+    const bool arrived = staged ? mbar_wait(&bar, parity, limit) : true;
     if (__syncthreads_or(!arrived)) {  // the CTA leaves together
       ok = false;
       break;
     }
-    if (staged) parity[stage] ^= 1u;
-    const int32_t *s_col = reinterpret_cast<const int32_t *>(smem_raw + stage * buf);
-    const C2<T> *s_val = reinterpret_cast<const C2<T> *>(smem_raw + stage * buf + (size_t)cap * sizeof(int32_t));
+    if (staged) parity ^= 1u;
+    const int32_t *s_col = reinterpret_cast<const int32_t *>(smem_raw);
+    const C2<T> *s_val = reinterpret_cast<const C2<T> *>(smem_raw + (size_t)cap * sizeof(int32_t));
     A sr = 0, si = 0;
     if (row < N) {
       const int b = __ldg(rp + row), e = __ldg(rp + row + 1);
       if (staged) {
         // batches of kBatch nonzeros per lane (the row's lanes take every
         // R-th one): all gathers of a batch are issued before the first is
-        // used (rows of the mesh graph fit one batch); the values are read
+        // used (a row of the mesh graph is one or two); the values are read
         // from shared memory when used, so only the gathered x of a batch
         // occupies registers
-        constexpr int kBatch = (sizeof(T) == 4 ? 16 : 8) / R;
+        constexpr int kBatch = 8 / R;
         for (int k0 = b - ks + lane_r; k0 < e - ks; k0 += kBatch * R) {
           const int cnt = (e - ks - k0 + R - 1) / R;
           C2<T> xv[kBatch];
@@ -495,16 +477,14 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     }
     if (row < N && lane_r == 0) part += (typename PartOf<Op, A>::type)op.finish(row, sr, si, pre);
     __syncthreads();  // the buffer's readers are done: it may be refilled
-    if (!kTwo && threadIdx.x == 0 && nxt(rb) < rb_end) issue(nxt(rb), 0);
+    if (threadIdx.x == 0 && nxt(rb) < rb_end) issue(nxt(rb));
   }
   if (!ok) {
-    // a wait gave up: record it, give the copies still in flight (this row
-    // block's and the next one's) a last wait at the default bound, so no
-    // copy lands in shared memory after the CTA has left, and leave (the
-    // results of this launch are invalid)
+    // a wait gave up: record it, give the copy still in flight a last wait at
+    // the default bound, so that it does not land in shared memory after the
+    // CTA has left, and leave (the results of this launch are invalid)
     if (threadIdx.x == 0) stage_fail(counter);
-    if (cur_staged) mbar_wait(&bar[stage], parity[stage]);
-    if (next_staged) mbar_wait(&bar[stage ^ 1], parity[stage ^ 1]);
+    if (staged) mbar_wait(&bar, parity);
     return;
   }
   if (Op::kReduce) {
@@ -631,7 +611,7 @@ void launch_spmv(bool warp, int N, const int32_t *rp, const int32_t *ci, const C
                                      100 * 1024));
       attr_set = true;
     }
-    const size_t smem = stage_count<T>() * stage_bytes<T>(cap);
+    const size_t smem = stage_bytes<T>(cap);
     launch_dep(overlap, row_block_apply<T, Op>,
                dim3(row_grid((const void *)row_block_apply<T, Op>, block_threads<T>(), smem, N)),
                dim3(block_threads<T>()), smem, st, N, rp, ci, val, x, cap, op, partials, counter, red_out);
