@@ -1323,15 +1323,11 @@ __global__ void dot_advance(int64_t n, const C2<T> *__restrict__ a, const C2<T> 
   if (grid_reduce(v, partials, counter, &s->rz, &total)) minres_advance(s, total);
 }
 
-template <typename T>
-int staging_cap_of(const std::vector<int32_t> &rp, int64_t n) {
-  int64_t mx = 0;
-  for (int64_t r0 = 0; r0 < n; r0 += kRows) {
-    const int64_t r1 = std::min<int64_t>(n, r0 + kRows);
-    mx = std::max<int64_t>(mx, rp[r1] - (rp[r0] & ~(int64_t)3));
-  }
-  mx = (mx + 3) & ~(int64_t)3;
-  return (int)std::min<int64_t>(mx, stage_limit<T>());
+// the longest 4-aligned range of nonzeros of a block of kRows rows
+int longest_block(const std::vector<int32_t> &rp, int64_t n) {
+  int32_t mx = 0;
+  for (int64_t r0 = 0; r0 < n; r0 += kRows) mx = std::max(mx, rp[std::min<int64_t>(n, r0 + kRows)] - (rp[r0] & ~3));
+  return mx;
 }
 
 }  // namespace
@@ -1341,7 +1337,7 @@ struct AmgLevel {
   int64_t n = 0, nnz = 0;
   const int32_t *rp = nullptr, *ci = nullptr;  // level 0: the mesh graph
   DevBuf<int32_t> rp_own, ci_own;
-  int cap32 = 0, cap64 = 0;
+  int block_nnz = 0;  // longest_block
   bool warp32 = false, warp64 = false;  // SpMV schedule (tuned on the first refresh)
   bool tuned32 = false, tuned64 = false;
   // transfer to the next level
@@ -1495,8 +1491,7 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
       A.rp = A.rp_own.p;
       A.ci = A.ci_own.p;
     }
-    A.cap32 = staging_cap_of<float>(h.rp, h.n);
-    A.cap64 = staging_cap_of<double>(h.rp, h.n);
+    A.block_nnz = longest_block(h.rp, h.n);
     if (l + 1 < L) {
       A.agg.upload(h.agg, st);
       A.mem_ptr.upload(h.mem_ptr, st);
@@ -1691,7 +1686,7 @@ void Amg::refresh() {
     if (tuned) continue;
     bool &warp = sizeof(T) == 4 ? A.warp32 : A.warp64;
     if (I.nls.spmv_schedule == 0)
-      warp = pick_warp_schedule<T>((int)A.n, A.rp, A.ci, I.off<T>(l), sizeof(T) == 4 ? A.cap32 : A.cap64,
+      warp = pick_warp_schedule<T>((int)A.n, A.rp, A.ci, I.off<T>(l), A.block_nnz,
                                    I.nls.red.partials.p, I.nls.red.counter.p, st);
     else
       warp = I.nls.spmv_schedule == 2;
@@ -1714,12 +1709,10 @@ template <typename T>
 void Amg::Impl::prime() {
   // shared-memory opt-in of every row kernel instantiation, set before any
   // stream capture
-  NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, ChebOp<T>>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-  NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, ChebMinresOp<T>>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-  NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, ResidOp<T>>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+  allow_staging<T, ChebOp<T>>();
+  allow_staging<T, ChebMinresOp<T>>();
+  allow_staging<T, ChebRowDotOp<T>>();
+  allow_staging<T, ResidOp<T>>();
 }
 
 // The cluster's size: 16 CTAs (above the portable 8) when the device runs
@@ -1849,9 +1842,8 @@ void Amg::Impl::launch_tail(const TailPlan<T> &P, const TailArgs<T> &a, bool ove
 template <typename T, class Op>
 void Amg::Impl::rows(int l, const C2<T> *x, const Op &op) {
   const AmgLevel &A = lev[l];
-  const int cap = sizeof(T) == 4 ? A.cap32 : A.cap64;
   const bool warp = l == 0 ? (sizeof(T) == 4 ? nls.warp32 : nls.warp64) : (sizeof(T) == 4 ? A.warp32 : A.warp64);
-  launch_spmv<T, Op>(warp, (int)A.n, A.rp, A.ci, off<T>(l), x, cap, op, nls.red.partials.p, nls.red.counter.p,
+  launch_spmv<T, Op>(warp, (int)A.n, A.rp, A.ci, off<T>(l), x, A.block_nnz, op, nls.red.partials.p, nls.red.counter.p,
                      Op::kReduce ? &nls.red.out.p[32] : nullptr, nls.stream, ovl());
   ++nls.launch_count;
 }

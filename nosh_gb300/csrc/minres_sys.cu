@@ -295,8 +295,7 @@ MinresSys<T>::MinresSys(NlsImpl &nls) : s(nls), N(nls.N), S(nls.nsys()) {
   NOSH_CUDA(cudaMallocHost(&h_active, sizeof(int)));
   NOSH_CUDA(cudaMallocHost(&h_err, sizeof(int)));
   NOSH_CUDA(cudaMallocHost(&h_state, sizeof(BatchState)));
-  NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, JacRowDotOp<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 100 * 1024));
+  allow_staging<T, JacRowDotOp<T>>();
   s.sync();
 }
 
@@ -314,7 +313,6 @@ template <typename T>
 void MinresSys<T>::iteration(int j, int maxit) {
   cudaStream_t st = s.stream;
   const int G = egrid(N);
-  const int cap = sizeof(T) == 4 ? s.cap32 : s.cap64;
   const C2<T> *val = sizeof(T) == 4 ? (const C2<T> *)s.d_keo32.p : (const C2<T> *)s.d_keo64.p;
   const T *jd = sizeof(T) == 4 ? (const T *)s.d_jd32.p : (const T *)s.d_jd64.p;
   const bool warp = sizeof(T) == 4 ? s.warp32 : s.warp64;
@@ -325,7 +323,7 @@ void MinresSys<T>::iteration(int j, int maxit) {
   JacRowDotOp<T> op{jd, (const C2<T> *)zc, (C2<T> *)u.p, rowdot.p, vsys.p, sc.p, (const C2<T> *)zn,
                     (C2<T> *)w[(j + 2) % 3].p, (const C2<T> *)w[j % 3].p, (const C2<T> *)w[(j + 1) % 3].p,
                     (C2<T> *)x.p, halt};
-  launch_spmv<T>(warp, (int)N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, (const C2<T> *)zc, cap, op, s.red.partials.p,
+  launch_spmv<T>(warp, (int)N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, (const C2<T> *)zc, s.mesh->max_block, op, s.red.partials.p,
                  s.red.counter.p, nullptr, st, ovl());
   ++s.launch_count;
   reduce(kLanczos, maxit);

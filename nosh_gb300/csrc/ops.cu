@@ -275,18 +275,11 @@ __global__ void export_kernel(int64_t N, const int32_t *__restrict__ rp,
   if (!placed) out[o] = C2<double>{diag ? diag[i] : 0.0, 0.0};
 }
 
-template <typename T>
-int staging_cap(const MeshImpl &m) {
-  // largest staged range of any row block, capped by the shared memory
-  static_assert(kRows == 128, "MeshImpl::max_block is of 128 rows");
-  return (int)std::min<int64_t>((m.max_block + 3) & ~3, stage_limit<T>());
-}
-
+static_assert(kRows == 128, "MeshImpl::max_block is of 128 rows");
 template <typename T, class Op>
-void launch_rows(const NlsImpl &s, const C2<T> *val, const C2<T> *x, const Op &op, int cap,
-                 double *red_out) {
-  launch_spmv<T, Op>(sizeof(T) == 4 ? s.warp32 : s.warp64, (int)s.N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, x, cap,
-                     op, s.red.partials.p, s.red.counter.p, red_out, s.stream);
+void launch_rows(const NlsImpl &s, const C2<T> *val, const C2<T> *x, const Op &op, double *red_out) {
+  launch_spmv<T, Op>(sizeof(T) == 4 ? s.warp32 : s.warp64, (int)s.N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, x,
+                     s.mesh->max_block, op, s.red.partials.p, s.red.counter.p, red_out, s.stream);
   ++s.launch_count;
 }
 
@@ -346,7 +339,7 @@ __global__ void history_dots(int64_t n, const double *x0, const double *x1, cons
 
 namespace dev {
 template <typename T>
-bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T> *val, int cap, double *partials,
+bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T> *val, int block_nnz, double *partials,
                         unsigned *counter, cudaStream_t st) {
   if (N <= 0) return false;
   DevBuf<C2<T>> xb, yb;
@@ -369,9 +362,9 @@ bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T>
   float best[2] = {1e30f, 1e30f};
   for (int round = 0; round < 3; round++)
     for (int w = 0; w < 2; w++) {
-      for (int r = 0; r < 2; r++) launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, cap, op, partials, counter, rb.p, st);
+      for (int r = 0; r < 2; r++) launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, block_nnz, op, partials, counter, rb.p, st);
       NOSH_CUDA(cudaEventRecord(e0, st));
-      for (int r = 0; r < 5; r++) launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, cap, op, partials, counter, rb.p, st);
+      for (int r = 0; r < 5; r++) launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, block_nnz, op, partials, counter, rb.p, st);
       NOSH_CUDA(cudaEventRecord(e1, st));
       NOSH_CUDA(cudaEventSynchronize(e1));
       float ms = 0.f;
@@ -417,8 +410,7 @@ int warp_grid(const void *kernel, int64_t n_rows) {
   return (int)std::max<int64_t>(1, std::min(blocks, resident_ctas(kernel, kWarpThreads, 0)));
 }
 
-int row_grid(const void *kernel, int threads, size_t smem, int64_t n_rows) {
-  const int64_t blocks = (n_rows + kRows - 1) / kRows;
+int row_grid(const void *kernel, int threads, size_t smem, int64_t blocks) {
   return (int)std::max<int64_t>(1, std::min(blocks, resident_ctas(kernel, threads, smem)));
 }
 }  // namespace dev
@@ -622,8 +614,6 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
   *h_stage_err = 0u;
   NOSH_CUDA(cudaMemcpyAsync(red.counter.p + kStageErrorSlot, &h_stage_err, sizeof(h_stage_err),
                             cudaMemcpyHostToDevice, s));
-  cap32 = staging_cap<float>(*m);
-  cap64 = staging_cap<double>(*m);
   tune_schedules();
   sum_kernel<<<reduce_grid(N), 256, 0, s>>>(N, m->d_cv.p, red.partials.p, red.counter.p, red.host);
   ++launch_count;
@@ -705,7 +695,7 @@ void NlsImpl::tune_schedules() {
   } else if (spmv_schedule == 2) {
     warp32 = warp64 = true;
   } else {
-    warp32 = pick_warp_schedule<float>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo32.p, cap32, red.partials.p,
+    warp32 = pick_warp_schedule<float>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo32.p, mesh->max_block, red.partials.p,
                                        red.counter.p, stream);
     // FP64 rows of a mesh graph are never faster in the warp schedule, whose
     // shuffles of sums go through the FP64 pipe: 127 us against 55 at 64^3 (14
@@ -713,7 +703,7 @@ void NlsImpl::tune_schedules() {
     // 64^3 handle's set-up; only longer rows, where a half-warp has more than
     // two rounds of work a row, are still timed.
     warp64 = mesh->max_row > 32 &&
-             pick_warp_schedule<double>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo64.p, cap64, red.partials.p,
+             pick_warp_schedule<double>((int)N, mesh->d_rp.p, mesh->d_ci.p, d_keo64.p, mesh->max_block, red.partials.p,
                                         red.counter.p, stream);
   }
 }
@@ -782,32 +772,30 @@ void NlsImpl::dkeo_refill(double mu) {
 
 void NlsImpl::keo_apply64(const double *x, double *y) {
   KeoOp<double> op{d_kdiag.p, (const C2<double> *)x, (C2<double> *)y};
-  launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap64, nullptr);
+  launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, nullptr);
 }
 
 void NlsImpl::dkeo_apply64(const double *x, double *y) {
   PlainOp<double> op{(C2<double> *)y};
-  launch_rows<double>(*this, d_dkeo64.p, (const C2<double> *)x, op, cap64,
-                      nullptr);
+  launch_rows<double>(*this, d_dkeo64.p, (const C2<double> *)x, op, nullptr);
 }
 
 void NlsImpl::compute_f64(const double *x, double g, double mu, double *f, int norm_slot, double *soff) {
   if (!(keo_mu == mu)) keo_refill(mu);
-  const int cap = cap64;
   if (norm_slot >= 0) {
     ResidualOp<true> op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f, (C2<double> *)soff};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap, red.host + norm_slot);
+    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, red.host + norm_slot);
   } else {
     ResidualOp<false> op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f,
                          (C2<double> *)soff};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap, nullptr);
+    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, nullptr);
   }
 }
 
 void NlsImpl::residual_update(const double *x, const float *dx, double g, double mu, double *f, double *soff) {
   if (!(keo_mu == mu)) keo_refill(mu);
   ResidualUpdateOp op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f, (C2<double> *)soff};
-  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)dx, op, cap32, red.host);
+  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)dx, op, red.host);
 }
 
 namespace {
@@ -926,40 +914,36 @@ void NlsImpl::ensure_diag32() {
 
 template <>
 void NlsImpl::jac_apply<double>(const double *x, double *y, double *dot_out) {
-  const int cap = cap64;
   if (dot_out) {
     BlockDiagOp<double, true> op{d_jd64.p, (const C2<double> *)x, (C2<double> *)y};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap, dot_out);
+    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, dot_out);
   } else {
     BlockDiagOp<double, false> op{d_jd64.p, (const C2<double> *)x, (C2<double> *)y};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap, nullptr);
+    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, nullptr);
   }
 }
 
 template <>
 void NlsImpl::jac_apply<float>(const float *x, float *y, double *dot_out) {
-  const int cap = cap32;
   if (dot_out) {
     BlockDiagOp<float, true> op{d_jd32.p, (const C2<float> *)x, (C2<float> *)y};
-    launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, cap, dot_out);
+    launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, dot_out);
   } else {
     BlockDiagOp<float, false> op{d_jd32.p, (const C2<float> *)x, (C2<float> *)y};
-    launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, cap, nullptr);
+    launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, nullptr);
   }
 }
 
 template <>
 void NlsImpl::reg_apply<double>(const double *x, double *y) {
   BlockDiagOp<double, false> op{d_rd64.p, (const C2<double> *)x, (C2<double> *)y};
-  launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, cap64,
-                      nullptr);
+  launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, nullptr);
 }
 
 template <>
 void NlsImpl::reg_apply<float>(const float *x, float *y) {
   BlockDiagOp<float, false> op{d_rd32.p, (const C2<float> *)x, (C2<float> *)y};
-  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, cap32,
-                     nullptr);
+  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, nullptr);
 }
 
 double NlsImpl::energy(const double *psi) {

@@ -198,8 +198,7 @@ Minres<T>::Minres(NlsImpl &nls) : s(nls), n2(2 * nls.N) {
   sc.alloc(1);
   NOSH_CUDA(cudaMallocHost(&h_rep, sizeof(MinresReport)));
   NOSH_CUDA(cudaMallocHost(&h_args, sizeof(MinresArgs)));
-  NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, JacMinresOp<T>>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+  allow_staging<T, JacMinresOp<T>>();
 }
 
 template <typename T>
@@ -235,7 +234,6 @@ void Minres<T>::iteration(int j) {
   // deferred w/x update of step j-1: its z is zn, its (w1, w2, w) buffers
   const int jm = (j + kChunk - 1) % 3;
   T *wa = w[jm].p, *wb = w[(jm + 1) % 3].p, *wc = w[(jm + 2) % 3].p;
-  const int cap = sizeof(T) == 4 ? s.cap32 : s.cap64;
   const C2<T> *val = sizeof(T) == 4 ? (const C2<T> *)s.d_keo32.p : (const C2<T> *)s.d_keo64.p;
   const T *jd = sizeof(T) == 4 ? (const T *)s.d_jd32.p : (const T *)s.d_jd64.p;
   JacMinresOp<T> op{jd, (const C2<T> *)zc, (C2<T> *)u.p, d, zn, wa, wb, wc, x.p, &d->done};
@@ -244,7 +242,7 @@ void Minres<T>::iteration(int j) {
   // were assembled before the solve)
   const bool overlap = s.overlap_launches && !s.timers[NOSH_KERNEL_JACOBIAN].on;
   launch_spmv<T>(sizeof(T) == 4 ? s.warp32 : s.warp64, (int)s.N, s.mesh->d_rp.p, s.mesh->d_ci.p, val,
-                 (const C2<T> *)zc, cap, op, s.red.partials.p, s.red.counter.p, &d->zu, st, overlap);
+                 (const C2<T> *)zc, s.mesh->max_block, op, s.red.partials.p, s.red.counter.p, &d->zu, st, overlap);
   ++s.launch_count;
   // values per vertex: z (2) and the diagonal block (3) read, u (2) written;
   // the fused w/x update reads z_prev, w2, w, x and writes w1, x (12).  The

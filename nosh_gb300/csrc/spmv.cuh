@@ -1,7 +1,7 @@
 // Row-block SpMV over the off-diagonal KEO graph with a fused per-vertex
 // epilogue (diagonal 2x2 block, residual nonlinearity, reductions).
 //
-// One CTA = kRows consecutive rows (row_threads<T>() threads per row),
+// One CTA = 128 threads on consecutive rows, 1 to 8 threads a row (row_lanes),
 // persistent over row blocks.  A row block's nonzeros [rp[r0], rp[r1]) are
 // contiguous: one thread stages them into shared memory with two bulk
 // asynchronous copies (TMA, cp.async.bulk: column ids and complex values)
@@ -32,18 +32,23 @@ __device__ __forceinline__ unsigned arrive_acq_rel(unsigned *counter) {
   return old;
 }
 
-constexpr int kRows = 128;
+constexpr int kRows = 128;  // rows of a row block at one thread a row, and threads of a CTA
 // Threads per row of the staged schedule (adjacent lanes, each taking every
-// row_threads-th nonzero).  One: two lanes per FP32 row (twice the warps
-// per SM for the gathers' latency, four CTAs per SM instead of five)
-// measured 4 % slower on the 64^3 smoother launch and 9 % on the 160^3 one.
-template <typename T>
-__host__ __device__ constexpr int row_threads() {
-  return 1;
-}
-template <typename T>
-__host__ __device__ constexpr int block_threads() {
-  return kRows * row_threads<T>();
+// n-th nonzero; a row block then has kRows / n rows), as a power of two: the
+// most that still fit one CTA on every multiprocessor and leave a lane
+// kLaneNnz nonzeros, up to 8.  One thread walks a long row of a small matrix
+// while most multiprocessors idle, and its row blocks may exceed the staging
+// buffer: the 1331 rows of some 27 nonzeros of a 32^3 hierarchy take 4.2
+// instead of 5.4 us a smoothing step (continuation there 16.4 -> 15.7 ms;
+// V-cycles at 48^3, 4913 such rows, 619 -> 607 us; 4 or 6 nonzeros a lane do
+// equally, 8 gains a tenth of it).  Short rows lose by the longer fold: 4225
+// rows of 6, 4.0 -> 4.5 us with four lanes.  In a grid that is full anyway two
+// lanes measured 4 % slower (FP32 smoother at 64^3).
+constexpr int kLaneNnz = 6;
+inline int row_lanes_log2(int64_t n, int block_nnz) {
+  int lr = 0;
+  while (lr < 3 && (n << (lr + 1)) <= (int64_t)kRows * kNumSMs && (block_nnz >> (lr + 1)) >= kLaneNnz * kRows) lr++;
+  return lr;
 }
 
 template <typename T>
@@ -357,15 +362,17 @@ __device__ __forceinline__ void stage_fail(const unsigned *counter) {
 // stage (cap > 0).
 constexpr int kStageWaitSlot = 14;
 
-template <typename T, class Op>
-__global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
+template <typename T, class Op, bool Lanes = false>
+__global__ void __launch_bounds__(kRows, stage_ctas<T>())
     row_block_apply(int N, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
                     const C2<T> *__restrict__ val, const C2<T> *__restrict__ x, int cap,
-                    Op op, double *partials, unsigned *counter, double *red_out) {
+                    Op op, double *partials, unsigned *counter, double *red_out, int log2_lanes) {
   using A = typename Acc<T>::type;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
-  const int nblocks = (N + kRows - 1) / kRows;
+  const int lr = Lanes ? log2_lanes : 0;
+  const int R = 1 << lr, rows = kRows >> lr;  // lanes of a row, rows of a block
+  const int nblocks = (N + rows - 1) / rows;
   if (threadIdx.x == 0) {
     mbar_init(&bar);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -374,7 +381,7 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
   __syncthreads();
   // row block -> its aligned nonzero range; staged when it fits
   auto range = [&](int rb, int &ks, int &n) {
-    const int r0 = rb * kRows, r1 = min(N, r0 + kRows);
+    const int r0 = rb * rows, r1 = min(N, r0 + rows);
     const int k0 = __ldg(rp + r0), k1 = __ldg(rp + r1);
     ks = k0 & ~3;  // 16-byte aligned start for both arrays
     n = k1 - ks;
@@ -424,10 +431,10 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
   for (int rb = rb0; rb < rb_end; rb = nxt(rb)) {
     int ks, n;
     range(rb, ks, n);
-    constexpr int R = row_threads<T>();
-    const int row = rb * kRows + (int)threadIdx.x / R, lane_r = (int)threadIdx.x % R;
+    const int row = rb * rows + ((int)threadIdx.x >> lr), lane_r = (int)threadIdx.x & (R - 1);
     typename Op::Pre pre{};
     if (row < N && lane_r == 0) pre = op.load(row);
+    const int b = row < N ? __ldg(rp + row) : 0, e = row < N ? __ldg(rp + row + 1) : 0;
     staged = n > 0 && n <= cap;
     const bool arrived = staged ? mbar_wait(&bar, parity, limit) : true;
     if (__syncthreads_or(!arrived)) {  // the CTA leaves together
@@ -439,24 +446,23 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
     const C2<T> *s_val = reinterpret_cast<const C2<T> *>(smem_raw + (size_t)cap * sizeof(int32_t));
     A sr = 0, si = 0;
     if (row < N) {
-      const int b = __ldg(rp + row), e = __ldg(rp + row + 1);
       if (staged) {
         // batches of kBatch nonzeros per lane (the row's lanes take every
         // R-th one): all gathers of a batch are issued before the first is
         // used (a row of the mesh graph is one or two); the values are read
         // from shared memory when used, so only the gathered x of a batch
         // occupies registers
-        constexpr int kBatch = 8 / R;
-        for (int k0 = b - ks + lane_r; k0 < e - ks; k0 += kBatch * R) {
-          const int cnt = (e - ks - k0 + R - 1) / R;
+        constexpr int kBatch = 8;
+        for (int k0 = b - ks + lane_r; k0 < e - ks; k0 += kBatch << lr) {
+          const int cnt = (e - ks - k0 + R - 1) >> lr;
           C2<T> xv[kBatch];
 #pragma unroll
           for (int u = 0; u < kBatch; u++)
-            if (u < cnt) xv[u] = ldg(x + s_col[k0 + u * R]);
+            if (u < cnt) xv[u] = ldg(x + s_col[k0 + (u << lr)]);
 #pragma unroll
           for (int u = 0; u < kBatch; u++) {
             if (u < cnt) {
-              const C2<T> v = s_val[k0 + u * R];
+              const C2<T> v = s_val[k0 + (u << lr)];
               row_mac(sr, si, v, xv[u]);
             }
           }
@@ -469,11 +475,15 @@ __global__ void __launch_bounds__(block_threads<T>(), stage_ctas<T>())
         }
       }
     }
-    // the row's lanes are adjacent: fold their partial sums into lane 0
-#pragma unroll
-    for (int o = R / 2; o > 0; o >>= 1) {
-      sr += __shfl_xor_sync(0xffffffffu, sr, o);
-      si += __shfl_xor_sync(0xffffffffu, si, o);
+    // the row's lanes are adjacent: fold their partial sums into lane 0, one
+    // component on the even lanes and the other on the odd ones
+    if (Lanes) {
+      const bool odd = lane_r & 1;
+      A v = odd ? si : sr;
+      v += __shfl_xor_sync(0xffffffffu, odd ? sr : si, 1);
+      for (int o = R / 2; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      sr = v;
+      si = __shfl_xor_sync(0xffffffffu, v, 1);
     }
     if (row < N && lane_r == 0) part += (typename PartOf<Op, A>::type)op.finish(row, sr, si, pre);
     __syncthreads();  // the buffer's readers are done: it may be refilled
@@ -586,35 +596,46 @@ int warp_grid(const void *kernel, int64_t n_rows);
 
 // Grid for a persistent row kernel of `threads` threads per CTA: the
 // resident capacity of the device for this kernel and shared-memory size,
-// capped by the number of row blocks.
-int row_grid(const void *kernel, int threads, size_t smem, int64_t n_rows);
+// capped by the number of row blocks n_blocks.
+int row_grid(const void *kernel, int threads, size_t smem, int64_t n_blocks);
+
+// Opts the staged kernels of Op into the largest staging buffer (done ahead of
+// a capture where the first launch may be in one).
+template <typename T, class Op>
+void allow_staging() {
+  for (auto *k : {row_block_apply<T, Op, false>, row_block_apply<T, Op, true>})
+    NOSH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes<T>(stage_limit<T>())));
+}
 
 // Launch the SpMV + epilogue over an off-diagonal CSR with one of the two
-// schedules (warp: row_warp_apply, else the staged row_block_apply with
-// staging capacity cap).
+// schedules (warp: row_warp_apply, else the staged row_block_apply); block_nnz:
+// the longest 4-aligned range of nonzeros of a block of kRows rows.
 //
 // With `overlap` the launch may start while the previous kernel of the stream
 // finishes (launch_dep); the staged schedule then copies its first row block
 // before waiting for it, so the previous kernel must not write this matrix.
 template <typename T, class Op>
 void launch_spmv(bool warp, int N, const int32_t *rp, const int32_t *ci, const C2<T> *val, const C2<T> *x,
-                 int cap, const Op &op, double *partials, unsigned *counter, double *red_out, cudaStream_t st,
-                 bool overlap = false) {
+                 int block_nnz, const Op &op, double *partials, unsigned *counter, double *red_out,
+                 cudaStream_t st, bool overlap = false) {
   if (warp) {
     const int grid = warp_grid((const void *)row_warp_apply<T, Op>, N);
     launch_dep(overlap, row_warp_apply<T, Op>, dim3(grid), dim3(kWarpThreads), 0, st, N, rp, ci, val, x, op,
                partials, counter, red_out);
   } else {
-    static bool attr_set = false;  // per instantiation; first call precedes any capture
+    const int lr = row_lanes_log2(N, block_nnz);
+    const auto kernel = lr > 0 ? row_block_apply<T, Op, true> : row_block_apply<T, Op, false>;
+    static bool attr_set = false;  // per instantiation
     if (!attr_set) {
-      NOSH_CUDA(cudaFuncSetAttribute(row_block_apply<T, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     100 * 1024));
+      allow_staging<T, Op>();
       attr_set = true;
     }
+    const int cap = std::min((block_nnz + 3) & ~3, stage_limit<T>());
     const size_t smem = stage_bytes<T>(cap);
-    launch_dep(overlap, row_block_apply<T, Op>,
-               dim3(row_grid((const void *)row_block_apply<T, Op>, block_threads<T>(), smem, N)),
-               dim3(block_threads<T>()), smem, st, N, rp, ci, val, x, cap, op, partials, counter, red_out);
+    // (kernels of one lane a row are compiled apart: with the lanes a parameter
+    // the FP32 ones lost 3 %)
+    launch_dep(overlap, kernel, dim3(row_grid((const void *)kernel, kRows, smem, div_up((int64_t)N << lr, kRows))),
+               dim3(kRows), smem, st, N, rp, ci, val, x, cap, op, partials, counter, red_out, lr);
   }
   NOSH_CUDA(cudaGetLastError());
 }
@@ -623,7 +644,7 @@ void launch_spmv(bool warp, int N, const int32_t *rp, const int32_t *ci, const C
 // after a warm-up) on y = A x + D x with <x, y> reduced, when the matrix
 // structure is set up.
 template <typename T>
-bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T> *val, int cap, double *partials,
+bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T> *val, int block_nnz, double *partials,
                         unsigned *counter, cudaStream_t st);
 
 // ---- epilogues --------------------------------------------------------
