@@ -661,76 +661,102 @@ __global__ void coarse_dense(int64_t n, const int32_t *__restrict__ rp, const in
   }
 }
 
-// In-place Gauss-Jordan inversion of an SPD matrix (no pivoting needed) in
-// shared memory, one CTA, m <= kDenseSmem, in the arithmetic type C (FP32 for
-// the mixed path: FP64 arithmetic is slow on GB300 and the coarsest operator
-// is well conditioned); writes the FP64 and FP32 copies.
-constexpr int kDenseSmem = 128;
+// Gauss-Jordan inversion of the coarsest level's SPD blocks (no pivoting
+// needed), kPivots pivots a launch, in the arithmetic type C (FP32 for the
+// mixed path: the coarsest operator is well conditioned).  A CTA owns
+// kPivotCols columns of a block: it inverts the pivot block P (every CTA does),
+// takes R = P^-1 times its columns' pivot rows and subtracts the pivot columns
+// times R from the other rows; a column of the pivot block itself starts from
+// the identity.  It reads src and writes dst, since every CTA reads the pivot
+// columns.  After the last launch the FP32 copy is written as well.
+//
+// Most of a launch's 13 us in FP64 is the chain of 16 reciprocals and updates
+// of P.  One CTA a block was bound by the FP64 pipe of its multiprocessor, m^3
+// multiply-adds: 661 -> 104 us for a block of 128 rows, 35 -> 26 us for one of
+// 32 (an FP64 continuation at 32^3 with two of the former 16.2 -> 14.8 ms).
+constexpr int kPivots = 16, kPivotCols = 2, kPivotThreads = 128;
 template <typename C>
-__global__ void gauss_jordan_spd_smem(const int64_t *__restrict__ boff, const int32_t *__restrict__ bd, double *Ag,
-                                      float *Afg, int *err) {
-  // one CTA per diagonal block of the coarsest level
-  const int m = bd[blockIdx.x];
-  double *A = Ag + boff[blockIdx.x];
-  float *Af = Afg + boff[blockIdx.x];
-  extern __shared__ __align__(16) unsigned char gj_raw[];
-  C *S = reinterpret_cast<C *>(gj_raw);
-  __shared__ C ip_s;
-  for (int q = threadIdx.x; q < m * m; q += blockDim.x) S[q] = (C)A[q];
-  __syncthreads();
-  for (int k = 0; k < m; k++) {
-    if (threadIdx.x == 0) {
-      const C piv = S[k * m + k];
-      if (!(piv > (C)0)) atomicOr(err, 16);
-      ip_s = (C)1 / piv;
+__global__ void __launch_bounds__(kPivotThreads)
+    gauss_jordan_step(const int64_t *__restrict__ boff, const int32_t *__restrict__ bd, int k0, int last,
+                      const double *__restrict__ src, double *__restrict__ dst, float *__restrict__ Afg, int *err) {
+  const int m = bd[blockIdx.x], j0 = blockIdx.y * kPivotCols;
+  if (j0 >= m) return;
+  const double *A = src + boff[blockIdx.x];
+  double *B = dst + boff[blockIdx.x];
+  float *Af = last ? Afg + boff[blockIdx.x] : nullptr;
+  const int nc = min(kPivotCols, m - j0), nk = min(kPivots, m - k0);
+  dep_sync();
+  if (nk <= 0) {  // a smaller block, inverted by an earlier launch
+    for (int q = threadIdx.x; q < m * kPivotCols; q += kPivotThreads) {
+      const int jj = q % kPivotCols;
+      const int64_t at = (int64_t)(q / kPivotCols) * m + j0 + jj;
+      if (jj >= nc) continue;
+      B[at] = A[at];
+      if (last) Af[at] = (float)A[at];
     }
-    __syncthreads();
-    const C ip = ip_s;
-    for (int j = threadIdx.x; j < m; j += blockDim.x) S[k * m + j] = (j == k) ? ip : S[k * m + j] * ip;
-    __syncthreads();
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-      const int i = q / m, j = q % m;
-      if (i == k || j == k) continue;
-      S[q] -= S[i * m + k] * S[k * m + j];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < m; i += blockDim.x)
-      if (i != k) S[i * m + k] = -S[i * m + k] * ip;
-    __syncthreads();
+    return;
   }
-  for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-    A[q] = (double)S[q];
-    Af[q] = (float)S[q];
-  }
-}
-
-// The same in global memory for larger blocks.
-__global__ void gauss_jordan_spd(const int64_t *__restrict__ boff, const int32_t *__restrict__ bd, double *Ag,
-                                 float *Afg, int *err) {
-  const int m = bd[blockIdx.x];
-  double *A = Ag + boff[blockIdx.x];
-  float *Af = Afg + boff[blockIdx.x];
-  for (int k = 0; k < m; k++) {
-    __syncthreads();
-    const double piv = A[(int64_t)k * m + k];
-    __syncthreads();
-    if (threadIdx.x == 0 && !(piv > 0.0)) atomicOr(err, 16);
-    const double ip = 1.0 / piv;
-    for (int j = threadIdx.x; j < m; j += blockDim.x)
-      A[(int64_t)k * m + j] = (j == k) ? ip : A[(int64_t)k * m + j] * ip;
-    __syncthreads();
-    for (int64_t q = threadIdx.x; q < (int64_t)m * m; q += blockDim.x) {
-      const int i = (int)(q / m), j = (int)(q % m);
-      if (i == k || j == k) continue;
-      A[q] -= A[(int64_t)i * m + k] * A[(int64_t)k * m + j];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < m; i += blockDim.x)
-      if (i != k) A[(int64_t)i * m + k] = -A[(int64_t)i * m + k] * ip;
+  __shared__ C P[2][kPivots][kPivots + 1], Y[kPivots][kPivotCols], R[kPivots][kPivotCols];
+  const int r = threadIdx.x / (kPivots / 2), c = threadIdx.x % (kPivots / 2) * 2;
+#pragma unroll
+  for (int q = 0; q < 2; q++) P[0][r][c + q] = r < nk && c + q < nk ? (C)A[(int64_t)(k0 + r) * m + k0 + c + q] : (C)0;
+  if (threadIdx.x < kPivots * kPivotCols) {
+    const int l = threadIdx.x / kPivotCols, jj = threadIdx.x % kPivotCols;
+    Y[l][jj] = l < nk && jj < nc ? (C)A[(int64_t)(k0 + l) * m + j0 + jj] : (C)0;
   }
   __syncthreads();
-  for (int64_t q = threadIdx.x; q < (int64_t)m * m; q += blockDim.x) Af[q] = (float)A[q];
+  for (int k = 0; k < nk; k++) {
+    const C(*S)[kPivots + 1] = P[k & 1];
+    const C piv = S[k][k];
+    if (threadIdx.x == 0 && blockIdx.y == 0 && !(piv > (C)0)) atomicOr(err, 16);
+    const C ip = (C)1 / piv;
+    const C f = r == k ? ip : -S[r][k] * ip;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const C a = c + q == k ? (C)0 : S[r][c + q], pk = c + q == k ? (C)1 : S[k][c + q];
+      P[(k & 1) ^ 1][r][c + q] = r == k ? pk * f : a + f * pk;
+    }
+    __syncthreads();
+  }
+  const C(*S)[kPivots + 1] = P[nk & 1];
+  if (threadIdx.x < kPivots * kPivotCols) {
+    const int l = threadIdx.x / kPivotCols, jj = threadIdx.x % kPivotCols, jp = j0 + jj - k0;
+    C v = 0;
+    if (jp >= 0 && jp < nk) {
+      v = l < nk ? S[l][jp] : (C)0;
+    } else {
+#pragma unroll
+      for (int q = 0; q < kPivots; q++) v += S[l][q] * Y[q][jj];
+    }
+    R[l][jj] = v;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < m; i += kPivotThreads) {
+    const int ip = i - k0;
+    const bool pivot_row = ip >= 0 && ip < nk;
+    C v[kPivotCols];
+#pragma unroll
+    for (int jj = 0; jj < kPivotCols; jj++) {
+      const int jp = j0 + jj - k0;
+      v[jj] = pivot_row ? R[ip][jj] : jj >= nc || (jp >= 0 && jp < nk) ? (C)0 : (C)A[(int64_t)i * m + j0 + jj];
+    }
+    if (!pivot_row)
+#pragma unroll
+      for (int q = 0; q < kPivots; q++) {
+        const C a = q < nk ? (C)A[(int64_t)i * m + k0 + q] : (C)0;
+#pragma unroll
+        for (int jj = 0; jj < kPivotCols; jj++) v[jj] -= a * R[q][jj];
+      }
+#pragma unroll
+    for (int jj = 0; jj < kPivotCols; jj++)
+      if (jj < nc) {
+        B[(int64_t)i * m + j0 + jj] = (double)v[jj];
+        if (last) Af[(int64_t)i * m + j0 + jj] = (float)v[jj];
+      }
+  }
 }
+// Blocks of more rows than this are inverted in FP64 on the mixed path too.
+constexpr int kDenseFp32 = 128;
 
 // Packed block-diagonal dense inverse: real row i of the coarsest level is
 // row rowoff[i] of the packed array, its block starts at real row bstart[i]
@@ -1388,6 +1414,7 @@ struct Amg::Impl {
   DevBuf<unsigned> arrive;
   ChebSpec cheb;
   DevBuf<double> dense;  // coarsest (2n)^2 FP64
+  DevBuf<double> dense2;  // the inversion's other buffer
   DevBuf<float> densef;
   // packed block-diagonal coarsest inverse: per block (offset, dim), per real
   // row (offset, block start, dim)
@@ -1557,13 +1584,10 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
     I.row_dim.upload(rdim, st);
     I.dense.alloc(total);
     I.densef.alloc(total);
+    I.dense2.alloc(total);
   }
   I.err.alloc(1);
   I.err.zero(st);
-  NOSH_CUDA(cudaFuncSetAttribute(gauss_jordan_spd_smem<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kDenseSmem * kDenseSmem * (int)sizeof(double)));
-  NOSH_CUDA(cudaFuncSetAttribute(gauss_jordan_spd_smem<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kDenseSmem * kDenseSmem * (int)sizeof(float)));
   s.sync();
 }
 
@@ -1693,15 +1717,16 @@ void Amg::refresh() {
     tuned = true;
   }
   const AmgLevel &C = I.lev.back();
+  const int steps = div_up(I.max_dim, kPivots);
+  double *buf[2] = {I.dense.p, I.dense2.p};  // the last step writes the first
   coarse_dense<T><<<div_up(C.n, 128), 128, 0, st>>>(C.n, C.rp, C.ci, I.off<T>(L - 1), I.dia<T>(L - 1),
-                                                     I.row_start.p, I.row_off.p, I.row_dim.p, I.dense.p);
-  ++I.nls.launch_count;
-  if (I.max_dim <= kDenseSmem)
-    gauss_jordan_spd_smem<T><<<I.nblk, 1024, (size_t)I.max_dim * I.max_dim * sizeof(T), st>>>(
-        I.blk_off.p, I.blk_dim.p, I.dense.p, I.densef.p, I.err.p);
-  else
-    gauss_jordan_spd<<<I.nblk, 1024, 0, st>>>(I.blk_off.p, I.blk_dim.p, I.dense.p, I.densef.p, I.err.p);
-  ++I.nls.launch_count;
+                                                     I.row_start.p, I.row_off.p, I.row_dim.p, buf[steps & 1]);
+  const auto step = I.max_dim <= kDenseFp32 ? gauss_jordan_step<T> : gauss_jordan_step<double>;
+  for (int k = 0; k < steps; k++)
+    launch_dep(I.ovl(), step, dim3(I.nblk, div_up(I.max_dim, kPivotCols)), dim3(kPivotThreads), 0, st, I.blk_off.p,
+               I.blk_dim.p, k * kPivots, (int)(k == steps - 1), (const double *)buf[(steps - k) & 1],
+               buf[(steps - k - 1) & 1], I.densef.p, I.err.p);
+  I.nls.launch_count += 1 + steps;
   NOSH_CUDA(cudaGetLastError());
 }
 
