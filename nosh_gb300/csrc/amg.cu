@@ -1659,6 +1659,7 @@ void Amg::Impl::ensure_vals() {
 template <typename T>
 void Amg::refresh() {
   Impl &I = *impl;
+  if (sizeof(T) == 4) I.nls.ensure_keo32();
   I.ensure_vals<T>();
   AmgVals<T> &V = I.vals<T>();
   cudaStream_t st = I.nls.stream;

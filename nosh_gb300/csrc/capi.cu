@@ -588,15 +588,22 @@ int nosh_jacobian_apply(nosh_nls nls, const double *X, double *Y, int nvec, int 
     check_apply_args(mode, alpha, beta, nvec);
     require(s.jac_ready, "Jacobian not built: call nosh_jacobian_rebuild first");
     if (s.precision != NOSH_PREC_FP64) s.ensure_diag32();
+    const size_t n = 2 * (size_t)s.N;
+    // mixed precision: up to kCastVectors device vectors are rounded in one
+    // launch, and a product overlaps the one before it (a rebuild and three
+    // products at 64^3 74 us; with a launch to round each vector and another to
+    // widen each product, each after the one before, 102)
+    const bool mixed = s.precision != NOSH_PREC_FP64;
+    const int group = mixed && usable_in_place(X) ? std::min<int>(nvec, s.kCastVectors) : 1;
     for (int k = 0; k < nvec; k++) {
-      const double *dx = stage_in(s, X + (size_t)k * 2 * s.N, s.d_in, 2 * s.N);
-      OutVec o(s, Y + (size_t)k * 2 * s.N, s.d_out, 2 * s.N);
-      if (s.precision == NOSH_PREC_FP64) {
-        s.jac_apply<double>(dx, o.dev);
+      const double *dx = stage_in(s, X + k * n, s.d_in, n);
+      OutVec o(s, Y + k * n, s.d_out, n);
+      if (!mixed) {
+        s.jac_apply(dx, o.dev);
       } else {
-        nosh::launch_f64_to_f32(dx, s.d_inf.p, 2 * s.N, s.stream);
-        s.jac_apply<float>(s.d_inf.p, s.d_outf.p);
-        nosh::launch_f32_to_f64(s.d_outf.p, o.dev, 2 * s.N, s.stream);
+        const int q = k % group;
+        if (q == 0) nosh::launch_f64_to_f32(dx, s.d_inf.p, std::min(group, nvec - k) * n, s.stream);
+        s.jac_apply32(s.d_inf.p + q * n, o.dev, true);
       }
       o.copy_back(s);
     }

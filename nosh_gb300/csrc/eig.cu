@@ -331,7 +331,7 @@ int lowest_eigenpairs(NlsImpl &s, const double *psi_dev, double g, double mu, in
     if (Ug && rows > 0) B.project_off(V, rows, Ug);
   };
   auto applyJ = [&](const double *V, double *AV, int rows) {
-    for (int j = 0; j < rows; j++) s.jac_apply<double>(V + (size_t)j * n, AV + (size_t)j * n);
+    for (int j = 0; j < rows; j++) s.jac_apply(V + (size_t)j * n, AV + (size_t)j * n);
     NOSH_CUDA(cudaGetLastError());
   };
   auto applyT = [&](const double *V, double *TV, int rows) {

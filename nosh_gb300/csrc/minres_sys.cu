@@ -359,6 +359,7 @@ int MinresSys<T>::solve(const T *b, double eta, const std::vector<double> &rtol_
   const int64_t n2 = 2 * N;
   const size_t bytes = n2 * sizeof(T);
   const int G = egrid(N);
+  if (sizeof(T) == 4) s.ensure_keo32();
   rtol.upload(rtol_host.data(), S, st);
   // (the flag falls several launches before the first one that looks at it:
   // the SpMV reads it ahead of its predecessor's completion)

@@ -1655,8 +1655,8 @@ void Mpnn::Impl::features(const double *const x[4], const double mu[4], double t
                                      (C2<double> *)vt.p);
     ++s.launch_count;
     s.jac_rebuild(vt.p, s.g0, t, false);
-    s.jac_apply<double>(vc.p, jc.p);
-    s.jac_apply<double>(vd.p, jd.p);
+    s.jac_apply(vc.p, jc.p);
+    s.jac_apply(vd.p, jd.p);
     gram3_kernel<<<reduce_grid(2 * N), 256, 0, st>>>(2 * N, jc.p, jd.p, rd.partials.p, rd.counter.p, gram.p);
     s.launch_count += 3;
   }

@@ -177,6 +177,8 @@ struct NlsImpl {
 
   // staging for host / misaligned vectors
   DevBuf<double> d_in, d_out, d_tmp;  // 2N each
+  // FP32 images of up to kCastVectors inputs, and of one output
+  static constexpr int kCastVectors = 4;
   DevBuf<float> d_inf, d_outf;
 
   Reducer red;
@@ -227,6 +229,11 @@ struct NlsImpl {
 
   // operators (device pointers to interleaved complex vectors)
   void keo_refill(double mu);
+  // the KEO's FP32 image: written with the FP64 values when the handle works
+  // in mixed precision (two conversions and a third of the writes of the
+  // launch), else on the first use
+  bool keo32_ok = true;
+  void ensure_keo32();
   void dkeo_refill(double mu);
   void keo_apply64(const double *x, double *y);
   void dkeo_apply64(const double *x, double *y);
@@ -258,8 +265,10 @@ struct NlsImpl {
   // mixed-precision solve
   void operators32_rebuild(const double *x, double g, double mu);
   void reg_rebuild(const double *x, double g, double mu, bool want32);
-  template <typename T>
-  void jac_apply(const T *x, T *y, double *dot_out = nullptr);
+  void jac_apply(const double *x, double *y);
+  // the FP32 product widened by the launch that forms it; overlap: the launch
+  // before it writes neither the KEO nor the diagonal
+  void jac_apply32(const float *x, double *y, bool overlap);
   template <typename T>
   void reg_apply(const T *x, T *y);
   double energy(const double *psi);

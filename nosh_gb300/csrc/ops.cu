@@ -109,6 +109,7 @@ __global__ void keo_assemble(int64_t E, const double *__restrict__ alpha, const 
   const int32_t f = pf[e], b = pb[e];
   val[f] = C2<double>{re, im};
   val[b] = C2<double>{re, -im};
+  if (!val32) return;
   val32[f] = C2<float>{(float)re, (float)im};
   val32[b] = C2<float>{(float)re, -(float)im};
 }
@@ -131,6 +132,21 @@ __global__ void dkeo_assemble64(int64_t E, const double *__restrict__ alpha,
   // complex v0 - i v1 at (v0,v1): w sin a + i w cos a; conjugate at (v1,v0)
   val[pf[e]] = C2<double>{w * s, w * c};
   val[pb[e]] = C2<double>{w * s, -w * c};
+}
+
+// The same from the KEO's values at the same parameter, -alpha e^{-+ i a}: the
+// derivative multiplies them by -+ i dp.  One launch of FP64 sines takes 60 us
+// at 64^3 (1.9 M edges, the FP64 pipe), this one 20.
+__global__ void dkeo_from_keo(int64_t E, const C2<double> *__restrict__ keo, const double *__restrict__ p,
+                              double dscale, const int32_t *__restrict__ pf, const int32_t *__restrict__ pb,
+                              C2<double> *__restrict__ val) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  const int32_t f = pf[e], b = pb[e];
+  const C2<double> k = keo[f];
+  const double q = p[e] * dscale, re = q * k.y, im = q * k.x;
+  val[f] = C2<double>{re, -im};
+  val[b] = C2<double>{re, im};
 }
 
 // ------------------------------------------------------------ diagonals
@@ -277,9 +293,10 @@ __global__ void export_kernel(int64_t N, const int32_t *__restrict__ rp,
 
 static_assert(kRows == 128, "MeshImpl::max_block is of 128 rows");
 template <typename T, class Op>
-void launch_rows(const NlsImpl &s, const C2<T> *val, const C2<T> *x, const Op &op, double *red_out) {
+void launch_rows(const NlsImpl &s, const C2<T> *val, const C2<T> *x, const Op &op, double *red_out,
+                 bool overlap = false) {
   launch_spmv<T, Op>(sizeof(T) == 4 ? s.warp32 : s.warp64, (int)s.N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, x,
-                     s.mesh->max_block, op, s.red.partials.p, s.red.counter.p, red_out, s.stream);
+                     s.mesh->max_block, op, s.red.partials.p, s.red.counter.p, red_out, s.stream, overlap);
   ++s.launch_count;
 }
 
@@ -607,7 +624,7 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
   d_in.alloc(2 * N);
   d_out.alloc(2 * N);
   d_tmp.alloc(2 * N);
-  d_inf.alloc(2 * N);
+  d_inf.alloc(2 * N * kCastVectors);
   d_outf.alloc(2 * N);
   red.init(div_up(N, kRows) + div_up(N, 256) + 1024, 64, s);
   NOSH_CUDA(cudaMallocHost(&h_stage_err, sizeof(unsigned)));
@@ -755,16 +772,30 @@ void NlsImpl::set_stage_wait_limit(int64_t polls) {
 void NlsImpl::keo_refill(double mu) {
   const double *ms = sys_off.empty() ? nullptr : d_mu_sys.p;
   keo_assemble<<<div_up(E, 256), 256, 0, stream>>>(E, d_alpha.p, d_p.p, mu, mesh->d_pos_fwd.p, mesh->d_pos_bwd.p,
-                                                    d_keo64.p, d_keo32.p, ms, d_esys.p);
+                                                    d_keo64.p, precision != NOSH_PREC_FP64 ? d_keo32.p : nullptr, ms,
+                                                    d_esys.p);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
   keo_mu = mu;
+  keo32_ok = precision != NOSH_PREC_FP64;
+}
+
+void NlsImpl::ensure_keo32() {
+  if (keo32_ok) return;
+  launch_f64_to_f32((const double *)d_keo64.p, (float *)d_keo32.p, 4 * E, stream);
+  ++launch_count;
+  keo32_ok = true;
 }
 
 void NlsImpl::dkeo_refill(double mu) {
-  dkeo_assemble64<<<div_up(E, 256), 256, 0, stream>>>(
-      E, d_alpha.p, d_p.p, mu, deriv_param == "mu" ? 1.0 : 0.0, mesh->d_pos_fwd.p,
-      mesh->d_pos_bwd.p, d_dkeo64.p, sys_off.empty() ? nullptr : d_mu_sys.p, d_esys.p);
+  const double dscale = deriv_param == "mu" ? 1.0 : 0.0;
+  if (keo_mu == mu)
+    dkeo_from_keo<<<div_up(E, 256), 256, 0, stream>>>(E, d_keo64.p, d_p.p, dscale, mesh->d_pos_fwd.p,
+                                                       mesh->d_pos_bwd.p, d_dkeo64.p);
+  else
+    dkeo_assemble64<<<div_up(E, 256), 256, 0, stream>>>(
+        E, d_alpha.p, d_p.p, mu, dscale, mesh->d_pos_fwd.p, mesh->d_pos_bwd.p, d_dkeo64.p,
+        sys_off.empty() ? nullptr : d_mu_sys.p, d_esys.p);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
   dkeo_mu = mu;
@@ -794,6 +825,7 @@ void NlsImpl::compute_f64(const double *x, double g, double mu, double *f, int n
 
 void NlsImpl::residual_update(const double *x, const float *dx, double g, double mu, double *f, double *soff) {
   if (!(keo_mu == mu)) keo_refill(mu);
+  ensure_keo32();
   ResidualUpdateOp op{d_kdiag.p, d_cvt.p, d_V.p, g, (const C2<double> *)x, (C2<double> *)f, (C2<double> *)soff};
   launch_rows<float>(*this, d_keo32.p, (const C2<float> *)dx, op, red.host);
 }
@@ -814,6 +846,7 @@ __global__ void abs_rowmax_kernel(int64_t n, const int32_t *__restrict__ rp, con
 double NlsImpl::keo_abs_rowmax() {
   if (abs_rowmax_ >= 0.0) return abs_rowmax_;
   if (!(keo_mu == keo_mu)) keo_refill(mu0);
+  ensure_keo32();
   DevBuf<unsigned long long> w(1);
   w.zero(stream);
   abs_rowmax_kernel<<<div_up(N, 256), 256, 0, stream>>>(N, mesh->d_rp.p, d_keo32.p, w.p);
@@ -869,6 +902,7 @@ void NlsImpl::jac_rebuild(const double *x, double g, double mu, bool want32) {
 
 void NlsImpl::operators32_rebuild(const double *x, double g, double mu) {
   if (!(keo_mu == mu)) keo_refill(mu);
+  ensure_keo32();
   jac_reg_diag_kernel<float><<<div_up(N, 256), 256, 0, stream>>>(N, d_kdiag.p, d_cvt.p, d_V.p, g,
                                                                   (const C2<double> *)x, d_jd32.p, d_rd32.p);
   ++launch_count;
@@ -902,6 +936,7 @@ void NlsImpl::reg_rebuild(const double *x, double g, double mu, bool want32) {
 }
 
 void NlsImpl::ensure_diag32() {
+  ensure_keo32();
   if (jac_ready && !jd32_ok) {
     launch_f64_to_f32(d_jd64.p, d_jd32.p, 3 * N, stream);
     jd32_ok = true;
@@ -912,26 +947,14 @@ void NlsImpl::ensure_diag32() {
   }
 }
 
-template <>
-void NlsImpl::jac_apply<double>(const double *x, double *y, double *dot_out) {
-  if (dot_out) {
-    BlockDiagOp<double, true> op{d_jd64.p, (const C2<double> *)x, (C2<double> *)y};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, dot_out);
-  } else {
-    BlockDiagOp<double, false> op{d_jd64.p, (const C2<double> *)x, (C2<double> *)y};
-    launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, nullptr);
-  }
+void NlsImpl::jac_apply(const double *x, double *y) {
+  BlockDiagOp<double, false> op{d_jd64.p, (const C2<double> *)x, (C2<double> *)y};
+  launch_rows<double>(*this, d_keo64.p, (const C2<double> *)x, op, nullptr);
 }
 
-template <>
-void NlsImpl::jac_apply<float>(const float *x, float *y, double *dot_out) {
-  if (dot_out) {
-    BlockDiagOp<float, true> op{d_jd32.p, (const C2<float> *)x, (C2<float> *)y};
-    launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, dot_out);
-  } else {
-    BlockDiagOp<float, false> op{d_jd32.p, (const C2<float> *)x, (C2<float> *)y};
-    launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, nullptr);
-  }
+void NlsImpl::jac_apply32(const float *x, double *y, bool overlap) {
+  BlockDiagOp<float, false, double> op{d_jd32.p, (const C2<float> *)x, (C2<double> *)y};
+  launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, nullptr, overlap && overlap_launches);
 }
 
 template <>
@@ -942,6 +965,7 @@ void NlsImpl::reg_apply<double>(const double *x, double *y) {
 
 template <>
 void NlsImpl::reg_apply<float>(const float *x, float *y) {
+  ensure_keo32();
   BlockDiagOp<float, false> op{d_rd32.p, (const C2<float> *)x, (C2<float> *)y};
   launch_rows<float>(*this, d_keo32.p, (const C2<float> *)x, op, nullptr);
 }

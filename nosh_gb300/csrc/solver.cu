@@ -265,6 +265,7 @@ void Minres<T>::wx_final(int j) {
 template <typename T>
 int Minres<T>::solve(const double *rhs, double scale, double rtol, int maxit, int &status, double &rel_res) {
   cudaStream_t st = s.stream;
+  if (sizeof(T) == 4) s.ensure_keo32();
   MinresScalars *d = sc.p;
   // with kernel timing on, the graphs carry event-record nodes around the
   // timed launches: captured anew when timing is switched

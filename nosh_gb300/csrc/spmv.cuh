@@ -681,12 +681,12 @@ struct PlainOp {
 
 // y = K_offdiag x + [[d0r, d1b], [d1b, d0i]] x_i (Jacobian or regularised
 // KEO; the diagonal blocks include K_ii); optionally sum_i <x_i, y_i>.
-template <typename T, bool kDot>
+template <typename T, bool kDot, typename Out = T>
 struct BlockDiagOp {
   static constexpr bool kReduce = kDot;
   const T *d;  // 3 per vertex
   const C2<T> *x;
-  C2<T> *y;
+  C2<Out> *y;
   struct Pre {
     C2<T> xi;
     T d0r, d0i, d1b;
@@ -695,7 +695,7 @@ struct BlockDiagOp {
   __device__ double finish(int i, T sr, T si, const Pre &p) const {
     const T yr = sr + p.d0r * p.xi.x + p.d1b * p.xi.y;
     const T yi = si + p.d1b * p.xi.x + p.d0i * p.xi.y;
-    y[i] = C2<T>{yr, yi};
+    y[i] = C2<Out>{(Out)yr, (Out)yi};
     return kDot ? (double)p.xi.x * (double)yr + (double)p.xi.y * (double)yi : 0.0;
   }
 };
