@@ -499,7 +499,9 @@ struct ChebMinresOp {
     const C2<T> z = cheb_apply<T>(i, step, sr, si, p, coef, d, xout);
     return (double)p.bi.x * (double)z.x + (double)p.bi.y * (double)z.y;
   }
-  __device__ void hook(double total) const { minres_advance(s, total); }
+  static constexpr int kHeadWords = kMinresHeadWords;
+  __device__ const double *head() const { return reinterpret_cast<const double *>(s); }
+  __device__ void hook(double total, const double *state) const { minres_advance(s, state, total); }
 };
 
 // The fine level's last step of a batch: also rowdot[i] = <b_i, x_i>.
@@ -1313,11 +1315,11 @@ __global__ void __launch_bounds__(kTailThreads)
                    : "memory");
     cluster_arrive();
     cluster_wait();
-    if (R.rank == 0 && threadIdx.x == 0) {
+    if (R.rank == 0 && threadIdx.x < 32) {
       dep_trigger();
       double t = 0.0;
       for (int q = 0; q < R.nct; q++) t += s_dot[q];
-      minres_advance(a.ms, t);
+      minres_advance(a.ms, reinterpret_cast<const double *>(a.ms), t);
     }
   } else {
     cluster_arrive();
@@ -1346,7 +1348,8 @@ __global__ void dot_advance(int64_t n, const C2<T> *__restrict__ a, const C2<T> 
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) v = (double)a[i].x * b[i].x + (double)a[i].y * b[i].y;
   double total = 0.0;
-  if (grid_reduce(v, partials, counter, &s->rz, &total)) minres_advance(s, total);
+  if (grid_reduce(v, partials, counter, &s->rz, &total))
+    minres_advance(s, reinterpret_cast<const double *>(s), total);
 }
 
 // the longest 4-aligned range of nonzeros of a block of kRows rows

@@ -182,13 +182,21 @@ __global__ void __launch_bounds__(kSysThreads)
     for (int q = c0 + threadIdx.x; q < c1; q += kSysThreads) v += __ldcg(cpart + q);
     v = block_sum(v, s32);
   }
+  if (threadIdx.x < 32) {
+    v = __shfl_sync(0xffffffffu, v, 0);
+    MinresScalars *s = sc + sy;
+    if (Mode == kInit) {
+      if (threadIdx.x == 0) sys_init(s, v, rtol[sy], maxit);
+    } else if (Mode == kLanczos) {
+      minres_lanczos_coefs(s, reinterpret_cast<const double *>(s), v);
+    } else {
+      minres_advance(s, reinterpret_cast<const double *>(s), v);
+    }
+    __threadfence();
+    __syncwarp();
+  }
   if (threadIdx.x == 0) {
     counter[sy] = 0u;
-    MinresScalars *s = sc + sy;
-    if (Mode == kInit) sys_init(s, v, rtol[sy], maxit);
-    else if (Mode == kLanczos) minres_lanczos_coefs(s, v);
-    else minres_advance(s, v);
-    __threadfence();
     last = atomicAdd(counter + S, 1u) == (unsigned)(S - 1);
     if (last) counter[S] = 0u;
     run = 0;

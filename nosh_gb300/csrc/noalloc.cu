@@ -51,7 +51,11 @@ double *scratch_on_current_device() {
 struct ResidualNormOp : ResidualOp<true> {
   static constexpr bool kHook = true;
   double *norm;
-  __device__ void hook(double total) const { *norm = sqrt(total); }
+  static constexpr int kHeadWords = 0;
+  __device__ const double *head() const { return nullptr; }
+  __device__ void hook(double total, const double *) const {
+    if (threadIdx.x == 0) *norm = sqrt(total);
+  }
 };
 
 // Device memory of `device` (or managed memory, reachable from every

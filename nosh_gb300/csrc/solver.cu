@@ -91,7 +91,8 @@ __global__ void dot_init(int64_t n, const T *__restrict__ a, const T *__restrict
   }
   for (; i < n; i += stride) v += (double)a[i] * (double)b[i];
   double total = 0.0;
-  if (grid_reduce(v, partials, counter, &s->rz, &total)) minres_init(s, total, args->rtol, args->maxit);
+  if (grid_reduce(v, partials, counter, &s->rz, &total) && threadIdx.x == 0)
+    minres_init(s, total, args->rtol, args->maxit);
 }
 
 // the host's view of the recurrence (pinned memory), before a poll
@@ -157,8 +158,12 @@ struct JacMinresOp {
     }
     return (double)(p.xi.x * yr + p.xi.y * yi);
   }
-  // the finishing thread turns <z, J z> into the Lanczos coefficients
-  __device__ void hook(double total) const { minres_lanczos_coefs(const_cast<MinresScalars *>(s), total); }
+  // the finishing warp turns <z, J z> into the Lanczos coefficients
+  static constexpr int kHeadWords = kMinresHeadWords;
+  __device__ const double *head() const { return reinterpret_cast<const double *>(s); }
+  __device__ void hook(double total, const double *state) const {
+    minres_lanczos_coefs(const_cast<MinresScalars *>(s), state, total);
+  }
 };
 
 template <typename T>

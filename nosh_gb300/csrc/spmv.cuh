@@ -58,10 +58,14 @@ template <> struct Acc<double> { using type = double; };
 
 // Grid-wide deterministic sum of one double per thread: block partials, then
 // the last CTA to arrive adds them in fixed order and stores *out.  Returns
-// true in exactly one thread (thread 0 of that last CTA), with the sum in
-// *total, so callers can continue with scalar work on the result.
-__device__ __forceinline__ bool grid_reduce(double v, double *partials, unsigned *counter,
-                                            double *out, double *total = nullptr) {
+// true in the first warp of that last CTA, with the sum in *total of all its
+// lanes, so callers can continue with scalar work on the result.  That work's
+// state (`words` <= 32 doubles at `head`) is fetched into s_head beside the
+// partials, whose loads are all under way before the first is added: their
+// latencies are the tail of the launch.
+__device__ __forceinline__ bool grid_reduce(double v, double *partials, unsigned *counter, double *out,
+                                            double *total = nullptr, const double *head = nullptr,
+                                            double *s_head = nullptr, int words = 0) {
   __shared__ double s32[32];
   __shared__ bool last;
   const double b = block_sum(v, s32);
@@ -71,30 +75,31 @@ __device__ __forceinline__ bool grid_reduce(double v, double *partials, unsigned
     last = (t == gridDim.x - 1);
   }
   __syncthreads();
-  bool finisher = false;
-  if (last) {
-    dep_trigger();
-    // four independent accumulators so the partial loads overlap (fixed
-    // order per thread: deterministic)
-    const unsigned G = gridDim.x, st = blockDim.x;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    unsigned j = threadIdx.x;
-    for (; j + 3 * st < G; j += 4 * st) {
-      a0 += __ldcg(partials + j);
-      a1 += __ldcg(partials + j + st);
-      a2 += __ldcg(partials + j + 2 * st);
-      a3 += __ldcg(partials + j + 3 * st);
-    }
-    for (; j < G; j += st) a0 += __ldcg(partials + j);
-    double s = block_sum((a0 + a1) + (a2 + a3), s32);
-    if (threadIdx.x == 0) {
-      *out = s;
-      *counter = 0u;
-      if (total) *total = s;
-      finisher = true;
-    }
+  if (!last) return false;
+  dep_trigger();
+  const unsigned G = gridDim.x, st = blockDim.x, tid = threadIdx.x;
+  const int hl = (int)tid - 32;
+  const double h = hl >= 0 && hl < words ? __ldcg(head + hl) : 0.0;
+  double a = 0.0;
+  for (unsigned j0 = 0; j0 < G; j0 += 4 * st) {
+    double t[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) t[k] = j0 + k * st + tid < G ? __ldcg(partials + j0 + k * st + tid) : 0.0;
+    a += t[0];
+    if (j0 + st < G) a += t[1];
+    if (j0 + 2 * st < G) a += t[2];
+    if (j0 + 3 * st < G) a += t[3];
   }
-  return finisher;
+  if (hl >= 0 && hl < words) s_head[hl] = h;
+  double s = block_sum(a, s32);  // (its barriers also publish s_head)
+  if (tid >= 32) return false;
+  s = __shfl_sync(0xffffffffu, s, 0);
+  if (tid == 0) {
+    *out = s;
+    *counter = 0u;
+  }
+  if (total) *total = s;
+  return true;
 }
 
 // The same for m <= K values at once (v[0..m-1], partials in columns
@@ -219,8 +224,8 @@ __device__ __forceinline__ void row_mac(double &sr, double &si, const C2<double>
 //   __device__ double finish(int row, acc sr, acc si, const Pre &)
 //                                                -- writes y[row], returns the
 //                                                   thread's partial
-// and, when kReduce, may provide kHook + hook(total): scalar work done by one
-// thread once the grid sum is known.
+// and, when kReduce, may provide kHook + hook(total, state): scalar work done
+// by one warp once the grid sum is known, on kHeadWords doubles from head().
 template <class Op, class = void>
 struct HasHook {
   static constexpr bool value = false;
@@ -230,13 +235,17 @@ struct HasHook<Op, decltype((void)Op::kHook, void())> {
   static constexpr bool value = Op::kHook;
 };
 template <class Op>
-__device__ __forceinline__ typename std::enable_if<HasHook<Op>::value>::type run_hook(const Op &op,
-                                                                                     double t) {
-  op.hook(t);
+__device__ __forceinline__ void reduce_rows(const Op &op, double part, double *partials, unsigned *counter,
+                                            double *red_out) {
+  if constexpr (HasHook<Op>::value) {
+    __shared__ double s_head[32];
+    double total = 0.0;
+    if (grid_reduce(part, partials, counter, red_out, &total, op.head(), s_head, Op::kHeadWords))
+      op.hook(total, s_head);
+  } else {
+    grid_reduce(part, partials, counter, red_out);
+  }
 }
-template <class Op>
-__device__ __forceinline__ typename std::enable_if<!HasHook<Op>::value>::type run_hook(const Op &,
-                                                                                      double) {}
 // An Op may also carry `const int *halt`: when it points at a value >= 2
 // the whole launch returns at once (MINRES iterations of a captured chunk
 // that follow convergence).
@@ -497,10 +506,7 @@ __global__ void __launch_bounds__(kRows, stage_ctas<T>())
     if (staged) mbar_wait(&bar, parity);
     return;
   }
-  if (Op::kReduce) {
-    double total = 0.0;
-    if (grid_reduce((double)part, partials, counter, red_out, &total)) run_hook(op, total);
-  }
+  if constexpr (Op::kReduce) reduce_rows(op, (double)part, partials, counter, red_out);
 }
 
 // Warp-cooperative schedule of the same SpMV + epilogue (no staging): a
@@ -585,10 +591,7 @@ __global__ void __launch_bounds__(kWarpThreads)
     }
     if (row < N) part += (typename PartOf<Op, A>::type)op.finish(row, msr, msi, pre);
   }
-  if (Op::kReduce) {
-    double total = 0.0;
-    if (grid_reduce((double)part, partials, counter, red_out, &total)) run_hook(op, total);
-  }
+  if constexpr (Op::kReduce) reduce_rows(op, (double)part, partials, counter, red_out);
 }
 
 // Resident CTAs of row_warp_apply on the device, capped by the work.
