@@ -216,7 +216,7 @@ int nosh_mesh_edges(nosh_mesh mesh, int32_t *edges) {
   return guarded([&] {
     auto &m = M(mesh);
     require(edges != nullptr, "null output");
-    std::memcpy(edges, m.edges().data(), 2 * m.E * sizeof(int32_t));
+    m.read(edges, m.d_edges, 2 * m.E);
   });
 }
 
@@ -238,8 +238,8 @@ int nosh_mesh_edge_gids_complex(nosh_mesh mesh, int32_t *idx) {
 int nosh_mesh_edge_data(nosh_mesh mesh, double *length, double *covolume) {
   return guarded([&] {
     auto &m = M(mesh);
-    if (length) std::memcpy(length, m.len().data(), m.E * sizeof(double));
-    if (covolume) std::memcpy(covolume, m.covol().data(), m.E * sizeof(double));
+    if (length) m.read(length, m.d_len, m.E);
+    if (covolume) m.read(covolume, m.d_covol, m.E);
   });
 }
 
@@ -247,7 +247,7 @@ int nosh_mesh_control_volumes(nosh_mesh mesh, double *cv) {
   return guarded([&] {
     auto &m = M(mesh);
     require(cv != nullptr, "null output");
-    std::memcpy(cv, m.cv().data(), m.N * sizeof(double));
+    m.read(cv, m.d_cv, m.N);
   });
 }
 

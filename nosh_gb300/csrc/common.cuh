@@ -40,13 +40,14 @@ template <typename T>
 struct DevBuf {
   T *p = nullptr;
   size_t n = 0;
+  bool owned = true;  // false: part of a DevSlab
   DevBuf() = default;
   explicit DevBuf(size_t count) { alloc(count); }
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
-  DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+  DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), owned(o.owned) { o.p = nullptr; o.n = 0; }
   DevBuf &operator=(DevBuf &&o) noexcept {
-    if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+    if (this != &o) { release(); p = o.p; n = o.n; owned = o.owned; o.p = nullptr; o.n = 0; }
     return *this;
   }
   ~DevBuf() { release(); }
@@ -63,9 +64,10 @@ struct DevBuf {
     n = count;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && owned) cudaFree(p);
     p = nullptr;
     n = 0;
+    owned = true;
   }
   void upload(const T *h, size_t count, cudaStream_t s) {
     if (count > n) alloc(count);
@@ -84,6 +86,36 @@ struct DevBuf {
   void zero(cudaStream_t s) {
     if (n) NOSH_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
   }
+};
+
+// One device allocation for several buffers: want() each, then commit().  The
+// slab outlives them (an allocation and its release cost 40 to 70 us for
+// buffers of megabytes, and a handle has dozens).
+struct DevSlab {
+  template <typename T>
+  void want(DevBuf<T> &b, size_t count) {
+    b.release();
+    if (count == 0) return;
+    b.n = count;
+    b.owned = false;
+    wants.push_back({reinterpret_cast<void **>(&b.p), bytes});
+    bytes += (count * sizeof(T) + kAlign - 1) / kAlign * kAlign;
+  }
+  void commit() {
+    mem.alloc(bytes);
+    for (const Want &w : wants) *w.p = mem.p + w.at;
+    wants.clear();
+  }
+
+ private:
+  static constexpr size_t kAlign = 512;
+  struct Want {
+    void **p;
+    size_t at;
+  };
+  DevBuf<char> mem;
+  std::vector<Want> wants;
+  size_t bytes = 0;
 };
 
 // True when p points to device (or managed) memory of the CUDA context.

@@ -571,12 +571,28 @@ void solve_hubs(int nvc, const int32_t *cells, const std::vector<int32_t> &hubs,
 void MeshImpl::build(const double *coords, const int32_t *cells) {
   cudaStream_t s = stream;
   const int64_t nk = nvc * T;
-  DevBuf<int32_t> d_cells;
+  slab_vertices.want(d_x, 3 * N);
+  slab_vertices.want(d_rp, N + 1);
+  slab_vertices.want(d_cv, N);
+  slab_vertices.commit();
+  DevBuf<double> coef_len, cv_part;
+  DevBuf<int> flags;  // geometry errors, hubs, longest row, longest row block
+  DevBuf<int32_t> d_cells, cnt, ptr, vc, nb, deg, up, hubs, ebase;
+  DevBuf<int64_t> tile;
+  DevSlab tmp;
+  tmp.want(coef_len, ne * T);
+  tmp.want(cv_part, nk);
+  tmp.want(flags, 4);
+  tmp.want(d_cells, nk);
+  for (DevBuf<int32_t> *b : {&cnt, &deg, &up, &hubs}) tmp.want(*b, N);
+  for (DevBuf<int32_t> *b : {&ptr, &ebase}) tmp.want(*b, N + 1);
+  tmp.want(vc, nk);
+  tmp.want(nb, (nvc - 1) * nk);
+  tmp.want(tile, div_up(N, kScanTile) + 1);
+  tmp.commit();
   d_cells.upload(cells, nk, s);
   d_x.upload(coords, 3 * N, s);
   // geometry of the cells
-  DevBuf<double> coef_len(ne * T), cv_part(nk);
-  DevBuf<int> flags(4);  // geometry errors, hubs, longest row, longest row block
   flags.zero(s);
   const int B = 128;
   if (nvc == 3)
@@ -584,8 +600,6 @@ void MeshImpl::build(const double *coords, const int32_t *cells) {
   else
     cell_geometry_kernel<4><<<div_up(T, B), B, 0, s>>>(T, d_cells.p, d_x.p, coef_len.p, cv_part.p, flags.p);
   // vertex -> (cell, slot) incidence and neighbours
-  DevBuf<int32_t> cnt(N), ptr(N + 1), vc(nk), nb((nvc - 1) * nk), deg(N), up(N), hubs(N), ebase(N + 1);
-  DevBuf<int64_t> tile(div_up(N, kScanTile) + 1);
   cnt.zero(s);
   count_incident<<<wide_grid(nk), 256, 0, s>>>(nk, d_cells.p, cnt.p);
   scan(N, cnt.p, ptr.p, tile.p, s);
@@ -610,7 +624,6 @@ void MeshImpl::build(const double *coords, const int32_t *cells) {
     solve_hubs(nvc, cells, hv, ptr, vc, nb, deg, up, s);
   }
   // row pointers and first edges
-  d_rp.alloc(N + 1);
   int64_t total[2];
   NOSH_CUDA(cudaMemcpyAsync(&total[0], tile.p + scan(N, deg.p, d_rp.p, tile.p, s), sizeof(int64_t),
                             cudaMemcpyDeviceToHost, s));
@@ -625,15 +638,15 @@ void MeshImpl::build(const double *coords, const int32_t *cells) {
   max_block = h[3];
   // column indices padded by kPad entries so that 128-bit staged loads of a
   // row block may run past its end
-  d_ci.alloc(2 * E + kPad);
+  slab_edges.want(d_ci, 2 * E + kPad);
+  slab_edges.want(d_edges, 2 * E);
+  slab_edges.want(d_pos_fwd, E);
+  slab_edges.want(d_pos_bwd, E);
+  slab_edges.want(d_nz_edge, 2 * E);
+  slab_edges.want(d_len, E);
+  slab_edges.want(d_covol, E);
+  slab_edges.commit();
   NOSH_CUDA(cudaMemsetAsync(d_ci.p + 2 * E, 0, kPad * sizeof(int32_t), s));
-  d_edges.alloc(2 * E);
-  d_pos_fwd.alloc(E);
-  d_pos_bwd.alloc(E);
-  d_nz_edge.alloc(2 * E);
-  d_len.alloc(E);
-  d_covol.alloc(E);
-  d_cv.alloc(N);
   graph_rows<<<div_up(16 * N, 256), 256, 0, s>>>(N, nvc, ptr.p, nb.p, d_rp.p, up.p, ebase.p, d_ci.p, d_edges.p,
                                                  d_pos_fwd.p, d_nz_edge.p);
   graph_back<<<div_up(E, 256), 256, 0, s>>>(E, d_edges.p, d_rp.p, d_ci.p, d_pos_bwd.p, d_nz_edge.p);

@@ -15,6 +15,7 @@ struct MeshImpl {
   // range of nonzeros of 128 consecutive rows from a multiple of 128
   int max_row = 0, max_block = 0;
 
+  DevSlab slab_vertices, slab_edges;  // memory of the buffers below
   // device: coordinates, edges (v0 < v1, lexicographic), geometry, the
   // off-diagonal KEO graph (row v: its sorted neighbours), each nonzero's edge
   // (~e if the row is v1), the nonzeros of (v0, v1) and (v1, v0) of each edge
@@ -39,8 +40,12 @@ struct MeshImpl {
   const std::vector<int32_t> &rp() { return fetch(h_rp_, d_rp, N + 1); }
   const std::vector<int32_t> &ci() { return fetch(h_ci_, d_ci, 2 * E); }
   const std::vector<double> &len() { return fetch(h_len_, d_len, E); }
-  const std::vector<double> &covol() { return fetch(h_covol_, d_covol, E); }
-  const std::vector<double> &cv() { return fetch(h_cv_, d_cv, N); }
+  // a caller's own copy
+  template <typename V>
+  void read(V *out, const DevBuf<V> &d, int64_t n) {
+    NOSH_CUDA(cudaMemcpyAsync(out, d.p, n * sizeof(V), cudaMemcpyDeviceToHost, stream));
+    NOSH_CUDA(cudaStreamSynchronize(stream));
+  }
 
   // complex graph with the diagonal (row_ptr[N+1], cols[N+2E])
   void complex_graph(int32_t *row_ptr, int32_t *cols);
@@ -48,14 +53,14 @@ struct MeshImpl {
  private:
   std::mutex fetch_mtx_;
   std::vector<int32_t> h_edges_, h_rp_, h_ci_;
-  std::vector<double> h_len_, h_covol_, h_cv_;
+  std::vector<double> h_len_;
   template <typename V>
   const std::vector<V> &fetch(std::vector<V> &h, const DevBuf<V> &d, int64_t n) {
     std::lock_guard<std::mutex> lock(fetch_mtx_);
     if ((int64_t)h.size() != n) {
-      h.resize(n);
-      NOSH_CUDA(cudaMemcpyAsync(h.data(), d.p, n * sizeof(V), cudaMemcpyDeviceToHost, stream));
-      NOSH_CUDA(cudaStreamSynchronize(stream));
+      std::vector<V> v(n);
+      read(v.data(), d, n);
+      h.swap(v);
     }
     return h;
   }

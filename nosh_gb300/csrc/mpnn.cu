@@ -1356,6 +1356,7 @@ struct Mpnn::Impl {
   // inference overlaps the solver; own reduction scratch for the features
   cudaStream_t stream;
   Reducer rd;
+  DevSlab slab;
   explicit Impl(NlsImpl &nls);
   void refresh_bf16();
   void forward(bool train);               // X -> pooled embedding
@@ -1370,7 +1371,10 @@ struct Mpnn::Impl {
 
 Mpnn::Impl::Impl(NlsImpl &nls) : s(nls), N(nls.N), nnz(2 * nls.E), stream(nls.stream) {
   cudaStream_t st = s.stream;
-  rd.init(2 * (vgrid(N) + 64), 4, st);  // history_dots: up to 8 slots of partials
+  rd.init(2 * (vgrid(N) + 64), 4, slab);  // history_dots: up to 8 slots of partials
+  slab.commit();
+  rd.counter.zero(st);
+  rd.out.zero(st);
   MeshImpl &m = *s.mesh;
   // normalisation of the edge features from the mesh and fields
   std::vector<double> alpha(s.E), p(s.E);

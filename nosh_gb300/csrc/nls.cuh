@@ -27,13 +27,15 @@ struct Reducer {
   ~Reducer() {
     if (host) cudaFreeHost(host);
   }
-  void init(int max_blocks, int nslots, cudaStream_t s) {
-    partials.alloc(max_blocks * 4 + 64);
-    counter.alloc(16);
-    counter.zero(s);
-    out.alloc(nslots);
-    out.zero(s);
-    if (!host) NOSH_CUDA(cudaMallocHost(&host, 16 * sizeof(double)));
+  // the buffers from the handle's slab (whose owner zeroes counter and out);
+  // behind the host slots one more double for the owner's failure word (a
+  // pinned allocation costs 130 to 240 us)
+  static constexpr int kHostSlots = 16;
+  void init(int max_blocks, int nslots, DevSlab &slab) {
+    slab.want(partials, max_blocks * 4 + 64);
+    slab.want(counter, 16);
+    slab.want(out, nslots);
+    if (!host) NOSH_CUDA(cudaMallocHost(&host, (kHostSlots + 1) * sizeof(double)));
   }
 };
 
@@ -152,6 +154,7 @@ struct NlsImpl {
   std::string deriv_param;
   double g0, mu0;
 
+  DevSlab slab;  // memory of the handle's own buffers
   // fields (FP64) and derived per-edge / per-vertex data
   DevBuf<double> d_A, d_V, d_t, d_cvt;  // 3N, N, N, N (cv * thickness)
   std::vector<double> h_V, h_t;

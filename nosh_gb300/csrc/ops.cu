@@ -74,11 +74,14 @@ __device__ __forceinline__ void edge_sincos(double x, double &s, double &c) {
   constexpr double s1 = -1.0 / 6, s2 = 1.0 / 120, s3 = -1.0 / 5040, s4 = 1.0 / 362880, s5 = -1.0 / 39916800;
   constexpr double c1 = -1.0 / 2, c2 = 1.0 / 24, c3 = -1.0 / 720, c4 = 1.0 / 40320, c5 = -1.0 / 3628800,
                    c6 = 1.0 / 479001600;
-  if (fabs(x) <= 0.02) {
+  // (the range by the high words: a comparison of doubles is an FP64
+  // instruction)
+  const int hx = __double2hiint(x) & 0x7fffffff;
+  if (hx < 0x3f947ae1) {  // |x| < 0.02
     const double x2 = x * x;
     s = fma(x * x2, fma(x2, fma(x2, s3, s2), s1), x);
     c = fma(x2, fma(x2, fma(x2, fma(x2, c4, c3), c2), c1), 1.0);
-  } else if (fabs(x) <= 0.1) {
+  } else if (hx < 0x3fb99999) {  // |x| < 0.1
     const double x2 = x * x;
     s = fma(x * x2, fma(x2, fma(x2, fma(x2, fma(x2, s5, s4), s3), s2), s1), x);
     c = fma(x2, fma(x2, fma(x2, fma(x2, fma(x2, fma(x2, c6, c5), c4), c3), c2), c1), 1.0);
@@ -362,10 +365,12 @@ bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T>
   DevBuf<C2<T>> xb, yb;
   DevBuf<T> db;
   DevBuf<double> rb;
-  xb.alloc(N);
-  yb.alloc(N);
-  db.alloc(3 * (int64_t)N);
-  rb.alloc(1);
+  DevSlab tmp;
+  tmp.want(xb, N);
+  tmp.want(yb, N);
+  tmp.want(db, 3 * (int64_t)N);
+  tmp.want(rb, 1);
+  tmp.commit();
   xb.zero(st);
   db.zero(st);
   // a representative epilogue: the diagonal block and a grid reduction, as
@@ -590,14 +595,24 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
   }
   h_V.assign(V, V + N);
   h_t.assign(t, t + N);
+  const size_t nz = 2 * E + kPad;
+  slab.want(d_A, 3 * N);
+  for (DevBuf<double> *b : {&d_V, &d_t, &d_cvt, &d_kdiag}) slab.want(*b, N);
+  for (DevBuf<double> *b : {&d_p, &d_alpha}) slab.want(*b, E);
+  slab.want(d_kdiagf, N);
+  slab.want(d_keo64, nz);
+  slab.want(d_keo32, nz);
+  slab.want(d_dkeo64, nz);
+  for (DevBuf<double> *b : {&d_jd64, &d_rd64}) slab.want(*b, 3 * N);
+  for (DevBuf<float> *b : {&d_jd32, &d_rd32}) slab.want(*b, 3 * N);
+  for (DevBuf<double> *b : {&d_in, &d_out, &d_tmp}) slab.want(*b, 2 * N);
+  slab.want(d_inf, 2 * N * kCastVectors);
+  slab.want(d_outf, 2 * N);
+  red.init(div_up(N, kRows) + div_up(N, 256) + 1024, 64, slab);
+  slab.commit();
   d_A.upload(mvp, 3 * N, s);
   d_V.upload(h_V, s);
   d_t.upload(h_t, s);
-  d_p.alloc(E);
-  d_alpha.alloc(E);
-  d_kdiag.alloc(N);
-  d_kdiagf.alloc(N);
-  d_cvt.alloc(N);
   edge_fields_kernel<<<div_up(E, 256), 256, 0, s>>>(E, m->d_edges.p, m->d_x.p, d_A.p, m->d_len.p,
                                                      m->d_covol.p, d_t.p, d_p.p, d_alpha.p);
   ++launch_count;
@@ -606,28 +621,12 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
                                                        d_cvt.p);
   ++launch_count;
   NOSH_CUDA(cudaGetLastError());
-  const size_t nz = 2 * E + kPad;
-  d_keo64.alloc(nz);
-  d_keo32.alloc(nz);
-  d_dkeo64.alloc(nz);
-  d_keo64.zero(s);
+  for (DevBuf<C2<double>> *b : {&d_keo64, &d_dkeo64}) b->zero(s);
   d_keo32.zero(s);
-  d_dkeo64.zero(s);
-  d_jd64.alloc(3 * N);
-  d_rd64.alloc(3 * N);
-  d_jd32.alloc(3 * N);
-  d_rd32.alloc(3 * N);
-  d_jd64.zero(s);
-  d_rd64.zero(s);
-  d_jd32.zero(s);
-  d_rd32.zero(s);
-  d_in.alloc(2 * N);
-  d_out.alloc(2 * N);
-  d_tmp.alloc(2 * N);
-  d_inf.alloc(2 * N * kCastVectors);
-  d_outf.alloc(2 * N);
-  red.init(div_up(N, kRows) + div_up(N, 256) + 1024, 64, s);
-  NOSH_CUDA(cudaMallocHost(&h_stage_err, sizeof(unsigned)));
+  for (DevBuf<double> *b : {&d_jd64, &d_rd64, &red.out}) b->zero(s);
+  for (DevBuf<float> *b : {&d_jd32, &d_rd32}) b->zero(s);
+  red.counter.zero(s);
+  h_stage_err = reinterpret_cast<unsigned *>(red.host + Reducer::kHostSlots);
   *h_stage_err = 0u;
   NOSH_CUDA(cudaMemcpyAsync(red.counter.p + kStageErrorSlot, &h_stage_err, sizeof(h_stage_err),
                             cudaMemcpyHostToDevice, s));
@@ -729,7 +728,6 @@ NlsImpl::~NlsImpl() {
   solver_state.reset();
   amg.reset();
   if (stream) cudaStreamDestroy(stream);
-  if (h_stage_err) cudaFreeHost(h_stage_err);
 }
 
 void NlsImpl::sync() {
