@@ -454,34 +454,42 @@ __global__ void __launch_bounds__(kRows, stage_ctas<T>())
     const int32_t *s_col = reinterpret_cast<const int32_t *>(smem_raw);
     const C2<T> *s_val = reinterpret_cast<const C2<T> *>(smem_raw + (size_t)cap * sizeof(int32_t));
     A sr = 0, si = 0;
-    if (row < N) {
-      if (staged) {
-        // batches of kBatch nonzeros per lane (the row's lanes take every
-        // R-th one): all gathers of a batch are issued before the first is
-        // used (a row of the mesh graph is one or two); the values are read
-        // from shared memory when used, so only the gathered x of a batch
-        // occupies registers
-        constexpr int kBatch = 8;
-        for (int k0 = b - ks + lane_r; k0 < e - ks; k0 += kBatch << lr) {
-          const int cnt = (e - ks - k0 + R - 1) >> lr;
-          C2<T> xv[kBatch];
+    if (staged) {
+      // batches of kBatch nonzeros per lane (the row's lanes take every R-th
+      // one): all gathers of a batch are issued before the first is used (a
+      // row of the mesh graph is one or two); the values are read from shared
+      // memory when used, so only the gathered x of a batch occupies registers
+      // An FP64 instruction whose lanes are all off still takes the pipe, so a
+      // batch goes by pairs of nonzeros, and a branch that the whole warp takes
+      // skips those beyond its longest row: rows of 14 paid for 16, rows of 6
+      // for 8.  J rebuild + apply at 160^3 643 -> 565 us, V-cycles at 48^3 611
+      // -> 563 us, 24 squares of 97^2 16.0 -> 14.9 ms.  FP32 predicates each
+      // nonzero (in pairs three products at 64^3 lost 2 %).
+      constexpr int kBatch = 8, kPair = sizeof(T) == 8 ? 2 : 1;
+      const int k0 = b - ks + lane_r, cnt = row < N ? (e - ks - k0 + R - 1) >> lr : 0;
+      const int most = __reduce_max_sync(0xffffffffu, cnt);
+      for (int q = 0; q < most; q += kBatch) {
+        C2<T> xv[kBatch];
 #pragma unroll
-          for (int u = 0; u < kBatch; u++)
-            if (u < cnt) xv[u] = ldg(x + s_col[k0 + (u << lr)]);
+        for (int g = 0; g < kBatch; g += kPair)
+          if (g == 0 || q + g < most) {
 #pragma unroll
-          for (int u = 0; u < kBatch; u++) {
-            if (u < cnt) {
-              const C2<T> v = s_val[k0 + (u << lr)];
-              row_mac(sr, si, v, xv[u]);
-            }
+            for (int u = g; u < g + kPair; u++)
+              if (q + u < cnt) xv[u] = ldg(x + s_col[k0 + ((q + u) << lr)]);
           }
-        }
-      } else {
-        for (int k = b + lane_r; k < e; k += R) {
-          const C2<T> v = ldg(val + k);
-          const C2<T> xv = ldg(x + __ldg(ci + k));
-          row_mac(sr, si, v, xv);
-        }
+#pragma unroll
+        for (int g = 0; g < kBatch; g += kPair)
+          if (g == 0 || q + g < most) {
+#pragma unroll
+            for (int u = g; u < g + kPair; u++)
+              if (q + u < cnt) row_mac(sr, si, s_val[k0 + ((q + u) << lr)], xv[u]);
+          }
+      }
+    } else if (row < N) {
+      for (int k = b + lane_r; k < e; k += R) {
+        const C2<T> v = ldg(val + k);
+        const C2<T> xv = ldg(x + __ldg(ci + k));
+        row_mac(sr, si, v, xv);
       }
     }
     // the row's lanes are adjacent: fold their partial sums into lane 0, one
