@@ -664,12 +664,10 @@ __global__ void coarse_dense(int64_t n, const int32_t *__restrict__ rp, const in
 }
 
 // Gauss-Jordan inversion of the coarsest level's SPD blocks (no pivoting
-// needed), kPivots pivots a launch, in the arithmetic type C (FP32 for the
-// mixed path: the coarsest operator is well conditioned).  A CTA owns
-// kPivotCols columns of a block: it inverts the pivot block P (every CTA does),
-// takes R = P^-1 times its columns' pivot rows and subtracts the pivot columns
-// times R from the other rows; a column of the pivot block itself starts from
-// the identity.  It reads src and writes dst, since every CTA reads the pivot
+// needed), kPivots pivots a launch, in FP64.  A CTA owns kPivotCols columns of
+// a block: it inverts the pivot block P (every CTA does), takes R = P^-1 times
+// its columns' pivot rows and subtracts the pivot columns times R from the
+// other rows; a column of the pivot block itself starts from the identity.  It reads src and writes dst, since every CTA reads the pivot
 // columns.  After the last launch the FP32 copy is written as well.
 //
 // Most of a launch's 13 us in FP64 is the chain of 16 reciprocals and updates
@@ -677,7 +675,6 @@ __global__ void coarse_dense(int64_t n, const int32_t *__restrict__ rp, const in
 // multiply-adds: 661 -> 104 us for a block of 128 rows, 35 -> 26 us for one of
 // 32 (an FP64 continuation at 32^3 with two of the former 16.2 -> 14.8 ms).
 constexpr int kPivots = 16, kPivotCols = 2, kPivotThreads = 128;
-template <typename C>
 __global__ void __launch_bounds__(kPivotThreads)
     gauss_jordan_step(const int64_t *__restrict__ boff, const int32_t *__restrict__ bd, int k0, int last,
                       const double *__restrict__ src, double *__restrict__ dst, float *__restrict__ Afg, int *err) {
@@ -698,34 +695,34 @@ __global__ void __launch_bounds__(kPivotThreads)
     }
     return;
   }
-  __shared__ C P[2][kPivots][kPivots + 1], Y[kPivots][kPivotCols], R[kPivots][kPivotCols];
+  __shared__ double P[2][kPivots][kPivots + 1], Y[kPivots][kPivotCols], R[kPivots][kPivotCols];
   const int r = threadIdx.x / (kPivots / 2), c = threadIdx.x % (kPivots / 2) * 2;
 #pragma unroll
-  for (int q = 0; q < 2; q++) P[0][r][c + q] = r < nk && c + q < nk ? (C)A[(int64_t)(k0 + r) * m + k0 + c + q] : (C)0;
+  for (int q = 0; q < 2; q++) P[0][r][c + q] = r < nk && c + q < nk ? A[(int64_t)(k0 + r) * m + k0 + c + q] : 0.0;
   if (threadIdx.x < kPivots * kPivotCols) {
     const int l = threadIdx.x / kPivotCols, jj = threadIdx.x % kPivotCols;
-    Y[l][jj] = l < nk && jj < nc ? (C)A[(int64_t)(k0 + l) * m + j0 + jj] : (C)0;
+    Y[l][jj] = l < nk && jj < nc ? A[(int64_t)(k0 + l) * m + j0 + jj] : 0.0;
   }
   __syncthreads();
   for (int k = 0; k < nk; k++) {
-    const C(*S)[kPivots + 1] = P[k & 1];
-    const C piv = S[k][k];
-    if (threadIdx.x == 0 && blockIdx.y == 0 && !(piv > (C)0)) atomicOr(err, 16);
-    const C ip = (C)1 / piv;
-    const C f = r == k ? ip : -S[r][k] * ip;
+    const double(*S)[kPivots + 1] = P[k & 1];
+    const double piv = S[k][k];
+    if (threadIdx.x == 0 && blockIdx.y == 0 && !(piv > 0.0)) atomicOr(err, 16);
+    const double ip = 1.0 / piv;
+    const double f = r == k ? ip : -S[r][k] * ip;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
-      const C a = c + q == k ? (C)0 : S[r][c + q], pk = c + q == k ? (C)1 : S[k][c + q];
+      const double a = c + q == k ? 0.0 : S[r][c + q], pk = c + q == k ? 1.0 : S[k][c + q];
       P[(k & 1) ^ 1][r][c + q] = r == k ? pk * f : a + f * pk;
     }
     __syncthreads();
   }
-  const C(*S)[kPivots + 1] = P[nk & 1];
+  const double(*S)[kPivots + 1] = P[nk & 1];
   if (threadIdx.x < kPivots * kPivotCols) {
     const int l = threadIdx.x / kPivotCols, jj = threadIdx.x % kPivotCols, jp = j0 + jj - k0;
-    C v = 0;
+    double v = 0;
     if (jp >= 0 && jp < nk) {
-      v = l < nk ? S[l][jp] : (C)0;
+      v = l < nk ? S[l][jp] : 0.0;
     } else {
 #pragma unroll
       for (int q = 0; q < kPivots; q++) v += S[l][q] * Y[q][jj];
@@ -736,29 +733,70 @@ __global__ void __launch_bounds__(kPivotThreads)
   for (int i = threadIdx.x; i < m; i += kPivotThreads) {
     const int ip = i - k0;
     const bool pivot_row = ip >= 0 && ip < nk;
-    C v[kPivotCols];
+    double v[kPivotCols];
 #pragma unroll
     for (int jj = 0; jj < kPivotCols; jj++) {
       const int jp = j0 + jj - k0;
-      v[jj] = pivot_row ? R[ip][jj] : jj >= nc || (jp >= 0 && jp < nk) ? (C)0 : (C)A[(int64_t)i * m + j0 + jj];
+      v[jj] = pivot_row ? R[ip][jj] : jj >= nc || (jp >= 0 && jp < nk) ? 0.0 : A[(int64_t)i * m + j0 + jj];
     }
     if (!pivot_row)
 #pragma unroll
       for (int q = 0; q < kPivots; q++) {
-        const C a = q < nk ? (C)A[(int64_t)i * m + k0 + q] : (C)0;
+        const double a = q < nk ? A[(int64_t)i * m + k0 + q] : 0.0;
 #pragma unroll
         for (int jj = 0; jj < kPivotCols; jj++) v[jj] -= a * R[q][jj];
       }
 #pragma unroll
     for (int jj = 0; jj < kPivotCols; jj++)
       if (jj < nc) {
-        B[(int64_t)i * m + j0 + jj] = (double)v[jj];
+        B[(int64_t)i * m + j0 + jj] = v[jj];
         if (last) Af[(int64_t)i * m + j0 + jj] = (float)v[jj];
       }
   }
 }
-// Blocks of more rows than this are inverted in FP64 on the mixed path too.
+// The same in FP32 on the mixed path, one CTA a block of up to kDenseFp32 rows
+// in shared memory (43 us for 54 rows, bound by its barriers); larger blocks
+// are inverted in FP64 there too.  An FP64 solve that follows on the handle
+// works with this inverse until its own refresh, and the rounding of the
+// elimination shows in its iterates: by blocks of pivots (20 us) they moved by
+// 1e-10 to 1e-9 relative, so the mixed path keeps this order.
 constexpr int kDenseFp32 = 128;
+__global__ void gauss_jordan_fp32(const int64_t *__restrict__ boff, const int32_t *__restrict__ bd, double *Ag,
+                                  float *Afg, int *err) {
+  // one CTA per diagonal block of the coarsest level
+  const int m = bd[blockIdx.x];
+  double *A = Ag + boff[blockIdx.x];
+  float *Af = Afg + boff[blockIdx.x];
+  extern __shared__ __align__(16) unsigned char gj_raw[];
+  float *S = reinterpret_cast<float *>(gj_raw);
+  __shared__ float ip_s;
+  for (int q = threadIdx.x; q < m * m; q += blockDim.x) S[q] = (float)A[q];
+  __syncthreads();
+  for (int k = 0; k < m; k++) {
+    if (threadIdx.x == 0) {
+      const float piv = S[k * m + k];
+      if (!(piv > 0.f)) atomicOr(err, 16);
+      ip_s = 1.f / piv;
+    }
+    __syncthreads();
+    const float ip = ip_s;
+    for (int j = threadIdx.x; j < m; j += blockDim.x) S[k * m + j] = (j == k) ? ip : S[k * m + j] * ip;
+    __syncthreads();
+    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
+      const int i = q / m, j = q % m;
+      if (i == k || j == k) continue;
+      S[q] -= S[i * m + k] * S[k * m + j];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x)
+      if (i != k) S[i * m + k] = -S[i * m + k] * ip;
+    __syncthreads();
+  }
+  for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
+    A[q] = (double)S[q];
+    Af[q] = S[q];
+  }
+}
 
 // Packed block-diagonal dense inverse: real row i of the coarsest level is
 // row rowoff[i] of the packed array, its block starts at real row bstart[i]
@@ -1591,6 +1629,8 @@ Amg::Amg(NlsImpl &s, const AmgOptions &o) : impl(new Impl(s, o)) {
   }
   I.err.alloc(1);
   I.err.zero(st);
+  NOSH_CUDA(cudaFuncSetAttribute(gauss_jordan_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kDenseFp32 * kDenseFp32 * (int)sizeof(float)));
   s.sync();
 }
 
@@ -1721,16 +1761,19 @@ void Amg::refresh() {
     tuned = true;
   }
   const AmgLevel &C = I.lev.back();
-  const int steps = div_up(I.max_dim, kPivots);
+  const bool fp32 = sizeof(T) == 4 && I.max_dim <= kDenseFp32;
+  const int steps = fp32 ? 0 : div_up(I.max_dim, kPivots);
   double *buf[2] = {I.dense.p, I.dense2.p};  // the last step writes the first
   coarse_dense<T><<<div_up(C.n, 128), 128, 0, st>>>(C.n, C.rp, C.ci, I.off<T>(L - 1), I.dia<T>(L - 1),
                                                      I.row_start.p, I.row_off.p, I.row_dim.p, buf[steps & 1]);
-  const auto step = I.max_dim <= kDenseFp32 ? gauss_jordan_step<T> : gauss_jordan_step<double>;
+  if (fp32)
+    gauss_jordan_fp32<<<I.nblk, 1024, (size_t)I.max_dim * I.max_dim * sizeof(float), st>>>(
+        I.blk_off.p, I.blk_dim.p, I.dense.p, I.densef.p, I.err.p);
   for (int k = 0; k < steps; k++)
-    launch_dep(I.ovl(), step, dim3(I.nblk, div_up(I.max_dim, kPivotCols)), dim3(kPivotThreads), 0, st, I.blk_off.p,
-               I.blk_dim.p, k * kPivots, (int)(k == steps - 1), (const double *)buf[(steps - k) & 1],
+    launch_dep(I.ovl(), gauss_jordan_step, dim3(I.nblk, div_up(I.max_dim, kPivotCols)), dim3(kPivotThreads), 0, st,
+               I.blk_off.p, I.blk_dim.p, k * kPivots, (int)(k == steps - 1), (const double *)buf[(steps - k) & 1],
                buf[(steps - k - 1) & 1], I.densef.p, I.err.p);
-  I.nls.launch_count += 1 + steps;
+  I.nls.launch_count += 1 + (fp32 ? 1 : steps);
   NOSH_CUDA(cudaGetLastError());
 }
 

@@ -2,7 +2,7 @@
 
 A hierarchy of one level is the inverse itself, so that the preconditioner
 solves K_reg x = b.  The inverse is of 2 N real rows: 8, 16 and 18, 32 and 34
-take one to three steps with whole and ragged last ones, 128 is the largest
+take one to three steps with whole and ragged last ones in FP64, 128 is the largest
 that the mixed path inverts in FP32, 130 the smallest it inverts in FP64 there;
 a batch has blocks of several sizes in one launch.  Forward error bound of a
 solve by an explicit inverse: 4 m cond(K) machine epsilons, and the rounding
