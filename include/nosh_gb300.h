@@ -73,7 +73,8 @@ int nosh_device_count(int *count);
  * and control volumes (compute_control_volumes_t_, src/mesh_tri.cpp:187-210 /
  * src/mesh_tetra.cpp:196-271).  coords: 3*N doubles; cells: T*verts_per_cell
  * vertex ids, verts_per_cell = 3 (triangles) or 4 (tetrahedra).  Geometry is
- * computed on the GPU in FP64; integer work on the host. */
+ * computed on the GPU in FP64, and so are the edges and the graph; vertices with
+ * more than 84 cells are finished on the host. */
 int nosh_mesh_create(const double *coords, int64_t num_vertices,
                      const int32_t *cells, int64_t num_cells,
                      int verts_per_cell, nosh_mesh *out);
