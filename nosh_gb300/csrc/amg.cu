@@ -667,8 +667,9 @@ __global__ void coarse_dense(int64_t n, const int32_t *__restrict__ rp, const in
 // needed), kPivots pivots a launch, in FP64.  A CTA owns kPivotCols columns of
 // a block: it inverts the pivot block P (every CTA does), takes R = P^-1 times
 // its columns' pivot rows and subtracts the pivot columns times R from the
-// other rows; a column of the pivot block itself starts from the identity.  It reads src and writes dst, since every CTA reads the pivot
-// columns.  After the last launch the FP32 copy is written as well.
+// other rows; a column of the pivot block itself starts from the identity.  It
+// reads src and writes dst, since every CTA reads the pivot columns.  After the
+// last launch the FP32 copy is written as well.
 //
 // Most of a launch's 13 us in FP64 is the chain of 16 reciprocals and updates
 // of P.  One CTA a block was bound by the FP64 pipe of its multiprocessor, m^3
@@ -1986,14 +1987,14 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
       // restriction + first step of level l+1, whose pre-smoothing must end
       // in its x buffer
       C2<T> *first = (deg % 2 == 1) ? V.x[l + 1].p : V.x2[l + 1].p;
-      launch_dep(ovl(), few ? restrict_first<T, 8> : restrict_first<T, 16>, dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
-                 A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p, V.coef[l + 1].p, V.d[l + 1].p, first,
+      launch_dep(ovl(), few ? restrict_first<T, 8> : restrict_first<T, 16>, dim3(div_up(Cl.n * (few ? 8 : 16), B)),
+                 dim3(B), 0, st, Cl.n, A.mem_ptr.p, A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p, V.coef[l + 1].p, V.d[l + 1].p, first,
                  halt);
       ++nls.launch_count;
       descend_ascend<T>(l + 1, V.b[l + 1].p, V.x[l + 1].p, nullptr);
     } else {
-      launch_dep(ovl(), few ? restrict_kernel<T, 8> : restrict_kernel<T, 16>, dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p,
-                 A.mem_idx.p, V.res[l].p, V.b[l + 1].p, halt);
+      launch_dep(ovl(), few ? restrict_kernel<T, 8> : restrict_kernel<T, 16>,
+                 dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p, A.mem_idx.p, V.res[l].p, V.b[l + 1].p, halt);
       const int m = (int)(2 * Cl.n);
       launch_dep(ovl(), dense_matvec<T>, dim3(div_up(m * kDenseLanes, B)), dim3(B), 0, st, m, dense_inv<T>(), dmap(),
                  (const T *)V.b[l + 1].p, (T *)V.x[l + 1].p, halt);

@@ -331,8 +331,8 @@ void MinresSys<T>::iteration(int j, int maxit) {
   JacRowDotOp<T> op{jd, (const C2<T> *)zc, (C2<T> *)u.p, rowdot.p, vsys.p, sc.p, (const C2<T> *)zn,
                     (C2<T> *)w[(j + 2) % 3].p, (const C2<T> *)w[j % 3].p, (const C2<T> *)w[(j + 1) % 3].p,
                     (C2<T> *)x.p, halt};
-  launch_spmv<T>(warp, (int)N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, (const C2<T> *)zc, s.mesh->max_block, op, s.red.partials.p,
-                 s.red.counter.p, nullptr, st, ovl());
+  launch_spmv<T>(warp, (int)N, s.mesh->d_rp.p, s.mesh->d_ci.p, val, (const C2<T> *)zc, s.mesh->max_block, op,
+                 s.red.partials.p, s.red.counter.p, nullptr, st, ovl());
   ++s.launch_count;
   reduce(kLanczos, maxit);
   if (!s.amg->apply_batch<T>(vsys.p, sc.p, halt, u.p, r_old, r_cur, zn, rowdot.p)) {

@@ -384,9 +384,11 @@ bool pick_warp_schedule(int N, const int32_t *rp, const int32_t *ci, const C2<T>
   float best[2] = {1e30f, 1e30f};
   for (int round = 0; round < 3; round++)
     for (int w = 0; w < 2; w++) {
-      for (int r = 0; r < 2; r++) launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, block_nnz, op, partials, counter, rb.p, st);
+      for (int r = 0; r < 2; r++)
+        launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, block_nnz, op, partials, counter, rb.p, st);
       NOSH_CUDA(cudaEventRecord(e0, st));
-      for (int r = 0; r < 5; r++) launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, block_nnz, op, partials, counter, rb.p, st);
+      for (int r = 0; r < 5; r++)
+        launch_spmv<T>(w == 1, N, rp, ci, val, xb.p, block_nnz, op, partials, counter, rb.p, st);
       NOSH_CUDA(cudaEventRecord(e1, st));
       NOSH_CUDA(cudaEventSynchronize(e1));
       float ms = 0.f;

@@ -6,9 +6,9 @@
 // contiguous: one thread stages them into shared memory with two bulk
 // asynchronous copies (TMA, cp.async.bulk: column ids and complex values)
 // completing on an mbarrier; the several CTAs of an SM overlap one another's
-// copies and arithmetic (stage_ctas).  The threads of a row then reduce its nonzeros out of shared memory and gather x through
-// the read-only path.  A row block whose nonzeros exceed the staging
-// capacity reads them directly.
+// copies and arithmetic (stage_ctas).  The threads of a row then reduce its
+// nonzeros out of shared memory and gather x through the read-only path.  A
+// row block whose nonzeros exceed the staging capacity reads them directly.
 #pragma once
 
 #include <utility>
@@ -615,7 +615,8 @@ int row_grid(const void *kernel, int threads, size_t smem, int64_t n_blocks);
 template <typename T, class Op>
 void allow_staging() {
   for (auto *k : {row_block_apply<T, Op, false>, row_block_apply<T, Op, true>})
-    NOSH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes<T>(stage_limit<T>())));
+    NOSH_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)stage_bytes<T>(stage_limit<T>())));
 }
 
 // Launch the SpMV + epilogue over an off-diagonal CSR with one of the two
