@@ -22,12 +22,16 @@ struct Error : std::runtime_error {
   Error(int c, const std::string &m) : std::runtime_error(m), code(c) {}
 };
 
+// (the runtime keeps the error of a failed call until it is asked for, so it
+// is taken here: the next call's check of its launches is not to find it)
 #define NOSH_CUDA(call)                                                      \
   do {                                                                       \
     cudaError_t e_ = (call);                                                 \
-    if (e_ != cudaSuccess)                                                   \
+    if (e_ != cudaSuccess) {                                                 \
+      cudaGetLastError();                                                    \
       throw ::nosh::Error(NOSH_ERR_CUDA, std::string(#call) + ": " +         \
                                              cudaGetErrorString(e_));        \
+    }                                                                        \
   } while (0)
 
 #define NOSH_CHECK(cond, code, msg)                                          \
@@ -57,6 +61,7 @@ struct DevBuf {
     cudaError_t e = cudaMalloc(&p, count * sizeof(T));
     if (e != cudaSuccess) {
       p = nullptr;
+      cudaGetLastError();
       throw Error(e == cudaErrorMemoryAllocation ? NOSH_ERR_NO_MEMORY
                                                  : NOSH_ERR_CUDA,
                   std::string("cudaMalloc: ") + cudaGetErrorString(e));

@@ -1,0 +1,86 @@
+"""A device allocation that fails, and the same call again.
+
+A child process preloads a cudaMalloc whose n-th call fails (the runtime's own
+answer to a request larger than the device).  For every n that an action
+reaches, the action returns NOSH_ERR_NO_MEMORY, and done again it gives the
+bits of an undisturbed run.
+"""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+CHILD = r"""
+import ctypes
+import sys
+
+import numpy as np
+
+import nosh_gb300 as ng
+from nosh_gb300 import meshgen
+
+shim = ctypes.CDLL(sys.argv[1])
+shim.fail_malloc_at.argtypes = [ctypes.c_long]
+shim.fail_malloc_real.argtypes = [ctypes.c_void_p]
+ng.lib()
+runtime = next(line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line)
+shim.fail_malloc_real(ctypes.cast(ctypes.CDLL(runtime).cudaMalloc, ctypes.c_void_p))
+x, cells, psi0 = meshgen.cube(8, 5)
+A = meshgen.mvp_constant_curl(x)
+p = {"g": 1.0, "mu": 0.3}
+
+
+def handle():
+    model = ng.nls(ng.mesh(x, cells), A, -1.0, 1.0, 1.0, mu=0.3, precision=ng.PREC_FP64)
+    model.set_spmv_schedule(ng.SPMV_STAGED)
+    return model
+
+
+def setup(state):
+    model = handle()
+    return [model.mesh.get_edge_data()[1], model.compute_f(psi0, p)]
+
+
+ACTIONS = {"setup": (lambda: None, setup)}
+prepare, act = ACTIONS[sys.argv[2]]
+reference = act(prepare())
+n = 0
+while True:
+    n += 1
+    assert n < 400
+    state = prepare()
+    shim.fail_malloc_at(n)
+    try:
+        out = act(state)
+        break  # no n-th allocation
+    except ng.NoshError as e:
+        assert e.code == ng.ERR_NO_MEMORY, (n, e.code, str(e))
+    finally:
+        shim.fail_malloc_at(0)
+    for a, b in zip(reference, act(state)):
+        assert np.array_equal(a, b), n
+assert n > 1
+print("failures", n - 1)
+"""
+
+
+def run_child(tmp_path, action):
+    shim = str(tmp_path / "fail_malloc.so")
+    subprocess.run([shutil.which("gcc") or "gcc", "-shared", "-fPIC", "-o", shim,
+                    os.path.join(HERE, "cpp", "fail_malloc.c")], check=True)
+    env = dict(os.environ, LD_PRELOAD=shim, PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", CHILD, shim, action], cwd=ROOT, env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "failures" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("action", ["setup"])
+def test_a_failed_allocation_leaves_no_trace(tmp_path, action):
+    run_child(tmp_path, action)
