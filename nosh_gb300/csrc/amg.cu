@@ -1718,8 +1718,10 @@ void Amg::refresh() {
   AmgVals<T> &V = I.vals<T>();
   cudaStream_t st = I.nls.stream;
   const int L = (int)I.lev.size();
+  // (counted where it is done: after a failure on the way the hierarchy, the
+  // coarsest inverse above all, may be half formed, and the next is full again)
   const bool partial = I.opt.reuse_period > 1 && L > 1 && V.refreshes % I.opt.reuse_period != 0;
-  ++V.refreshes;
+  const int64_t done = std::exchange(V.refreshes, 0) + 1;
   if (!V.rowabs_ready) {
     V.rowabs0.alloc(I.lev[0].n);
     row_abs_sums<T><<<div_up(I.lev[0].n, 256), 256, 0, st>>>(I.lev[0].n, I.lev[0].rp, I.off<T>(0), V.rowabs0.p);
@@ -1737,6 +1739,7 @@ void Amg::refresh() {
                                                                 V.rowabs0.p, I.cheb, V.coef[0].p);
     ++I.nls.launch_count;
     NOSH_CUDA(cudaGetLastError());
+    V.refreshes = done;
     return;
   }
   for (int l = 0; l < L; l++) {
@@ -1786,6 +1789,7 @@ void Amg::refresh() {
                buf[(steps - k - 1) & 1], I.densef.p, I.err.p);
   I.nls.launch_count += 1 + (fp32 ? 1 : steps);
   NOSH_CUDA(cudaGetLastError());
+  V.refreshes = done;
 }
 
 template <typename T>

@@ -48,7 +48,14 @@ def setup(state):
     return [model.mesh.get_edge_data()[1], model.compute_f(psi0, p)]
 
 
-ACTIONS = {"setup": (lambda: None, setup)}
+def newton(model):
+    psi = psi0.copy()
+    st = model.newton(psi, p, tol=1e-10)
+    assert st["status"] == 0, st
+    return [psi]
+
+
+ACTIONS = {"setup": (lambda: None, setup), "newton": (handle, newton)}
 prepare, act = ACTIONS[sys.argv[2]]
 reference = act(prepare())
 n = 0
@@ -81,6 +88,6 @@ def run_child(tmp_path, action):
     assert r.returncode == 0 and "failures" in r.stdout, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("action", ["setup"])
+@pytest.mark.parametrize("action", ["setup", "newton"])
 def test_a_failed_allocation_leaves_no_trace(tmp_path, action):
     run_child(tmp_path, action)
