@@ -1019,14 +1019,15 @@ __global__ void __launch_bounds__(256) encoder_wgrad(int64_t n, const float *__r
 // a fixed order (deterministic).
 constexpr int kGradSegs = 1 + 3 * LAYERS;
 struct GradSeg {
-  const float *part;
-  int64_t dst;
+  int64_t src, dst;           // first partial, first gradient entry
   int nparts, count, block0;  // block0: the segment's first block
 };
 struct GradPlan {
   GradSeg seg[kGradSegs];
+  int blocks = 0;      // of reduce_parts
+  int64_t floats = 0;  // partials of all segments, side by side
 };
-__global__ void reduce_parts(GradPlan plan, float *__restrict__ grad) {
+__global__ void reduce_parts(GradPlan plan, const float *__restrict__ part, float *__restrict__ grad) {
   __shared__ float red[8][33];
   int g = 0;
   while (g + 1 < kGradSegs && (int)blockIdx.x >= plan.seg[g + 1].block0) g++;
@@ -1035,7 +1036,7 @@ __global__ void reduce_parts(GradPlan plan, float *__restrict__ grad) {
   float s = 0.f;
   if (q < sg.count) {
 #pragma unroll 4
-    for (int b = threadIdx.y; b < sg.nparts; b += 8) s += sg.part[(int64_t)b * sg.count + q];
+    for (int b = threadIdx.y; b < sg.nparts; b += 8) s += part[sg.src + (int64_t)b * sg.count + q];
   }
   red[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
@@ -1346,7 +1347,7 @@ struct Mpnn::Impl {
   DevBuf<float> part, pool;
   GradPlan grad_plan{};
   CastPlan cast_plan{};
-  int cast_max = 0, grad_blocks = 0;
+  int cast_max = 0;
   int enc_grid = 0, agg_grid = 0, upd_grid = 0, node_grid = 0, edge_grid = 0, encw_grid = 0;
   void ensure_training();
   int pool_parts = 0;  // pool partial rows written by the last forward
@@ -1485,7 +1486,9 @@ void Mpnn::Impl::refresh_bf16() {
   NOSH_CUDA(cudaGetLastError());
 }
 
-// the training pass's buffers, launch shapes and gradient segments
+// The training pass's launch shapes, gradient segments and buffers.  dH, whose
+// size says that all is there, is allocated last and the segments are planned
+// afresh: a call whose allocation failed can be made again.
 void Mpnn::Impl::ensure_training() {
   if (dH.n) return;
   cudaStream_t st = s.stream;
@@ -1509,12 +1512,12 @@ void Mpnn::Impl::ensure_training() {
                        persistent_grid((const void *)edge_backward_b, 0, div_up(N, 16), kEdgeThreads));
   encw_grid = (int)std::min<int64_t>(4 * kNumSMs, div_up(N, 64));
   // every segment's partials side by side, reduced together at the end
-  int64_t o = 0;
+  GradPlan plan;
   int g = 0;
   auto seg = [&](int64_t dst, int nparts, int count) {
-    grad_plan.seg[g++] = GradSeg{(const float *)(o * sizeof(float)), dst, nparts, count, grad_blocks};
-    grad_blocks += div_up(count, 32);
-    o += (int64_t)nparts * count;
+    plan.seg[g++] = GradSeg{plan.floats, dst, nparts, count, plan.blocks};
+    plan.blocks += div_up(count, 32);
+    plan.floats += (int64_t)nparts * count;
   };
   for (int l = 0; l < LAYERS; l++) {
     seg(L.wu[l], node_grid, kUpdOut);    // W_u, b_u
@@ -1522,8 +1525,8 @@ void Mpnn::Impl::ensure_training() {
     seg(L.wa[l], node_grid, kMsgOut);    // W_a, W_b
   }
   seg(L.enc_w, encw_grid, kEncOut);
-  part.alloc(o);
-  for (GradSeg &q : grad_plan.seg) q.part = part.p + (int64_t)((uintptr_t)q.part / sizeof(float));
+  grad_plan = plan;
+  part.alloc(plan.floats);
   dH.alloc(N * H);
   NOSH_CUDA(cudaStreamSynchronize(st));
 }
@@ -1569,8 +1572,8 @@ double Mpnn::Impl::backward_and_step(float lr) {
   readout_launch(true);  // loss, readout gradients, dz
   for (int l = LAYERS - 1; l >= 0; l--) {
     // h_{l+1} = h_l + R_l, R_l = relu([h_l, M_l] W_u + b_u)
-    float *pu = const_cast<float *>(grad_plan.seg[3 * l].part), *pe = const_cast<float *>(grad_plan.seg[3 * l + 1].part),
-          *pm = const_cast<float *>(grad_plan.seg[3 * l + 2].part);
+    float *pu = part.p + grad_plan.seg[3 * l].src, *pe = part.p + grad_plan.seg[3 * l + 1].src,
+          *pm = part.p + grad_plan.seg[3 * l + 2].src;
     auto upd = l == LAYERS - 1 ? update_backward<true> : update_backward<false>;
     upd<<<node_grid, kNodeThreads, kUpdBwdSmem, st>>>(N, Hs[l].p, Mb[l].p, gate[l].p, dz.p, wt.p + wtb_um[l],
                                                       wt.p + wtb_uh[l], dH.p, dM.p, pu);
@@ -1584,8 +1587,8 @@ double Mpnn::Impl::backward_and_step(float lr) {
     s.launch_count += 4;
   }
   // encoder: h0 = relu(X W + b)
-  encoder_wgrad<<<encw_grid, 256, 0, st>>>(N, X.p, Hs[0].p, dH.p, const_cast<float *>(grad_plan.seg[3 * LAYERS].part));
-  reduce_parts<<<grad_blocks, dim3(32, 8), 0, st>>>(grad_plan, grads.p);
+  encoder_wgrad<<<encw_grid, 256, 0, st>>>(N, X.p, Hs[0].p, dH.p, part.p + grad_plan.seg[3 * LAYERS].src);
+  reduce_parts<<<grad_plan.blocks, dim3(32, 8), 0, st>>>(grad_plan, part.p, grads.p);
   s.launch_count += 2;
   if (lr > 0.f) {
     adam_t++;

@@ -55,7 +55,18 @@ def newton(model):
     return [psi]
 
 
-ACTIONS = {"setup": (lambda: None, setup), "newton": (handle, newton)}
+def network():
+    model = handle()
+    return model, ng.mpnn(model)
+
+
+def training(state):
+    X = np.random.default_rng(1).standard_normal((state[0].mesh.num_vertices, 10)).astype(np.float32)
+    return state[1].loss_grad(X, np.array([2.0, 0.5, 1.0]))
+
+
+ACTIONS = {"setup": (lambda: None, setup), "newton": (handle, newton),
+           "training": (network, training)}
 prepare, act = ACTIONS[sys.argv[2]]
 reference = act(prepare())
 n = 0
@@ -88,6 +99,6 @@ def run_child(tmp_path, action):
     assert r.returncode == 0 and "failures" in r.stdout, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("action", ["setup", "newton"])
+@pytest.mark.parametrize("action", ["setup", "newton", "training"])
 def test_a_failed_allocation_leaves_no_trace(tmp_path, action):
     run_child(tmp_path, action)
