@@ -1655,7 +1655,8 @@ void Mpnn::Impl::features(const double *const x[4], const double mu[4], double t
     // what Newton starts from; a state-space (cv-weighted) error favoured
     // the cubic combination, whose amplified high-frequency noise the
     // residual penalises.
-    if (vc.n < (size_t)(2 * N))
+    // (jd, the last of them, says that all are there)
+    if (jd.n < (size_t)(2 * N))
       for (DevBuf<double> *b : {&vc, &vd, &vt, &jc, &jd}) b->alloc(2 * N);
     sample_fields<<<G, 256, 0, st>>>(N, dots.p, Ls.p, (const C2<double> *)x[0], (const C2<double> *)x[1],
                                      (const C2<double> *)target, sq.p, (C2<double> *)vc.p, (C2<double> *)vd.p,

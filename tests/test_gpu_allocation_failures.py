@@ -65,8 +65,26 @@ def training(state):
     return state[1].loss_grad(X, np.array([2.0, 0.5, 1.0]))
 
 
+def continuation():
+    model = handle()
+    psi = newton(model)[0]
+    go = ng.continuation(model, psi, p["mu"])
+    go.learning(4, 2, 1e-3)
+    for k in range(3):
+        go.advance(p["mu"] + 0.01 * (k + 1))
+    return go
+
+
+def learning_step(go):
+    # (the fourth step is the first that trains; its state stands when the
+    # training after it fails, so the second try is the step after it)
+    st = go.advance(go.mu + 0.01)
+    return [st["status"] == 0, np.isfinite(go.last_prediction()["train_loss"])]
+
+
 ACTIONS = {"setup": (lambda: None, setup), "newton": (handle, newton),
-           "training": (network, training)}
+           "training": (network, training),
+           "learning_step": (continuation, learning_step)}
 prepare, act = ACTIONS[sys.argv[2]]
 reference = act(prepare())
 n = 0
@@ -99,6 +117,6 @@ def run_child(tmp_path, action):
     assert r.returncode == 0 and "failures" in r.stdout, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("action", ["setup", "newton", "training"])
+@pytest.mark.parametrize("action", ["setup", "newton", "training", "learning_step"])
 def test_a_failed_allocation_leaves_no_trace(tmp_path, action):
     run_child(tmp_path, action)
