@@ -1440,6 +1440,7 @@ template <typename T>
 struct AmgVals {
   bool ready = false;
   int64_t refreshes = 0;  // numeric refreshes so far
+  int64_t built = -1;     // the rebuild (NlsImpl::reg_builds) the last one followed
   std::vector<DevBuf<C2<T>>> off;  // level >= 1
   std::vector<DevBuf<T>> dia;      // level >= 1
   std::vector<DevBuf<T>> dinv, coef;
@@ -1722,6 +1723,7 @@ void Amg::refresh() {
   // coarsest inverse above all, may be half formed, and the next is full again)
   const bool partial = I.opt.reuse_period > 1 && L > 1 && V.refreshes % I.opt.reuse_period != 0;
   const int64_t done = std::exchange(V.refreshes, 0) + 1;
+  V.built = -1;
   if (!V.rowabs_ready) {
     V.rowabs0.alloc(I.lev[0].n);
     row_abs_sums<T><<<div_up(I.lev[0].n, 256), 256, 0, st>>>(I.lev[0].n, I.lev[0].rp, I.off<T>(0), V.rowabs0.p);
@@ -1740,6 +1742,7 @@ void Amg::refresh() {
     ++I.nls.launch_count;
     NOSH_CUDA(cudaGetLastError());
     V.refreshes = done;
+    V.built = I.nls.reg_builds;
     return;
   }
   for (int l = 0; l < L; l++) {
@@ -1790,6 +1793,12 @@ void Amg::refresh() {
   I.nls.launch_count += 1 + (fp32 ? 1 : steps);
   NOSH_CUDA(cudaGetLastError());
   V.refreshes = done;
+  V.built = I.nls.reg_builds;
+}
+
+template <typename T>
+void Amg::ensure() {
+  if (impl->vals<T>().built != impl->nls.reg_builds) refresh<T>();
 }
 
 template <typename T>
@@ -2158,6 +2167,8 @@ bool Amg::apply_batch(const int32_t *vsys, const MinresScalars *sc, const int *h
 
 template void Amg::refresh<float>();
 template void Amg::refresh<double>();
+template void Amg::ensure<float>();
+template void Amg::ensure<double>();
 template void Amg::apply<float>(const float *, float *);
 template void Amg::apply<double>(const double *, double *);
 template void Amg::presmooth<float>(const float *, float *);

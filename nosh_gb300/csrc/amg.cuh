@@ -26,6 +26,10 @@ struct Amg {
   // numeric refresh from the current regularised KEO (nls.d_rd*, d_keo*)
   template <typename T>
   void refresh();
+  // refresh() unless this precision's hierarchy follows the last rebuild of
+  // the regularised KEO already (the rebuild was for the other precision)
+  template <typename T>
+  void ensure();
   // z = V-cycle(r); r, z device vectors of 2N (interleaved complex)
   template <typename T>
   void apply(const T *r, T *z);

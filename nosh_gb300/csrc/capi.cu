@@ -612,6 +612,19 @@ int nosh_jacobian_apply(nosh_nls nls, const double *X, double *Y, int nvec, int 
 }
 
 // -------------------------------------------------------- preconditioner
+// The hierarchy in the handle's precision at the operator's last rebuild, which
+// may have been in the other one (the precision set since, a Newton solve of
+// its own precision).
+static void ensure_cycle(nosh::NlsImpl &s) {
+  require(s.reg_ready && s.amg, "preconditioner not built: call nosh_keo_regularized_rebuild");
+  if (s.precision == NOSH_PREC_FP64) {
+    s.amg->ensure<double>();
+  } else {
+    s.ensure_diag32();
+    s.amg->ensure<float>();
+  }
+}
+
 int nosh_keo_regularized_rebuild(nosh_nls nls, const double *p, const double *x) {
   return guarded([&] {
     auto &s = N(nls);
@@ -630,8 +643,7 @@ int nosh_keo_regularized_apply(nosh_nls nls, const double *X, double *Y, int nve
   return guarded([&] {
     auto &s = NC(nls);
     check_apply_args(mode, alpha, beta, nvec);
-    require(s.reg_ready && s.amg, "preconditioner not built: call nosh_keo_regularized_rebuild");
-    if (s.precision != NOSH_PREC_FP64) s.ensure_diag32();
+    ensure_cycle(s);
     for (int k = 0; k < nvec; k++) {
       const double *dx = stage_in(s, X + (size_t)k * 2 * s.N, s.d_in, 2 * s.N);
       OutVec o(s, Y + (size_t)k * 2 * s.N, s.d_out, 2 * s.N);
@@ -666,8 +678,7 @@ int nosh_eig_lowest(nosh_nls nls, const double *psi, const double *p, int k, dou
 int nosh_keo_regularized_smoother_apply(nosh_nls nls, const double *x, double *y) {
   return guarded([&] {
     auto &s = NC(nls);
-    require(s.reg_ready && s.amg, "preconditioner not built: call nosh_keo_regularized_rebuild");
-    if (s.precision != NOSH_PREC_FP64) s.ensure_diag32();
+    ensure_cycle(s);
     const double *dx = stage_in(s, x, s.d_in, 2 * s.N);
     OutVec o(s, y, s.d_out, 2 * s.N);
     if (s.precision == NOSH_PREC_FP64) {

@@ -176,6 +176,9 @@ struct NlsImpl {
   // rounds them before an FP32 apply)
   bool jd32_ok = false, rd32_ok = false;
   void ensure_diag32();
+  // rebuilds of the regularised KEO so far (the preconditioner's hierarchies,
+  // one a precision, record the one they follow)
+  int64_t reg_builds = 0;
   double reg_g = 0.0;
 
   // staging for host / misaligned vectors

@@ -911,6 +911,7 @@ void NlsImpl::operators32_rebuild(const double *x, double g, double mu) {
   // points want their own rebuild
   jac_ready = reg_ready = false;
   jd32_ok = rd32_ok = true;
+  ++reg_builds;
 }
 
 void NlsImpl::operators64_rebuild(const double *x, double g, double mu) {
@@ -922,6 +923,7 @@ void NlsImpl::operators64_rebuild(const double *x, double g, double mu) {
   reg_g = g;
   jac_ready = reg_ready = true;
   jd32_ok = rd32_ok = false;
+  ++reg_builds;
 }
 
 void NlsImpl::reg_rebuild(const double *x, double g, double mu, bool want32) {
@@ -933,6 +935,7 @@ void NlsImpl::reg_rebuild(const double *x, double g, double mu, bool want32) {
   reg_g = g;
   reg_ready = true;
   rd32_ok = want32;
+  ++reg_builds;
 }
 
 void NlsImpl::ensure_diag32() {
