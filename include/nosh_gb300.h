@@ -194,11 +194,13 @@ int nosh_nls_set_forcing_aim(nosh_nls nls, double aim);
 int nosh_nls_set_launch_overlap(nosh_nls nls, int enable);
 /* Diagnostics (no counterpart in the reference, whose Tpetra SpMV has no
  * bounded wait): the bound, in mbarrier polls, of the waits of the staged
- * SpMV schedule for the copies of its matrix rows into shared memory; the
- * default is 2^20, and polls < 0 restores it.  A wait that runs out leaves
- * its launch early and flags it; the call that ran that launch returns
- * NOSH_ERR_CUDA at its next synchronisation, and the handle stays usable.
- * polls = 0 makes every staged wait give up at once (tests of that path). */
+ * SpMV schedule for the copies of its matrix rows into shared memory, and of
+ * the resident coarse cycle's waits for the vectors that its thread blocks send
+ * one another; the default is 2^20, and polls < 0 restores it.  A wait that
+ * runs out ends its launch with invalid results and flags it; the call that
+ * ran that launch returns NOSH_ERR_CUDA at its next synchronisation, and the
+ * handle stays usable.  polls = 0 makes every such wait give up at once (tests
+ * of that path). */
 int nosh_nls_set_stage_wait_limit(nosh_nls nls, int64_t polls);
 /* Index-check mode (the reference's debug builds assert sizes on the host,
  * e.g. src/jacobian_operator.cpp:68-86; there is no device counterpart).

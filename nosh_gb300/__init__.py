@@ -480,8 +480,9 @@ class nls:
 
     def set_stage_wait_limit(self, polls):
         """Diagnostics: bound (mbarrier polls) of the staged SpMV's waits for
-        its row copies; < 0 restores the default, 0 makes them give up at
-        once (see nosh_nls_set_stage_wait_limit)."""
+        its row copies and the resident coarse cycle's for its vectors; < 0
+        restores the default, 0 makes them give up at once (see
+        nosh_nls_set_stage_wait_limit)."""
         _check(_lib.nosh_nls_set_stage_wait_limit(self._h, int(polls)))
 
     def stream(self) -> int:

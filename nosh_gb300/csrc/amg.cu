@@ -847,6 +847,12 @@ __global__ void dense_matvec(int m, const T *__restrict__ Ainv, DenseMap D, cons
 // of the phase that reads it: each sends its rows of that phase only after
 // its own reads, and nobody goes on without all rows.
 //
+// The waits are bounded.  A thread whose wait runs out flags it to the host,
+// waits for nothing more and goes through the remaining phases all the same
+// (their results are invalid), so every CTA sends all that the others expect.
+// At the end it waits once more, with a bound, for all of it: no store is to
+// land in the shared memory of a CTA that has left.
+//
 // A row is summed by LN lanes: even lanes its real component, odd lanes its
 // imaginary one (two FMAs a nonzero each, no reduction between the two), and
 // LN/2 parts of the row.  FP64 takes just enough lanes for a warp on each of
@@ -891,7 +897,8 @@ struct TailArgs {
   const C2<T> *r_cur;
   C2<T> *z;            // kOutVector, kOutMinres
   MinresScalars *ms;
-  unsigned *fail;      // (pinned host memory) set when a wait for a phase's vector gives up
+  unsigned *fail;           // (pinned host memory) set when a wait for a phase's vector gives up
+  const unsigned *counter;  // kStageWaitSlot: diagnostic override of the waits' bound
 };
 
 // The coarsest level's dense inverse in shared memory (byte offsets): the own
@@ -948,6 +955,8 @@ struct TailTeam {
   int rank, nct;  // CTA of the cluster, CTAs in it
   int lane, warp;
   unsigned *fail;
+  uint32_t polls;  // bound of a wait; 0 once one has run out
+  bool lost;       // one has
   template <typename T>
   __device__ __forceinline__ int rows_of(const LevelDesc<T> &A) const {
     return max(0, min(A.rw, A.n - rank * A.rw));
@@ -962,10 +971,10 @@ struct TailTeam {
     const uint32_t at = sm_addr + o + row * (uint32_t)sizeof(C2<T>), bar = bars + 8u * ph;
     for (int q = li; q < nct; q += LN) st_async(at, bar, q, w);
   }
-  // the whole vector of phase ph has arrived here
-  __device__ __forceinline__ void wait(int ph) const {
+  // polls until phase ph's vector is here or the bound is reached
+  __device__ __forceinline__ bool arrived(int ph, uint32_t &bound) const {
     const uint32_t a = bars + 8u * ph;
-    for (uint32_t it = 0; it < kStageWaitPolls; it++) {
+    for (; bound > 0; bound--) {
       uint32_t done;
       asm volatile(
           "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
@@ -973,9 +982,24 @@ struct TailTeam {
           : "=r"(done)
           : "r"(a)
           : "memory");
-      if (done) return;
+      if (done) return true;
     }
+    return false;
+  }
+  // the whole vector of phase ph has arrived here
+  __device__ __forceinline__ void wait(int ph) {
+    uint32_t bound = polls;
+    if (arrived(ph, bound) || lost) return;
     *(volatile unsigned *)fail = 1u;
+    lost = true;
+    polls = 0;
+  }
+  // all that is under way to this CTA has landed: the vectors of the n phases
+  // but `unused` (at most the default bound, over all of them)
+  __device__ __forceinline__ void drain(int n, int unused) const {
+    uint32_t bound = kStageWaitPolls;
+    for (int ph = 0; ph < n && bound > 0; ph++)
+      if (ph != unused) arrived(ph, bound);
   }
 };
 
@@ -1135,6 +1159,11 @@ __global__ void __launch_bounds__(kTailThreads)
   R.sm_addr = smem_addr(tail_sm);
   R.bars = R.sm_addr + s_bar;
   R.fail = a.fail;
+  {
+    const unsigned o = __ldcg(a.counter + kStageWaitSlot);
+    R.polls = o ? o - 1 : kStageWaitPolls;
+    R.lost = false;
+  }
   {
     unsigned r, n;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -1374,6 +1403,8 @@ __global__ void __launch_bounds__(kTailThreads)
     cluster_arrive();
     cluster_wait();
   }
+  // (the first level's last step goes to memory unless it is prolonged)
+  if (R.lost) R.drain(nph, a.out == kOutProlong ? -1 : per - 1);
 }
 
 // plain MINRES pieces for the single-level case
@@ -1498,7 +1529,7 @@ struct Amg::Impl {
     AmgVals<T> &V = vals<T>();
     return V.plan[V.plan[1].lt >= 0 && (nls.timers[0].on || nls.timers[1].on) ? 1 : 0];
   }
-  template <typename T> void launch_tail(const TailPlan<T> &P, const TailArgs<T> &a, bool overlap);
+  template <typename T> void launch_tail(const TailPlan<T> &P, TailArgs<T> a, bool overlap);
   // V-cycle launches overlap their predecessors (launch_dep) unless the
   // handle turned that off or times kernels with events between launches
   bool ovl() const { return nls.overlap_launches && !nls.timers[0].on && !nls.timers[1].on; }
@@ -1928,7 +1959,9 @@ void Amg::Impl::build_plan(TailPlan<T> &P, int first) {
 }
 
 template <typename T>
-void Amg::Impl::launch_tail(const TailPlan<T> &P, const TailArgs<T> &a, bool overlap) {
+void Amg::Impl::launch_tail(const TailPlan<T> &P, TailArgs<T> a, bool overlap) {
+  a.fail = nls.h_stage_err + 1;
+  a.counter = nls.red.counter.p;
   launch_cluster_dep(overlap, tail_ctas, resident_vcycle<T>, dim3(kTailThreads), P.smem, nls.stream,
                      (const LevelDesc<T> *)P.desc.p, P.lt, (int)lev.size(), std::max(opt.smooth_degree, 1),
                      dense_inv<T>(), dmap(), P.dense, P.s_bar, a, halt);
@@ -1984,7 +2017,6 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
   const TailPlan<T> &P = plan<T>();
   if (!grid_coarse && l + 1 == P.lt) {
     TailArgs<T> a{};
-    a.fail = nls.h_stage_err;
     a.head = kHeadRestrict;
     a.out = kOutProlong;
     a.f_res = V.res[l].p;
@@ -2058,7 +2090,6 @@ void Amg::apply(const T *r, T *z) {
     // the whole cycle resident; no overlap: it stages the block inverses,
     // which the refresh before it may have written
     TailArgs<T> a{};
-    a.fail = I.nls.h_stage_err;
     a.head = kHeadVector;
     a.out = kOutVector;
     a.b = (const C2<T> *)r;
@@ -2122,7 +2153,6 @@ void Amg::apply_minres(MinresScalars *ms, const T *u, T *r_old, const T *r_cur, 
   I.halt = &ms->done;
   if (const TailPlan<T> &P = I.plan<T>(); P.lt == 0) {
     TailArgs<T> a{};
-    a.fail = I.nls.h_stage_err;
     a.head = kHeadLanczos;
     a.out = kOutMinres;
     a.b = (const C2<T> *)u;

@@ -28,7 +28,7 @@ struct Reducer {
     if (host) cudaFreeHost(host);
   }
   // the buffers from the handle's slab (whose owner zeroes counter and out);
-  // behind the host slots one more double for the owner's failure word (a
+  // behind the host slots one more double for the owner's two failure words (a
   // pinned allocation costs 130 to 240 us)
   static constexpr int kHostSlots = 16;
   void init(int max_blocks, int nslots, DevSlab &slab) {
@@ -283,12 +283,14 @@ struct NlsImpl {
   void export_values(const C2<double> *offdiag, const double *diag, double *out);
 
   // Waits for the handle's stream.  A kernel that gave up one of its bounded
-  // waits (a staged SpMV's copies, the resident cycle's vectors) has set
-  // *h_stage_err: then it throws NOSH_ERR_CUDA after clearing the flag and the
-  // reduction counters, so the handle stays usable.
+  // waits (a staged SpMV's copies, the resident cycle's vectors) has set its
+  // word of h_stage_err: then it throws NOSH_ERR_CUDA after clearing the words
+  // and the reduction counters, so the handle stays usable.
   void sync();
   [[noreturn]] void stage_failure();
-  unsigned *h_stage_err = nullptr;  // pinned, one word, written by the failing kernel
+  // pinned, written by the failing kernel: [0] staged SpMV, [1] resident cycle
+  unsigned *h_stage_err = nullptr;
+  bool wait_failed() const { return (h_stage_err[0] | h_stage_err[1]) != 0u; }
   // diagnostics: bound of the staging waits (polls; < 0 restores the default)
   void set_stage_wait_limit(int64_t polls);
   // index-check mode: the KEO graph is validated on the device before every

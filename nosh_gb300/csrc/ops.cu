@@ -629,7 +629,7 @@ NlsImpl::NlsImpl(MeshImpl *m, const double *mvp, double mu, const double *V, dou
   for (DevBuf<float> *b : {&d_jd32, &d_rd32}) b->zero(s);
   red.counter.zero(s);
   h_stage_err = reinterpret_cast<unsigned *>(red.host + Reducer::kHostSlots);
-  *h_stage_err = 0u;
+  h_stage_err[0] = h_stage_err[1] = 0u;
   NOSH_CUDA(cudaMemcpyAsync(red.counter.p + kStageErrorSlot, &h_stage_err, sizeof(h_stage_err),
                             cudaMemcpyHostToDevice, s));
   tune_schedules();
@@ -738,7 +738,7 @@ void NlsImpl::sync() {
     return;
   }
   NOSH_CUDA(cudaStreamSynchronize(stream));
-  if (*h_stage_err) stage_failure();
+  if (wait_failed()) stage_failure();
 }
 
 void NlsImpl::stage_failure() {
@@ -747,10 +747,12 @@ void NlsImpl::stage_failure() {
   // the wait-bound override stay)
   NOSH_CUDA(cudaMemsetAsync(red.counter.p, 0, kStageErrorSlot * sizeof(unsigned), stream));
   NOSH_CUDA(cudaStreamSynchronize(stream));
-  if (h_stage_err) *h_stage_err = 0;
-  throw Error(NOSH_ERR_CUDA,
-              "an SpMV staging copy did not complete within its wait bound: the results of this call are "
-              "invalid (the handle stays usable)");
+  const bool staging = h_stage_err[0] != 0u;
+  h_stage_err[0] = h_stage_err[1] = 0u;
+  throw Error(NOSH_ERR_CUDA, std::string(staging ? "an SpMV staging copy did not complete"
+                                                 : "a vector of the resident coarse cycle did not arrive") +
+                                 " within its wait bound: the results of this call are invalid (the handle "
+                                 "stays usable)");
 }
 
 void NlsImpl::check_indices() {

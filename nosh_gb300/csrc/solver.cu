@@ -368,12 +368,12 @@ int Minres<T>::solve(const double *rhs, double scale, double rtol, int maxit, in
       }
     }
     first = false;
-    if (h_rep->done || *s.h_stage_err != 0 || it >= maxit + kChunk) break;
+    if (h_rep->done || s.wait_failed() || it >= maxit + kChunk) break;
   }
   // converged on the last issued iteration: its w/x update is still due
   // (h is the next part; the last issued iteration ends the part before it)
   if (h_rep->wx_pending) wx_final(((h + kParts - 1) % kParts + 1) * kPart - 1);
-  if (*s.h_stage_err != 0) s.stage_failure();
+  if (s.wait_failed()) s.stage_failure();
   if (h_rep->amg_err != 0) {
     s.amg->clear_error();
     throw Error(NOSH_ERR_BREAKDOWN,

@@ -56,3 +56,35 @@ def test_resident_cycle(name, prec, tol, degree):
     model.profile(False)
     assert np.abs(grid - Ma).max() <= tol * np.abs(grid).max()
     assert np.array_equal(M.apply(a), Ma)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("name", ["square9", "cube11", "square65"])
+def test_waits_that_run_out(name, prec):
+    """With a bound of 0 polls every wait of the resident cycle gives up at
+    once: the call returns NOSH_ERR_CUDA and names the cycle, alone and in a
+    solve, and with the bound restored the handle gives the same bits as
+    before.  (The warp schedule has no waits of its own.)"""
+    import nosh_gb300 as ng
+
+    x, c, psi = MESHES[name]()
+    m = O.finish_mesh(x, c)
+    A = O.mvp_constant_curl(m.x)
+    model = ng.nls(ng.mesh(m.x, m.cells), A, -1.0, 1.0, 1.0, mu=0.3, precision=prec)
+    model.set_spmv_schedule(ng.SPMV_WARP)
+    model.set_amg_options(coarse_size=40)
+    M = model.create_W_prec()
+    M.rebuild({"g": 1.0, "mu": 0.3}, psi)
+    a = np.random.default_rng(11).standard_normal(2 * m.N)
+    Ma = M.apply(a)
+    model.set_stage_wait_limit(0)
+    for call in (lambda: M.apply(a), lambda: model.newton(psi.copy(), {"g": 1.0, "mu": 0.3})):
+        with pytest.raises(ng.NoshError) as e:
+            call()
+        assert e.value.code == ng.ERR_CUDA and "resident coarse cycle" in str(e.value)
+    model.set_stage_wait_limit(-1)
+    M.rebuild({"g": 1.0, "mu": 0.3}, psi)
+    assert np.array_equal(M.apply(a), Ma)
+    sol = psi.copy()
+    st = model.newton(sol, {"g": 1.0, "mu": 0.3}, tol=1e-10)
+    assert st["status"] == 0 and np.linalg.norm(O.Problem(m, A).compute_f(sol, 1.0, 0.3)) <= 2e-10
