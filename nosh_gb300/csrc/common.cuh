@@ -128,7 +128,8 @@ bool is_device_pointer(const void *p);
 
 // ------------------------------------------------------- host parallelism
 // f(begin, end) over a static partition of [0, n) on the host cores, at least
-// `grain` elements each (a thread costs about 20 us to start).
+// `grain` elements each (a thread costs about 20 us to start).  f does not
+// throw.  Parts for which no thread is to be had run on this one.
 template <class F>
 void parallel_ranges(int64_t n, int64_t grain, F &&f) {
   const unsigned hw = std::thread::hardware_concurrency();
@@ -139,8 +140,13 @@ void parallel_ranges(int64_t n, int64_t grain, F &&f) {
   }
   std::vector<std::thread> th;
   th.reserve(nt - 1);
-  for (int64_t t = 1; t < nt; t++) th.emplace_back([=, &f] { f(n * t / nt, n * (t + 1) / nt); });
+  int64_t t = 1;
+  try {
+    for (; t < nt; t++) th.emplace_back([=, &f] { f(n * t / nt, n * (t + 1) / nt); });
+  } catch (const std::exception &) {
+  }
   f((int64_t)0, n / nt);
+  for (; t < nt; t++) f(n * t / nt, n * (t + 1) / nt);
   for (auto &x : th) x.join();
 }
 

@@ -85,3 +85,34 @@ def test_version():
     import nosh_gb300 as ng
 
     assert ng.lib().nosh_version() >= 100
+
+
+NO_THREADS = r"""
+import resource
+import numpy as np
+import nosh_gb300 as ng
+
+n = 1 << 20  # cells: enough for several threads to look through them
+cells = np.tile(np.array([[0, 1, 2]], np.int32), (n, 1))
+cells[-1, 1] = 3
+x = np.zeros((3, 3))
+ng.lib()
+pages = int(open("/proc/self/statm").read().split()[0])
+room = pages * resource.getpagesize() + (4 << 20)  # (a thread's stack is 8 MB)
+resource.setrlimit(resource.RLIMIT_AS, (room, room))
+try:
+    ng.mesh(x, cells)
+except ng.NoshError as e:
+    assert e.code == ng.ERR_INVALID and str(3 * n - 2) in str(e), str(e)
+    print("reported")
+"""
+
+
+def test_no_thread_to_be_had():
+    """A mesh is checked on several host threads; where the system starts
+    none, the caller's own does the work."""
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", NO_THREADS], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and "reported" in r.stdout, r.stdout + r.stderr
