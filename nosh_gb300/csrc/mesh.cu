@@ -537,34 +537,83 @@ int64_t scan(int64_t n, const int32_t *in, int32_t *out, int64_t *tile, cudaStre
 }
 inline int wide_grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(div_up(n, 256), 16 * kNumSMs)); }
 
-// The vertices with too many cells for the warp kernel: sorted codes and
-// neighbours from the host.
-void solve_hubs(int nvc, const int32_t *cells, const std::vector<int32_t> &hubs, const DevBuf<int32_t> &ptr,
-                DevBuf<int32_t> &vc, DevBuf<int32_t> &nb, DevBuf<int32_t> &deg, DevBuf<int32_t> &up, cudaStream_t s) {
-  std::vector<int32_t> code, u;
-  for (const int32_t v : hubs) {
-    int32_t pb[2];
-    NOSH_CUDA(cudaMemcpyAsync(pb, ptr.p + v, sizeof(pb), cudaMemcpyDeviceToHost, s));
-    NOSH_CUDA(cudaStreamSynchronize(s));
-    code.resize(pb[1] - pb[0]);
-    NOSH_CUDA(cudaMemcpyAsync(code.data(), vc.p + pb[0], code.size() * 4, cudaMemcpyDeviceToHost, s));
-    NOSH_CUDA(cudaStreamSynchronize(s));
-    std::sort(code.begin(), code.end());
-    u.clear();
-    for (const int32_t k : code)
-      for (int q = 0; q < nvc; q++) {
-        const int32_t w = cells[(int64_t)(k / nvc) * nvc + q];
-        if (w != v) u.push_back(w);
-      }
-    std::sort(u.begin(), u.end());
-    u.erase(std::unique(u.begin(), u.end()), u.end());
-    const int32_t d = (int32_t)u.size(), a = (int32_t)(u.end() - std::upper_bound(u.begin(), u.end(), v));
-    NOSH_CUDA(cudaMemcpyAsync(vc.p + pb[0], code.data(), code.size() * 4, cudaMemcpyHostToDevice, s));
-    NOSH_CUDA(cudaMemcpyAsync(nb.p + (int64_t)(nvc - 1) * pb[0], u.data(), u.size() * 4, cudaMemcpyHostToDevice, s));
-    NOSH_CUDA(cudaMemcpyAsync(deg.p + v, &d, 4, cudaMemcpyHostToDevice, s));
-    NOSH_CUDA(cudaMemcpyAsync(up.p + v, &a, 4, cudaMemcpyHostToDevice, s));
-    NOSH_CUDA(cudaStreamSynchronize(s));
+// The vertices with too many cells for the warp kernel: their codes are sorted
+// and their neighbours found on the host's cores, all hubs in one copy out and
+// one back.  A mesh of 10000 fans of 100 triangles 6.2 ms; 350 with the hubs one
+// after the other, each with copies and waits of its own, and 45 with all of the
+// topology on the host's cores.  One fan 0.39 ms (0.35).
+struct Hubs {
+  DevBuf<int32_t> off, codes, nb, deg, up;  // hub h: codes [off[h], off[h + 1])
+};
+__global__ void hub_sizes(int64_t nh, const int32_t *__restrict__ hubs, const int32_t *__restrict__ ptr, int32_t *size) {
+  const int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (h < nh) size[h] = ptr[hubs[h] + 1] - ptr[hubs[h]];
+}
+// a CTA per hub
+__global__ void hub_gather(const int32_t *__restrict__ hubs, const int32_t *__restrict__ ptr,
+                           const int32_t *__restrict__ vc, const int32_t *__restrict__ off, int32_t *codes) {
+  const int b = ptr[hubs[blockIdx.x]], o = off[blockIdx.x], d = off[blockIdx.x + 1] - o;
+  for (int q = threadIdx.x; q < d; q += blockDim.x) codes[o + q] = vc[b + q];
+}
+__global__ void hub_scatter(int nvc, const int32_t *__restrict__ hubs, const int32_t *__restrict__ ptr,
+                            const int32_t *__restrict__ off, const int32_t *__restrict__ codes,
+                            const int32_t *__restrict__ hub_nb, const int32_t *__restrict__ hub_deg,
+                            const int32_t *__restrict__ hub_up, int32_t *vc, int32_t *nb, int32_t *deg, int32_t *up) {
+  const int v = hubs[blockIdx.x], b = ptr[v], o = off[blockIdx.x], d = off[blockIdx.x + 1] - o, m = hub_deg[blockIdx.x];
+  for (int q = threadIdx.x; q < d; q += blockDim.x) vc[b + q] = codes[o + q];
+  for (int q = threadIdx.x; q < m; q += blockDim.x)
+    nb[(int64_t)(nvc - 1) * b + q] = hub_nb[(int64_t)(nvc - 1) * o + q];
+  if (threadIdx.x == 0) {
+    deg[v] = m;
+    up[v] = hub_up[blockIdx.x];
   }
+}
+void solve_hubs(int nvc, const int32_t *cells, int nh, const DevBuf<int32_t> &hubs, const DevBuf<int32_t> &ptr,
+                DevBuf<int32_t> &vc, DevBuf<int32_t> &nb, DevBuf<int32_t> &deg, DevBuf<int32_t> &up, cudaStream_t s) {
+  std::vector<int32_t> hv(nh), off(nh + 1, 0), h_deg(nh), h_up(nh);
+  Hubs D;
+  D.deg.alloc(nh);
+  D.up.alloc(nh);
+  D.off.alloc(nh + 1);
+  hub_sizes<<<div_up(nh, 256), 256, 0, s>>>(nh, hubs.p, ptr.p, D.deg.p);
+  NOSH_CUDA(cudaGetLastError());
+  hubs.download(hv.data(), nh, s);
+  D.deg.download(off.data() + 1, nh, s);
+  NOSH_CUDA(cudaStreamSynchronize(s));
+  for (int h = 0; h < nh; h++) off[h + 1] += off[h];  // (at most the codes of all vertices: 32 bits)
+  const int64_t total = off[nh];
+  std::vector<int32_t> codes(total), adj((nvc - 1) * total);
+  D.codes.alloc(total);
+  D.nb.alloc((nvc - 1) * total);
+  D.off.upload(off, s);
+  hub_gather<<<nh, 128, 0, s>>>(hubs.p, ptr.p, vc.p, D.off.p, D.codes.p);
+  NOSH_CUDA(cudaGetLastError());
+  D.codes.download(codes.data(), total, s);
+  NOSH_CUDA(cudaStreamSynchronize(s));
+  parallel_ranges(nh, 16, [&](int64_t h0, int64_t h1) {
+    for (int64_t h = h0; h < h1; h++) {
+      const int32_t v = hv[h];
+      std::sort(codes.begin() + off[h], codes.begin() + off[h + 1]);
+      int32_t *u = adj.data() + (int64_t)(nvc - 1) * off[h], *e = u;
+      for (int32_t k = off[h]; k < off[h + 1]; k++)
+        for (int q = 0; q < nvc; q++) {
+          const int32_t w = cells[(int64_t)(codes[k] / nvc) * nvc + q];
+          if (w != v) *e++ = w;
+        }
+      std::sort(u, e);
+      e = std::unique(u, e);
+      h_deg[h] = (int32_t)(e - u);
+      h_up[h] = (int32_t)(e - std::upper_bound(u, e, v));
+    }
+  });
+  D.codes.upload(codes, s);
+  D.nb.upload(adj, s);
+  D.deg.upload(h_deg, s);
+  D.up.upload(h_up, s);
+  hub_scatter<<<nh, 128, 0, s>>>(nvc, hubs.p, ptr.p, D.off.p, D.codes.p, D.nb.p, D.deg.p, D.up.p, vc.p, nb.p, deg.p,
+                                 up.p);
+  NOSH_CUDA(cudaGetLastError());
+  NOSH_CUDA(cudaStreamSynchronize(s));
 }
 }  // namespace
 
@@ -617,12 +666,7 @@ void MeshImpl::build(const double *coords, const int32_t *cells) {
   flags.download(h, 2, s);
   NOSH_CUDA(cudaStreamSynchronize(s));
   NOSH_CHECK(h[0] == 0, NOSH_ERR_MESH, "degenerate cell(s) in the mesh (flags " + std::to_string(h[0]) + ")");
-  if (h[1] > 0) {
-    std::vector<int32_t> hv(h[1]);
-    hubs.download(hv.data(), hv.size(), s);
-    NOSH_CUDA(cudaStreamSynchronize(s));
-    solve_hubs(nvc, cells, hv, ptr, vc, nb, deg, up, s);
-  }
+  if (h[1] > 0) solve_hubs(nvc, cells, h[1], hubs, ptr, vc, nb, deg, up, s);
   // row pointers and first edges
   int64_t total[2];
   NOSH_CUDA(cudaMemcpyAsync(&total[0], tile.p + scan(N, deg.p, d_rp.p, tile.p, s), sizeof(int64_t),

@@ -85,6 +85,45 @@ def test_topology_and_geometry_match_oracle(name):
     assert np.abs(f - ref).max() <= 10 * tol * np.abs(ref).max()
 
 
+def _fans(sizes):
+    xs, cs, n = [], [], 0
+    for k, s in enumerate(sizes):
+        x, c = _fan(s)
+        xs.append(x + [3.0 * k, 0.0, 0.0])
+        cs.append(c + n)
+        n += len(x)
+    return np.vstack(xs), np.vstack(cs).astype(np.int32)
+
+
+def test_many_hubs():
+    """more hubs than one host thread takes, among vertices that are none"""
+    import nosh_gb300 as ng
+
+    x, c = _permuted(*_fans(range(60, 140)), 7)
+    o = O.finish_mesh(x, c)
+    m = ng.mesh(x, c)
+    assert np.array_equal(m.my_edges(), o.edges)
+    ln, cov = m.get_edge_data()
+    assert np.abs(cov - o.covolume).max() <= 1e-9 * np.abs(o.covolume).max()
+    assert np.abs(m.control_volumes() - o.cv).max() <= 1e-9 * np.abs(o.cv).max()
+
+
+def test_time_of_many_hubs():
+    """10000 hubs are found together, in about 6 ms; one after the other, each
+    with copies of its own, they take 340, the bound is 100"""
+    import time
+
+    import nosh_gb300 as ng
+
+    x, c = _fans([85] * 10000)
+    best = 1.0
+    for _ in range(4):
+        t = time.perf_counter()
+        ng.mesh(x, c)
+        best = min(best, time.perf_counter() - t)
+    assert best < 0.1, best
+
+
 def test_vertices_outside_every_cell():
     """a vertex of no cell has an empty row, wherever it stands"""
     import nosh_gb300 as ng
