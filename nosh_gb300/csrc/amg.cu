@@ -1497,7 +1497,12 @@ struct Amg::Impl {
   DevBuf<unsigned long long> lmax_bits;
   DevBuf<unsigned> arrive;
   ChebSpec cheb;
-  DevBuf<double> dense;  // coarsest (2n)^2 FP64
+  // The coarsest level's inverse, FP64 (2n)^2 and FP32: of the operators of the
+  // precision inverse_of (in bytes) that was refreshed in full last.  A solve
+  // takes it as it is (any SPD inverse preconditions), an apply of the V-cycle
+  // by itself has its own formed first (ensure).
+  DevBuf<double> dense;
+  size_t inverse_of = 0;
   DevBuf<double> dense2;  // the inversion's other buffer
   DevBuf<float> densef;
   // packed block-diagonal coarsest inverse: per block (offset, dim), per real
@@ -1510,6 +1515,7 @@ struct Amg::Impl {
   Impl(NlsImpl &s, const AmgOptions &o) : nls(s), opt(o) {}
   template <typename T> AmgVals<T> &vals();
   template <typename T> void ensure_vals();
+  template <typename T> void invert_coarsest();
   template <typename T> const C2<T> *off(int l);
   template <typename T> const T *dia(int l);
   template <typename T> const T *dense_inv();
@@ -1808,28 +1814,38 @@ void Amg::refresh() {
       warp = I.nls.spmv_schedule == 2;
     tuned = true;
   }
-  const AmgLevel &C = I.lev.back();
-  const bool fp32 = sizeof(T) == 4 && I.max_dim <= kDenseFp32;
-  const int steps = fp32 ? 0 : div_up(I.max_dim, kPivots);
-  double *buf[2] = {I.dense.p, I.dense2.p};  // the last step writes the first
-  coarse_dense<T><<<div_up(C.n, 128), 128, 0, st>>>(C.n, C.rp, C.ci, I.off<T>(L - 1), I.dia<T>(L - 1),
-                                                     I.row_start.p, I.row_off.p, I.row_dim.p, buf[steps & 1]);
-  if (fp32)
-    gauss_jordan_fp32<<<I.nblk, 1024, (size_t)I.max_dim * I.max_dim * sizeof(float), st>>>(
-        I.blk_off.p, I.blk_dim.p, I.dense.p, I.densef.p, I.err.p);
-  for (int k = 0; k < steps; k++)
-    launch_dep(I.ovl(), gauss_jordan_step, dim3(I.nblk, div_up(I.max_dim, kPivotCols)), dim3(kPivotThreads), 0, st,
-               I.blk_off.p, I.blk_dim.p, k * kPivots, (int)(k == steps - 1), (const double *)buf[(steps - k) & 1],
-               buf[(steps - k - 1) & 1], I.densef.p, I.err.p);
-  I.nls.launch_count += 1 + (fp32 ? 1 : steps);
-  NOSH_CUDA(cudaGetLastError());
+  I.invert_coarsest<T>();
   V.refreshes = done;
   V.built = I.nls.reg_builds;
+}
+
+// The dense inverse of the coarsest level's operators of precision T.
+template <typename T>
+void Amg::Impl::invert_coarsest() {
+  const AmgLevel &C = lev.back();
+  const bool fp32 = sizeof(T) == 4 && max_dim <= kDenseFp32;
+  const int L = (int)lev.size();
+  cudaStream_t st = nls.stream;
+  const int steps = fp32 ? 0 : div_up(max_dim, kPivots);
+  double *buf[2] = {dense.p, dense2.p};  // the last step writes the first
+  coarse_dense<T><<<div_up(C.n, 128), 128, 0, st>>>(C.n, C.rp, C.ci, off<T>(L - 1), dia<T>(L - 1),
+                                                     row_start.p, row_off.p, row_dim.p, buf[steps & 1]);
+  if (fp32)
+    gauss_jordan_fp32<<<nblk, 1024, (size_t)max_dim * max_dim * sizeof(float), st>>>(
+        blk_off.p, blk_dim.p, dense.p, densef.p, err.p);
+  for (int k = 0; k < steps; k++)
+    launch_dep(ovl(), gauss_jordan_step, dim3(nblk, div_up(max_dim, kPivotCols)), dim3(kPivotThreads), 0, st,
+               blk_off.p, blk_dim.p, k * kPivots, (int)(k == steps - 1), (const double *)buf[(steps - k) & 1],
+               buf[(steps - k - 1) & 1], densef.p, err.p);
+  nls.launch_count += 1 + (fp32 ? 1 : steps);
+  NOSH_CUDA(cudaGetLastError());
+  inverse_of = sizeof(T);
 }
 
 template <typename T>
 void Amg::ensure() {
   if (impl->vals<T>().built != impl->nls.reg_builds) refresh<T>();
+  if (impl->inverse_of != sizeof(T)) impl->invert_coarsest<T>();
 }
 
 template <typename T>

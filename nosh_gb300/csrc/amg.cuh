@@ -26,8 +26,10 @@ struct Amg {
   // numeric refresh from the current regularised KEO (nls.d_rd*, d_keo*)
   template <typename T>
   void refresh();
-  // refresh() unless this precision's hierarchy follows the last rebuild of
-  // the regularised KEO already (the rebuild was for the other precision)
+  // For an apply of the V-cycle by itself: refresh() unless this precision's
+  // hierarchy follows the last rebuild of the regularised KEO already (the
+  // rebuild was for the other precision), and the coarsest inverse anew when
+  // the other precision formed the one that stands
   template <typename T>
   void ensure();
   // z = V-cycle(r); r, z device vectors of 2N (interleaved complex)

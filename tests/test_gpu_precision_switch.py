@@ -101,3 +101,18 @@ def test_preconditioner_of_a_mixed_handle_after_an_fp64_solve(gen):
     fp64 = M.apply(v)
     assert np.isfinite(mixed).all() and v @ mixed > 0
     assert np.abs(mixed - fp64).max() <= 1e-4 * np.abs(fp64).max()
+
+
+@pytest.mark.parametrize("first", [0, 1])
+@pytest.mark.parametrize("gen", sorted(CYCLES))
+def test_a_solve_in_the_other_precision_leaves_the_cycle_alone(gen, first):
+    """The V-cycle rebuilt at the same state is the same, to the bit, after a
+    solve of the other precision at another state and parameter."""
+    p = {"g": 1.0, "mu": 0.3}
+    model, psi, v = _handle(CYCLES[gen], first)
+    M = model.create_W_prec()
+    M.rebuild(p, psi)
+    want = M.apply(v)
+    model.newton(1.1 * psi, {"g": 1.0, "mu": 0.5}, precision=1 - first)
+    M.rebuild(p, psi)
+    assert np.array_equal(M.apply(v), want)
