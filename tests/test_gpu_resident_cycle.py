@@ -88,3 +88,41 @@ def test_waits_that_run_out(name, prec):
     sol = psi.copy()
     st = model.newton(sol, {"g": 1.0, "mu": 0.3}, tol=1e-10)
     assert st["status"] == 0 and np.linalg.norm(O.Problem(m, A).compute_f(sol, 1.0, 0.3)) <= 2e-10
+
+
+# the first level that runs resident for the mesh alone
+FIRST = {"square33": 0, "square45": 0, "square65": 1, "cube11": 0, "cube17": 1}
+
+
+@pytest.mark.parametrize("prec,tol", [(0, 1e-12), (1, 1e-4)])
+@pytest.mark.parametrize("name", sorted(FIRST))
+def test_resident_against_every_level_on_the_grid(name, prec, tol):
+    """A union of equal meshes is block diagonal with equal blocks, so every
+    block of its V-cycle is the V-cycle of the mesh alone: the same levels,
+    aggregates and Chebyshev bounds.  With so many copies that the coarsest
+    level has more than 1024 nodes the union has no level in the resident kernel;
+    the mesh alone has all but its fine level there, or that as well.
+    Tolerances as above."""
+    import nosh_gb300 as ng
+
+    x, c, psi = MESHES[name]()
+    m = O.finish_mesh(x, c)
+    r = np.random.default_rng(3).standard_normal(2 * m.N)
+    p = {"g": 1.0, "mu": 0.3}
+    out = []
+    for many in (False, True):
+        k = 1025 // out[0][1][-1] + 1 if many else 1
+        X = np.tile(m.x, (k, 1))
+        cells = (m.cells[None] + m.N * np.arange(k)[:, None, None]).reshape(-1, m.cells.shape[1]).astype(np.int32)
+        model = ng.nls(ng.mesh(X, cells), O.mvp_constant_curl(X), -1.0, 1.0, 1.0, mu=0.3, precision=prec)
+        model.set_spmv_schedule(ng.SPMV_STAGED)
+        model.set_amg_options(coarse_size=40)
+        if many:
+            model.set_systems(m.N * np.arange(k + 1), np.full(k, 0.3))
+        M = model.create_W_prec()
+        M.rebuild(p, np.tile(psi, k))
+        sizes, tail = model.amg_levels()
+        out.append((M.apply(np.tile(r, k)).reshape(k, -1), np.array(sizes), tail))
+    (alone, sizes, tail), (union, usizes, _) = out
+    assert tail == FIRST[name] and np.array_equal(usizes, len(union) * sizes) and usizes[-1] > 1024, (sizes, tail)
+    assert np.abs(union - alone).max() <= tol * np.abs(alone).max()
