@@ -505,7 +505,10 @@ int nosh_mpnn_loss_grad(nosh_mpnn net, const float *X, const double *gram,
  * run from its captured graphs (captured anew when timing is switched), the
  * events are event-record nodes of those graphs, and only the launches that
  * did work are counted (not those that return at once after convergence
- * inside a captured part). */
+ * inside a captured part).  Launches do not overlap then, and a mesh of up to
+ * 2048 vertices, whose whole V-cycle is otherwise one resident launch, keeps
+ * its fine level's launches: the figures are of those, not of the cycle that
+ * the handle runs with timing off. */
 int nosh_nls_profile_enable(nosh_nls nls, int enable);
 /* Launch count, summed device time and summed algorithmic bytes (the bytes
  * the kernel must move at minimum: matrix, indices and the vectors it reads

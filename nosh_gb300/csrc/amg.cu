@@ -14,7 +14,7 @@
 //  * block-Jacobi Chebyshev smoothing (same polynomial before and after the
 //    coarse correction, so the V-cycle is a fixed SPD operator as MINRES
 //    requires); Gershgorin bound for lambda_max(D^-1 A);
-//  * coarsest level: dense inverse (Gauss-Jordan, FP64) applied as a matvec.
+//  * coarsest level: dense inverse (Gauss-Jordan) applied as a matvec.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -406,12 +406,6 @@ __device__ __forceinline__ C2<T> cheb_apply(int64_t i, int k, T sr, T si, const 
   const C2<T> xo{p.xi.x + dn.x, p.xi.y + dn.y};
   xout[i] = xo;
   return xo;
-}
-template <typename T>
-__device__ __forceinline__ C2<T> cheb_elem(int64_t i, int k, T sr, T si, const T *dia, const T *dinv,
-                                           const T *coef, const C2<T> *b, const C2<T> *xin, C2<T> *d,
-                                           C2<T> *xout) {
-  return cheb_apply<T>(i, k, sr, si, cheb_load<T>(i, k, dia, dinv, b, xin, d), coef, d, xout);
 }
 
 template <typename T>
@@ -2049,13 +2043,14 @@ void Amg::Impl::descend_ascend(int l, const C2<T> *b, C2<T> *x, MinresScalars *m
       // in its x buffer
       C2<T> *first = (deg % 2 == 1) ? V.x[l + 1].p : V.x2[l + 1].p;
       launch_dep(ovl(), few ? restrict_first<T, 8> : restrict_first<T, 16>, dim3(div_up(Cl.n * (few ? 8 : 16), B)),
-                 dim3(B), 0, st, Cl.n, A.mem_ptr.p, A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p, V.coef[l + 1].p, V.d[l + 1].p, first,
-                 halt);
+                 dim3(B), 0, st, Cl.n, A.mem_ptr.p, A.mem_idx.p, V.res[l].p, V.b[l + 1].p, V.dinv[l + 1].p,
+                 V.coef[l + 1].p, V.d[l + 1].p, first, halt);
       ++nls.launch_count;
       descend_ascend<T>(l + 1, V.b[l + 1].p, V.x[l + 1].p, nullptr);
     } else {
       launch_dep(ovl(), few ? restrict_kernel<T, 8> : restrict_kernel<T, 16>,
-                 dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p, A.mem_idx.p, V.res[l].p, V.b[l + 1].p, halt);
+                 dim3(div_up(Cl.n * (few ? 8 : 16), B)), dim3(B), 0, st, Cl.n, A.mem_ptr.p, A.mem_idx.p, V.res[l].p,
+                 V.b[l + 1].p, halt);
       const int m = (int)(2 * Cl.n);
       launch_dep(ovl(), dense_matvec<T>, dim3(div_up(m * kDenseLanes, B)), dim3(B), 0, st, m, dense_inv<T>(), dmap(),
                  (const T *)V.b[l + 1].p, (T *)V.x[l + 1].p, halt);

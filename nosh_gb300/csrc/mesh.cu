@@ -545,7 +545,8 @@ inline int wide_grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int6
 struct Hubs {
   DevBuf<int32_t> off, codes, nb, deg, up;  // hub h: codes [off[h], off[h + 1])
 };
-__global__ void hub_sizes(int64_t nh, const int32_t *__restrict__ hubs, const int32_t *__restrict__ ptr, int32_t *size) {
+__global__ void hub_sizes(int64_t nh, const int32_t *__restrict__ hubs, const int32_t *__restrict__ ptr,
+                          int32_t *size) {
   const int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (h < nh) size[h] = ptr[hubs[h] + 1] - ptr[hubs[h]];
 }

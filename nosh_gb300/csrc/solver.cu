@@ -6,8 +6,8 @@
 // Vectors live in HBM in the operator precision (FP32 in the mixed path,
 // FP64 in the plain path); every recurrence scalar is FP64 and stays in
 // device memory: the reductions finish in the last CTA of the producing
-// kernel, and one single-thread kernel advances the Givens recurrence, so
-// the host only polls a convergence flag.
+// kernel, whose first warp advances the Givens recurrence, so the host only
+// polls a convergence flag.
 //
 // Newton: full step (NOX "Line Search Based" / "Full Step",
 // examples/conf.xml:168-174), NormF two-norm test (conf.xml:178-189) on the

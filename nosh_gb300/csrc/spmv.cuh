@@ -341,14 +341,15 @@ __host__ __device__ constexpr size_t stage_bytes(int cap) {
 // has one buffer, and the other CTAs of its SM run under its copies: two
 // buffers left room for fewer CTAs, and the gathers, whose latency bounds the
 // FP32 kernel, and the FP64 pipe, which bounds the other, waited.
-// FP64, a tetrahedral mesh: two buffers (72 KB) fit three CTAs, one fits five
-// (register bound).  J rebuild + apply at 160^3 776 -> 699 us, V-cycles at 48^3
-// 925 -> 868 us; six CTAs (80 registers) gained 1 % more there and lost 3 % on a
-// 32^3 continuation.
+// FP64, a tetrahedral mesh: two buffers (72 KB) fit three CTAs, one fits four
+// (the smoother's step, 110 registers) or five (the residual, 95).  J rebuild +
+// apply at 160^3 776 -> 699 us, V-cycles at 48^3 925 -> 868 us; six CTAs (80
+// registers) gained 1 % more there and lost 3 % on a 32^3 continuation.
 // FP32: two buffers with 16 gathers in flight a row (88 registers) fit five
-// CTAs, one with 8 gathers (72 registers) seven.  A mixed continuation step at
+// CTAs, one with 8 gathers seven (the Jacobian, 70 registers) or eight (the
+// smoother's step, 64).  A mixed continuation step at
 // 64^3 73.3 -> 70.5 ms; one buffer with 16 gathers and five or six CTAs 71.1
-// and 71.9, with 8 gathers and eight CTAs (64 registers) 71.2.
+// and 71.9, with 8 gathers and all held to eight CTAs 71.2.
 template <typename T>
 __host__ __device__ constexpr int stage_ctas() {
   return sizeof(T) == 4 ? 7 : 4;
