@@ -655,15 +655,22 @@ void NlsImpl::set_systems(const int64_t *offsets, int64_t num, const double *mu)
     NOSH_CHECK(sa == sb, NOSH_ERR_INVALID, "an edge joins two systems");
     es[e] = (int32_t)sa;
   }
+  // (all of it or none: the handle stays as it was when an allocation fails)
+  DevBuf<int64_t> d_off(num + 1);
+  DevBuf<int32_t> d_es(E);
+  DevBuf<double> d_mu(num), d_norm(num);
+  d_off.upload(offsets, num + 1, stream);
+  d_es.upload(es, stream);
+  d_mu.upload(mu, num, stream);
+  sync();
   sys_off.assign(offsets, offsets + num + 1);
-  d_sys_off.upload(sys_off, stream);
-  d_esys.upload(es, stream);
-  d_mu_sys.upload(mu, num, stream);
-  d_sys_norm.alloc(num);
+  d_sys_off = std::move(d_off);
+  d_esys = std::move(d_es);
+  d_mu_sys = std::move(d_mu);
+  d_sys_norm = std::move(d_norm);
   h_sys_norm.assign(num, 0.0);
   keo_mu = std::nan("");
   dkeo_mu = std::nan("");
-  sync();
 }
 
 namespace {

@@ -55,6 +55,27 @@ def newton(model):
     return [psi]
 
 
+def union():
+    X, C, n = np.concatenate([x, x]), np.concatenate([cells, cells + len(x)]).astype(np.int32), len(x)
+    model = ng.nls(ng.mesh(X, C), meshgen.mvp_constant_curl(X), -1.0, 1.0, 1.0, mu=0.3, precision=ng.PREC_FP64)
+    model.set_spmv_schedule(ng.SPMV_STAGED)
+    return model, np.array([0, n, 2 * n])
+
+
+def systems(state):
+    model, offsets = state
+    try:
+        model.set_systems(offsets, np.array([0.2, 0.4]))
+    except ng.NoshError:
+        # the handle is still the single system that it was
+        model.newton(np.concatenate([psi0, psi0]), p, tol=1e-10)
+        raise
+    psi = np.concatenate([psi0, psi0])
+    st = model.newton(psi, p, tol=1e-10)
+    assert st["status"] == 0, st
+    return [psi]
+
+
 def network():
     model = handle()
     return model, ng.mpnn(model)
@@ -82,7 +103,7 @@ def learning_step(go):
     return [st["status"] == 0, np.isfinite(go.last_prediction()["train_loss"])]
 
 
-ACTIONS = {"setup": (lambda: None, setup), "newton": (handle, newton),
+ACTIONS = {"setup": (lambda: None, setup), "newton": (handle, newton), "systems": (union, systems),
            "training": (network, training),
            "learning_step": (continuation, learning_step)}
 prepare, act = ACTIONS[sys.argv[2]]
@@ -111,12 +132,12 @@ def run_child(tmp_path, action):
     shim = str(tmp_path / "fail_malloc.so")
     subprocess.run([shutil.which("gcc") or "gcc", "-shared", "-fPIC", "-o", shim,
                     os.path.join(HERE, "cpp", "fail_malloc.c")], check=True)
-    env = dict(os.environ, LD_PRELOAD=shim, PYTHONPATH=ROOT)
+    env = dict(os.environ, LD_PRELOAD=shim)
     r = subprocess.run([sys.executable, "-c", CHILD, shim, action], cwd=ROOT, env=env, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "failures" in r.stdout, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("action", ["setup", "newton", "training", "learning_step"])
+@pytest.mark.parametrize("action", ["setup", "newton", "systems", "training", "learning_step"])
 def test_a_failed_allocation_leaves_no_trace(tmp_path, action):
     run_child(tmp_path, action)
